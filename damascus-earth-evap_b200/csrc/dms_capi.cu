@@ -218,6 +218,16 @@ void Apply_Lane_Options(RunParams& p, const dms_run_opts* o)
 	p.final_wait = o->final_wait ? static_cast<int>(o->final_wait) : 32;
 }
 
+// Threads per block when the caller leaves the choice open, one block per SM either way.  With a lane
+// per trajectory in one 128-thread block per SM, every warp has a scheduler of its own and a pass is
+// bound by its dependent chain; beyond that, 512-thread blocks run their 16 warps in lockstep
+// (dms_lane.cuh).  Measured, Capture mode m = 1 GeV, sigma = 1e-35 cm^2, FP64, 128 against 512 threads:
+// 1 024 trajectories 2.1 / 2.3 ms, 4 096 2.9 / 3.2 ms, 16 384 4.2 / 4.1 ms, 65 536 10.6 / 6.3 ms.
+int Default_Threads(uint64_t total, int sm_count)
+{
+	return total <= 128 * static_cast<uint64_t>(sm_count) ? 128 : MAX_THREADS;
+}
+
 // One persistent launch over the given work; polls for completion, enforcing the wall-clock
 // limit through the mapped cancel flag.
 int Launch_And_Wait(dms_ctx* ctx, const dms_run_opts* o, RunParams& p)
@@ -228,18 +238,24 @@ int Launch_And_Wait(dms_ctx* ctx, const dms_run_opts* o, RunParams& p)
 	if(o->max_trajectory_wall_time_s > 0.0 && p.wall_limit_ns == 0)
 		p.wall_limit_ns = 1;
 	Apply_Lane_Options(p, o);
-	const int threads = o->threads_per_block ? static_cast<int>(o->threads_per_block) : 128;
 	const bool mixed = o->precision == DMS_PRECISION_MIXED;
+	int threads = o->threads_per_block ? static_cast<int>(o->threads_per_block) : 128;
+	if(o->threads_per_block == 0 && o->blocks_per_sm == 0)
+		threads = Default_Threads(p.total, ctx->sm_count);
 	const int max_per_sm = mixed ? Trajectory_Mixed_Max_Blocks_Per_SM(threads) : Trajectory_Max_Blocks_Per_SM(threads);
 	if(max_per_sm <= 0)
 		return Fail(ctx, DMS_ERR_CUDA, "trajectory kernel cannot be resident with this block size");
-	int per_sm = o->blocks_per_sm ? static_cast<int>(o->blocks_per_sm) : max_per_sm;
+	int per_sm = o->blocks_per_sm ? static_cast<int>(o->blocks_per_sm) : o->threads_per_block ? max_per_sm : 1;
 	per_sm = per_sm > max_per_sm ? max_per_sm : per_sm;
 	int blocks = ctx->sm_count * per_sm;
-	const uint64_t needed_blocks = (p.total + threads - 1) / threads;
-	if(static_cast<uint64_t>(blocks) > needed_blocks)
-		blocks = static_cast<int>(std::max<uint64_t>(1, needed_blocks));
-	const size_t lanes = static_cast<size_t>(blocks) * threads;
+	// a launch with fewer trajectories than lanes spreads them over all of its warps: fewer lanes per
+	// warp diverge less, and its idle lanes help in the collective steps
+	const uint64_t warps = static_cast<uint64_t>(blocks) * (threads / 32);
+	p.lanes_per_warp = static_cast<int>(std::min<uint64_t>(32, (p.total + warps - 1) / warps));
+	const uint64_t per_block = static_cast<uint64_t>(threads / 32) * p.lanes_per_warp;
+	blocks = static_cast<int>(std::min<uint64_t>(blocks, (p.total + per_block - 1) / per_block));
+	p.lockstep_min = threads / 16;
+	const size_t lanes = static_cast<size_t>(blocks) * (threads / 32) * p.lanes_per_warp;
 	int rc = Ensure_Lanes(ctx, lanes);
 	if(rc != DMS_OK)
 		return rc;
@@ -519,13 +535,21 @@ int dms_load_solar_model(dms_ctx* ctx, const char* path)
 	if(!err.empty())
 		return Fail(ctx, DMS_ERR_IO, err);
 	const size_t n = t.n, nt = static_cast<size_t>(t.n) * DMS_NUM_TARGETS;
-	const size_t doubles = 9 * n + 2 * nt + DMS_NUM_TARGETS;
+	// the packed knots come first (32-byte aligned, as the allocation)
+	const size_t doubles = 4 * n + 9 * n + 2 * nt + DMS_NUM_TARGETS;
 	const size_t bytes = doubles * sizeof(double) + sizeof(uint16_t) * t.bucket_index.size();
 	std::vector<char> host(bytes);
 	double* h = reinterpret_cast<double*>(host.data());
+	for(size_t i = 0; i < n; i++)
+	{
+		h[4 * i + 0] = i + 1 < n ? t.r[i] : INFINITY;
+		h[4 * i + 1] = t.gm[i];
+		h[4 * i + 2] = i + 1 < n ? t.gm_s[i] : 0.0;
+		h[4 * i + 3] = t.vesc2[i];
+	}
 	const std::vector<double>* parts[11] = {&t.r, &t.gm, &t.gm_s, &t.temp, &t.temp_s, &t.vesc2, &t.vesc2_s, &t.ne, &t.ne_s, &t.nt, &t.nt_s};
 	size_t offsets[11];
-	size_t off = 0;
+	size_t off = 4 * n;
 	for(int k = 0; k < 11; k++)
 	{
 		offsets[k] = off;
@@ -551,6 +575,8 @@ int dms_load_solar_model(dms_ctx* ctx, const char* path)
 	S.n = t.n;
 	S.nbuckets = t.nbuckets;
 	S.bucket_single_step = t.bucket_single_step;
+	S.fast_tables = t.fast_tables;
+	S.gm_pack = reinterpret_cast<const Knot*>(dd);
 	S.bucket_scale = static_cast<double>(t.nbuckets) / DMS_RSUN_KM;
 	S.r = dd + offsets[0];
 	S.gm = dd + offsets[1];
@@ -1280,9 +1306,12 @@ int dms_run_records_noalloc(dms_ctx* ctx, const dms_run_opts* opts, int point_id
 	rc = Noalloc_Scratch(ctx, &scratch);
 	if(rc != DMS_OK)
 		return rc;
-	const int threads = 32;
-	const int blocks = static_cast<int>((count + threads - 1) / threads);
-	const uint64_t lanes = static_cast<uint64_t>(blocks) * threads;
+	// one trajectory per warp, four warps per block: the lanes that take work number at most
+	// DMS_NOALLOC_MAX_TRAJECTORIES.  (127 histories: 106 ms in blocks of one full warp.)
+	const int threads = 128;
+	const int blocks = static_cast<int>((count + 3) / 4);
+	const uint64_t lanes = static_cast<uint64_t>(blocks) * 4;
+	static_assert(DMS_NOALLOC_MAX_TRAJECTORIES % 4 == 0, "the lanes of whole blocks fit the scratch");
 
 	RunParams p{};
 	p.S = ctx->dsolar;
@@ -1307,6 +1336,7 @@ int dms_run_records_noalloc(dms_ctx* ctx, const dms_run_opts* opts, int point_id
 	if(opts->max_trajectory_wall_time_s > 0.0 && p.wall_limit_ns == 0)
 		p.wall_limit_ns = 1;
 	p.ic_max_attempts = 1 << 20;
+	p.lanes_per_warp = 1;
 	Apply_Lane_Options(p, opts);
 	p.counters = ctx->d_counters;
 	p.hists = ctx->d_hists;

@@ -58,6 +58,7 @@ struct DevSolar
 	int n;                 // knots
 	int nbuckets;
 	int bucket_single_step;  // 1: the knot interval of x is its bucket's base or the base + 1
+	int fast_tables;         // 1: also gm_pack holds, and its G*M values suit dms_fastmath.cuh
 	double bucket_scale;   // nbuckets / R_sun
 	const double* r;
 	const double* gm;
@@ -72,6 +73,7 @@ struct DevSolar
 	const double* nt_s;
 	const double* target_mass; // DMS_NUM_TARGETS isotope masses [GeV]
 	const uint16_t* bucket;
+	const struct Knot* gm_pack;  // {r, G*M, G*M slope, v_esc^2} per knot, 32-byte aligned; the last r is infinity
 };
 
 struct DevPoint
@@ -664,435 +666,73 @@ enum RkResult : int
 	RK_FORCED = 2,
 };
 
-// Arithmetic policies of the RK45 attempt: IEEE division and square root as written, or the
-// certified straight-line forms of dms_fastmath.cuh (bit-identical whenever `good` stays set;
-// the caller repeats the attempt with IeeeMath otherwise).
-struct IeeeMath
+// G*M(r) through the packed table S.gm_pack ({r, G*M, slope, v_esc^2} per knot, 32 bytes): both
+// candidate intervals of the radius' bucket are loaded with one 256-bit load each and the interval
+// of knot_index is selected, without a branch or a conversion instruction.  Same value as solar_gm
+// for 0 <= r < inf; for other r some finite value (the index is clamped).
+struct Knot
 {
-	struct Rcp
-	{
-		double b;
-	};
-	__device__ __forceinline__ Rcp rcp(double b) const { return Rcp{b}; }
-	__device__ __forceinline__ double div(double a, const Rcp& d) const { return a / d.b; }
-	__device__ __forceinline__ double div(double a, double b) const { return a / b; }
-	__device__ __forceinline__ double root(double x) const { return sqrt(x); }
+	double r, gm, gm_s, vesc2;
 };
 
-struct CertMath
+__device__ __forceinline__ Knot load_knot(const Knot* p)
 {
-	bool good = true;
-	using Rcp = fast::Recip;
-	__device__ __forceinline__ Rcp rcp(double b) const { return fast::recip(b); }
-	__device__ __forceinline__ double div(double a, const Rcp& d) { return fast::div(a, d, good); }
-	__device__ __forceinline__ double div(double a, double b) { return fast::div(a, b, good); }
-	__device__ __forceinline__ double root(double x) { return fast::sqrt(x, good); }
-};
-
-// RK45_Next_Step_Size (src/Simulation_Trajectory.cpp:477-502) under an arithmetic policy;
-// pow(c, 0.25) is sqrt(sqrt(c)) as in dms_pow_quarter.
-template <class M>
-__device__ __forceinline__ double next_step_size_t(M& m, double current, double e0, double e1, double e2)
-{
-	if(!isfinite(e0) || !isfinite(e1) || !isfinite(e2))
-		return DMS_RK45_MIN_STEP_FACTOR * current;
-	double factor = DMS_RK45_MAX_STEP_FACTOR;
-	double c;
-	if(e0 > 0.0)
-	{
-		c = 0.84 * m.root(m.root(m.div(DMS_RK45_TOL_R_KM, e0)));
-		if(isfinite(c) && c < factor) factor = c;
-	}
-	if(e1 > 0.0)
-	{
-		c = 0.84 * m.root(m.root(m.div(DMS_RK45_TOL_V_KMS, e1)));
-		if(isfinite(c) && c < factor) factor = c;
-	}
-	if(e2 > 0.0)
-	{
-		c = 0.84 * m.root(m.root(m.div(DMS_RK45_TOL_PHI, e2)));
-		if(isfinite(c) && c < factor) factor = c;
-	}
-	if(factor > DMS_RK45_MAX_STEP_FACTOR) factor = DMS_RK45_MAX_STEP_FACTOR;
-	if(factor < DMS_RK45_MIN_STEP_FACTOR) factor = DMS_RK45_MIN_STEP_FACTOR;
-	return sanitized_step(factor * current);
+	Knot k;
+	asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(k.r), "=d"(k.gm), "=d"(k.gm_s), "=d"(k.vesc2) : "l"(p));
+	return k;
 }
 
-// dv/dt and dphi/dt of one stage at radius r: J*J/r/r/r - gm/r/r with r clamped to >= 1 km, and
-// J/r/r (0 in radial mode, for J = 0 or r <= 0), the reference's divisions in its order.  The
-// quotients by the same r share one reciprocal under CertMath.
-template <class M>
-__device__ __forceinline__ void stage_rates(M& m, const Prop& p, double r, double gm, double& dv, double& dphi, bool want_phi)
+__device__ __forceinline__ int bucket_base(const DevSolar& S, double r)
 {
-	const double rc = r < 1.0 ? 1.0 : r;
-	const auto R = m.rcp(rc);
-	dv = m.div(m.div(m.div(p.J * p.J, R), R), R) - m.div(m.div(gm, R), R);
-	dphi = 0.0;
-	if(want_phi && !(p.radial_mode || p.J == 0.0 || r <= 0.0))
-		dphi = r < 1.0 ? m.div(m.div(p.J, r), r) : m.div(m.div(p.J, R), R);
-}
-
-// The attempt with the six stages written out: a longer instruction stream (more
-// instruction-cache pressure with many warps) but a shorter dependent chain for a lane that
-// runs alone.
-template <class M>
-__device__ __forceinline__ int rk45_attempt_t(const DevSolar& S, Prop& p, int inner, M& m)
-{
-	{
-		const double dt = p.time_step;
-		double kr0, kr1, kr2, kr3, kr4, kr5, kv0, kv1, kv2, kv3, kv4, kv5, kp0, kp2, kp3, kp4, kp5, ri, a, b;
-		kr0 = dt * p.v_radial;
-		stage_rates(m, p, p.radius, solar_gm(S, p.radius), a, b, true);
-		kv0 = dt * a;
-		kp0 = dt * b;
-		ri = p.radius + kr0 / 4.0;
-		kr1 = dt * (p.v_radial + kv0 / 4.0);
-		stage_rates(m, p, ri, solar_gm(S, ri), a, b, false);
-		kv1 = dt * a;
-		ri = p.radius + 3.0 / 32.0 * kr0 + 9.0 / 32.0 * kr1;
-		kr2 = dt * (p.v_radial + 3.0 / 32.0 * kv0 + 9.0 / 32.0 * kv1);
-		stage_rates(m, p, ri, solar_gm(S, ri), a, b, true);
-		kv2 = dt * a;
-		kp2 = dt * b;
-		ri = p.radius + 1932.0 / 2197.0 * kr0 - 7200.0 / 2197.0 * kr1 + 7296.0 / 2197.0 * kr2;
-		kr3 = dt * (p.v_radial + 1932.0 / 2197.0 * kv0 - 7200.0 / 2197.0 * kv1 + 7296.0 / 2197.0 * kv2);
-		stage_rates(m, p, ri, solar_gm(S, ri), a, b, true);
-		kv3 = dt * a;
-		kp3 = dt * b;
-		ri = p.radius + 439.0 / 216.0 * kr0 - 8.0 * kr1 + 3680.0 / 513.0 * kr2 - 845.0 / 4104.0 * kr3;
-		kr4 = dt * (p.v_radial + 439.0 / 216.0 * kv0 - 8.0 * kv1 + 3680.0 / 513.0 * kv2 - 845.0 / 4104.0 * kv3);
-		stage_rates(m, p, ri, solar_gm(S, ri), a, b, true);
-		kv4 = dt * a;
-		kp4 = dt * b;
-		ri = p.radius - 8.0 / 27.0 * kr0 + 2.0 * kr1 - 3544.0 / 2565.0 * kr2 + 1859.0 / 4104.0 * kr3 - 11.0 / 40.0 * kr4;
-		kr5 = dt * (p.v_radial - 8.0 / 27.0 * kv0 + 2.0 * kv1 - 3544.0 / 2565.0 * kv2 + 1859.0 / 4104.0 * kv3 - 11.0 / 40.0 * kv4);
-		stage_rates(m, p, ri, solar_gm(S, ri), a, b, true);
-		kv5 = dt * a;
-		kp5 = dt * b;
-		const double r4 = p.radius + 25.0 / 216.0 * kr0 + 1408.0 / 2565.0 * kr2 + 2197.0 / 4104.0 * kr3 - 1.0 / 5.0 * kr4;
-		const double v4 = p.v_radial + 25.0 / 216.0 * kv0 + 1408.0 / 2565.0 * kv2 + 2197.0 / 4104.0 * kv3 - 1.0 / 5.0 * kv4;
-		const double p4 = p.phi + 25.0 / 216.0 * kp0 + 1408.0 / 2565.0 * kp2 + 2197.0 / 4104.0 * kp3 - 1.0 / 5.0 * kp4;
-		const double r5 = p.radius + 16.0 / 135.0 * kr0 + 6656.0 / 12825.0 * kr2 + 28561.0 / 56430.0 * kr3 - 9.0 / 50.0 * kr4 + 2.0 / 55.0 * kr5;
-		const double v5 = p.v_radial + 16.0 / 135.0 * kv0 + 6656.0 / 12825.0 * kv2 + 28561.0 / 56430.0 * kv3 - 9.0 / 50.0 * kv4 + 2.0 / 55.0 * kv5;
-		const double p5 = p.phi + 16.0 / 135.0 * kp0 + 6656.0 / 12825.0 * kp2 + 28561.0 / 56430.0 * kp3 - 9.0 / 50.0 * kp4 + 2.0 / 55.0 * kp5;
-		const double e0 = fabs(r5 - r4), e1 = fabs(v5 - v4), e2 = fabs(p5 - p4);
-		const double new_step = next_step_size_t(m, dt, e0, e1, e2);
-		const bool within = isfinite(e0) && e0 <= DMS_RK45_TOL_R_KM && isfinite(e1) && e1 <= DMS_RK45_TOL_V_KMS && isfinite(e2) && e2 <= DMS_RK45_TOL_PHI;
-		if(within)
-		{
-			p.time = p.time + dt;
-			p.radius = r4 < 0.0 ? 0.0 : r4;
-			p.v_radial = v4;
-			p.phi = p4;
-			p.time_step = new_step;
-			return RK_ACCEPTED;
-		}
-		if(new_step < DMS_RK45_ABS_MIN_STEP_S || inner >= DMS_RK45_MAX_INNER_RETRIES)
-		{
-			const bool ok = isfinite(r4) && isfinite(v4) && isfinite(p4);
-			p.time = p.time + DMS_RK45_ABS_MIN_STEP_S;
-			if(ok)
-			{
-				p.radius = r4 < 0.0 ? 0.0 : r4;
-				p.v_radial = v4;
-				p.phi = p4;
-			}
-			p.time_step = DMS_RK45_ABS_MIN_STEP_S;
-			return RK_FORCED;
-		}
-		p.time_step = new_step;
-		return RK_RETRY;
-	}
-}
-
-__device__ __forceinline__ int rk45_attempt_unrolled(const DevSolar& S, Prop& p, int inner)
-{
-	IeeeMath m;
-	return rk45_attempt_t(S, p, inner, m);
-}
-
-// The IEEE attempt, out of line: the fallback of rk45_attempt_certified.
-static __device__ __noinline__ int rk45_attempt_ieee(const DevSolar& S, Prop& p, int inner)
-{
-	IeeeMath m;
-	return rk45_attempt_t(S, p, inner, m);
-}
-
-// Solar_Model::Mass as G*M for tables whose buckets hold at most one knot
-// (S.bucket_single_step): both candidate intervals are loaded with the bucket's base and the
-// interval of the search in knot_index is selected, so the lookup has no branch.  Same value
-// as solar_gm.
-__device__ __forceinline__ double solar_gm_select(const DevSolar& S, double r)
-{
-	const double x = r < 0.0 ? 0.0 : r;
-	const double xc = !(x >= 0.0) ? 0.0 : (x > DMS_RSUN_KM ? DMS_RSUN_KM : x);
-	int b = static_cast<int>(xc * S.bucket_scale);
-	b = b > S.nbuckets ? S.nbuckets : b;
+	double whole;
+	unsigned int b = fast::floor_index(r * S.bucket_scale, whole);
+	b = b > static_cast<unsigned int>(S.nbuckets) ? static_cast<unsigned int>(S.nbuckets) : b;
 	int i = __ldg(S.bucket + b);
 	DMS_CHECK_INDEX(i, 0, S.n - 1, BOUNDS_KNOT);
-	const double r0 = __ldg(S.r + i), r1 = __ldg(S.r + i + 1);
-	const double y0 = __ldg(S.gm + i), y1 = __ldg(S.gm + i + 1);
-	const double s0 = __ldg(S.gm_s + i), s1 = __ldg(S.gm_s + i + 1);
-	const bool up = (i < S.n - 2) & (r1 <= x);
-	const double v = up ? y1 + (x - r1) * s1 : y0 + (x - r0) * s0;
-	return !isfinite(r) ? NAN : (r > DMS_RSUN_KM ? DMS_GMSUN_KM3S2 : v);
+	return i;
 }
 
-// One stage's dv/dt = J*J/r/r/r - gm/r/r (r clamped to >= 1 km) and, when wanted,
-// dphi/dt = J/r/r (0 in radial mode, for J = 0 or r <= 0), with the certified division and
-// without branches: every quotient by r shares one reciprocal.  A stage with 0 < r < 1 km (where
-// the reference divides J by the unclamped r) clears `good`, which hands the attempt to IEEE.
+__device__ __forceinline__ double solar_gm_fast(const DevSolar& S, double r)
+{
+	const Knot* k = S.gm_pack + bucket_base(S, r);
+	const Knot k0 = load_knot(k), k1 = load_knot(k + 1);
+	const bool up = k1.r <= r;  // the last knot is stored as infinity: no step beyond the last interval
+	const double r0 = up ? k1.r : k0.r, y0 = up ? k1.gm : k0.gm, s0 = up ? k1.gm_s : k0.gm_s;
+	const double v = y0 + (r - r0) * s0;
+	return r > DMS_RSUN_KM ? DMS_GMSUN_KM3S2 : v;
+}
+
+// v_esc^2(r) inside the Sun (0 <= r <= R_sun), as table_eval(S, S.vesc2, S.vesc2_s, r).
+__device__ __forceinline__ double solar_vesc2_fast(const DevSolar& S, double r)
+{
+	const int i = bucket_base(S, r);
+	const Knot k0 = load_knot(S.gm_pack + i), k1 = load_knot(S.gm_pack + i + 1);
+	const bool up = k1.r <= r;
+	const double slope = __ldg(S.vesc2_s + i + (up ? 1 : 0));
+	return (up ? k1.vesc2 : k0.vesc2) + (r - (up ? k1.r : k0.r)) * slope;
+}
+
+// One stage's dv/dt = J*J/r/r/r - gm/r/r and dphi/dt = J/r/r, each division rounded as the
+// reference rounds it; the quotients share one reciprocal.  A radius below 1 km (where the
+// reference clamps it) or not finite clears `good`, which hands the attempt to IEEE arithmetic.
 template <bool WANT_PHI>
-__device__ __forceinline__ void cert_stage(const DevSolar& S, const Prop& p, double r, double& dv, double& dphi, bool& good)
+__device__ __forceinline__ void fast_stage(const DevSolar& S, double J, double JJ, double r, double& dv, double& dphi, bool& good)
 {
-	const double gm = solar_gm_select(S, r);
-	const double rc = r < 1.0 ? 1.0 : r;
-	const fast::Recip R = fast::recip(rc);
-	const double jj = p.J * p.J;
-	dv = fast::div(fast::div(fast::div(jj, R, good), R, good), R, good) - fast::div(fast::div(gm, R, good), R, good);
-	dphi = 0.0;
+	const double gm = solar_gm_fast(S, r);
+	good &= (r >= 1.0) & (r < 0x1p100);
+	const fast::Recip R = fast::recip(r, good);
+	dv = fast::div(fast::div(fast::div(JJ, R), R), R) - fast::div(fast::div(gm, R), R);
 	if(WANT_PHI)
-	{
-		const bool zero = (p.radial_mode != 0) | (p.J == 0.0) | (r <= 0.0);
-		const double q = fast::div(fast::div(p.J, R, good), R, good);
-		dphi = zero ? 0.0 : q;
-		good &= zero | (r >= 1.0);
-	}
+		dphi = fast::div(fast::div(J, R), R);
 }
 
-// The factor of RK45_Next_Step_Size for one error component without branches: 0.84 (tol/e)^(1/4)
-// when e > 0 and the result is finite, else +inf (no limit); e outside (0, inf) divides 1.
-__device__ __forceinline__ double cert_step_factor(double tol, double e, bool& good)
+// tol / e of one error component of RK45_Next_Step_Size, +inf when the component sets no limit.
+__device__ __forceinline__ double fast_tolerance_ratio(double tol, double e, bool& good)
 {
-	const bool use = (e > 0.0) & isfinite(e);
-	const double c = 0.84 * fast::sqrt(fast::sqrt(fast::div(tol, use ? e : 1.0, good), good), good);
-	return (use & isfinite(c)) ? c : INFINITY;
-}
-
-// The written-out attempt of rk45_attempt_t with the certified division and square root and
-// no branch before its final accept / retry decision, so that the compiler can overlap the
-// stages that do not depend on one another: the radius of stage j needs the slopes of stages
-// up to j - 2 only, so stages 0 and 1, 2 and 3, 4 and 5 are independent pairs.  `good` is
-// cleared when any certificate fails; p is then unchanged and the caller repeats the attempt
-// with IEEE arithmetic.
-__device__ __forceinline__ int rk45_attempt_cert(const DevSolar& S, Prop& p, int inner, bool& good)
-{
-	const double dt = p.time_step;
-	double kr0, kr1, kr2, kr3, kr4, kr5, kv0, kv1, kv2, kv3, kv4, kv5, kp0, kp1, kp2, kp3, kp4, kp5, ri, a;
-	kr0 = dt * p.v_radial;
-	cert_stage<true>(S, p, p.radius, a, kp0, good);
-	kv0 = dt * a;
-	kp0 = dt * kp0;
-	ri = p.radius + kr0 / 4.0;
-	kr1 = dt * (p.v_radial + kv0 / 4.0);
-	cert_stage<false>(S, p, ri, a, kp1, good);
-	kv1 = dt * a;
-	ri = p.radius + 3.0 / 32.0 * kr0 + 9.0 / 32.0 * kr1;
-	kr2 = dt * (p.v_radial + 3.0 / 32.0 * kv0 + 9.0 / 32.0 * kv1);
-	cert_stage<true>(S, p, ri, a, kp2, good);
-	kv2 = dt * a;
-	kp2 = dt * kp2;
-	ri = p.radius + 1932.0 / 2197.0 * kr0 - 7200.0 / 2197.0 * kr1 + 7296.0 / 2197.0 * kr2;
-	kr3 = dt * (p.v_radial + 1932.0 / 2197.0 * kv0 - 7200.0 / 2197.0 * kv1 + 7296.0 / 2197.0 * kv2);
-	cert_stage<true>(S, p, ri, a, kp3, good);
-	kv3 = dt * a;
-	kp3 = dt * kp3;
-	ri = p.radius + 439.0 / 216.0 * kr0 - 8.0 * kr1 + 3680.0 / 513.0 * kr2 - 845.0 / 4104.0 * kr3;
-	kr4 = dt * (p.v_radial + 439.0 / 216.0 * kv0 - 8.0 * kv1 + 3680.0 / 513.0 * kv2 - 845.0 / 4104.0 * kv3);
-	cert_stage<true>(S, p, ri, a, kp4, good);
-	kv4 = dt * a;
-	kp4 = dt * kp4;
-	ri = p.radius - 8.0 / 27.0 * kr0 + 2.0 * kr1 - 3544.0 / 2565.0 * kr2 + 1859.0 / 4104.0 * kr3 - 11.0 / 40.0 * kr4;
-	kr5 = dt * (p.v_radial - 8.0 / 27.0 * kv0 + 2.0 * kv1 - 3544.0 / 2565.0 * kv2 + 1859.0 / 4104.0 * kv3 - 11.0 / 40.0 * kv4);
-	cert_stage<true>(S, p, ri, a, kp5, good);
-	kv5 = dt * a;
-	kp5 = dt * kp5;
-	const double r4 = p.radius + 25.0 / 216.0 * kr0 + 1408.0 / 2565.0 * kr2 + 2197.0 / 4104.0 * kr3 - 1.0 / 5.0 * kr4;
-	const double v4 = p.v_radial + 25.0 / 216.0 * kv0 + 1408.0 / 2565.0 * kv2 + 2197.0 / 4104.0 * kv3 - 1.0 / 5.0 * kv4;
-	const double p4 = p.phi + 25.0 / 216.0 * kp0 + 1408.0 / 2565.0 * kp2 + 2197.0 / 4104.0 * kp3 - 1.0 / 5.0 * kp4;
-	const double r5 = p.radius + 16.0 / 135.0 * kr0 + 6656.0 / 12825.0 * kr2 + 28561.0 / 56430.0 * kr3 - 9.0 / 50.0 * kr4 + 2.0 / 55.0 * kr5;
-	const double v5 = p.v_radial + 16.0 / 135.0 * kv0 + 6656.0 / 12825.0 * kv2 + 28561.0 / 56430.0 * kv3 - 9.0 / 50.0 * kv4 + 2.0 / 55.0 * kv5;
-	const double p5 = p.phi + 16.0 / 135.0 * kp0 + 6656.0 / 12825.0 * kp2 + 28561.0 / 56430.0 * kp3 - 9.0 / 50.0 * kp4 + 2.0 / 55.0 * kp5;
-	const double e0 = fabs(r5 - r4), e1 = fabs(v5 - v4), e2 = fabs(p5 - p4);
-	// RK45_Next_Step_Size (src/Simulation_Trajectory.cpp:477-502) as selects: the factor is
-	// limited by each component in turn, clamped to [0.1, 4], and the step sanitised; non-finite
-	// errors give 0.1 x the current step
-	double factor = DMS_RK45_MAX_STEP_FACTOR;
-	const double c0 = cert_step_factor(DMS_RK45_TOL_R_KM, e0, good);
-	factor = c0 < factor ? c0 : factor;
-	const double c1 = cert_step_factor(DMS_RK45_TOL_V_KMS, e1, good);
-	factor = c1 < factor ? c1 : factor;
-	const double c2 = cert_step_factor(DMS_RK45_TOL_PHI, e2, good);
-	factor = c2 < factor ? c2 : factor;
-	factor = factor > DMS_RK45_MAX_STEP_FACTOR ? DMS_RK45_MAX_STEP_FACTOR : factor;
-	factor = factor < DMS_RK45_MIN_STEP_FACTOR ? DMS_RK45_MIN_STEP_FACTOR : factor;
-	const double grown = factor * dt;
-	const double sane = (!isfinite(grown) | (grown <= 0.0)) ? DMS_RK45_DEFAULT_STEP_S
-	                    : (grown < DMS_RK45_ABS_MAX_STEP_S ? grown : DMS_RK45_ABS_MAX_STEP_S);
-	const bool finite_err = isfinite(e0) & isfinite(e1) & isfinite(e2);
-	const double new_step = finite_err ? sane : DMS_RK45_MIN_STEP_FACTOR * dt;
-	const bool within = finite_err & (e0 <= DMS_RK45_TOL_R_KM) & (e1 <= DMS_RK45_TOL_V_KMS) & (e2 <= DMS_RK45_TOL_PHI);
-	if(!good)
-		return RK_RETRY;
-	if(within)
-	{
-		p.time = p.time + dt;
-		p.radius = r4 < 0.0 ? 0.0 : r4;
-		p.v_radial = v4;
-		p.phi = p4;
-		p.time_step = new_step;
-		return RK_ACCEPTED;
-	}
-	if(new_step < DMS_RK45_ABS_MIN_STEP_S || inner >= DMS_RK45_MAX_INNER_RETRIES)
-	{
-		const bool ok = isfinite(r4) && isfinite(v4) && isfinite(p4);
-		p.time = p.time + DMS_RK45_ABS_MIN_STEP_S;
-		if(ok)
-		{
-			p.radius = r4 < 0.0 ? 0.0 : r4;
-			p.v_radial = v4;
-			p.phi = p4;
-		}
-		p.time_step = DMS_RK45_ABS_MIN_STEP_S;
-		return RK_FORCED;
-	}
-	p.time_step = new_step;
-	return RK_RETRY;
-}
-
-// The attempt of rk45_attempt_cert computed by two lanes of a warp: an owner (role 1, the lane
-// whose propagator steps) and a helper (role 2, an idle lane), `partner` being the other lane of
-// the pair.  Every lane of the warp calls it (the exchanges are warp shuffles); lanes without a
-// pair (role 0) compute nothing that is kept.  The radius of stage j needs the slopes of the
-// stages up to j - 2 only, so the owner computes stages 0, 2, 4 and the helper 1, 3, 5, three
-// rounds instead of six, exchanging the new slopes after each round; the owner then forms the
-// solutions, the helper two of the three step-size factors.  Every value is formed by the same
-// operations in the same order as in rk45_attempt_cert, so the result is the same bits.  Only
-// the owner's p is changed; `good` (owner) is cleared when a certificate of either lane failed.
-__device__ __forceinline__ int rk45_attempt_pair(const DevSolar& S, Prop& p, int inner, int role, int partner, bool& good)
-{
-	constexpr unsigned int FULL = 0xffffffffu;
-	const int me = threadIdx.x & 31;
-	const int src = role == 2 ? partner : me;
-	Prop q = p;
-	q.time_step = __shfl_sync(FULL, p.time_step, src);
-	q.radius = __shfl_sync(FULL, p.radius, src);
-	q.v_radial = __shfl_sync(FULL, p.v_radial, src);
-	q.J = __shfl_sync(FULL, p.J, src);
-	q.radial_mode = __shfl_sync(FULL, p.radial_mode, src);
-	const bool odd = role == 2;
-	const int other = role == 0 ? me : partner;
-	const double dt = q.time_step;
-	const double R = q.radius, V = q.v_radial;
-	double a, b;
-	const double kr0 = dt * V;
-	// first pair: stage 0 (owner) | stage 1 (helper)
-	const double r_s1 = R + kr0 / 4.0;
-	cert_stage<true>(S, q, odd ? r_s1 : R, a, b, good);
-	const double kv_m1 = dt * a, kp_m1 = dt * b;
-	const double kv_o1 = __shfl_sync(FULL, kv_m1, other);
-	const double kv0 = odd ? kv_o1 : kv_m1, kv1 = odd ? kv_m1 : kv_o1;
-	const double kr1 = dt * (V + kv0 / 4.0);
-	const double kr2 = dt * (V + 3.0 / 32.0 * kv0 + 9.0 / 32.0 * kv1);
-	// second pair: stage 2 | stage 3
-	const double r_s2 = R + 3.0 / 32.0 * kr0 + 9.0 / 32.0 * kr1;
-	const double r_s3 = R + 1932.0 / 2197.0 * kr0 - 7200.0 / 2197.0 * kr1 + 7296.0 / 2197.0 * kr2;
-	cert_stage<true>(S, q, odd ? r_s3 : r_s2, a, b, good);
-	const double kv_m2 = dt * a, kp_m2 = dt * b;
-	const double kv_o2 = __shfl_sync(FULL, kv_m2, other);
-	const double kv2 = odd ? kv_o2 : kv_m2, kv3 = odd ? kv_m2 : kv_o2;
-	const double kr3 = dt * (V + 1932.0 / 2197.0 * kv0 - 7200.0 / 2197.0 * kv1 + 7296.0 / 2197.0 * kv2);
-	const double kr4 = dt * (V + 439.0 / 216.0 * kv0 - 8.0 * kv1 + 3680.0 / 513.0 * kv2 - 845.0 / 4104.0 * kv3);
-	// third pair: stage 4 | stage 5
-	const double r_s4 = R + 439.0 / 216.0 * kr0 - 8.0 * kr1 + 3680.0 / 513.0 * kr2 - 845.0 / 4104.0 * kr3;
-	const double r_s5 = R - 8.0 / 27.0 * kr0 + 2.0 * kr1 - 3544.0 / 2565.0 * kr2 + 1859.0 / 4104.0 * kr3 - 11.0 / 40.0 * kr4;
-	cert_stage<true>(S, q, odd ? r_s5 : r_s4, a, b, good);
-	const double kv_m3 = dt * a, kp_m3 = dt * b;
-	// both lanes gather every slope: the owner's kp of rounds 1-3 are kp0, kp2, kp4, the
-	// helper's kp3, kp5 (its round-1 dphi belongs to stage 1, which has none)
-	const double kv_o3 = __shfl_sync(FULL, kv_m3, other);
-	const double kp_o1 = __shfl_sync(FULL, kp_m1, other);
-	const double kp_o2 = __shfl_sync(FULL, kp_m2, other);
-	const double kp_o3 = __shfl_sync(FULL, kp_m3, other);
-	const double kv4 = odd ? kv_o3 : kv_m3, kv5 = odd ? kv_m3 : kv_o3;
-	const double kp0 = odd ? kp_o1 : kp_m1;
-	const double kp2 = odd ? kp_o2 : kp_m2, kp3 = odd ? kp_m2 : kp_o2;
-	const double kp4 = odd ? kp_o3 : kp_m3, kp5 = odd ? kp_m3 : kp_o3;
-	const double kr5 = dt * (V - 8.0 / 27.0 * kv0 + 2.0 * kv1 - 3544.0 / 2565.0 * kv2 + 1859.0 / 4104.0 * kv3 - 11.0 / 40.0 * kv4);
-	const double r4 = R + 25.0 / 216.0 * kr0 + 1408.0 / 2565.0 * kr2 + 2197.0 / 4104.0 * kr3 - 1.0 / 5.0 * kr4;
-	const double v4 = V + 25.0 / 216.0 * kv0 + 1408.0 / 2565.0 * kv2 + 2197.0 / 4104.0 * kv3 - 1.0 / 5.0 * kv4;
-	const double p4 = p.phi + 25.0 / 216.0 * kp0 + 1408.0 / 2565.0 * kp2 + 2197.0 / 4104.0 * kp3 - 1.0 / 5.0 * kp4;
-	const double r5 = R + 16.0 / 135.0 * kr0 + 6656.0 / 12825.0 * kr2 + 28561.0 / 56430.0 * kr3 - 9.0 / 50.0 * kr4 + 2.0 / 55.0 * kr5;
-	const double v5 = V + 16.0 / 135.0 * kv0 + 6656.0 / 12825.0 * kv2 + 28561.0 / 56430.0 * kv3 - 9.0 / 50.0 * kv4 + 2.0 / 55.0 * kv5;
-	const double p5 = p.phi + 16.0 / 135.0 * kp0 + 6656.0 / 12825.0 * kp2 + 28561.0 / 56430.0 * kp3 - 9.0 / 50.0 * kp4 + 2.0 / 55.0 * kp5;
-	const double e0 = fabs(r5 - r4), e1 = fabs(v5 - v4), e2 = fabs(p5 - p4);
-	// the step-size factors: c0 and c2 on the owner, c1 (and c2 again) on the helper, whose e2
-	// needs the owner's phi
-	const double phi_o = __shfl_sync(FULL, p.phi, src);
-	const double p4h = phi_o + 25.0 / 216.0 * kp0 + 1408.0 / 2565.0 * kp2 + 2197.0 / 4104.0 * kp3 - 1.0 / 5.0 * kp4;
-	const double p5h = phi_o + 16.0 / 135.0 * kp0 + 6656.0 / 12825.0 * kp2 + 28561.0 / 56430.0 * kp3 - 9.0 / 50.0 * kp4 + 2.0 / 55.0 * kp5;
-	const double e2h = fabs(p5h - p4h);
-	const double cA = cert_step_factor(odd ? DMS_RK45_TOL_V_KMS : DMS_RK45_TOL_R_KM, odd ? e1 : e0, good);
-	const double cB = cert_step_factor(DMS_RK45_TOL_PHI, e2h, good);
-	const double c1 = __shfl_sync(FULL, cA, other), c2 = cB;
-	const int helper_good = __shfl_sync(FULL, static_cast<int>(good), other);
-	if(role != 1)
-		return RK_RETRY;
-	good = good && helper_good != 0;
-	const double c0 = cA;
-	double factor = DMS_RK45_MAX_STEP_FACTOR;
-	factor = c0 < factor ? c0 : factor;
-	factor = c1 < factor ? c1 : factor;
-	factor = c2 < factor ? c2 : factor;
-	factor = factor > DMS_RK45_MAX_STEP_FACTOR ? DMS_RK45_MAX_STEP_FACTOR : factor;
-	factor = factor < DMS_RK45_MIN_STEP_FACTOR ? DMS_RK45_MIN_STEP_FACTOR : factor;
-	const double grown = factor * dt;
-	const double sane = (!isfinite(grown) | (grown <= 0.0)) ? DMS_RK45_DEFAULT_STEP_S
-	                    : (grown < DMS_RK45_ABS_MAX_STEP_S ? grown : DMS_RK45_ABS_MAX_STEP_S);
-	const bool finite_err = isfinite(e0) & isfinite(e1) & isfinite(e2);
-	const double new_step = finite_err ? sane : DMS_RK45_MIN_STEP_FACTOR * dt;
-	const bool within = finite_err & (e0 <= DMS_RK45_TOL_R_KM) & (e1 <= DMS_RK45_TOL_V_KMS) & (e2 <= DMS_RK45_TOL_PHI);
-	if(!good)
-		return RK_RETRY;
-	if(within)
-	{
-		p.time = p.time + dt;
-		p.radius = r4 < 0.0 ? 0.0 : r4;
-		p.v_radial = v4;
-		p.phi = p4;
-		p.time_step = new_step;
-		return RK_ACCEPTED;
-	}
-	if(new_step < DMS_RK45_ABS_MIN_STEP_S || inner >= DMS_RK45_MAX_INNER_RETRIES)
-	{
-		const bool ok = isfinite(r4) && isfinite(v4) && isfinite(p4);
-		p.time = p.time + DMS_RK45_ABS_MIN_STEP_S;
-		if(ok)
-		{
-			p.radius = r4 < 0.0 ? 0.0 : r4;
-			p.v_radial = v4;
-			p.phi = p4;
-		}
-		p.time_step = DMS_RK45_ABS_MIN_STEP_S;
-		return RK_FORCED;
-	}
-	p.time_step = new_step;
-	return RK_RETRY;
-}
-
-// One attempt with the certified straight-line division and square root; when any certificate
-// fails (or the tables' buckets can hold two knots), the attempt is repeated from the same
-// state with IEEE arithmetic.  Either way the result is bit-identical with rk45_attempt_unrolled.
-__device__ __forceinline__ int rk45_attempt_certified(const DevSolar& S, Prop& p, int inner)
-{
-	bool good = S.bucket_single_step != 0;
-	if(good)
-	{
-		const int rk = rk45_attempt_cert(S, p, inner, good);
-		if(good)
-			return rk;
-	}
-	return rk45_attempt_ieee(S, p, inner);
+	const bool in = (e > 0x1p-400) & (e < 0x1p400);
+	good &= in | !(e > 0.0);
+	const double q = fast::div(tol, fast::recip(in ? e : 1.0, good));
+	return in ? q : INFINITY;
 }
 
 // Runge-Kutta-Fehlberg 4(5) coefficients of src/Simulation_Trajectory.cpp:1492-1540: stage
@@ -1108,7 +748,8 @@ __constant__ double RKF_A[6][5] = {
 __constant__ double RKF_B4[6] = {25.0 / 216.0, 0.0, 1408.0 / 2565.0, 2197.0 / 4104.0, -(1.0 / 5.0), 0.0};
 __constant__ double RKF_B5[6] = {16.0 / 135.0, 0.0, 6656.0 / 12825.0, 28561.0 / 56430.0, -(9.0 / 50.0), 2.0 / 55.0};
 
-__device__ __forceinline__ int rk45_attempt(const DevSolar& S, Prop& p, int inner)
+// The attempt with IEEE division and square root, out of line: the fallback of rk45_attempt.
+static __device__ __noinline__ int rk45_attempt_ieee(const DevSolar& S, Prop& p, int inner)
 {
 	{
 		const double dt = p.time_step;
@@ -1165,6 +806,85 @@ __device__ __forceinline__ int rk45_attempt(const DevSolar& S, Prop& p, int inne
 		p.time_step = new_step;
 		return RK_RETRY;
 	}
+}
+
+// The attempt with the six stages written out and the straight-line division and square root of
+// dms_fastmath.cuh: no branch before its accept / retry decision.  The radius of stage j needs
+// the slopes of stages up to j - 2 only, so the compiler overlaps stages 0 and 1, 2 and 3, 4 and 5,
+// which is what a lane that runs alone needs; with every lane busy it executes about 30 % fewer
+// instructions than a loop over the stages with IEEE operations.  The step-size factor is
+// 0.84 (tol / e)^(1/4) limited by each of three components; every operation of that expression
+// rounds monotonically, so the smallest ratio gives the smallest factor and one root serves all.
+// When a condition of the arithmetic fails the step is repeated by rk45_attempt_ieee; the results
+// are the same bits.
+__device__ __forceinline__ int rk45_attempt(const DevSolar& S, Prop& p, int inner)
+{
+	const double dt = p.time_step, R = p.radius, V = p.v_radial, PHI = p.phi, J = p.J;
+	const double JJ = J * J;
+	bool good = (S.fast_tables != 0) & ((J == 0.0) | ((J > 0x1p-200) & (J < 0x1p200)));
+	double kr0, kr1, kr2, kr3, kr4, kr5, kv0, kv1, kv2, kv3, kv4, kv5, kp0, kp2, kp3, kp4, kp5, a, b = 0.0;
+	kr0 = dt * V;
+	fast_stage<true>(S, J, JJ, R, a, b, good);
+	kv0 = dt * a;
+	kp0 = dt * b;
+	kr1 = dt * (V + kv0 / 4.0);
+	fast_stage<false>(S, J, JJ, R + kr0 / 4.0, a, b, good);
+	kv1 = dt * a;
+	kr2 = dt * (V + 3.0 / 32.0 * kv0 + 9.0 / 32.0 * kv1);
+	fast_stage<true>(S, J, JJ, R + 3.0 / 32.0 * kr0 + 9.0 / 32.0 * kr1, a, b, good);
+	kv2 = dt * a;
+	kp2 = dt * b;
+	kr3 = dt * (V + 1932.0 / 2197.0 * kv0 - 7200.0 / 2197.0 * kv1 + 7296.0 / 2197.0 * kv2);
+	fast_stage<true>(S, J, JJ, R + 1932.0 / 2197.0 * kr0 - 7200.0 / 2197.0 * kr1 + 7296.0 / 2197.0 * kr2, a, b, good);
+	kv3 = dt * a;
+	kp3 = dt * b;
+	kr4 = dt * (V + 439.0 / 216.0 * kv0 - 8.0 * kv1 + 3680.0 / 513.0 * kv2 - 845.0 / 4104.0 * kv3);
+	fast_stage<true>(S, J, JJ, R + 439.0 / 216.0 * kr0 - 8.0 * kr1 + 3680.0 / 513.0 * kr2 - 845.0 / 4104.0 * kr3, a, b, good);
+	kv4 = dt * a;
+	kp4 = dt * b;
+	kr5 = dt * (V - 8.0 / 27.0 * kv0 + 2.0 * kv1 - 3544.0 / 2565.0 * kv2 + 1859.0 / 4104.0 * kv3 - 11.0 / 40.0 * kv4);
+	fast_stage<true>(S, J, JJ, R - 8.0 / 27.0 * kr0 + 2.0 * kr1 - 3544.0 / 2565.0 * kr2 + 1859.0 / 4104.0 * kr3 - 11.0 / 40.0 * kr4, a, b, good);
+	kv5 = dt * a;
+	kp5 = dt * b;
+	const double r4 = R + 25.0 / 216.0 * kr0 + 1408.0 / 2565.0 * kr2 + 2197.0 / 4104.0 * kr3 - 1.0 / 5.0 * kr4;
+	const double v4 = V + 25.0 / 216.0 * kv0 + 1408.0 / 2565.0 * kv2 + 2197.0 / 4104.0 * kv3 - 1.0 / 5.0 * kv4;
+	const double p4 = PHI + 25.0 / 216.0 * kp0 + 1408.0 / 2565.0 * kp2 + 2197.0 / 4104.0 * kp3 - 1.0 / 5.0 * kp4;
+	const double r5 = R + 16.0 / 135.0 * kr0 + 6656.0 / 12825.0 * kr2 + 28561.0 / 56430.0 * kr3 - 9.0 / 50.0 * kr4 + 2.0 / 55.0 * kr5;
+	const double v5 = V + 16.0 / 135.0 * kv0 + 6656.0 / 12825.0 * kv2 + 28561.0 / 56430.0 * kv3 - 9.0 / 50.0 * kv4 + 2.0 / 55.0 * kv5;
+	const double p5 = PHI + 16.0 / 135.0 * kp0 + 6656.0 / 12825.0 * kp2 + 28561.0 / 56430.0 * kp3 - 9.0 / 50.0 * kp4 + 2.0 / 55.0 * kp5;
+	const double e0 = fabs(r5 - r4), e1 = fabs(v5 - v4), e2 = fabs(p5 - p4);
+	// RK45_Next_Step_Size (src/Simulation_Trajectory.cpp:477-502): a ratio of 10^6 or more already
+	// gives more than the largest factor
+	double ratio = 1.0e6;
+	const double q0 = fast_tolerance_ratio(DMS_RK45_TOL_R_KM, e0, good);
+	const double q1 = fast_tolerance_ratio(DMS_RK45_TOL_V_KMS, e1, good);
+	const double q2 = fast_tolerance_ratio(DMS_RK45_TOL_PHI, e2, good);
+	ratio = q0 < ratio ? q0 : ratio;
+	ratio = q1 < ratio ? q1 : ratio;
+	ratio = q2 < ratio ? q2 : ratio;
+	double factor = 0.84 * fast::sqrt(fast::sqrt(ratio, good), good);
+	factor = factor > DMS_RK45_MAX_STEP_FACTOR ? DMS_RK45_MAX_STEP_FACTOR : factor;
+	factor = factor < DMS_RK45_MIN_STEP_FACTOR ? DMS_RK45_MIN_STEP_FACTOR : factor;
+	// a non-finite error has cleared `good` or set no limit; dt is finite and positive (sanitized_step)
+	const double grown = factor * dt;
+	const double new_step = grown < DMS_RK45_ABS_MAX_STEP_S ? grown : DMS_RK45_ABS_MAX_STEP_S;
+	const bool within = (e0 <= DMS_RK45_TOL_R_KM) & (e1 <= DMS_RK45_TOL_V_KMS) & (e2 <= DMS_RK45_TOL_PHI);
+	good &= (e0 < INFINITY) & (e1 < INFINITY) & (e2 < INFINITY) & (grown > 0.0);
+	if(!good)
+		return rk45_attempt_ieee(S, p, inner);
+	if(within)
+	{
+		p.time = p.time + dt;
+		p.radius = r4 < 0.0 ? 0.0 : r4;
+		p.v_radial = v4;
+		p.phi = p4;
+		p.time_step = new_step;
+		return RK_ACCEPTED;
+	}
+	if(new_step < DMS_RK45_ABS_MIN_STEP_S || inner >= DMS_RK45_MAX_INNER_RETRIES)
+		return rk45_attempt_ieee(S, p, inner);  // the forced acceptance (rare)
+	p.time_step = new_step;
+	return RK_RETRY;
 }
 
 __device__ __forceinline__ double prop_radius(const Prop& p) { return p.radius < 0.0 ? 0.0 : p.radius; }

@@ -263,6 +263,11 @@ std::string Load_Solar_Tables(const std::string& path, SolarTables& t)
 	}
 	if(Knot_Search(t.r, DMS_RSUN_KM) > t.bucket_index[t.nbuckets] + 1)
 		t.bucket_single_step = 0;
+	const auto in_range = [](double x) { return x == 0.0 || (x >= 0x1p-300 && x <= 0x1p+300); };
+	t.fast_tables = t.bucket_single_step;
+	for(int i = 0; i < n; i++)
+		if(!in_range(t.gm[i]) || (i < n - 1 && !in_range(t.gm_s[i])))
+			t.fast_tables = 0;
 	return "";
 }
 

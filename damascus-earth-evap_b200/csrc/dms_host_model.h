@@ -33,6 +33,9 @@ struct SolarTables
 	// base + 1 (no bucket holds two knots)
 	int nbuckets = 0;
 	int bucket_single_step = 0;
+	// 1 when, besides, every G*M value and slope is 0 or within [2^-300, 2^300]: the range of the
+	// device's straight-line division (dms_fastmath.cuh)
+	int fast_tables = 0;
 	std::vector<uint16_t> bucket_index;
 };
 

@@ -19,569 +19,637 @@ namespace
 using namespace lane;
 using StrictLane = LaneT<Prop, Event>;
 
-// The written-out attempt: with the certified straight-line division and square root
-// (DMS_CERTIFIED_MATH = 1, the default; IEEE fallback per attempt) or with IEEE arithmetic.
-__device__ __forceinline__ int rk45_attempt_written_out(const DevSolar& S, Prop& p, int inner)
+
+// ---------------------------------------------------------------------------------------------
+// One pass of the Propagate_Freely loop body (src/Simulation_Trajectory.cpp:876-1116), split at the
+// RK45 retry loop: when no step is in progress the pre-step bounds are applied and a step is opened
+// (step_begin); every pass makes one RK45 attempt; an accepted attempt runs the optical-depth,
+// boundary and commit logic (strict_step).  The propagator keeps the state at the start of the step
+// until the step is committed, so a rejected step has nothing to restore.
+//
+// The pass is one straight path of about 1 500 instructions: with every lane busy the kernel is bound
+// by instruction supply (an SM fetches full rate from 32 KB of instruction cache; measured
+// with a straight-line FP32 loop: 1.2-1.4 cycles per instruction of a warp up to 32 KB, 3.2 up to
+// 128 KB, 6 beyond).  What is rare in a pass sits in the non-inlined functions below.
+
+// The event, speed and scattering rate at the propagator's state, at the start of a free segment
+// (later steps take them from the step before).
+static __device__ __noinline__ void fresh_state(const DevSolar& S, const DevPoint* __restrict__ P, StrictLane& L)
 {
-#if DMS_CERTIFIED_MATH
-	return rk45_attempt_certified(S, p, inner);
-#else
-	return rk45_attempt_unrolled(S, p, inner);
-#endif
+	if(!L.before_valid)
+		L.before = prop_event(L.pr);
+	L.before_valid = L.before_valid ? L.before_valid : 1;
+	const double r = prop_radius(L.pr);
+	L.next_speed = prop_speed(L.pr);
+	L.next_rate = r >= DMS_RSUN_KM ? 0.0 : rate_total(S, P, r, L.next_speed);
+	L.next_valid = 1;
 }
 
-// commit_accepted_event, src/Simulation_Trajectory.cpp:842-874.  Returns the capture energy of
-// the committed event when it was evaluated (NaN otherwise) so that the uncaptured-bound guard
-// that follows the commit reuses the same value.
-__device__ __forceinline__ double commit_event(const DevSolar& S, double m_dm, int capture_mode, StrictLane& L, double2* hist, const Event& local)
+// Ends the trajectory at the propagator's state.
+static __device__ __noinline__ int end_at_propagator(StrictLane& L, int reason)
 {
-	const double r_now = ev_radius(local);
-	const double v_now = ev_speed(local);
-	if(!capture_mode)
+	set_final(L, prop_event(L.pr), true, reason);
+	return PH_FINAL;
+}
+
+// The bounds of a step that starts at or outside the surface.
+static __device__ __noinline__ double outside_step(const StrictLane& L, double r, double step, double boundary)
+{
+	const double cap = step_cap(r, L.next_speed, boundary);
+	step = step < cap ? step : cap;
+	const double along = dot3(L.before.x, L.before.v);
+	if(r > DMS_RSUN_KM && along < 0.0)
 	{
-		const double v2 = v_now * v_now;
+		const double est = (r - DMS_RSUN_KM) / (-(along / r));
+		if(isfinite(est) && est > 0.0)
+		{
+			const double lim = est > DMS_RK45_ABS_MIN_STEP_S ? est : DMS_RK45_ABS_MIN_STEP_S;
+			step = lim < step ? lim : step;
+		}
+	}
+	return step;
+}
+
+// Pre-step bounds (src/Simulation_Trajectory.cpp:873-927).  Returns PH_STEP when an attempt is due,
+// else the lane's next phase.
+__device__ __forceinline__ int step_begin(const RunParams& R, const DevPoint* __restrict__ P, StrictLane& L)
+{
+	if(!(L.seg_steps < R.max_free_steps))
+	{
+		if(L.before_valid == 2)  // otherwise L.cur holds the last committed event
+		{
+			L.cur = L.before;
+			L.cur.t += L.origin;
+		}
+		L.reason = DMS_REASON_MAX_FREE_STEPS;
+		return PH_FINAL;
+	}
+	if(wall_time_exceeded(R, L))  // "before_step", src/Simulation_Trajectory.cpp:873-874
+		return end_at_propagator(L, DMS_REASON_WALL_TIME_LIMIT);
+	if(!L.next_valid)
+		fresh_state(R.S, P, L);
+	const double r = prop_radius(L.pr);
+	double step = sanitized_step(L.pr.time_step);
+	double rate = 0.0;
+	if(r >= DMS_RSUN_KM)
+		step = outside_step(L, r, step, R.boundary);
+	else
+	{
+		rate = L.next_rate;
+		if(!isfinite(rate) || rate < 0.0)
+			return end_at_propagator(L, DMS_REASON_NUMERICAL_FAILURE);
+		const double tau_limit = R.capture_mode ? DMS_CAPTURE_MAX_OPTICAL_DEPTH_STEP : DMS_MAX_OPTICAL_DEPTH_STEP;
+		// the quotient is formed only where it can be the smaller one
+		if(rate * step * (1.0 + 0x1p-50) > tau_limit)
+		{
+			const double lim = tau_limit / rate;
+			step = lim < step ? lim : step;
+		}
+	}
+	L.rate_before = rate;
+	L.pr.time_step = step;
+	L.in_rk = 1;
+	L.rk_inner = 0;
+	return PH_STEP;
+}
+
+// A step as an accepted attempt leaves it: the propagator after it, the events and radii before
+// and after it, and its interval inside the Sun.
+struct StepCtx
+{
+	Event before, after;
+	double r_before, r_after, v_after, dt, s0, s1;
+};
+
+// Event_In_3D and the speed of a propagator with J = 0, a radius below 1 km or a value outside the
+// range of dms_fastmath.cuh.
+static __device__ __noinline__ void event_and_speed_general(const Prop& p, Event& e, double& speed)
+{
+	speed = prop_speed(p);
+	e = prop_event(p);
+}
+
+__device__ __forceinline__ void event_and_speed(const Prop& p, Event& e, double& speed)
+{
+	bool ok = (p.J > 0x1p-200) & (p.J < 0x1p200) & (p.radius >= 1.0) & (p.radius < 0x1p100) & (p.radial_mode == 0);
+	const fast::Recip R = fast::recip(p.radius, ok);
+	if(!ok)
+	{
+		event_and_speed_general(p, e, speed);
+		return;
+	}
+	// prop_speed and prop_event with the quotients by the radius sharing its reciprocal
+	speed = sqrt(p.v_radial * p.v_radial + fast::div(fast::div(p.J * p.J, R), R));
+	const double safe = p.radius;
+	double sp, cp;
+	dms_sincos(p.phi, &sp, &cp);
+	const double vt = fast::div(p.J, R);
+	const double vx = p.v_radial * cp - vt * sp;
+	const double vy = p.v_radial * sp + vt * cp;
+	e.t = p.time;
+	e.x = mk(safe * (cp * p.ax.x + sp * p.ay.x), safe * (cp * p.ax.y + sp * p.ay.y), safe * (cp * p.ax.z + sp * p.ay.z));
+	e.v = mk(vx * p.ax.x + vy * p.ay.x, vx * p.ax.y + vy * p.ay.y, vx * p.ax.z + vy * p.ay.z);
+}
+
+// Solar_Interior_Fraction_Interval for a chord with an end outside the Sun.
+static __device__ __noinline__ bool interior_interval_outside(const Event& a, const Event& b, double ra, double rb, double& s0, double& s1)
+{
+	return interior_interval(a, b, ra, rb, s0, s1);
+}
+
+static __device__ __noinline__ double rate_total_general(const DevSolar& S, const DevPoint* __restrict__ P, double r, double v)
+{
+	return rate_total(S, P, r, v);
+}
+
+// rate_total at 0 <= r, v; r at or beyond the surface gives 0 (Scattering_Rate_At_Fraction).
+__device__ __forceinline__ double rate_inside(const DevSolar& S, const DevPoint* __restrict__ P, double r, double v)
+{
+	if(r >= DMS_RSUN_KM)
+		return 0.0;
+	if(!((r < DMS_RSUN_KM) & (v <= __ldg(&P->grid_vmax))))
+		return rate_total_general(S, P, r, v);  // no grid, a speed beyond it or a NaN
+	const double rc = r * __ldg(&P->grid_inv_r), vc = v * __ldg(&P->grid_inv_v);
+	const unsigned int N = static_cast<unsigned int>(__ldg(&P->grid_n));
+	double whole;
+	unsigned int ri = fast::floor_index(rc, whole);
+	double rf = rc - whole;
+	if(ri > N - 2)
+	{
+		ri = N - 2;
+		rf = rc - static_cast<double>(ri);
+	}
+	unsigned int vi = fast::floor_index(vc, whole);
+	double vf = vc - whole;
+	if(vi > N - 2)
+	{
+		vi = N - 2;
+		vf = vc - static_cast<double>(vi);
+	}
+	DMS_CHECK_INDEX(ri, 0u, N - 1, BOUNDS_GRID);
+	DMS_CHECK_INDEX(vi, 0u, N - 1, BOUNDS_GRID);
+	const double* g = reinterpret_cast<const double*>(__ldg(reinterpret_cast<const unsigned long long*>(&P->grid))) + static_cast<size_t>(ri) * N + vi;
+	const double g00 = __ldg(g), g01 = __ldg(g + 1);
+	const double g10 = __ldg(g + N), g11 = __ldg(g + N + 1);
+	const double lower_rate = g00 + vf * (g01 - g00);
+	const double upper_rate = g10 + vf * (g11 - g10);
+	const double rate = lower_rate + rf * (upper_rate - lower_rate);
+	return isfinite(rate) ? (rate > 0.0 ? rate : 0.0) : NAN;
+}
+
+// One piece-boundary rate of a step (Scattering_Rate_At_Fraction at fraction f of the chord a - b)
+// or, with `next`, the scattering rate at the state after the step (ra, va), which the next step's
+// head needs.
+__device__ __forceinline__ double piece_rate(const DevSolar& S, const DevPoint* __restrict__ P, const Vec3& ax, const Vec3& av, const Vec3& bx,
+                                             const Vec3& bv, double f, bool next, double ra, double va)
+{
+	f = clamp_unit(f);
+	const double x = ax.x + f * (bx.x - ax.x), vx = av.x + f * (bv.x - av.x);
+	const double y = ax.y + f * (bx.y - ax.y), vy = av.y + f * (bv.y - av.y);
+	const double z = ax.z + f * (bx.z - ax.z), vz = av.z + f * (bv.z - av.z);
+	double r = sqrt(x * x + y * y + z * z), v = sqrt(vx * vx + vy * vy + vz * vz);
+	r = next ? ra : r;
+	v = next ? va : v;
+	return rate_inside(S, P, r, v);
+}
+
+// The optical depth of a step: the trapezoid sum over its pieces (dtau), the two-piece estimate
+// (tau2), whether a rate was invalid, and the rate at the state after the step.
+struct Depth
+{
+	double dtau, tau2, next_rate;
+	bool invalid;
+};
+
+// Adds piece boundary i of `pieces` (2 or 4) at fraction f with its rate to the sums of
+// Build_Optical_Depth_Pieces (src/Simulation_Trajectory.cpp:347-414), in the reference's order.
+struct DepthSums
+{
+	double f_prev, r_prev, f_0, r_0, f_2, r_2, tau2_a;
+	__device__ __forceinline__ void add(Depth& d, int i, int pieces, double f, double rate, double dt)
+	{
+		d.invalid |= !isfinite(rate) | (rate < 0.0);
+		if(i > 0 && f > f_prev)
+			d.dtau += 0.5 * (r_prev + rate) * (dt * (f - f_prev));
+		if(pieces >= 4)
+		{
+			if(i == 0)
+			{
+				f_0 = f;
+				r_0 = rate;
+			}
+			else if(i == 2)
+			{
+				f_2 = f;
+				r_2 = rate;
+				tau2_a = 0.5 * (r_0 + r_2) * (dt * (f_2 - f_0));
+			}
+			else if(i == 4)
+				d.tau2 = tau2_a + 0.5 * (r_2 + rate) * (dt * (f - f_2));
+		}
+		else if(i > 0)
+			d.tau2 += 0.5 * (r_prev + rate) * (dt * (f - f_prev));
+		f_prev = f;
+		r_prev = rate;
+	}
+};
+
+// The depth of one lane's step, its boundary rates one after another.
+__device__ __forceinline__ void lane_depth(const RunParams& R, const DevPoint* __restrict__ P, const StepCtx& c, double rate_before, bool first_known,
+                                           int pieces, Depth& d)
+{
+	const double fraction = 1.0 / static_cast<double>(pieces), span = c.s1 - c.s0;  // 1/2 or 1/4, exact
+	DepthSums sums = {};
+#pragma unroll 1
+	for(int i = 0; i <= pieces + 1; i++)
+	{
+		const double f = c.s0 + static_cast<double>(i) * fraction * span;
+		double rate = rate_before;
+		if(i > 0 || !first_known)
+			rate = piece_rate(R.S, P, c.before.x, c.before.v, c.after.x, c.after.v, f, i > pieces, c.r_after, c.v_after);
+		if(i <= pieces)
+			sums.add(d, i, pieces, f, rate, c.dt);
+		else
+			d.next_rate = rate;
+	}
+}
+
+// The depths of the steps of the lanes in `dm`, each boundary rate of each step on a lane of its own
+// (the whole warp calls this): the owners of a round put their events into shared memory, 30 or 32
+// lanes form one rate each, and every owner sums its own.  The same lookups with the same
+// arguments as lane_depth, so the same numbers.  A rate is a dependent chain of some 600 cycles, so
+// a warp with few finished steps is done in one chain per round instead of five.
+constexpr int COOP_SLOT = 16;    // doubles of a step handed over
+constexpr int COOP_SLOTS = 8;    // most steps of a round (Capture mode: 4 rates each)
+constexpr int COOP_BUFFER = COOP_SLOT * COOP_SLOTS + 32;
+__device__ __forceinline__ void warp_depth(const RunParams& R, const DevPoint* __restrict__ P, const StepCtx& c, double rate_before, bool first_known,
+                                           int pieces, unsigned int dm, bool mine, double* buffer, Depth& d)
+{
+	const double fraction = 1.0 / static_cast<double>(pieces);
+	const int rates = pieces + 2, slots = 32 / rates;
+	const int me = threadIdx.x & 31;
+	const int rank = __popc(dm & ((1u << me) - 1u));
+	const int steps = __popc(dm);
+	const int slot_of_job = me / rates, j = me - slot_of_job * rates;
+	for(int base = 0; base < steps; base += slots)
+	{
+		const int slot = rank - base;
+		const bool owner = mine && slot >= 0 && slot < slots;
+		if(owner)
+		{
+			double* b = buffer + slot * COOP_SLOT;
+			b[0] = c.before.x.x; b[1] = c.before.x.y; b[2] = c.before.x.z;
+			b[3] = c.before.v.x; b[4] = c.before.v.y; b[5] = c.before.v.z;
+			b[6] = c.after.x.x; b[7] = c.after.x.y; b[8] = c.after.x.z;
+			b[9] = c.after.v.x; b[10] = c.after.v.y; b[11] = c.after.v.z;
+			b[12] = c.s0 + 0.0; b[13] = c.s1 - c.s0;
+			b[14] = c.r_after; b[15] = c.v_after;
+		}
+		// the point of each slot's owner
+		const int owner_lane = slot_of_job < slots && base + slot_of_job < steps ? nth_set_bit(dm, base + slot_of_job) : me;
+		const DevPoint* Po = reinterpret_cast<const DevPoint*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(P), owner_lane));
+		__syncwarp();
+		double rate = 0.0;
+		if(slot_of_job < slots && base + slot_of_job < steps)
+		{
+			const double* b = buffer + slot_of_job * COOP_SLOT;
+			rate = piece_rate(R.S, Po, mk(b[0], b[1], b[2]), mk(b[3], b[4], b[5]), mk(b[6], b[7], b[8]), mk(b[9], b[10], b[11]),
+			                  b[12] + static_cast<double>(j) * fraction * b[13], j > pieces, b[14], b[15]);
+		}
+		buffer[COOP_SLOT * COOP_SLOTS + me] = rate;
+		__syncwarp();
+		if(owner)
+		{
+			const double* q = buffer + COOP_SLOT * COOP_SLOTS + slot * rates;
+			const double span = c.s1 - c.s0;
+			DepthSums sums = {};
+			for(int i = 0; i <= pieces; i++)
+				sums.add(d, i, pieces, c.s0 + static_cast<double>(i) * fraction * span, i == 0 && first_known ? rate_before : q[i], c.dt);
+			d.next_rate = q[rates - 1];
+		}
+		__syncwarp();
+	}
+}
+
+// A step whose optical depth exceeds the limit or whose two estimates differ too much: the step is
+// taken again, shorter (src/Simulation_Trajectory.cpp:975-1011).
+static __device__ __noinline__ int depth_reject(StrictLane& L, const Event& before, double dtau, double rel, bool reject_acc, double dt, double tau_limit)
+{
+	L.retries++;
+	if(L.retries > DMS_MAX_OPTICAL_DEPTH_RETRIES)
+	{
+		set_final(L, before, true, DMS_REASON_NUMERICAL_FAILURE);
+		return PH_FINAL;
+	}
+	double factor = DMS_RK45_MAX_STEP_FACTOR;
+	if(dtau > tau_limit && dtau > 0.0 && 0.8 * tau_limit / dtau < factor)
+		factor = 0.8 * tau_limit / dtau;
+	if(reject_acc && rel > 0.0 && 0.8 * sqrt(DMS_OPTICAL_DEPTH_REL_TOL / rel) < factor)
+		factor = 0.8 * sqrt(DMS_OPTICAL_DEPTH_REL_TOL / rel);
+	if(factor > 1.0) factor = 1.0;
+	if(factor < DMS_RK45_MIN_STEP_FACTOR) factor = DMS_RK45_MIN_STEP_FACTOR;
+	L.pr.time_step = sanitized_step(factor * dt);
+	return PH_STEP;  // L.before and the speed and rate at it still describe the propagator
+}
+
+// The scattering point of a step whose depth reaches the remaining one (src/Simulation_Trajectory.cpp:
+// 1013-1044).  The boundary rates are formed again: the same lookups, the same numbers.
+static __device__ __noinline__ void scatter_point(const DevSolar& S, const DevPoint* __restrict__ P, const StepCtx& c, double rate_before, bool first_known,
+                                                  bool depth, int pieces, double remaining, Event& accepted)
+{
+	if(depth)
+	{
+		const double fraction = 1.0 / static_cast<double>(pieces), span = c.s1 - c.s0;
+		double f_prev = c.s0, r_prev = rate_before;
+		if(!first_known)
+			r_prev = rate_at_fraction(S, P, c.before, c.after, f_prev);
+#pragma unroll 1
+		for(int k = 1; k <= pieces; k++)
+		{
+			const double f = c.s0 + static_cast<double>(k) * fraction * span;
+			const double rate = rate_at_fraction(S, P, c.before, c.after, f);
+			if(f > f_prev)
+			{
+				const double pdt = c.dt * (f - f_prev);
+				const double ptau = 0.5 * (r_prev + rate) * pdt;
+				if(ptau >= remaining)
+				{
+					const double lf = solve_linear_rate(r_prev, rate, pdt, remaining);
+					accepted = interpolate_event(c.before, c.after, f_prev + lf * (f - f_prev));
+					return;
+				}
+				remaining -= ptau;
+			}
+			f_prev = f;
+			r_prev = rate;
+		}
+	}
+	accepted = interpolate_event(c.before, c.after, c.s1);
+}
+
+__device__ void commit_event(const RunParams& R, double m_dm, StrictLane& L, double2* hist, const Event& local, double r_now, double& E);
+
+// A step that ends at or beyond the boundary radius (src/Simulation_Trajectory.cpp:1046-1086).
+enum Boundary : int
+{
+	BOUNDARY_INSIDE = 0,    // nothing to do
+	BOUNDARY_ESCAPE = 1,    // `accepted` is the outward escape
+	BOUNDARY_RETURN = 2,    // the bound orbit was carried back to the boundary; the segment goes on
+	BOUNDARY_FAILURE = 3,
+};
+static __device__ __noinline__ int boundary_step(const RunParams& R, double m_dm, StrictLane& L, double2* hist, const StepCtx& c, Event& accepted)
+{
+	const DevSolar& S = R.S;
+	Event ev = c.after;
+	double r_b = c.r_after, v_b = c.v_after;
+	if(c.r_before < R.boundary && c.r_after >= R.boundary && c.r_after > c.r_before)
+	{
+		const double f = (R.boundary - c.r_before) / (c.r_after - c.r_before);
+		ev = interpolate_event(c.before, c.after, f);
+		r_b = ev_radius(ev);
+		v_b = ev_speed(ev);
+	}
+	if(!(r_b >= R.boundary && r_b >= c.r_before))
+		return BOUNDARY_INSIDE;
+	if(v_b > solar_vesc(S, r_b))
+	{
+		accepted = ev;
+		return BOUNDARY_ESCAPE;
+	}
+	Event abs_b = ev;
+	abs_b.t += L.origin;
+	if(uncaptured_bound(S, m_dm, L, abs_b))
+	{
+		set_final(L, abs_b, false, DMS_REASON_NUMERICAL_FAILURE);
+		return BOUNDARY_FAILURE;
+	}
+	Event inbound;
+	if(!bound_kepler_return(ev, inbound))
+		return BOUNDARY_INSIDE;
+	L.seg_steps++;
+	L.steps++;
+	L.retries = 0;
+	double E;
+	commit_event(R, m_dm, L, hist, ev, ev_radius(ev), E);
+	// reset_propagator_at_absolute_event, src/Simulation_Trajectory.cpp:814-822
+	L.cur = inbound;
+	L.cur.t += L.origin;
+	L.origin = L.cur.t;
+	Event local = inbound;
+	local.t = 0.0;
+	prop_init(L.pr, local);
+	L.before_valid = 0;
+	L.next_valid = 0;
+	if(!R.capture_mode && L.prev_time >= 0.0)
+		L.prev_time = 0.0;
+	return BOUNDARY_RETURN;
+}
+
+static __device__ __noinline__ double capture_energy_general(const DevSolar& S, double m_dm, double r, double v) { return capture_energy_eV(S, m_dm, r, v); }
+static __device__ __noinline__ double solar_vesc_general(const DevSolar& S, double r) { return solar_vesc(S, r); }
+
+// commit_accepted_event (src/Simulation_Trajectory.cpp:842-874).  E receives the capture energy of the
+// committed event where the uncaptured-bound guard that follows needs its value: it is left at +1 for
+// an uncaptured particle that is clearly faster than the escape speed (only the sign matters there).
+__device__ __forceinline__ void commit_event_inline(const RunParams& R, double m_dm, StrictLane& L, double2* hist, const Event& local, double r_now, double& E)
+{
+	const double v2 = dot3(local.v, local.v);
+	const double v_now = sqrt(v2);
+	const double vv = v_now * v_now;
+	if(!R.capture_mode)
+	{
 		if(L.prev_time >= 0.0)
 			accumulate_bincount(L, hist, L.prev_r, L.prev_v2, local.t - L.prev_time);
 		L.prev_time = local.t;
 		L.prev_r = r_now;
-		L.prev_v2 = v2;
+		L.prev_v2 = vv;
 	}
-	const double t_abs = local.t + L.origin;
-	// Update_Capture_State(..., allow_new_capture = false), src/Simulation_Trajectory.cpp:689-721
-	if(capture_mode && !L.is_captured)
-		return NAN;
-	const double E = capture_energy_eV(S, m_dm, r_now, v_now);
-	if(L.is_captured && isfinite(L.free_flight_E))
+	// v_esc^2 before the root of Local_Escape_Speed and its square
+	const bool table = (r_now <= DMS_RSUN_KM) & (R.S.fast_tables != 0);
+	const double w = table ? solar_vesc2_fast(R.S, r_now) : NAN;
+	if(!L.is_captured)
+	{
+		E = 1.0;
+		// outside the Sun v_esc^2 = 2 G M / r: compared without the division
+		const double have = table ? vv : vv * r_now, need = table ? w : 2 * DMS_GMSUN_KM3S2;
+		if(!((have > need * (1.0 + 0x1p-40)) & (vv < 1.0e200) & (r_now < 0x1p100)))
+			E = capture_energy_general(R.S, m_dm, r_now, v_now);
+		return;
+	}
+	// capture_energy_eV
+	const double vesc = table ? sqrt(w) : solar_vesc_general(R.S, r_now);
+	E = fast::div_const(0.5 * m_dm * fast::div_const(vv - vesc * vesc, DMS_C_KMS * DMS_C_KMS), 1.0e-9);
+	if(isfinite(L.free_flight_E))
 	{
 		const double drift = fabs(E - L.free_flight_E);
-		if(isfinite(drift) && drift > L.max_drift_eV)
-			L.max_drift_eV = drift;
-		const double ref = fabs(L.free_flight_E);
-		const double scale = ref > DMS_FREE_ENERGY_DRIFT_REL_E_SCALE_EV ? ref : DMS_FREE_ENERGY_DRIFT_REL_E_SCALE_EV;
-		const double rel = drift / scale;
-		if(isfinite(rel) && rel > L.max_drift_rel)
-			L.max_drift_rel = rel;
-	}
-	if(L.bound_state && L.is_captured)
-		L.t_last_bound = t_abs;
-	return E;
-}
-
-// One pass of the Propagate_Freely loop body, src/Simulation_Trajectory.cpp:876-1116, split at the
-// RK45 retry loop: when no step is in progress the pre-step bounds are applied and a step is
-// opened (free_step_begin); every pass makes one RK45 attempt; only a finished step runs the
-// optical-depth, boundary and commit logic (free_step_finish).  free_step_begin returns PH_STEP
-// when an attempt is due, else the lane's next phase.
-__device__ __forceinline__ int free_step_begin(const RunParams& R, const DevPoint* __restrict__ P, StrictLane& L)
-{
-	const DevSolar& S = R.S;
-	const int capture_mode = R.capture_mode;
-	const double tau_limit = capture_mode ? DMS_CAPTURE_MAX_OPTICAL_DEPTH_STEP : DMS_MAX_OPTICAL_DEPTH_STEP;
-	if(!L.in_rk)
-	{
-		// speed and rate at the propagator's state, formed by the previous step's finish (tail of
-		// a launch) from the same propagator
-		const bool cached = L.next_valid != 0;
-		L.next_valid = 0;
-		if(!(L.seg_steps < R.max_free_steps))
+		if(isfinite(drift))
 		{
-			L.reason = DMS_REASON_MAX_FREE_STEPS;  // L.cur holds the last committed event
-			return PH_FINAL;
-		}
-		if(wall_time_exceeded(R, L))  // "before_step", src/Simulation_Trajectory.cpp:873-874
-		{
-			set_final(L, prop_event(L.pr), true, DMS_REASON_WALL_TIME_LIMIT);
-			return PH_FINAL;
-		}
-		if(!L.before_valid)
-		{
-			L.before = prop_event(L.pr);
-			L.before_valid = 1;
-		}
-		const double r_before = prop_radius(L.pr);
-		const double v_before = cached ? L.next_speed : prop_speed(L.pr);
-		L.rate_before = 0.0;
-		if(r_before >= DMS_RSUN_KM)
-		{
-			const double cap = step_cap(r_before, v_before, R.boundary);
-			const double ts = sanitized_step(L.pr.time_step);
-			L.pr.time_step = ts < cap ? ts : cap;
-			const double vr = (r_before > 0.0) ? dot3(L.before.x, L.before.v) / r_before : 0.0;
-			if(r_before > DMS_RSUN_KM && vr < 0.0)
+			if(drift > L.max_drift_eV)
+				L.max_drift_eV = drift;
+			const double ref = fabs(L.free_flight_E);
+			const double scale = ref > DMS_FREE_ENERGY_DRIFT_REL_E_SCALE_EV ? ref : DMS_FREE_ENERGY_DRIFT_REL_E_SCALE_EV;
+			// the quotient is formed only where it can be the larger one
+			if(drift * (1.0 + 0x1p-50) >= L.max_drift_rel * scale)
 			{
-				const double est = (r_before - DMS_RSUN_KM) / (-vr);
-				if(isfinite(est) && est > 0.0)
-				{
-					const double lim = est > DMS_RK45_ABS_MIN_STEP_S ? est : DMS_RK45_ABS_MIN_STEP_S;
-					if(lim < L.pr.time_step) L.pr.time_step = lim;
-				}
+				const double rel = drift / scale;
+				if(isfinite(rel) && rel > L.max_drift_rel)
+					L.max_drift_rel = rel;
 			}
 		}
+	}
+	if(L.bound_state)
+		L.t_last_bound = local.t + L.origin;
+}
+
+__device__ __noinline__ void commit_event(const RunParams& R, double m_dm, StrictLane& L, double2* hist, const Event& local, double r_now, double& E)
+{
+	commit_event_inline(R, m_dm, L, hist, local, r_now, E);
+}
+
+// Steps of a warp whose depths are formed by the whole warp rather than by each lane: one round of
+// lookups serves 5 steps (8 in Capture mode) and costs a third more than one lookup of lane_depth,
+// which makes 5 (3) of them one after another.
+constexpr int COOP_MAX_STEPS = 15;
+
+// One pass for every lane of the warp (all 32 call it); returns the lane's next phase.
+__device__ __forceinline__ int strict_step(const RunParams& R, const DevPoint* __restrict__ P, double m_dm, StrictLane& L, double2* hist, int phase,
+                                           double* buffer)
+{
+	const int capture_mode = R.capture_mode;
+	const int pieces = capture_mode ? DMS_CAPTURE_OPTICAL_DEPTH_PIECES : DMS_MAX_OPTICAL_DEPTH_PIECES;
+	const double tau_limit = capture_mode ? DMS_CAPTURE_MAX_OPTICAL_DEPTH_STEP : DMS_MAX_OPTICAL_DEPTH_STEP;
+	StepCtx c;
+	Prop q;
+	bool done = false, interior = false, depth = false;
+	int reason = 0;
+	if(phase == PH_STEP && !L.in_rk)
+		phase = step_begin(R, P, L);
+	if(phase == PH_STEP)
+	{
+		q = L.pr;
+		L.rk_inner++;
+		const int rk = rk45_attempt(R.S, q, L.rk_inner);
+		if(rk == RK_RETRY)
+			L.pr.time_step = q.time_step;
 		else
 		{
-			L.pr.time_step = sanitized_step(L.pr.time_step);
-			L.rate_before = cached ? L.next_rate : rate_total(S, P, r_before, v_before);
-			if(!isfinite(L.rate_before) || L.rate_before < 0.0)
+			done = true;
+			L.in_rk = 0;
+			L.attempts += static_cast<uint64_t>(L.rk_inner);
+			c.before = L.before;
+			c.before.t = L.pr.time;
+			c.r_before = prop_radius(L.pr);
+			c.dt = q.time - L.pr.time;
+			c.r_after = prop_radius(q);
+			event_and_speed(q, c.after, c.v_after);
+			// the checks after an attempt, src/Simulation_Trajectory.cpp:930-960
+			if(rk == RK_FORCED)
+				reason = DMS_REASON_NUMERICAL_FAILURE;
+			else if(!isfinite(c.r_after) || !isfinite(c.v_after) || !isfinite(c.dt) || c.dt <= 0.0)
+				reason = DMS_REASON_NON_FINITE_STATE;
+			else if(c.v_after > DMS_V_MAX_C * DMS_C_KMS)
+				reason = DMS_REASON_SPEED_LIMIT;
+			else if(wall_time_exceeded(R, L))  // "after_rk45_step", src/Simulation_Trajectory.cpp:953-954
+				reason = DMS_REASON_WALL_TIME_LIMIT;
+			else
 			{
-				set_final(L, prop_event(L.pr), true, DMS_REASON_NUMERICAL_FAILURE);
-				return PH_FINAL;
+				c.s0 = 0.0;
+				c.s1 = 1.0;
+				interior = true;
+				if(!(c.r_before < DMS_RSUN_KM && c.r_after < DMS_RSUN_KM))
+				{
+					c.s1 = 0.0;
+					interior = interior_interval_outside(c.before, c.after, c.r_before, c.r_after, c.s0, c.s1);
+				}
+				depth = interior && c.s1 > c.s0;
 			}
-			if(L.rate_before > 0.0 && tau_limit / L.rate_before < L.pr.time_step)
-				L.pr.time_step = tau_limit / L.rate_before;
 		}
-		// the RK step changes only these propagator fields
-		L.b_time = L.pr.time;
-		L.b_radius = L.pr.radius;
-		L.b_phi = L.pr.phi;
-		L.b_vr = L.pr.v_radial;
-		L.b_step = L.pr.time_step;
-		L.pr.time_step = sanitized_step(L.pr.time_step);  // head of Runge_Kutta_45_Step, :1489
-		L.in_rk = 1;
-		L.rk_inner = 0;
 	}
-	return PH_STEP;
-}
-
-// One RK45 attempt of the lane's open step (the lane alone).
-__device__ __forceinline__ int free_step_attempt(const DevSolar& S, StrictLane& L, int drained)
-{
-	L.rk_inner++;
-#if DMS_RK_UNROLLED == 2
-	return drained ? rk45_attempt_written_out(S, L.pr, L.rk_inner) : rk45_attempt(S, L.pr, L.rk_inner);
-#elif DMS_RK_UNROLLED == 1
-	(void)drained;
-	return rk45_attempt_written_out(S, L.pr, L.rk_inner);
-#else
-	(void)drained;
-	return rk45_attempt(S, L.pr, L.rk_inner);
-#endif
-}
-
-// The rest of the pass after an attempt with result rk: a retry keeps the step open; a
-// finished step runs the optical-depth, boundary and commit logic.
-// The trapezoid sums of the depth loop in free_step_finish over rates that are already formed:
-// the same additions in the same order.
-template <int PIECES>
-__device__ __forceinline__ void depth_sums(const double (&fr)[DMS_MAX_OPTICAL_DEPTH_PIECES + 1], const double (&rt)[DMS_MAX_OPTICAL_DEPTH_PIECES + 1],
-                                           double actual_dt, double& dtau, double& tau2, bool& invalid)
-{
-	double tau2_a = 0.0;
-#pragma unroll
-	for(int i = 0; i <= PIECES; i++)
+	const unsigned int dm = __ballot_sync(0xffffffffu, depth);
+	Depth d = {0.0, 0.0, 0.0, false};
+	const bool first_known = depth && c.r_before < DMS_RSUN_KM && c.s0 <= 1.0e-12;
+	if(dm != 0u)
 	{
-		const double f = fr[i], rate = rt[i];
-		if(!isfinite(rate) || rate < 0.0)
-			invalid = true;
-		if(i > 0 && f > fr[i - 1])
-			dtau += 0.5 * (rt[i - 1] + rate) * (actual_dt * (f - fr[i - 1]));
-		if(PIECES >= 4)
-		{
-			if(i == 2)
-				tau2_a = 0.5 * (rt[0] + rt[2]) * (actual_dt * (fr[2] - fr[0]));
-			else if(i == 4)
-				tau2 = tau2_a + 0.5 * (rt[2] + rate) * (actual_dt * (f - fr[2]));
-		}
-		else if(i > 0)
-			tau2 += 0.5 * (rt[i - 1] + rate) * (actual_dt * (f - fr[i - 1]));
+		if(__popc(dm) <= COOP_MAX_STEPS)
+			warp_depth(R, P, c, L.rate_before, first_known, pieces, dm, depth, buffer, d);
+		else if(depth)
+			lane_depth(R, P, c, L.rate_before, first_known, pieces, d);
 	}
-}
-
-// A finished RK45 step as the head of free_step_finish leaves it for the tail: the events and
-// radii before and after it and its interior interval.
-struct FinishCtx
-{
-	Event before, after;
-	double r_before, rate_before, actual_dt, r_after, v_after, s0, s1;
-	int interior;  // the chord enters the Sun (interior_interval)
-	int depth;     // with a positive span and duration: the piece rates are formed
-};
-
-constexpr int PH_CONTINUE = -1;  // free_step_finish_head: the step goes on to its tail
-
-// The checks after an attempt (src/Simulation_Trajectory.cpp:930-960) and the interior interval.
-__device__ __forceinline__ int free_step_finish_head(const RunParams& R, StrictLane& L, int rk, FinishCtx& c)
-{
-	if(rk == RK_RETRY)
-		return PH_STEP;
-	L.in_rk = 0;
-	L.attempts += static_cast<uint64_t>(L.rk_inner);
-	c.before = L.before;
-	c.r_before = L.b_radius < 0.0 ? 0.0 : L.b_radius;
-	c.rate_before = L.rate_before;
-	c.actual_dt = L.pr.time - L.b_time;
-	c.r_after = prop_radius(L.pr);
-	c.v_after = prop_speed(L.pr);
-	c.after = prop_event(L.pr);
-	if(rk == RK_FORCED)
+	if(!done)
+		return phase;
+	if(d.invalid || !isfinite(d.dtau) || d.dtau < 0.0)
+		reason = DMS_REASON_NUMERICAL_FAILURE;
+	if(reason != 0)
 	{
-		set_final(L, c.after, true, DMS_REASON_NUMERICAL_FAILURE);
+		set_final(L, c.after, true, reason);
 		return PH_FINAL;
 	}
-	if(!isfinite(c.r_after) || !isfinite(c.v_after) || !isfinite(c.actual_dt) || c.actual_dt <= 0.0)
-	{
-		set_final(L, c.after, true, DMS_REASON_NON_FINITE_STATE);
-		return PH_FINAL;
-	}
-	if(c.v_after > DMS_V_MAX_C * DMS_C_KMS)
-	{
-		set_final(L, c.after, true, DMS_REASON_SPEED_LIMIT);
-		return PH_FINAL;
-	}
-	if(wall_time_exceeded(R, L))  // "after_rk45_step", src/Simulation_Trajectory.cpp:953-954
-	{
-		set_final(L, c.after, true, DMS_REASON_WALL_TIME_LIMIT);
-		return PH_FINAL;
-	}
-	c.s0 = 0.0;
-	c.s1 = 0.0;
-	c.interior = interior_interval(c.before, c.after, c.r_before, c.r_after, c.s0, c.s1) ? 1 : 0;
-	c.depth = (c.interior && c.s1 > c.s0 && c.actual_dt > 0.0) ? 1 : 0;
-	return PH_CONTINUE;
-}
-
-// The optical depth, boundary and commit logic of a finished step (src/Simulation_Trajectory.cpp:
-// 960-1116) from its piece boundaries fr and rates rt, their trapezoid sums dtau (pieces) and
-// tau2 (two-piece estimate) and whether a rate was invalid.  next_ok: next_rate is the scattering
-// rate at the propagator's state (rate_total at r_after, v_after), for the next step's head.
-__device__ __forceinline__ int free_step_finish_tail(const RunParams& R, double m_dm, StrictLane& L, double2* hist,
-                                                     const FinishCtx& c, const double (&fr)[DMS_MAX_OPTICAL_DEPTH_PIECES + 1],
-                                                     const double (&rt)[DMS_MAX_OPTICAL_DEPTH_PIECES + 1], double dtau, double tau2, bool invalid,
-                                                     bool next_ok, double next_rate)
-{
-	const DevSolar& S = R.S;
-	const int capture_mode = R.capture_mode;
-	const double tau_limit = capture_mode ? DMS_CAPTURE_MAX_OPTICAL_DEPTH_STEP : DMS_MAX_OPTICAL_DEPTH_STEP;
-	bool scattering = false, reflection = false;
 	Event accepted = c.after;
-	if(c.interior)
+	bool scattering = false;
+	if(interior)
 	{
-		// Build_Optical_Depth_Pieces, src/Simulation_Trajectory.cpp:347-414
-		const int pieces = capture_mode ? DMS_CAPTURE_OPTICAL_DEPTH_PIECES : DMS_MAX_OPTICAL_DEPTH_PIECES;
-		if(invalid || !isfinite(dtau) || dtau < 0.0)
+		const double scale = d.dtau > DMS_OPTICAL_DEPTH_ABS_TOL ? d.dtau : DMS_OPTICAL_DEPTH_ABS_TOL;
+		const double apart = fabs(d.dtau - d.tau2);
+		const bool reject_depth = d.dtau > tau_limit;
+		if(reject_depth || apart > (DMS_OPTICAL_DEPTH_REL_TOL * (1.0 - 0x1p-50)) * scale)
 		{
-			set_final(L, c.after, true, DMS_REASON_NUMERICAL_FAILURE);
-			return PH_FINAL;
+			const double rel = apart / scale;
+			const bool reject_acc = !capture_mode && rel > DMS_OPTICAL_DEPTH_REL_TOL;
+			if(reject_depth || reject_acc)
+				return depth_reject(L, c.before, d.dtau, rel, reject_acc, c.dt, tau_limit);
 		}
-		const double scale = dtau > DMS_OPTICAL_DEPTH_ABS_TOL ? dtau : DMS_OPTICAL_DEPTH_ABS_TOL;
-		const double rel = fabs(dtau - tau2) / scale;
-		const bool reject_depth = dtau > tau_limit;
-		const bool reject_acc = !capture_mode && rel > DMS_OPTICAL_DEPTH_REL_TOL;
-		if(reject_depth || reject_acc)
+		if(d.dtau >= L.tau)
 		{
-			L.retries++;
-			if(L.retries > DMS_MAX_OPTICAL_DEPTH_RETRIES)
-			{
-				set_final(L, c.before, true, DMS_REASON_NUMERICAL_FAILURE);
-				return PH_FINAL;
-			}
-			L.pr.time = L.b_time;
-			L.pr.radius = L.b_radius;
-			L.pr.phi = L.b_phi;
-			L.pr.v_radial = L.b_vr;
-			L.pr.time_step = L.b_step;
-			double factor = DMS_RK45_MAX_STEP_FACTOR;
-			if(dtau > tau_limit && dtau > 0.0 && 0.8 * tau_limit / dtau < factor)
-				factor = 0.8 * tau_limit / dtau;
-			if(reject_acc && rel > 0.0 && 0.8 * sqrt(DMS_OPTICAL_DEPTH_REL_TOL / rel) < factor)
-				factor = 0.8 * sqrt(DMS_OPTICAL_DEPTH_REL_TOL / rel);
-			if(factor > 1.0) factor = 1.0;
-			if(factor < DMS_RK45_MIN_STEP_FACTOR) factor = DMS_RK45_MIN_STEP_FACTOR;
-			L.pr.time_step = sanitized_step(factor * c.actual_dt);
-			return PH_STEP;  // L.before still describes the restored propagator
-		}
-		if(dtau >= L.tau)
-		{
-			double remaining = L.tau;
-			for(int k = 0; k < pieces; k++)
-			{
-				if(!(fr[k + 1] > fr[k]))
-					continue;
-				const double pdt = c.actual_dt * (fr[k + 1] - fr[k]);
-				const double ptau = 0.5 * (rt[k] + rt[k + 1]) * pdt;
-				if(ptau >= remaining)
-				{
-					const double lf = solve_linear_rate(rt[k], rt[k + 1], pdt, remaining);
-					const double f = fr[k] + lf * (fr[k + 1] - fr[k]);
-					accepted = interpolate_event(c.before, c.after, f);
-					scattering = true;
-					break;
-				}
-				remaining -= ptau;
-			}
-			if(!scattering)
-			{
-				accepted = interpolate_event(c.before, c.after, c.s1);
-				scattering = true;
-			}
+			scatter_point(R.S, P, c, L.rate_before, first_known, depth, pieces, L.tau, accepted);
+			scattering = true;
 		}
 		else
-			L.tau -= dtau;
+			L.tau -= d.dtau;
 	}
-	if(!scattering)
+	int boundary = BOUNDARY_INSIDE;
+	if(!scattering && c.r_after >= R.boundary)
 	{
-		Event boundary_ev = c.after;
-		double r_b = c.r_after, v_b = c.v_after;
-		if(c.r_before < R.boundary && c.r_after >= R.boundary && c.r_after > c.r_before)
-		{
-			const double f = (R.boundary - c.r_before) / (c.r_after - c.r_before);
-			boundary_ev = interpolate_event(c.before, c.after, f);
-			r_b = ev_radius(boundary_ev);
-			v_b = ev_speed(boundary_ev);
-		}
-		if(r_b >= R.boundary && r_b >= c.r_before && v_b > solar_vesc(S, r_b))
-		{
-			accepted = boundary_ev;
-			reflection = true;
-		}
-		else if(r_b >= R.boundary && r_b >= c.r_before)
-		{
-			Event abs_b = boundary_ev;
-			abs_b.t += L.origin;
-			if(uncaptured_bound(S, m_dm, L, abs_b))
-			{
-				set_final(L, abs_b, false, DMS_REASON_NUMERICAL_FAILURE);
-				return PH_FINAL;
-			}
-			Event inbound;
-			if(bound_kepler_return(boundary_ev, inbound))
-			{
-				L.seg_steps++;
-				L.steps++;
-				L.retries = 0;
-				commit_event(S, m_dm, capture_mode, L, hist, boundary_ev);
-				// reset_propagator_at_absolute_event, src/Simulation_Trajectory.cpp:814-822
-				L.cur = inbound;
-				L.cur.t += L.origin;
-				L.origin = L.cur.t;
-				Event local = inbound;
-				local.t = 0.0;
-				prop_init(L.pr, local);
-				L.before_valid = 0;
-				if(!capture_mode && L.prev_time >= 0.0)
-					L.prev_time = 0.0;
-				return PH_STEP;
-			}
-		}
+		boundary = boundary_step(R, m_dm, L, hist, c, accepted);
+		if(boundary == BOUNDARY_RETURN)
+			return PH_STEP;
+		if(boundary == BOUNDARY_FAILURE)
+			return PH_FINAL;
 	}
 	L.seg_steps++;
 	L.steps++;
 	L.retries = 0;
-	double E = commit_event(S, m_dm, capture_mode, L, hist, accepted);
-	L.cur = accepted;
-	L.cur.t += L.origin;
-	if(!L.is_captured)
+	const double r_now = ev_radius(accepted);
+	double E;
+	commit_event_inline(R, m_dm, L, hist, accepted, r_now, E);
+	// abort_if_uncaptured_bound on the committed event, src/Simulation_Trajectory.cpp:767-778, 1108
+	const bool bound = !L.is_captured && !(isfinite(E) && E >= 0.0);
+	if(bound | scattering | (boundary == BOUNDARY_ESCAPE))
 	{
-		// abort_if_uncaptured_bound on the committed event, src/Simulation_Trajectory.cpp:767-778, 1108
-		if(isnan(E))
-			E = capture_energy_eV(S, m_dm, ev_radius(L.cur), ev_speed(L.cur));
-		if(!(isfinite(E) && E >= 0.0))
-		{
+		L.cur = accepted;
+		L.cur.t += L.origin;
+		if(bound)
 			L.reason = DMS_REASON_NUMERICAL_FAILURE;
-			return PH_FINAL;
-		}
-	}
-	if(reflection)
-	{
-		L.reason = DMS_REASON_OUTWARD_ESCAPE;
+		else if(!scattering)
+			L.reason = DMS_REASON_OUTWARD_ESCAPE;
+		else if(r_now < DMS_RSUN_KM)
+			return PH_SCATTER;  // Simulate, src/Simulation_Trajectory.cpp:1313-1346; Sample_Target runs in the lane loop
+		else
+			L.reason = DMS_REASON_SCATTER;
 		return PH_FINAL;
 	}
-	if(scattering)
-	{
-		// Simulate, src/Simulation_Trajectory.cpp:1313-1346
-		if(!(ev_radius(L.cur) < DMS_RSUN_KM))
-		{
-			L.reason = DMS_REASON_SCATTER;
-			return PH_FINAL;
-		}
-		return PH_SCATTER;  // Sample_Target runs warp-cooperatively in the lane loop
-	}
+	L.pr.time = q.time;
+	L.pr.radius = q.radius;
+	L.pr.phi = q.phi;
+	L.pr.v_radial = q.v_radial;
+	L.pr.time_step = q.time_step;
 	L.before = c.after;
-	// the propagator is left as the attempt made it: the next step starts from its speed and rate
-	L.next_valid = next_ok ? 1 : 0;
+	L.before_valid = 2;
+	// the next step starts from this speed and rate; without a depth the rate at a state inside the
+	// Sun is not known yet
 	L.next_speed = c.v_after;
-	L.next_rate = next_rate;
+	L.next_rate = d.next_rate;
+	L.next_valid = depth || c.r_after >= DMS_RSUN_KM;
 	return PH_STEP;
-}
-
-// A finished step on one lane: the piece rates one after another (one copy of the lookup).
-__device__ __forceinline__ int free_step_finish(const RunParams& R, const DevPoint* __restrict__ P, double m_dm, StrictLane& L,
-                                                double2* hist, int rk)
-{
-	const DevSolar& S = R.S;
-	const int capture_mode = R.capture_mode;
-	FinishCtx c;
-	const int ph = free_step_finish_head(R, L, rk, c);
-	if(ph != PH_CONTINUE)
-		return ph;
-	const int pieces = capture_mode ? DMS_CAPTURE_OPTICAL_DEPTH_PIECES : DMS_MAX_OPTICAL_DEPTH_PIECES;
-	const bool use_cached = c.r_before < DMS_RSUN_KM && c.s0 <= 1.0e-12;
-	const double span = c.s1 - c.s0;
-	double fr[DMS_MAX_OPTICAL_DEPTH_PIECES + 1], rt[DMS_MAX_OPTICAL_DEPTH_PIECES + 1];
-	bool invalid = false;
-	double dtau = 0.0, tau2 = 0.0;
-	if(c.depth)
-	{
-		// One loop over the piece boundaries (one copy of the rate lookup); the trapezoid
-		// sums are formed as the rates arrive, in the reference's order.  The arrays keep
-		// the boundaries for the scattering-point search, which is rare.
-		double fr_prev = 0.0, rt_prev = 0.0, fr_0 = 0.0, rt_0 = 0.0, fr_2 = 0.0, rt_2 = 0.0, tau2_a = 0.0;
-#pragma unroll 1
-		for(int i = 0; i <= pieces; i++)
-		{
-			const double f = c.s0 + static_cast<double>(i) / static_cast<double>(pieces) * span;
-			const double rate = (i == 0 && use_cached) ? c.rate_before : rate_at_fraction(S, P, c.before, c.after, f);
-			fr[i] = f;
-			rt[i] = rate;
-			if(!isfinite(rate) || rate < 0.0)
-				invalid = true;
-			if(i > 0 && f > fr_prev)
-				dtau += 0.5 * (rt_prev + rate) * (c.actual_dt * (f - fr_prev));
-			if(pieces >= 4)
-			{
-				// two-piece estimate over [0, 2] and [2, 4]
-				if(i == 0)
-				{
-					fr_0 = f;
-					rt_0 = rate;
-				}
-				else if(i == 2)
-				{
-					fr_2 = f;
-					rt_2 = rate;
-					tau2_a = 0.5 * (rt_0 + rt_2) * (c.actual_dt * (fr_2 - fr_0));
-				}
-				else if(i == 4)
-					tau2 = tau2_a + 0.5 * (rt_2 + rate) * (c.actual_dt * (f - fr_2));
-			}
-			else if(i > 0)
-				tau2 += 0.5 * (rt_prev + rate) * (c.actual_dt * (f - fr_prev));
-			fr_prev = f;
-			rt_prev = rate;
-		}
-	}
-	return free_step_finish_tail(R, m_dm, L, hist, c, fr, rt, dtau, tau2, invalid, false, 0.0);
-}
-
-// One piece-boundary rate of a step (rate_at_fraction at fraction f) or, for the job `next`, the
-// scattering rate at the propagator's state after the step (rate_total at ra, va, as the next
-// step's head forms it when ra is inside the Sun); the two share the code path, so that the lanes
-// of a warp that form them run converged.
-__device__ __forceinline__ double depth_job_rate(const DevSolar& S, const DevPoint* __restrict__ P, const Event& a, const Event& b, double f,
-                                                 bool next, double ra, double va)
-{
-	f = clamp_unit(f);
-	const double x = a.x.x + f * (b.x.x - a.x.x), vx = a.v.x + f * (b.v.x - a.v.x);
-	const double y = a.x.y + f * (b.x.y - a.x.y), vy = a.v.y + f * (b.v.y - a.v.y);
-	const double z = a.x.z + f * (b.x.z - a.x.z), vz = a.v.z + f * (b.v.z - a.v.z);
-	double r2 = 0.0, v2 = 0.0;
-	r2 += x * x;
-	v2 += vx * vx;
-	r2 += y * y;
-	v2 += vy * vy;
-	r2 += z * z;
-	v2 += vz * vz;
-	double r = sqrt(r2 > 0.0 ? r2 : 0.0), v = sqrt(v2 > 0.0 ? v2 : 0.0);
-	if(next)
-	{
-		r = ra;
-		v = va;
-	}
-	if(r >= DMS_RSUN_KM)
-		return 0.0;
-	return rate_total(S, P, r, v);
-}
-
-__device__ __forceinline__ double shfl_d(double v, int src) { return __shfl_sync(0xffffffffu, v, src); }
-
-// The piece rates of every lane of the warp in `dm` (the lanes whose finished step needs them),
-// formed by the whole warp at once: job j of a step (j = 0..PIECES, the boundaries; PIECES + 1,
-// the next step's rate) runs on its own lane with the step's events broadcast from its owner,
-// in as many rounds of 32 jobs as the steps need.  Each lookup is the function and arguments of
-// the one-lane loop, so the rates are the same numbers.  Every lane of the warp calls this.
-template <int PIECES>
-__device__ __forceinline__ void coop_depth_rates(const RunParams& R, const DevPoint* __restrict__ P, const FinishCtx& c, bool depth,
-                                                 unsigned int dm, double (&fr)[DMS_MAX_OPTICAL_DEPTH_PIECES + 1],
-                                                 double (&rt)[DMS_MAX_OPTICAL_DEPTH_PIECES + 1], double& next_rate)
-{
-	constexpr int J = PIECES + 2;
-	const int me = threadIdx.x & 31;
-	const int jobs = __popc(dm) * J;
-	const int rank = __popc(dm & ((1u << me) - 1u));  // among the lanes of dm (when depth)
-	const double span = c.s1 - c.s0;
-	for(int base = 0; base < jobs; base += 32)
-	{
-		const int job = base + me;
-		const bool active = job < jobs;
-		const int oi = active ? job / J : 0;
-		const int j = active ? job - oi * J : 0;
-		const int owner = nth_set_bit(dm, oi);
-		Event a, b;
-		a.x = mk(shfl_d(c.before.x.x, owner), shfl_d(c.before.x.y, owner), shfl_d(c.before.x.z, owner));
-		a.v = mk(shfl_d(c.before.v.x, owner), shfl_d(c.before.v.y, owner), shfl_d(c.before.v.z, owner));
-		b.x = mk(shfl_d(c.after.x.x, owner), shfl_d(c.after.x.y, owner), shfl_d(c.after.x.z, owner));
-		b.v = mk(shfl_d(c.after.v.x, owner), shfl_d(c.after.v.y, owner), shfl_d(c.after.v.z, owner));
-		const double s0 = shfl_d(c.s0, owner), sp = shfl_d(span, owner);
-		const double ra = shfl_d(c.r_after, owner), va = shfl_d(c.v_after, owner);
-		const DevPoint* Po = reinterpret_cast<const DevPoint*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(P), owner));
-		double rate = 0.0;
-		if(active)
-			rate = depth_job_rate(R.S, Po, a, b, s0 + static_cast<double>(j) / static_cast<double>(PIECES) * sp, j == J - 1, ra, va);
-#pragma unroll
-		for(int jj = 0; jj < J; jj++)
-		{
-			const int src = rank * J + jj - base;
-			const bool here = depth && src >= 0 && src < 32;
-			const double v = shfl_d(rate, here ? src : me);
-			if(here)
-			{
-				if(jj < J - 1)
-					rt[jj] = v;
-				else
-					next_rate = v;
-			}
-		}
-	}
-	if(depth)
-	{
-#pragma unroll
-		for(int i = 0; i <= PIECES; i++)
-			fr[i] = c.s0 + static_cast<double>(i) / static_cast<double>(PIECES) * span;
-		if(c.r_before < DMS_RSUN_KM && c.s0 <= 1.0e-12)
-			rt[0] = c.rate_before;
-	}
-}
-
-// A finished step on every lane of the warp that holds one (want), the piece rates formed by the
-// whole warp (coop_depth_rates).  Every lane of the warp calls this; the others only help.
-__device__ __forceinline__ int free_step_finish_warp(const RunParams& R, const DevPoint* __restrict__ P, double m_dm, StrictLane& L,
-                                                     double2* hist, int rk, bool want)
-{
-	FinishCtx c = {};
-	int ph = PH_STEP;
-	if(want)
-		ph = free_step_finish_head(R, L, rk, c);
-	const bool depth = want && ph == PH_CONTINUE && c.depth;
-	const unsigned int dm = __ballot_sync(0xffffffffu, depth);
-	double fr[DMS_MAX_OPTICAL_DEPTH_PIECES + 1], rt[DMS_MAX_OPTICAL_DEPTH_PIECES + 1];
-	double next_rate = 0.0, dtau = 0.0, tau2 = 0.0;
-	bool invalid = false;
-	if(dm != 0u)
-	{
-		if(R.capture_mode)
-			coop_depth_rates<DMS_CAPTURE_OPTICAL_DEPTH_PIECES>(R, P, c, depth, dm, fr, rt, next_rate);
-		else
-			coop_depth_rates<DMS_MAX_OPTICAL_DEPTH_PIECES>(R, P, c, depth, dm, fr, rt, next_rate);
-	}
-	if(depth)
-	{
-		if(R.capture_mode)
-			depth_sums<DMS_CAPTURE_OPTICAL_DEPTH_PIECES>(fr, rt, c.actual_dt, dtau, tau2, invalid);
-		else
-			depth_sums<DMS_MAX_OPTICAL_DEPTH_PIECES>(fr, rt, c.actual_dt, dtau, tau2, invalid);
-	}
-	if(want && ph == PH_CONTINUE)
-		return free_step_finish_tail(R, m_dm, L, hist, c, fr, rt, dtau, tau2, invalid, depth, next_rate);
-	return ph;
 }
 
 // Initial_Conditions + Hyperbolic_Kepler_Shift of every work index (src/Data_Generation.cpp:747-761,
@@ -613,112 +681,14 @@ __global__ void __launch_bounds__(128) initial_state_kernel(const RunParams R)
 	R.init[w] = st;
 }
 
-// ---------------------------------------------------------------------------------------------
-// Tail pipeline.  A lane that runs alone spends its step on one dependent chain, and the
-// divergent paths of a warp do not overlap, but two warps do.  So once a block has drained, a
-// warp whose lanes are all done stays as the block's helper: a stepping lane (the owner) hands it
-// its propagator through shared memory, the helper makes the step's head (free_step_begin) and
-// its RK45 attempts (paired on its lanes 0 and 1), and the owner adopts the result.  Right after
-// adopting, the owner hands over the next step's start, computed as if the step it is about to
-// finish ends plainly (the propagator unchanged, one more free step), and finishes the step
-// meanwhile.  It adopts that speculative result only when its state is then bit for bit the one
-// the speculation started from; otherwise it discards it and hands over its actual state.  The
-// helper runs the same functions on the same values, so the results are the same.  One owner per
-// block; every wait is bounded by the global timer, and a wait that runs out detaches the owner,
-// which then steps on its own.
-enum PipeState : int
-{
-	PIPE_NONE = 0,      // no helper
-	PIPE_FREE = 1,      // a helper waits for an owner
-	PIPE_ATTACHED = 2,
-	PIPE_CLOSED = 3,
-};
-
-struct PipeBox
-{
-	int state, job, done;  // job / done: sequence numbers of the hand-over and of its result
-	int begin_phase, rk, rk_inner;
-	const DevPoint* P;
-	uint64_t seg_in;
-	Prop pr_in, pr_out;
-	Event before_out;
-	double b_time, b_radius, b_phi, b_vr, b_step, rate_before;
-};
-
-__device__ __forceinline__ PipeBox& pipe_box()
-{
-	__shared__ PipeBox box;
-	return box;
-}
-
-// bounds of the waits, in SM clock cycles (about 2 GHz)
-constexpr long long PIPE_WAIT_CYCLES = 2000000ll;            // an owner's wait for a result (~1 ms, 100 steps)
-constexpr long long PIPE_IDLE_FREE_CYCLES = 400000ll;        // a helper without owner leaves after ~0.2 ms
-constexpr long long PIPE_IDLE_ATTACHED_CYCLES = 10000000ll;  // ~5 ms (an owner hands over every step)
-
-__device__ __forceinline__ bool pipe_wait(const PipeBox& b, int seq)
-{
-	const long long t0 = clock64();
-	while(*reinterpret_cast<const volatile int*>(&b.done) != seq)
-	{
-		if(clock64() - t0 > PIPE_WAIT_CYCLES)
-			return false;
-		__nanosleep(32);  // leaves the issue slots to the other warps of the SM
-	}
-	__threadfence_block();
-	return true;
-}
-
-__device__ __forceinline__ bool same_prop(const Prop& a, const Prop& b)
-{
-	auto eq = [](double x, double y) { return __double_as_longlong(x) == __double_as_longlong(y); };
-	return eq(a.time, b.time) && eq(a.radius, b.radius) && eq(a.phi, b.phi) && eq(a.v_radial, b.v_radial) && eq(a.J, b.J) &&
-	       eq(a.time_step, b.time_step) && eq(a.ax.x, b.ax.x) && eq(a.ax.y, b.ax.y) && eq(a.ax.z, b.ax.z) && eq(a.ay.x, b.ay.x) &&
-	       eq(a.ay.y, b.ay.y) && eq(a.ay.z, b.ay.z) && a.radial_mode == b.radial_mode;
-}
-
 struct StrictStep
 {
-	// the lane loop runs a step as begin / attempt / finish and may pair the attempt of a lane
-	// with an idle lane of its warp (rk45_attempt_pair)
-	static constexpr bool pairs = DMS_PAIRED_ATTEMPTS != 0 && DMS_CERTIFIED_MATH != 0 && DMS_RK_UNROLLED >= 1;
-	__device__ __forceinline__ int begin(const RunParams& R, const DevPoint* __restrict__ P, StrictLane& L) const
+	static constexpr bool collective = true;  // the whole warp makes a pass
+	static constexpr int buffer = COOP_BUFFER;
+	__device__ __forceinline__ int operator()(const RunParams& R, const DevPoint* __restrict__ P, double m_dm, StrictLane& L, double2* hist, int phase,
+	                                          double* buffer) const
 	{
-		return free_step_begin(R, P, L);
-	}
-	__device__ __forceinline__ int attempt(const DevSolar& S, StrictLane& L, int drained) const
-	{
-		return free_step_attempt(S, L, drained);
-	}
-	// all lanes of the warp call this; role 1 = owner (its attempt), 2 = helper, 0 = neither
-	__device__ __forceinline__ int pair_attempt(const DevSolar& S, StrictLane& L, int role, int partner) const
-	{
-		if(role == 1)
-			L.rk_inner++;
-		bool good = S.bucket_single_step != 0;
-		const int rk = rk45_attempt_pair(S, L.pr, L.rk_inner, role, partner, good);
-		if(role == 1 && !good)
-			return rk45_attempt_ieee(S, L.pr, L.rk_inner);
-		return rk;
-	}
-	__device__ __forceinline__ int finish(const RunParams& R, const DevPoint* __restrict__ P, double m_dm, StrictLane& L, double2* hist,
-	                                      int rk) const
-	{
-		return free_step_finish(R, P, m_dm, L, hist, rk);
-	}
-	// the finish of the paired attempts: all lanes of the warp call this (want: the lane's own)
-	__device__ __forceinline__ int finish_warp(const RunParams& R, const DevPoint* __restrict__ P, double m_dm, StrictLane& L, double2* hist,
-	                                           int rk, bool want) const
-	{
-		return free_step_finish_warp(R, P, m_dm, L, hist, rk, want);
-	}
-	__device__ __forceinline__ int operator()(const RunParams& R, const DevPoint* __restrict__ P, double m_dm, StrictLane& L, double2* hist,
-	                                          int drained) const
-	{
-		const int ph = begin(R, P, L);
-		if(ph != PH_STEP)
-			return ph;
-		return finish(R, P, m_dm, L, hist, attempt(R.S, L, drained));
+		return strict_step(R, P, m_dm, L, hist, phase, buffer);
 	}
 	__device__ __forceinline__ double channel(const DevSolar& S, const DevPoint* __restrict__ P, int i, double dr, double T, double v, int k) const
 	{
@@ -728,182 +698,9 @@ struct StrictStep
 	{
 		return scatter_with_target(S, P, D, e, target);
 	}
-
-	// ---- tail pipeline (see PipeBox) ----
-	static constexpr bool pipeline = DMS_TAIL_PIPELINE != 0 && pairs;
-	__device__ __forceinline__ void pipe_init() const
-	{
-		PipeBox& b = pipe_box();
-		b.state = PIPE_NONE;
-		b.job = 0;
-		b.done = 0;
-	}
-	// all lanes of a warp whose lanes are all done call this; it returns when the warp leaves
-	// (it was not needed as the helper, or it has served its last owner)
-	__device__ void pipe_serve(const RunParams& R, StrictLane& L) const
-	{
-		PipeBox& b = pipe_box();
-		const int me = threadIdx.x & 31;
-		int became = 0;
-		if(me == 0)
-			became = atomicCAS(&b.state, PIPE_NONE, PIPE_FREE) == PIPE_NONE ? 1 : 0;
-		if(__shfl_sync(0xffffffffu, became, 0) == 0)
-			return;
-		// a helper that served before this one left every hand-over answered (done == job)
-		int last = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile int*>(&b.job), 0);
-		long long idle_since = clock64();
-		for(unsigned int poll = 0;; poll++)
-		{
-			const int job = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile int*>(&b.job), 0);
-			if(job != last)
-			{
-				__threadfence_block();
-				pipe_job(R, L, b);
-				__threadfence_block();
-				if(me == 0)
-					*reinterpret_cast<volatile int*>(&b.done) = job;
-				last = job;
-				idle_since = clock64();
-				continue;
-			}
-			const int st = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile int*>(&b.state), 0);
-			const long long idle = clock64() - idle_since;
-			// the cancel flag lives in host memory: read it rarely
-			const bool cancelled = (poll & 4095u) == 4095u && __any_sync(0xffffffffu, *R.cancel != 0);
-			if(cancelled || (st == PIPE_FREE && idle > PIPE_IDLE_FREE_CYCLES) || (st != PIPE_FREE && idle > PIPE_IDLE_ATTACHED_CYCLES))
-			{
-				int closed = 1;
-				if(me == 0)
-				{
-					// without an owner the box is left for a warp that is done later; an owner may
-					// attach meanwhile, and then the helper stays
-					if(st == PIPE_FREE && !cancelled)
-						closed = atomicCAS(&b.state, PIPE_FREE, PIPE_NONE) == PIPE_FREE ? 1 : 0;
-					else
-						atomicExch(&b.state, PIPE_CLOSED);
-				}
-				if(__shfl_sync(0xffffffffu, closed, 0))
-					return;
-				continue;
-			}
-			__nanosleep(64);
-		}
-	}
-	// the helper's work for one hand-over: the step's head on lane 0 (its own lane state as
-	// scratch), then the RK45 attempts paired on lanes 0 and 1 until one is not retried
-	__device__ __forceinline__ void pipe_job(const RunParams& R, StrictLane& L, PipeBox& b) const
-	{
-		const int me = threadIdx.x & 31;
-		int ph = PH_STEP;
-		if(me == 0)
-		{
-			L.pr = b.pr_in;
-			L.seg_steps = b.seg_in;
-			L.before_valid = 0;  // the head forms Event_In_3D of the propagator (= the owner's cached one)
-			L.next_valid = 0;
-			L.in_rk = 0;
-			ph = free_step_begin(R, b.P, L);
-		}
-		ph = __shfl_sync(0xffffffffu, ph, 0);
-		int rk = RK_RETRY, passes = 0;
-		if(ph == PH_STEP)
-		{
-			const int role = me == 0 ? 1 : (me == 1 ? 2 : 0);
-			const int partner = me == 0 ? 1 : 0;
-			while(rk == RK_RETRY && passes <= DMS_RK45_MAX_INNER_RETRIES + 1)
-			{
-				rk = __shfl_sync(0xffffffffu, pair_attempt(R.S, L, role, partner), 0);
-				passes++;
-			}
-		}
-		if(me == 0)
-		{
-			b.begin_phase = (ph == PH_STEP && rk == RK_RETRY) ? PH_FINAL : ph;  // a step that never ended: the owner steps alone
-			b.rk = rk;
-			b.rk_inner = L.rk_inner;
-			b.pr_out = L.pr;
-			b.before_out = L.before;
-			b.b_time = L.b_time;
-			b.b_radius = L.b_radius;
-			b.b_phi = L.b_phi;
-			b.b_vr = L.b_vr;
-			b.b_step = L.b_step;
-			b.rate_before = L.rate_before;
-		}
-	}
-	__device__ __forceinline__ bool pipe_attach() const
-	{
-		PipeBox& b = pipe_box();
-		return *reinterpret_cast<volatile int*>(&b.state) == PIPE_FREE && atomicCAS(&b.state, PIPE_FREE, PIPE_ATTACHED) == PIPE_FREE;
-	}
-	__device__ __forceinline__ int pipe_post(const DevPoint* __restrict__ P, const Prop& pr, uint64_t seg) const
-	{
-		PipeBox& b = pipe_box();
-		b.P = P;
-		b.pr_in = pr;
-		b.seg_in = seg;
-		__threadfence_block();
-		const int seq = b.job + 1;
-		*reinterpret_cast<volatile int*>(&b.job) = seq;
-		return seq;
-	}
-	__device__ __forceinline__ void pipe_adopt(const PipeBox& b, StrictLane& L) const
-	{
-		L.pr = b.pr_out;
-		L.before = b.before_out;
-		L.before_valid = 1;
-		L.next_valid = 0;
-		L.b_time = b.b_time;
-		L.b_radius = b.b_radius;
-		L.b_phi = b.b_phi;
-		L.b_vr = b.b_vr;
-		L.b_step = b.b_step;
-		L.rate_before = b.rate_before;
-		L.in_rk = 1;
-		L.rk_inner = b.rk_inner;
-	}
-	// the owner's step start: 1 = adopted (rk set), 0 = make the head here, -1 = detached
-	__device__ __forceinline__ int pipe_step(const DevPoint* __restrict__ P, StrictLane& L, int& spec, int& rk) const
-	{
-		PipeBox& b = pipe_box();
-		if(*reinterpret_cast<volatile int*>(&b.state) != PIPE_ATTACHED)
-		{
-			spec = 0;
-			return -1;  // the helper has left
-		}
-		if(spec != 0)
-		{
-			const int s = spec;
-			spec = 0;
-			if(!pipe_wait(b, s))
-				return -1;
-			if(b.begin_phase == PH_STEP && b.P == P && b.seg_in == L.seg_steps && same_prop(b.pr_in, L.pr))
-			{
-				pipe_adopt(b, L);
-				rk = b.rk;
-				return 1;
-			}
-		}
-		const int s = pipe_post(P, L.pr, L.seg_steps);
-		if(!pipe_wait(b, s))
-			return -1;
-		if(b.begin_phase != PH_STEP)
-			return 0;
-		pipe_adopt(b, L);
-		rk = b.rk;
-		return 1;
-	}
-	__device__ __forceinline__ void pipe_release(int& spec) const
-	{
-		PipeBox& b = pipe_box();
-		if(spec != 0)
-			pipe_wait(b, spec);
-		spec = 0;
-		atomicCAS(&b.state, PIPE_ATTACHED, PIPE_FREE);
-	}
 };
 
-__global__ void __launch_bounds__(128, DMS_TRAJ_MIN_BLOCKS) trajectory_kernel(const RunParams R)
+__global__ void __launch_bounds__(MAX_THREADS, 1) trajectory_kernel(const RunParams R)
 {
 	lane_loop<StrictLane>(R, StrictStep());
 }
@@ -1008,8 +805,10 @@ __global__ void certified_math_check_kernel(uint64_t n, uint64_t seed, unsigned 
 		}
 		if(h3 & 1)
 			a = -a;
-		bool ok = true;
-		const double q = fast::div(a, b, ok);
+		// the operand range of fast::div: other pairs count as fallbacks
+		const double aa = fabs(a), ab = fabs(b);
+		bool ok = (ab >= 0x1p-100) & (ab < 0x1p100) & (((aa >= 0x1p-700) & (aa <= 0x1p400)) | (__double_as_longlong(a) == 0));
+		const double q = fast::div(a, fast::recip(b, ok));
 		const double ref = a / b;
 		if(!ok)
 			c[1]++;

@@ -5,54 +5,11 @@
 
 #include "dms_device.cuh"
 
-// Minimum resident 128-thread blocks per SM the trajectory kernels are compiled for (caps
-// their registers at 65536 / (128 * n)).
-#ifndef DMS_TRAJ_MIN_BLOCKS
-#define DMS_TRAJ_MIN_BLOCKS 4
-#endif
-// RK45 form of the kernels: 0 = one loop over the six stages (a short hot loop: fewer
-// instruction-cache misses with every lane busy), 1 = the stages written out (a shorter
-// dependent chain for a lane that runs alone), 2 = the loop while the work queue still has
-// items and the written-out stages once the block has seen it drained (a lane's fetch, or the
-// queue head read every 64 iterations).  With the FP64 tail attempts paired across two lanes
-// (DMS_PAIRED_ATTEMPTS), form 2 is the default: measured 13 % more accepted steps per second
-// with every lane busy than form 1, the same time per step for a lane that runs alone.
-#ifndef DMS_RK_UNROLLED
-#define DMS_RK_UNROLLED 2
-#endif
-// FP64 RK45 attempts with the certified straight-line division and square root of
-// dms_fastmath.cuh (1) or with IEEE `/` and sqrt (0); the results are the same bits.
-#ifndef DMS_CERTIFIED_MATH
-#define DMS_CERTIFIED_MATH 1
-#endif
-// FP64 attempts of lanes that run with idle lanes beside them are computed by two lanes
-// (rk45_attempt_pair) when 1; always by the lane alone when 0.  The same bits either way.
-#ifndef DMS_PAIRED_ATTEMPTS
-#define DMS_PAIRED_ATTEMPTS 1
-#endif
-// Pairing applies to warps with at most DMS_PAIR_MAX_LANES attempting lanes (up to 16, every
-// one paired with an idle lane) and, when DMS_PAIR_ONLY_DRAINED, only once the block has seen
-// the work queue drained (the tail of a launch).
-#ifndef DMS_PAIR_MAX_LANES
-#define DMS_PAIR_MAX_LANES 16
-#endif
-#ifndef DMS_PAIR_ONLY_DRAINED
-#define DMS_PAIR_ONLY_DRAINED 1
-#endif
-#ifndef DMS_RK_UNROLLED_MIXED
-#define DMS_RK_UNROLLED_MIXED 1
-#endif
-// The FP64 tail pipeline (a second warp of a drained block makes a lone lane's step head and
-// attempts while the lane finishes its previous step) when 1.
-#ifndef DMS_TAIL_PIPELINE
-#define DMS_TAIL_PIPELINE 1
-#endif
-#ifndef DMS_TRAJ_MIN_BLOCKS_MIXED
-#define DMS_TRAJ_MIN_BLOCKS_MIXED 4
-#endif
-
 namespace dms
 {
+
+// The largest block of the trajectory kernels: all 16 warps that their registers allow per SM.
+constexpr int MAX_THREADS = 512;
 
 // Status bits written by the kernels (device status word).
 enum : unsigned int
@@ -109,6 +66,8 @@ struct RunParams
 	// the warp batching of scatterings and terminations
 	uint32_t queue_chunk;
 	int scatter_batch, scatter_wait, final_batch, final_wait;
+	int lanes_per_warp;  // lanes of a warp that take trajectories (32, fewer in a spread launch)
+	int lockstep_min;    // lanes at work below which a block's warps leave the lockstep once the queue is empty
 	int ic_max_attempts;
 	// accumulators (accumulate mode)
 	unsigned long long* counters;   // n_points x DMS_NUM_COUNTERS

@@ -59,8 +59,7 @@ __device__ __forceinline__ double commit_event_mixed(const DevSolar& S, const De
 // RK45 retry loop: when no step is in progress the pre-step bounds are applied and a step is
 // opened; every pass makes one RK45 attempt; only a finished step runs the optical-depth,
 // boundary and commit logic.  Returns the next phase of the lane.
-__device__ __forceinline__ int free_step_mixed(const RunParams& R, const DevPoint* __restrict__ P, double m_dm, MixedLane& L, double2* hist,
-                                               int drained)
+__device__ __forceinline__ int free_step_mixed(const RunParams& R, const DevPoint* __restrict__ P, double m_dm, MixedLane& L, double2* hist)
 {
 	const DevSolar& S = R.S;
 	const DevSolarF F{R.sf_r, R.sf_gm, R.sf_gm_s, R.sf_vesc2, R.sf_vesc2_s};
@@ -130,12 +129,7 @@ __device__ __forceinline__ int free_step_mixed(const RunParams& R, const DevPoin
 		L.rk_inner = 0;
 	}
 	L.rk_inner++;
-#if DMS_RK_UNROLLED_MIXED == 2
-	const int rk = drained ? rk45_attempt_f<true>(S, F, L.pr, L.rk_inner) : rk45_attempt_f<false>(S, F, L.pr, L.rk_inner);
-#else
-	(void)drained;
-	const int rk = rk45_attempt_f<DMS_RK_UNROLLED_MIXED == 1>(S, F, L.pr, L.rk_inner);
-#endif
+	const int rk = rk45_attempt_f<true>(S, F, L.pr, L.rk_inner);
 	if(rk == RK_RETRY)
 		return PH_STEP;
 	L.in_rk = 0;
@@ -363,12 +357,11 @@ __device__ __forceinline__ int free_step_mixed(const RunParams& R, const DevPoin
 
 struct MixedStep
 {
-	static constexpr bool pairs = false;
-	static constexpr bool pipeline = false;
-	__device__ __forceinline__ int operator()(const RunParams& R, const DevPoint* __restrict__ P, double m_dm, MixedLane& L, double2* hist,
-	                                          int drained) const
+	static constexpr bool collective = false;
+	static constexpr int buffer = 0;
+	__device__ __forceinline__ int operator()(const RunParams& R, const DevPoint* __restrict__ P, double m_dm, MixedLane& L, double2* hist) const
 	{
-		return free_step_mixed(R, P, m_dm, L, hist, drained);
+		return free_step_mixed(R, P, m_dm, L, hist);
 	}
 	__device__ __forceinline__ double channel(const DevSolar& S, const DevPoint* __restrict__ P, int i, double dr, double T, double v, int k) const
 	{
@@ -380,7 +373,7 @@ struct MixedStep
 	}
 };
 
-__global__ void __launch_bounds__(128, DMS_TRAJ_MIN_BLOCKS_MIXED) trajectory_kernel_mixed(const RunParams R)
+__global__ void __launch_bounds__(MAX_THREADS, 1) trajectory_kernel_mixed(const RunParams R)
 {
 	lane_loop<MixedLane>(R, MixedStep());
 }

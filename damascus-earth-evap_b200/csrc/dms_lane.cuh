@@ -83,6 +83,13 @@ __device__ __forceinline__ bool wall_time_exceeded(const RunParams& R, const Lan
 	return R.wall_limit_ns != 0 && global_timer_ns() - L.wall_start > R.wall_limit_ns;
 }
 
+// Position of the (n+1)-th set bit of m (n from 0); m must have more than n set bits.
+__device__ __forceinline__ int nth_set_bit(unsigned int m, int n)
+{
+	for(int t = 0; t < n; t++) m &= m - 1u;
+	return __ffs(m) - 1;
+}
+
 template <class Lane>
 __device__ __forceinline__ void accumulate_bincount(Lane& L, double2* hist, double r, double v2, double dt)
 {
@@ -93,7 +100,10 @@ __device__ __forceinline__ void accumulate_bincount(Lane& L, double2* hist, doub
 	if(isfinite(r) && r >= 0.0 && r < DMS_BIN_MAX_KM)
 	{
 		if constexpr(Lane::exact_bins)
-			bin = static_cast<int>(r / DMS_BIN_WIDTH_KM);
+		{
+			double whole;
+			bin = static_cast<int>(fast::floor_index(fast::div_const(r, DMS_BIN_WIDTH_KM), whole));
+		}
 		else
 			bin = static_cast<int>(r * (1.0 / DMS_BIN_WIDTH_KM));
 		if(bin < 0) bin = 0;
@@ -669,28 +679,28 @@ __device__ __forceinline__ int finish_scatter(const RunParams& R, const DevPoint
 }
 
 
-// Position of the (n+1)-th set bit of m (n from 0); m must have more than n set bits.
-__device__ __forceinline__ int nth_set_bit(unsigned int m, int n)
-{
-	for(int t = 0; t < n; t++) m &= m - 1u;
-	return __ffs(m) - 1;
-}
-
 template <class Lane, class Step>
 __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 {
-	const int lane_id = blockIdx.x * blockDim.x + threadIdx.x;
-	double2* hist = R.lane_hist + static_cast<size_t>(lane_id) * DMS_NUM_BINS;
-	__shared__ double coop_rates[4][DMS_NUM_TARGETS + 1];  // blocks of at most 128 threads
+	// the first R.lanes_per_warp lanes of every warp take trajectories (and own a histogram row);
+	// the others only help in the warp's collective steps
+	const int in_warp = threadIdx.x & 31;
+	const bool takes_work = in_warp < R.lanes_per_warp;
+	const int warp_id = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+	double2* hist = R.lane_hist + static_cast<size_t>(warp_id * R.lanes_per_warp + (takes_work ? in_warp : 0)) * DMS_NUM_BINS;
+	// per warp: the 64 channel rates of a scattering, or the steps and rates of Step's own lookups
+	constexpr int BUFFER = Step::buffer > DMS_NUM_TARGETS + 1 ? Step::buffer : DMS_NUM_TARGETS + 1;
+	__shared__ double coop_rates[MAX_THREADS / 32][BUFFER];
 	double* rates = coop_rates[threadIdx.x >> 5];
-	// set once a lane of the block finds the work queue empty: the launch is in its tail, where
-	// the lanes left run alone and the free step takes its shorter-chain form
-	__shared__ int queue_drained;
-	if(threadIdx.x == 0)
-		queue_drained = 0;
-	if constexpr(Step::pipeline)
-		if(threadIdx.x == 0)
-			step.pipe_init();
+	// Lockstep: the warps of a block with more than one warp per scheduler make every pass together,
+	// so that an instruction fetched once serves all of them.  The block votes on its rare phases:
+	// lanes stepping, at a scattering point and at a termination, counted per pass (two sets, one
+	// being cleared while the other is filled).
+	__shared__ int votes[2][4];
+	if(threadIdx.x < 8)
+		votes[threadIdx.x >> 2][threadIdx.x & 3] = 0;
+	bool lockstep = blockDim.x > 128;
+	int passes_scatter = 0, passes_final = 0;  // passes since the block's last scattering (termination) phase
 	__syncthreads();
 	Lane L;
 	FlushJob job;
@@ -698,16 +708,10 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 	job.b1 = -1;
 	const DevPoint* P = R.points;
 	double m_dm = 0.0;
-	int phase = PH_FETCH;
-	int scatter_wait = 0;
-	int final_wait = 0;
+	int phase = takes_work ? PH_FETCH : PH_DONE;
 	// the lane's claimed ids [q_next, q_end): R.queue_chunk ids per claim
 	uint64_t q_next = 0, q_end = 0;
 	const unsigned int lane_bit = 1u << (threadIdx.x & 31);
-	// tail pipeline: this lane owns the block's helper warp; pipe_spec is the hand-over of the
-	// next step's start made before the current finish (0 = none)
-	bool pipe_owner = false;
-	int pipe_spec = 0;
 	// Every lane stays in the loop until its whole warp is done (a lane without work waits in
 	// PH_DONE), and leaves only together with the others.  So the warp's collective steps
 	// below (batching votes, cooperative target sampling into the warp's shared rates, the
@@ -716,32 +720,111 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 	constexpr unsigned int FULL_WARP = 0xffffffffu;
 	for(uint64_t iter = 0;; iter++)
 	{
-		if(__all_sync(FULL_WARP, phase == PH_DONE))
+		bool go_scatter = false, go_final = false;
+		if(lockstep)
 		{
-			if constexpr(Step::pipeline)
-				if(R.wall_limit_ns == 0 && blockDim.x > 32)
-					step.pipe_serve(R, L);  // the warp may stay as the block's helper
-			break;
-		}
-#if DMS_RK_UNROLLED == 2 || DMS_RK_UNROLLED_MIXED == 2
-		// a block whose lanes are all held by long trajectories learns of the drained queue from
-		// the queue head itself (one read per warp every 64 iterations)
-		if((iter & 63) == 63 && (threadIdx.x & 31) == 0 &&
-		   *reinterpret_cast<volatile unsigned long long*>(R.queue_head) >= R.total)
-			*reinterpret_cast<volatile int*>(&queue_drained) = 1;
-#endif
-		if((iter & 1023) == 1023)
-		{
-			if(__any_sync(FULL_WARP, *R.cancel != 0))
+			int* v = votes[iter & 1];
+			const unsigned int b_step = __ballot_sync(FULL_WARP, phase == PH_STEP || phase == PH_FETCH || phase == PH_SEGMENT);
+			const unsigned int b_scatter = __ballot_sync(FULL_WARP, phase == PH_SCATTER);
+			const unsigned int b_final = __ballot_sync(FULL_WARP, phase == PH_FINAL);
+			if(in_warp == 0)
 			{
-				atomicOr(R.status, STATUS_CANCELLED);
+				if(b_step) atomicAdd(v + 0, __popc(b_step));
+				if(b_scatter) atomicAdd(v + 1, __popc(b_scatter));
+				if(b_final) atomicAdd(v + 2, __popc(b_final));
+				// one thread looks whether the queue is empty and whether the host cancelled
+				if(threadIdx.x == 0)
+				{
+					int flags = (iter & 15) == 15 && *reinterpret_cast<volatile unsigned long long*>(R.queue_head) >= R.total ? 1 : 0;
+					flags |= (iter & 1023) == 1023 && *R.cancel != 0 ? 2 : 0;
+					v[3] = flags;
+				}
+			}
+			__syncthreads();
+			const int n_step = v[0], n_scatter = v[1], n_final = v[2], flags = v[3];
+			if(threadIdx.x < 3)
+				votes[(iter & 1) ^ 1][threadIdx.x] = 0;
+			const int lanes = blockDim.x >> 5;
+			passes_scatter++;
+			passes_final++;
+			go_scatter = n_scatter != 0 && (n_scatter >= R.scatter_batch * lanes / 2 || n_step == 0 || passes_scatter >= R.scatter_wait);
+			go_final = n_final != 0 && (n_final >= R.final_batch * lanes / 2 || n_step == 0 || passes_final >= R.final_wait);
+			if(go_scatter)
+				passes_scatter = 0;
+			if(go_final)
+				passes_final = 0;
+			if(flags & 2)
+			{
+				if(in_warp == 0)
+					atomicOr(R.status, STATUS_CANCELLED);
 				break;
 			}
-			if(iter > R.iteration_budget)
+			if((iter & 1023) == 1023 && iter > R.iteration_budget)
 			{
 				atomicOr(R.status, STATUS_BUDGET);
 				break;
 			}
+			// few lanes left and no more work: the warps go on by themselves
+			if((flags & 1) && n_step + n_scatter + n_final <= R.lockstep_min)
+				lockstep = false;
+			if(n_step + n_scatter + n_final == 0)
+				break;
+		}
+		else
+		{
+			if(__all_sync(FULL_WARP, phase == PH_DONE))
+				break;
+			if((iter & 1023) == 1023)
+			{
+				if(__any_sync(FULL_WARP, *R.cancel != 0))
+				{
+					atomicOr(R.status, STATUS_CANCELLED);
+					break;
+				}
+				if(iter > R.iteration_budget)
+				{
+					atomicOr(R.status, STATUS_BUDGET);
+					break;
+				}
+			}
+			const unsigned int stepping = __ballot_sync(FULL_WARP, phase == PH_STEP || phase == PH_FETCH || phase == PH_SEGMENT);
+			const unsigned int waiting = __ballot_sync(FULL_WARP, phase == PH_SCATTER);
+			const unsigned int ending = __ballot_sync(FULL_WARP, phase == PH_FINAL);
+			// lanes wait until several lanes of the warp are there, or one has waited long enough, or no
+			// lane is stepping
+			if(waiting != 0u)
+			{
+				passes_scatter++;
+				go_scatter = __popc(waiting) >= R.scatter_batch || stepping == 0u || passes_scatter >= R.scatter_wait;
+				if(go_scatter)
+					passes_scatter = 0;
+			}
+			if(ending != 0u)
+			{
+				passes_final++;
+				go_final = __popc(ending) >= R.final_batch || stepping == 0u || passes_final >= R.final_wait;
+				if(go_final)
+					passes_final = 0;
+			}
+		}
+		// Scatterings and terminations run for many lanes at once.  A lane's draws do not depend on
+		// when it scatters.
+		if(go_scatter)
+		{
+			int target = TARGET_FAILED;
+			cooperative_targets(R, L, phase, rates, target, step, FULL_WARP);
+			if(phase == PH_SCATTER)
+				phase = finish_scatter(R, P, m_dm, L, target, step);
+		}
+		if(go_final)
+		{
+			if(phase == PH_FINAL)
+			{
+				write_back_bin(L, hist);
+				finalize(R, P, m_dm, L, job);
+				phase = PH_FETCH;
+			}
+			cooperative_flush(hist, job, FULL_WARP);
 		}
 		if(phase == PH_FETCH)
 		{
@@ -766,154 +849,19 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 			}
 			const uint64_t w = q_next++;
 			if(w >= R.total)
-			{
-				*reinterpret_cast<volatile int*>(&queue_drained) = 1;
 				phase = PH_DONE;
-			}
 			else
 				phase = start_trajectory(R, L, w, P, m_dm);
 		}
 		if(phase == PH_SEGMENT)
 			phase = segment_start(R, P, m_dm, L);
-		if constexpr(Step::pairs)
+		if constexpr(Step::collective)
 		{
-			// A step is opened per lane; its RK45 attempt then runs paired when at most half of
-			// the warp is attempting: every attempting lane takes an idle lane of its warp as a
-			// helper for the independent stages (rk45_attempt_pair), which shortens the dependent
-			// chain of a lane that runs alone, the tail of a launch.  Same results either way.  With
-			// Step::pipeline a lane that steps alone in its warp may instead hand its step head and
-			// attempts to the block's helper warp (see PipeBox); such a lane is busy ("piped")
-			// without attempting here.
-			const int drained = *reinterpret_cast<volatile int*>(&queue_drained);
-			bool want = false;
-			bool piped = false;  // the step's head and attempts came from the helper warp
-			int rk_piped = RK_RETRY;
-			if constexpr(Step::pipeline)
-			{
-				// only a lane that steps alone in its warp owns the helper: an owner's waits hold its
-				// whole warp.  An owner that ends its trajectory or stops being alone releases it.
-				const unsigned int stepping = __ballot_sync(FULL_WARP, phase == PH_STEP);
-				const bool alone = phase == PH_STEP && stepping == lane_bit;
-				if(pipe_owner && !alone && phase != PH_SCATTER && phase != PH_SEGMENT)
-				{
-					step.pipe_release(pipe_spec);
-					pipe_owner = false;
-				}
-				if(alone && !L.in_rk && drained && R.wall_limit_ns == 0)
-				{
-					if(!pipe_owner)
-						pipe_owner = step.pipe_attach();
-					if(pipe_owner)
-					{
-						const int r = step.pipe_step(P, L, pipe_spec, rk_piped);
-						piped = r == 1;
-						if(r < 0)
-							pipe_owner = false;  // the helper did not answer: step alone
-					}
-				}
-			}
-			if(phase == PH_STEP)
-			{
-				if(piped)
-					want = true;
-				else
-				{
-					const int ph = step.begin(R, P, L);
-					want = ph == PH_STEP;
-					if(!want)
-						phase = ph;
-				}
-			}
-			if constexpr(Step::pipeline)
-			{
-				// hand over the next step's start now, so that it is made during this finish
-				if(piped && rk_piped == RK_ACCEPTED)
-					pipe_spec = step.pipe_post(P, L.pr, L.seg_steps + 1);
-			}
-			const unsigned int att = __ballot_sync(FULL_WARP, want && !piped);
-			const unsigned int busy = __ballot_sync(FULL_WARP, want);
-			const int n_att = __popc(att);
-			// every attempting lane needs an idle lane (a piped lane is busy without attempting)
-			if(busy != 0u && n_att <= DMS_PAIR_MAX_LANES && n_att + __popc(busy) <= 32 && (drained || !DMS_PAIR_ONLY_DRAINED))
-			{
-				const int me = threadIdx.x & 31;
-				int role = 0, partner = me;
-				const unsigned int below = lane_bit - 1u;
-				if(want && !piped)
-				{
-					role = 1;
-					partner = nth_set_bit(~busy, __popc(att & below));
-				}
-				else if(!want)
-				{
-					const int q = __popc(~busy & below);
-					if(q < n_att)
-					{
-						role = 2;
-						partner = nth_set_bit(att, q);
-					}
-				}
-				// (a warp whose only busy lane was piped has no attempt to make)
-				const int rk = n_att != 0 ? step.pair_attempt(R.S, L, role, partner) : RK_RETRY;
-				// the finished steps' piece rates are formed by the whole warp
-				const int ph = step.finish_warp(R, P, m_dm, L, hist, piped ? rk_piped : rk, want);
-				if(want)
-					phase = ph;
-			}
-			else if(want)
-				phase = step.finish(R, P, m_dm, L, hist, piped ? rk_piped : step.attempt(R.S, L, drained));
+			if(__any_sync(FULL_WARP, phase == PH_STEP))
+				phase = step(R, P, m_dm, L, hist, phase, rates);
 		}
 		else if(phase == PH_STEP)
-			phase = step(R, P, m_dm, L, hist, *reinterpret_cast<volatile int*>(&queue_drained));
-		// Scatterings wait until several lanes of the warp have one (or one has waited
-		// R.scatter_wait iterations, or no lane is stepping), so that the scattering code
-		// runs for many lanes at once.  A lane's draws do not depend on when it scatters.
-		{
-			const unsigned int grp = FULL_WARP;
-			const unsigned int waiting = __ballot_sync(grp, phase == PH_SCATTER);
-			if(waiting != 0u)
-			{
-				const unsigned int stepping = __ballot_sync(grp, phase == PH_STEP);
-				const bool go = __popc(waiting) >= R.scatter_batch || stepping == 0u ||
-				                __any_sync(grp, phase == PH_SCATTER && scatter_wait >= R.scatter_wait);
-				if(go)
-				{
-					int target = TARGET_FAILED;
-					cooperative_targets(R, L, phase, rates, target, step, grp);
-					if(phase == PH_SCATTER)
-					{
-						phase = finish_scatter(R, P, m_dm, L, target, step);
-						scatter_wait = 0;
-					}
-				}
-				else if(phase == PH_SCATTER)
-					scatter_wait++;
-			}
-		}
-		// terminations are batched the same way
-		{
-			const unsigned int grp = FULL_WARP;
-			const unsigned int ending = __ballot_sync(grp, phase == PH_FINAL);
-			if(ending != 0u)
-			{
-				const unsigned int stepping = __ballot_sync(grp, phase == PH_STEP);
-				const bool go = __popc(ending) >= R.final_batch || stepping == 0u ||
-				                __any_sync(grp, phase == PH_FINAL && final_wait >= R.final_wait);
-				if(go)
-				{
-					if(phase == PH_FINAL)
-					{
-						write_back_bin(L, hist);
-						finalize(R, P, m_dm, L, job);
-						phase = PH_FETCH;
-						final_wait = 0;
-					}
-					cooperative_flush(hist, job, grp);
-				}
-				else if(phase == PH_FINAL)
-					final_wait++;
-			}
-		}
+			phase = step(R, P, m_dm, L, hist);
 	}
 	const bool in_trajectory = phase != PH_FETCH && phase != PH_DONE;
 	if(in_trajectory && L.bmax >= L.bmin)

@@ -218,14 +218,21 @@ void Apply_Lane_Options(RunParams& p, const dms_run_opts* o)
 	p.final_wait = o->final_wait ? static_cast<int>(o->final_wait) : 32;
 }
 
-// Threads per block when the caller leaves the choice open, one block per SM either way.  With a lane
-// per trajectory in one 128-thread block per SM, every warp has a scheduler of its own and a pass is
-// bound by its dependent chain; beyond that, 512-thread blocks run their 16 warps in lockstep
-// (dms_lane.cuh).  Measured, Capture mode m = 1 GeV, sigma = 1e-35 cm^2, FP64, 128 against 512 threads:
-// 1 024 trajectories 2.1 / 2.3 ms, 4 096 2.9 / 3.2 ms, 16 384 4.2 / 4.1 ms, 65 536 10.6 / 6.3 ms.
-int Default_Threads(uint64_t total, int sm_count)
+// Threads of the one block per SM.  With a lane per trajectory in 128 threads, every warp has a
+// scheduler of its own and a pass is bound by its dependent chain (the latency form of the kernel);
+// beyond that, 512 threads run their 16 warps in lockstep (the throughput form, dms_lane.cuh).
+// Measured, Capture mode m = 1 GeV, sigma = 1e-35 cm^2, FP64, 128 against 512 threads: 1 024 trajectories
+// 2.1 / 2.3 ms, 4 096 2.9 / 3.2 ms, 16 384 4.2 / 4.1 ms, 65 536 10.6 / 6.3 ms.  threads_per_block and
+// blocks_per_sm ask for the lanes per SM: blocks of one SM run as one block.
+int Block_Threads(const dms_run_opts* o, uint64_t total, int sm_count)
 {
-	return total <= 128 * static_cast<uint64_t>(sm_count) ? 128 : MAX_THREADS;
+	const int fitting = total <= LATENCY_THREADS * static_cast<uint64_t>(sm_count) ? LATENCY_THREADS : MAX_THREADS;
+	if(o->threads_per_block == 0 && o->blocks_per_sm == 0)
+		return fitting;
+	const int threads = o->threads_per_block ? static_cast<int>(o->threads_per_block) : LATENCY_THREADS;
+	const int most = MAX_THREADS / threads;
+	const int per_sm = o->blocks_per_sm ? static_cast<int>(std::min<uint32_t>(o->blocks_per_sm, most)) : most;
+	return std::min(threads * per_sm, fitting);
 }
 
 // One persistent launch over the given work; polls for completion, enforcing the wall-clock
@@ -239,15 +246,8 @@ int Launch_And_Wait(dms_ctx* ctx, const dms_run_opts* o, RunParams& p)
 		p.wall_limit_ns = 1;
 	Apply_Lane_Options(p, o);
 	const bool mixed = o->precision == DMS_PRECISION_MIXED;
-	int threads = o->threads_per_block ? static_cast<int>(o->threads_per_block) : 128;
-	if(o->threads_per_block == 0 && o->blocks_per_sm == 0)
-		threads = Default_Threads(p.total, ctx->sm_count);
-	const int max_per_sm = mixed ? Trajectory_Mixed_Max_Blocks_Per_SM(threads) : Trajectory_Max_Blocks_Per_SM(threads);
-	if(max_per_sm <= 0)
-		return Fail(ctx, DMS_ERR_CUDA, "trajectory kernel cannot be resident with this block size");
-	int per_sm = o->blocks_per_sm ? static_cast<int>(o->blocks_per_sm) : o->threads_per_block ? max_per_sm : 1;
-	per_sm = per_sm > max_per_sm ? max_per_sm : per_sm;
-	int blocks = ctx->sm_count * per_sm;
+	const int threads = Block_Threads(o, p.total, ctx->sm_count);
+	int blocks = ctx->sm_count;
 	// a launch with fewer trajectories than lanes spreads them over all of its warps: fewer lanes per
 	// warp diverge less, and its idle lanes help in the collective steps
 	const uint64_t warps = static_cast<uint64_t>(blocks) * (threads / 32);
@@ -389,6 +389,7 @@ void Fill_Dev_Point(const PointConstants& c, double* grid, DevPoint& d)
 	d.grid_inv_r = c.grid_inv_r;
 	d.grid_inv_v = c.grid_inv_v;
 	d.grid_vmax = c.grid_vmax;
+	d.grid_last = c.grid_n - 2.0;
 	d.grid = grid;
 	d.grid_n = c.grid_n;
 	for(int k = 0; k < DMS_NUM_TARGETS; k++) d.sigma_t[k] = c.sigma_target[k];

@@ -85,6 +85,7 @@ struct DevPoint
 	double n_esc;
 	double avg_speed, eta0;
 	double grid_inv_r, grid_inv_v, grid_vmax;
+	double grid_last;      // grid_n - 2
 	const double* grid;    // grid_n x grid_n, radius-major
 	const float* grid_f;   // FP32 image of grid (mixed-precision kernel)
 	int grid_n;
@@ -712,29 +713,6 @@ __device__ __forceinline__ double solar_vesc2_fast(const DevSolar& S, double r)
 	return (up ? k1.vesc2 : k0.vesc2) + (r - (up ? k1.r : k0.r)) * slope;
 }
 
-// One stage's dv/dt = J*J/r/r/r - gm/r/r and dphi/dt = J/r/r, each division rounded as the
-// reference rounds it; the quotients share one reciprocal.  A radius below 1 km (where the
-// reference clamps it) or not finite clears `good`, which hands the attempt to IEEE arithmetic.
-template <bool WANT_PHI>
-__device__ __forceinline__ void fast_stage(const DevSolar& S, double J, double JJ, double r, double& dv, double& dphi, bool& good)
-{
-	const double gm = solar_gm_fast(S, r);
-	good &= (r >= 1.0) & (r < 0x1p100);
-	const fast::Recip R = fast::recip(r, good);
-	dv = fast::div(fast::div(fast::div(JJ, R), R), R) - fast::div(fast::div(gm, R), R);
-	if(WANT_PHI)
-		dphi = fast::div(fast::div(J, R), R);
-}
-
-// tol / e of one error component of RK45_Next_Step_Size, +inf when the component sets no limit.
-__device__ __forceinline__ double fast_tolerance_ratio(double tol, double e, bool& good)
-{
-	const bool in = (e > 0x1p-400) & (e < 0x1p400);
-	good &= in | !(e > 0.0);
-	const double q = fast::div(tol, fast::recip(in ? e : 1.0, good));
-	return in ? q : INFINITY;
-}
-
 // Runge-Kutta-Fehlberg 4(5) coefficients of src/Simulation_Trajectory.cpp:1492-1540: stage
 // weights a[i][j] (stage i from the slopes of stages j < i) and the 4th / 5th order weights.
 // Zero weights are absent from the reference's sums and are skipped here.
@@ -808,83 +786,144 @@ static __device__ __noinline__ int rk45_attempt_ieee(const DevSolar& S, Prop& p,
 	}
 }
 
-// The attempt with the six stages written out and the straight-line division and square root of
-// dms_fastmath.cuh: no branch before its accept / retry decision.  The radius of stage j needs
-// the slopes of stages up to j - 2 only, so the compiler overlaps stages 0 and 1, 2 and 3, 4 and 5,
-// which is what a lane that runs alone needs; with every lane busy it executes about 30 % fewer
-// instructions than a loop over the stages with IEEE operations.  The step-size factor is
+// Row j: the weights of slope j in the stages j + 1 ... 5 (0 beyond), then in the 4th and 5th order
+// solutions.
+__constant__ double RKF_SLOPE[6][8] = {
+	{1.0 / 4.0, 3.0 / 32.0, 1932.0 / 2197.0, 439.0 / 216.0, -(8.0 / 27.0), 25.0 / 216.0, 16.0 / 135.0, 0.0},
+	{9.0 / 32.0, -(7200.0 / 2197.0), -8.0, 2.0, 0.0, 0.0, 0.0, 0.0},
+	{7296.0 / 2197.0, 3680.0 / 513.0, -(3544.0 / 2565.0), 0.0, 0.0, 1408.0 / 2565.0, 6656.0 / 12825.0, 0.0},
+	{-(845.0 / 4104.0), 1859.0 / 4104.0, 0.0, 0.0, 0.0, 2197.0 / 4104.0, 28561.0 / 56430.0, 0.0},
+	{-(11.0 / 40.0), 0.0, 0.0, 0.0, 0.0, -(1.0 / 5.0), -(9.0 / 50.0), 0.0},
+	{0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 2.0 / 55.0, 0.0}};
+
+// One attempt with the straight-line division and square root of dms_fastmath.cuh.  The stages are
+// one loop: every later stage's radius and radial speed, and the two solutions, are accumulators that
+// start at the step's initial value and receive weight * slope as each slope becomes known, the
+// reference's additions in its order (a weight of 0 adds a zero; x + (-a) * k equals x - a * k).  The
+// radius of stage j + 1 needs the slopes of stages up to j - 1 only, so its G*M is looked up while stage
+// j divides.  UNROLL = 1 keeps the loop (130 instructions, where six stages written out are 570): 16 warps
+// share the instruction cache and the pass of the trajectory kernel fits it.  UNROLL = 6 lets the compiler
+// overlap the stages: a lane that runs alone takes 5.25 instead of 5.80 us per step.  The step-size factor is
 // 0.84 (tol / e)^(1/4) limited by each of three components; every operation of that expression
-// rounds monotonically, so the smallest ratio gives the smallest factor and one root serves all.
+// rounds monotonically, so the component with the largest e / tol gives the smallest factor, and one
+// quotient and one root serve all (two components closer than 2^-40 are left to IEEE arithmetic).
 // When a condition of the arithmetic fails the step is repeated by rk45_attempt_ieee; the results
 // are the same bits.
+template <int UNROLL>
 __device__ __forceinline__ int rk45_attempt(const DevSolar& S, Prop& p, int inner)
 {
-	const double dt = p.time_step, R = p.radius, V = p.v_radial, PHI = p.phi, J = p.J;
+	const double dt = p.time_step, J = p.J;
 	const double JJ = J * J;
 	bool good = (S.fast_tables != 0) & ((J == 0.0) | ((J > 0x1p-200) & (J < 0x1p200)));
-	double kr0, kr1, kr2, kr3, kr4, kr5, kv0, kv1, kv2, kv3, kv4, kv5, kp0, kp2, kp3, kp4, kp5, a, b = 0.0;
-	kr0 = dt * V;
-	fast_stage<true>(S, J, JJ, R, a, b, good);
-	kv0 = dt * a;
-	kp0 = dt * b;
-	kr1 = dt * (V + kv0 / 4.0);
-	fast_stage<false>(S, J, JJ, R + kr0 / 4.0, a, b, good);
-	kv1 = dt * a;
-	kr2 = dt * (V + 3.0 / 32.0 * kv0 + 9.0 / 32.0 * kv1);
-	fast_stage<true>(S, J, JJ, R + 3.0 / 32.0 * kr0 + 9.0 / 32.0 * kr1, a, b, good);
-	kv2 = dt * a;
-	kp2 = dt * b;
-	kr3 = dt * (V + 1932.0 / 2197.0 * kv0 - 7200.0 / 2197.0 * kv1 + 7296.0 / 2197.0 * kv2);
-	fast_stage<true>(S, J, JJ, R + 1932.0 / 2197.0 * kr0 - 7200.0 / 2197.0 * kr1 + 7296.0 / 2197.0 * kr2, a, b, good);
-	kv3 = dt * a;
-	kp3 = dt * b;
-	kr4 = dt * (V + 439.0 / 216.0 * kv0 - 8.0 * kv1 + 3680.0 / 513.0 * kv2 - 845.0 / 4104.0 * kv3);
-	fast_stage<true>(S, J, JJ, R + 439.0 / 216.0 * kr0 - 8.0 * kr1 + 3680.0 / 513.0 * kr2 - 845.0 / 4104.0 * kr3, a, b, good);
-	kv4 = dt * a;
-	kp4 = dt * b;
-	kr5 = dt * (V - 8.0 / 27.0 * kv0 + 2.0 * kv1 - 3544.0 / 2565.0 * kv2 + 1859.0 / 4104.0 * kv3 - 11.0 / 40.0 * kv4);
-	fast_stage<true>(S, J, JJ, R - 8.0 / 27.0 * kr0 + 2.0 * kr1 - 3544.0 / 2565.0 * kr2 + 1859.0 / 4104.0 * kr3 - 11.0 / 40.0 * kr4, a, b, good);
-	kv5 = dt * a;
-	kp5 = dt * b;
-	const double r4 = R + 25.0 / 216.0 * kr0 + 1408.0 / 2565.0 * kr2 + 2197.0 / 4104.0 * kr3 - 1.0 / 5.0 * kr4;
-	const double v4 = V + 25.0 / 216.0 * kv0 + 1408.0 / 2565.0 * kv2 + 2197.0 / 4104.0 * kv3 - 1.0 / 5.0 * kv4;
-	const double p4 = PHI + 25.0 / 216.0 * kp0 + 1408.0 / 2565.0 * kp2 + 2197.0 / 4104.0 * kp3 - 1.0 / 5.0 * kp4;
-	const double r5 = R + 16.0 / 135.0 * kr0 + 6656.0 / 12825.0 * kr2 + 28561.0 / 56430.0 * kr3 - 9.0 / 50.0 * kr4 + 2.0 / 55.0 * kr5;
-	const double v5 = V + 16.0 / 135.0 * kv0 + 6656.0 / 12825.0 * kv2 + 28561.0 / 56430.0 * kv3 - 9.0 / 50.0 * kv4 + 2.0 / 55.0 * kv5;
-	const double p5 = PHI + 16.0 / 135.0 * kp0 + 6656.0 / 12825.0 * kp2 + 28561.0 / 56430.0 * kp3 - 9.0 / 50.0 * kp4 + 2.0 / 55.0 * kp5;
+	double R0 = p.radius, R1 = R0, R2 = R0, R3 = R0, R4 = R0, R5 = R0;
+	double V0 = p.v_radial, V1 = V0, V2 = V0, V3 = V0, V4 = V0, V5 = V0;
+	double r4 = R0, v4 = V0, p4 = p.phi, r5 = R0, v5 = V0, p5 = p4;
+	double gm = solar_gm_fast(S, R0);
+#pragma unroll UNROLL
+	for(int j = 0; j < 6; j++)
+	{
+		const double* w = RKF_SLOPE[j];
+		const double r = R0, kr = dt * V0;
+		R0 = R1 + w[0] * kr;
+		R1 = R2 + w[1] * kr;
+		R2 = R3 + w[2] * kr;
+		R3 = R4 + w[3] * kr;
+		R4 = R5 + w[4] * kr;
+		r4 = r4 + w[5] * kr;
+		r5 = r5 + w[6] * kr;
+		const double gm_next = solar_gm_fast(S, R0);
+		// dv/dt = J*J/r/r/r - gm/r/r and dphi/dt = J/r/r, each division rounded as the reference rounds
+		// it; the quotients share one reciprocal.  A radius below 1 km (where the reference clamps it) or
+		// not finite hands the attempt to IEEE arithmetic.
+		good &= fast::in_radius_range(r);
+		const fast::Recip D = fast::recip(r, good);
+		const double kv = dt * (fast::div(fast::div(fast::div(JJ, D), D), D) - fast::div(fast::div(gm, D), D));
+		const double kp = dt * fast::div(fast::div(J, D), D);
+		V0 = V1 + w[0] * kv;
+		V1 = V2 + w[1] * kv;
+		V2 = V3 + w[2] * kv;
+		V3 = V4 + w[3] * kv;
+		V4 = V5 + w[4] * kv;
+		v4 = v4 + w[5] * kv;
+		v5 = v5 + w[6] * kv;
+		p4 = p4 + w[5] * kp;
+		p5 = p5 + w[6] * kp;
+		gm = gm_next;
+	}
 	const double e0 = fabs(r5 - r4), e1 = fabs(v5 - v4), e2 = fabs(p5 - p4);
-	// RK45_Next_Step_Size (src/Simulation_Trajectory.cpp:477-502): a ratio of 10^6 or more already
-	// gives more than the largest factor
-	double ratio = 1.0e6;
-	const double q0 = fast_tolerance_ratio(DMS_RK45_TOL_R_KM, e0, good);
-	const double q1 = fast_tolerance_ratio(DMS_RK45_TOL_V_KMS, e1, good);
-	const double q2 = fast_tolerance_ratio(DMS_RK45_TOL_PHI, e2, good);
-	ratio = q0 < ratio ? q0 : ratio;
-	ratio = q1 < ratio ? q1 : ratio;
-	ratio = q2 < ratio ? q2 : ratio;
+	// RK45_Next_Step_Size (src/Simulation_Trajectory.cpp:477-502)
+	static_assert(DMS_RK45_TOL_R_KM == 1.0, "the radial error is its own ratio");
+	const double m1 = e1 * (1.0 / DMS_RK45_TOL_V_KMS), m2 = e2 * (1.0 / DMS_RK45_TOL_PHI);
+	double e = e0, tol = DMS_RK45_TOL_R_KM, m = e0, next = m1;
+	if(m1 > m)
+	{
+		next = m;
+		m = m1;
+		e = e1;
+		tol = DMS_RK45_TOL_V_KMS;
+	}
+	if(m2 > m)
+	{
+		next = m;
+		m = m2;
+		e = e2;
+		tol = DMS_RK45_TOL_PHI;
+	}
+	else
+		next = m2 > next ? m2 : next;
+	// m < 1e-7 gives more than the largest factor whatever the component
+	const bool small = m < 1.0e-7;
+	good &= (m < 0x1p400) & (small | (next < m * (1.0 - 0x1p-40))) & (e0 < INFINITY) & (e1 < INFINITY) & (e2 < INFINITY);
+	const double ratio = fast::div(tol, fast::recip(small ? 1.0e-8 : e, good));
 	double factor = 0.84 * fast::sqrt(fast::sqrt(ratio, good), good);
-	factor = factor > DMS_RK45_MAX_STEP_FACTOR ? DMS_RK45_MAX_STEP_FACTOR : factor;
+	factor = (factor > DMS_RK45_MAX_STEP_FACTOR) | small ? DMS_RK45_MAX_STEP_FACTOR : factor;
 	factor = factor < DMS_RK45_MIN_STEP_FACTOR ? DMS_RK45_MIN_STEP_FACTOR : factor;
-	// a non-finite error has cleared `good` or set no limit; dt is finite and positive (sanitized_step)
+	// dt is finite and positive (sanitized_step)
 	const double grown = factor * dt;
 	const double new_step = grown < DMS_RK45_ABS_MAX_STEP_S ? grown : DMS_RK45_ABS_MAX_STEP_S;
 	const bool within = (e0 <= DMS_RK45_TOL_R_KM) & (e1 <= DMS_RK45_TOL_V_KMS) & (e2 <= DMS_RK45_TOL_PHI);
-	good &= (e0 < INFINITY) & (e1 < INFINITY) & (e2 < INFINITY) & (grown > 0.0);
+	// the forced acceptance at the smallest step or the last retry is rare and left to it as well
+	good &= (grown > 0.0) & (within | ((new_step >= DMS_RK45_ABS_MIN_STEP_S) & (inner < DMS_RK45_MAX_INNER_RETRIES)));
 	if(!good)
 		return rk45_attempt_ieee(S, p, inner);
-	if(within)
-	{
-		p.time = p.time + dt;
-		p.radius = r4 < 0.0 ? 0.0 : r4;
-		p.v_radial = v4;
-		p.phi = p4;
-		p.time_step = new_step;
-		return RK_ACCEPTED;
-	}
-	if(new_step < DMS_RK45_ABS_MIN_STEP_S || inner >= DMS_RK45_MAX_INNER_RETRIES)
-		return rk45_attempt_ieee(S, p, inner);  // the forced acceptance (rare)
 	p.time_step = new_step;
-	return RK_RETRY;
+	if(!within)
+		return RK_RETRY;
+	p.time = p.time + dt;
+	p.radius = r4 < 0.0 ? 0.0 : r4;
+	p.v_radial = v4;
+	p.phi = p4;
+	return RK_ACCEPTED;
+}
+
+// dms_sincos for |x| < 2^20: the same operations, the quadrant from the bits of the rounded quotient
+// instead of a conversion and a four-way branch.
+__device__ __forceinline__ void sincos_fast(double x, double& s, double& c)
+{
+	const double t = __dadd_rd(x * DMS_TWO_OVER_PI + 0.5, 6755399441055744.0);  // floor, in the low bits
+	const double k = t - 6755399441055744.0;
+	const double r = ((x - k * DMS_PIO2_1) - k * DMS_PIO2_2) - k * DMS_PIO2_3;
+	const int q = __double2loint(t);
+	const double sr = dms_sin_kernel(r), cr = dms_cos_kernel(r);
+	const double a = (q & 1) ? cr : sr, b = (q & 1) ? sr : cr;
+	s = (q & 2) ? -a : a;
+	c = ((q + 1) & 2) ? -b : b;
+}
+
+// sqrt() out of line: the fallback of fast::sqrt.
+static __device__ __noinline__ double sqrt_general(double x) { return sqrt(x); }
+
+// sqrt of two values at once, without a branch unless a certificate fails.
+__device__ __forceinline__ void sqrt2(double a, double b, double& ra, double& rb)
+{
+	bool ok = true;
+	ra = fast::sqrt(a, ok);
+	rb = fast::sqrt(b, ok);
+	if(!ok)
+	{
+		ra = sqrt_general(a);
+		rb = sqrt_general(b);
+	}
 }
 
 __device__ __forceinline__ double prop_radius(const Prop& p) { return p.radius < 0.0 ? 0.0 : p.radius; }

@@ -14,10 +14,10 @@
 //    ones (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000
 //    processor", IBM J. Res. Dev. 34, 1990; J.-M. Muller et al., "Handbook of Floating-Point
 //    Arithmetic", 2010, sec. 4.7).
-//  * quotient: q0 = RN(a y) is within two ulp of a / b, q1 = RN(q0 + (a - b q0) y) within one, and
-//    Markstein's theorem then gives q2 = RN(q1 + (a - b q1) y) = RN(a / b) for y = RN(1/b).
-//    Neither operand, quotient nor remainder may leave the normal range; the callers keep
-//    1 <= b < 2^100 and a = 0 or 2^-700 <= |a| <= 2^400.  A zero dividend gives +0.
+//  * quotient: with y = RN(1/b) and its residual l = (1 - b y) y, q0 = RN(a y + RN(a l)) is within one ulp of
+//    a / b, and Markstein's theorem then gives q = RN(q0 + (a - b q0) y) = RN(a / b).  Neither operand,
+//    quotient nor remainder may leave the normal range; the callers keep 1 <= b < 2^100 and a = 0 or
+//    2^-700 <= |a| <= 2^400.  A zero dividend gives +0.
 //  * square root: Goldschmidt iterations from rsqrt.approx.ftz.f64 and Markstein's correction step
 //    s = RN(g + (x - g^2) h), with a certificate instead of a theorem: the rounding error of that
 //    last sum, which is exactly representable, must stay below half the spacing of the doubles
@@ -47,11 +47,11 @@ __device__ __forceinline__ double rsqrt_approx(double x)
 	return y;
 }
 
-// RN(1/b), shared by every quotient with divisor b.  `ok` is cleared when the significand of b
-// may be all ones (its low word is: one divisor in 2^32).
+// RN(1/b) and its residual, shared by every quotient with divisor b.  `ok` is cleared when the
+// significand of b may be all ones (its low word is: one divisor in 2^32).
 struct Recip
 {
-	double b, y;
+	double b, y, l;
 };
 
 __device__ __forceinline__ Recip recip(double b, bool& ok)
@@ -64,6 +64,7 @@ __device__ __forceinline__ Recip recip(double b, bool& ok)
 	y = __fma_rn(y, e, y);
 	e = __fma_rn(-b, y, 1.0);
 	r.y = __fma_rn(y, e, y);
+	r.l = __dmul_rn(__fma_rn(-b, r.y, 1.0), r.y);
 	ok &= __double2loint(b) != -1;
 	return r;
 }
@@ -71,15 +72,24 @@ __device__ __forceinline__ Recip recip(double b, bool& ok)
 // RN(a / b) for operands in the range above.
 __device__ __forceinline__ double div(double a, const Recip& d)
 {
-	double q = __dmul_rn(a, d.y);
-	double r = __fma_rn(-d.b, q, a);
-	q = __fma_rn(r, d.y, q);
-	r = __fma_rn(-d.b, q, a);
-	return __fma_rn(r, d.y, q);
+	const double q = __fma_rn(a, d.y, __dmul_rn(a, d.l));
+	return __fma_rn(__fma_rn(-d.b, q, a), d.y, q);
 }
 
-// RN(a / b) for a constant divisor: its correctly rounded reciprocal is formed at compile time.
-__device__ __forceinline__ double div_const(double a, double b) { return div(a, Recip{b, 1.0 / b}); }
+// RN(a / b) for a constant divisor with the residual l of its correctly rounded reciprocal.
+__device__ __forceinline__ double div_const(double a, double b)
+{
+	const double y = 1.0 / b;
+	const double q = __dmul_rn(a, y);
+	const double q1 = __fma_rn(__fma_rn(-b, q, a), y, q);
+	return __fma_rn(__fma_rn(-b, q1, a), y, q1);
+}
+
+// Whether 1 <= x < 2^100, from the exponent alone.
+__device__ __forceinline__ bool in_radius_range(double x)
+{
+	return static_cast<unsigned int>(__double2hiint(x)) - 0x3ff00000u < 100u << 20;
+}
 
 // RN(sqrt(x)) when ok stays set.
 __device__ __forceinline__ double sqrt(double x, bool& ok)

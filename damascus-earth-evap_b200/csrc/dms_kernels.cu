@@ -52,6 +52,8 @@ static __device__ __noinline__ int end_at_propagator(StrictLane& L, int reason)
 	return PH_FINAL;
 }
 
+static __device__ __noinline__ double div_general(double a, double b) { return a / b; }
+
 // The bounds of a step that starts at or outside the surface.
 static __device__ __noinline__ double outside_step(const StrictLane& L, double r, double step, double boundary)
 {
@@ -102,7 +104,10 @@ __device__ __forceinline__ int step_begin(const RunParams& R, const DevPoint* __
 		// the quotient is formed only where it can be the smaller one
 		if(rate * step * (1.0 + 0x1p-50) > tau_limit)
 		{
-			const double lim = tau_limit / rate;
+			bool ok = (rate > 0x1p-200) & (rate < 0x1p100);
+			double lim = fast::div(tau_limit, fast::recip(rate, ok));
+			if(!ok)
+				lim = div_general(tau_limit, rate);
 			step = lim < step ? lim : step;
 		}
 	}
@@ -131,18 +136,18 @@ static __device__ __noinline__ void event_and_speed_general(const Prop& p, Event
 
 __device__ __forceinline__ void event_and_speed(const Prop& p, Event& e, double& speed)
 {
-	bool ok = (p.J > 0x1p-200) & (p.J < 0x1p200) & (p.radius >= 1.0) & (p.radius < 0x1p100) & (p.radial_mode == 0);
+	bool ok = (p.J > 0x1p-200) & (p.J < 0x1p200) & fast::in_radius_range(p.radius) & (p.radial_mode == 0) & (fabs(p.phi) < 0x1p20);
 	const fast::Recip R = fast::recip(p.radius, ok);
+	// prop_speed and prop_event with the quotients by the radius sharing its reciprocal
+	speed = fast::sqrt(p.v_radial * p.v_radial + fast::div(fast::div(p.J * p.J, R), R), ok);
 	if(!ok)
 	{
 		event_and_speed_general(p, e, speed);
 		return;
 	}
-	// prop_speed and prop_event with the quotients by the radius sharing its reciprocal
-	speed = sqrt(p.v_radial * p.v_radial + fast::div(fast::div(p.J * p.J, R), R));
 	const double safe = p.radius;
 	double sp, cp;
-	dms_sincos(p.phi, &sp, &cp);
+	sincos_fast(p.phi, sp, cp);
 	const double vt = fast::div(p.J, R);
 	const double vx = p.v_radial * cp - vt * sp;
 	const double vy = p.v_radial * sp + vt * cp;
@@ -171,21 +176,12 @@ __device__ __forceinline__ double rate_inside(const DevSolar& S, const DevPoint*
 		return rate_total_general(S, P, r, v);  // no grid, a speed beyond it or a NaN
 	const double rc = r * __ldg(&P->grid_inv_r), vc = v * __ldg(&P->grid_inv_v);
 	const unsigned int N = static_cast<unsigned int>(__ldg(&P->grid_n));
-	double whole;
-	unsigned int ri = fast::floor_index(rc, whole);
-	double rf = rc - whole;
-	if(ri > N - 2)
-	{
-		ri = N - 2;
-		rf = rc - static_cast<double>(ri);
-	}
-	unsigned int vi = fast::floor_index(vc, whole);
-	double vf = vc - whole;
-	if(vi > N - 2)
-	{
-		vi = N - 2;
-		vf = vc - static_cast<double>(vi);
-	}
+	const double last = __ldg(&P->grid_last);  // N - 2
+	double wr, wv;
+	unsigned int ri = fast::floor_index(rc, wr), vi = fast::floor_index(vc, wv);
+	ri = ri > N - 2 ? N - 2 : ri;
+	vi = vi > N - 2 ? N - 2 : vi;
+	const double rf = rc - (wr > last ? last : wr), vf = vc - (wv > last ? last : wv);
 	DMS_CHECK_INDEX(ri, 0u, N - 1, BOUNDS_GRID);
 	DMS_CHECK_INDEX(vi, 0u, N - 1, BOUNDS_GRID);
 	const double* g = reinterpret_cast<const double*>(__ldg(reinterpret_cast<const unsigned long long*>(&P->grid))) + static_cast<size_t>(ri) * N + vi;
@@ -207,7 +203,8 @@ __device__ __forceinline__ double piece_rate(const DevSolar& S, const DevPoint* 
 	const double x = ax.x + f * (bx.x - ax.x), vx = av.x + f * (bv.x - av.x);
 	const double y = ax.y + f * (bx.y - ax.y), vy = av.y + f * (bv.y - av.y);
 	const double z = ax.z + f * (bx.z - ax.z), vz = av.z + f * (bv.z - av.z);
-	double r = sqrt(x * x + y * y + z * z), v = sqrt(vx * vx + vy * vy + vz * vz);
+	double r, v;
+	sqrt2(x * x + y * y + z * z, vx * vx + vy * vy + vz * vz, r, v);
 	r = next ? ra : r;
 	v = next ? va : v;
 	return rate_inside(S, P, r, v);
@@ -221,34 +218,32 @@ struct Depth
 	bool invalid;
 };
 
-// Adds piece boundary i of `pieces` (2 or 4) at fraction f with its rate to the sums of
-// Build_Optical_Depth_Pieces (src/Simulation_Trajectory.cpp:347-414), in the reference's order.
+// Adds piece boundary i at fraction f with its rate to the sums of Build_Optical_Depth_Pieces
+// (src/Simulation_Trajectory.cpp:347-414), in the reference's order.  The two-piece estimate is over
+// [0, 2] and [2, 4] of four pieces; with two pieces (Capture mode) it is the sum itself and not used.
 struct DepthSums
 {
-	double f_prev, r_prev, f_0, r_0, f_2, r_2, tau2_a;
-	__device__ __forceinline__ void add(Depth& d, int i, int pieces, double f, double rate, double dt)
+	double f_prev, r_prev, f_0, r_0;
+	__device__ __forceinline__ void add(Depth& d, int i, double f, double rate, double dt)
 	{
-		d.invalid |= !isfinite(rate) | (rate < 0.0);
-		if(i > 0 && f > f_prev)
-			d.dtau += 0.5 * (r_prev + rate) * (dt * (f - f_prev));
-		if(pieces >= 4)
+		d.invalid |= !(rate >= 0.0) | !(rate < INFINITY);
+		if(i == 0)
 		{
-			if(i == 0)
+			f_0 = f;
+			r_0 = rate;
+			d.tau2 = 0.0;
+		}
+		else
+		{
+			if(f > f_prev)
+				d.dtau += 0.5 * (r_prev + rate) * (dt * (f - f_prev));
+			if((i & 1) == 0)
 			{
+				d.tau2 += 0.5 * (r_0 + rate) * (dt * (f - f_0));
 				f_0 = f;
 				r_0 = rate;
 			}
-			else if(i == 2)
-			{
-				f_2 = f;
-				r_2 = rate;
-				tau2_a = 0.5 * (r_0 + r_2) * (dt * (f_2 - f_0));
-			}
-			else if(i == 4)
-				d.tau2 = tau2_a + 0.5 * (r_2 + rate) * (dt * (f - f_2));
 		}
-		else if(i > 0)
-			d.tau2 += 0.5 * (r_prev + rate) * (dt * (f - f_prev));
 		f_prev = f;
 		r_prev = rate;
 	}
@@ -268,7 +263,7 @@ __device__ __forceinline__ void lane_depth(const RunParams& R, const DevPoint* _
 		if(i > 0 || !first_known)
 			rate = piece_rate(R.S, P, c.before.x, c.before.v, c.after.x, c.after.v, f, i > pieces, c.r_after, c.v_after);
 		if(i <= pieces)
-			sums.add(d, i, pieces, f, rate, c.dt);
+			sums.add(d, i, f, rate, c.dt);
 		else
 			d.next_rate = rate;
 	}
@@ -279,7 +274,7 @@ __device__ __forceinline__ void lane_depth(const RunParams& R, const DevPoint* _
 // lanes form one rate each, and every owner sums its own.  The same lookups with the same
 // arguments as lane_depth, so the same numbers.  A rate is a dependent chain of some 600 cycles, so
 // a warp with few finished steps is done in one chain per round instead of five.
-constexpr int COOP_SLOT = 16;    // doubles of a step handed over
+constexpr int COOP_SLOT = 18;    // doubles of a step handed over
 constexpr int COOP_SLOTS = 8;    // most steps of a round (Capture mode: 4 rates each)
 constexpr int COOP_BUFFER = COOP_SLOT * COOP_SLOTS + 32;
 __device__ __forceinline__ void warp_depth(const RunParams& R, const DevPoint* __restrict__ P, const StepCtx& c, double rate_before, bool first_known,
@@ -290,7 +285,7 @@ __device__ __forceinline__ void warp_depth(const RunParams& R, const DevPoint* _
 	const int me = threadIdx.x & 31;
 	const int rank = __popc(dm & ((1u << me) - 1u));
 	const int steps = __popc(dm);
-	const int slot_of_job = me / rates, j = me - slot_of_job * rates;
+	const int slot_of_job = pieces == 4 ? (me * 43) >> 8 : me >> 2, j = me - slot_of_job * rates;  // me / rates
 	for(int base = 0; base < steps; base += slots)
 	{
 		const int slot = rank - base;
@@ -302,18 +297,16 @@ __device__ __forceinline__ void warp_depth(const RunParams& R, const DevPoint* _
 			b[3] = c.before.v.x; b[4] = c.before.v.y; b[5] = c.before.v.z;
 			b[6] = c.after.x.x; b[7] = c.after.x.y; b[8] = c.after.x.z;
 			b[9] = c.after.v.x; b[10] = c.after.v.y; b[11] = c.after.v.z;
-			b[12] = c.s0 + 0.0; b[13] = c.s1 - c.s0;
+			b[12] = c.s0; b[13] = c.s1 - c.s0;
 			b[14] = c.r_after; b[15] = c.v_after;
+			b[16] = __longlong_as_double(reinterpret_cast<long long>(P));
 		}
-		// the point of each slot's owner
-		const int owner_lane = slot_of_job < slots && base + slot_of_job < steps ? nth_set_bit(dm, base + slot_of_job) : me;
-		const DevPoint* Po = reinterpret_cast<const DevPoint*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(P), owner_lane));
 		__syncwarp();
 		double rate = 0.0;
 		if(slot_of_job < slots && base + slot_of_job < steps)
 		{
 			const double* b = buffer + slot_of_job * COOP_SLOT;
-			rate = piece_rate(R.S, Po, mk(b[0], b[1], b[2]), mk(b[3], b[4], b[5]), mk(b[6], b[7], b[8]), mk(b[9], b[10], b[11]),
+			rate = piece_rate(R.S, reinterpret_cast<const DevPoint*>(__double_as_longlong(b[16])), mk(b[0], b[1], b[2]), mk(b[3], b[4], b[5]), mk(b[6], b[7], b[8]), mk(b[9], b[10], b[11]),
 			                  b[12] + static_cast<double>(j) * fraction * b[13], j > pieces, b[14], b[15]);
 		}
 		buffer[COOP_SLOT * COOP_SLOTS + me] = rate;
@@ -323,18 +316,31 @@ __device__ __forceinline__ void warp_depth(const RunParams& R, const DevPoint* _
 			const double* q = buffer + COOP_SLOT * COOP_SLOTS + slot * rates;
 			const double span = c.s1 - c.s0;
 			DepthSums sums = {};
-			for(int i = 0; i <= pieces; i++)
-				sums.add(d, i, pieces, c.s0 + static_cast<double>(i) * fraction * span, i == 0 && first_known ? rate_before : q[i], c.dt);
+			sums.add(d, 0, c.s0, first_known ? rate_before : q[0], c.dt);
+			sums.add(d, 1, c.s0 + fraction * span, q[1], c.dt);
+			sums.add(d, 2, c.s0 + 2.0 * fraction * span, q[2], c.dt);
+			if(pieces == 4)
+			{
+				sums.add(d, 3, c.s0 + 3.0 * fraction * span, q[3], c.dt);
+				sums.add(d, 4, c.s0 + 4.0 * fraction * span, q[4], c.dt);
+			}
 			d.next_rate = q[rates - 1];
 		}
 		__syncwarp();
 	}
 }
 
+constexpr int PH_CONTINUE = -1;  // depth_reject: the step stands
+
 // A step whose optical depth exceeds the limit or whose two estimates differ too much: the step is
 // taken again, shorter (src/Simulation_Trajectory.cpp:975-1011).
-static __device__ __noinline__ int depth_reject(StrictLane& L, const Event& before, double dtau, double rel, bool reject_acc, double dt, double tau_limit)
+static __device__ __noinline__ int depth_reject(StrictLane& L, const Event& before, double dtau, double apart, double scale, bool capture_mode, double dt,
+                                                double tau_limit)
 {
+	const double rel = apart / scale;
+	const bool reject_acc = !capture_mode && rel > DMS_OPTICAL_DEPTH_REL_TOL;
+	if(!(dtau > tau_limit) && !reject_acc)
+		return PH_CONTINUE;
 	L.retries++;
 	if(L.retries > DMS_MAX_OPTICAL_DEPTH_RETRIES)
 	{
@@ -387,7 +393,7 @@ static __device__ __noinline__ void scatter_point(const DevSolar& S, const DevPo
 	accepted = interpolate_event(c.before, c.after, c.s1);
 }
 
-__device__ void commit_event(const RunParams& R, double m_dm, StrictLane& L, double2* hist, const Event& local, double r_now, double& E);
+__device__ void commit_event(const RunParams& R, double m_dm, StrictLane& L, double2* hist, const Event& local);
 
 // A step that ends at or beyond the boundary radius (src/Simulation_Trajectory.cpp:1046-1086).
 enum Boundary : int
@@ -429,8 +435,7 @@ static __device__ __noinline__ int boundary_step(const RunParams& R, double m_dm
 	L.seg_steps++;
 	L.steps++;
 	L.retries = 0;
-	double E;
-	commit_event(R, m_dm, L, hist, ev, ev_radius(ev), E);
+	commit_event(R, m_dm, L, hist, ev);
 	// reset_propagator_at_absolute_event, src/Simulation_Trajectory.cpp:814-822
 	L.cur = inbound;
 	L.cur.t += L.origin;
@@ -445,65 +450,76 @@ static __device__ __noinline__ int boundary_step(const RunParams& R, double m_dm
 	return BOUNDARY_RETURN;
 }
 
-static __device__ __noinline__ double capture_energy_general(const DevSolar& S, double m_dm, double r, double v) { return capture_energy_eV(S, m_dm, r, v); }
 static __device__ __noinline__ double solar_vesc_general(const DevSolar& S, double r) { return solar_vesc(S, r); }
 
-// commit_accepted_event (src/Simulation_Trajectory.cpp:842-874).  E receives the capture energy of the
-// committed event where the uncaptured-bound guard that follows needs its value: it is left at +1 for
-// an uncaptured particle that is clearly faster than the escape speed (only the sign matters there).
-__device__ __forceinline__ void commit_event_inline(const RunParams& R, double m_dm, StrictLane& L, double2* hist, const Event& local, double r_now, double& E)
+// drift / scale of Update_Capture_State where it can be the larger one.
+static __device__ __noinline__ void relative_drift(StrictLane& L, double drift, double scale)
 {
-	const double v2 = dot3(local.v, local.v);
-	const double v_now = sqrt(v2);
-	const double vv = v_now * v_now;
+	const double rel = drift / scale;
+	if(isfinite(rel) && rel > L.max_drift_rel)
+		L.max_drift_rel = rel;
+}
+
+// Update_Capture_State(..., allow_new_capture = false) of a captured particle and the bincount, the
+// parts of commit_accepted_event (src/Simulation_Trajectory.cpp:842-874, 640-721) at radius r and speed v.
+__device__ __forceinline__ void commit_event_inline(const RunParams& R, double m_dm, StrictLane& L, double2* hist, double t, double r, double v)
+{
+	const double vv = v * v;
 	if(!R.capture_mode)
 	{
 		if(L.prev_time >= 0.0)
-			accumulate_bincount(L, hist, L.prev_r, L.prev_v2, local.t - L.prev_time);
-		L.prev_time = local.t;
-		L.prev_r = r_now;
+			accumulate_bincount(L, hist, L.prev_r, L.prev_v2, t - L.prev_time);
+		L.prev_time = t;
+		L.prev_r = r;
 		L.prev_v2 = vv;
 	}
-	// v_esc^2 before the root of Local_Escape_Speed and its square
-	const bool table = (r_now <= DMS_RSUN_KM) & (R.S.fast_tables != 0);
-	const double w = table ? solar_vesc2_fast(R.S, r_now) : NAN;
 	if(!L.is_captured)
-	{
-		E = 1.0;
-		// outside the Sun v_esc^2 = 2 G M / r: compared without the division
-		const double have = table ? vv : vv * r_now, need = table ? w : 2 * DMS_GMSUN_KM3S2;
-		if(!((have > need * (1.0 + 0x1p-40)) & (vv < 1.0e200) & (r_now < 0x1p100)))
-			E = capture_energy_general(R.S, m_dm, r_now, v_now);
 		return;
-	}
-	// capture_energy_eV
-	const double vesc = table ? sqrt(w) : solar_vesc_general(R.S, r_now);
-	E = fast::div_const(0.5 * m_dm * fast::div_const(vv - vesc * vesc, DMS_C_KMS * DMS_C_KMS), 1.0e-9);
-	if(isfinite(L.free_flight_E))
-	{
-		const double drift = fabs(E - L.free_flight_E);
-		if(isfinite(drift))
-		{
-			if(drift > L.max_drift_eV)
-				L.max_drift_eV = drift;
-			const double ref = fabs(L.free_flight_E);
-			const double scale = ref > DMS_FREE_ENERGY_DRIFT_REL_E_SCALE_EV ? ref : DMS_FREE_ENERGY_DRIFT_REL_E_SCALE_EV;
-			// the quotient is formed only where it can be the larger one
-			if(drift * (1.0 + 0x1p-50) >= L.max_drift_rel * scale)
-			{
-				const double rel = drift / scale;
-				if(isfinite(rel) && rel > L.max_drift_rel)
-					L.max_drift_rel = rel;
-			}
-		}
-	}
 	if(L.bound_state)
-		L.t_last_bound = local.t + L.origin;
+		L.t_last_bound = t + L.origin;
+	if(!isfinite(L.free_flight_E))
+		return;
+	// capture_energy_eV
+	bool ok = (r <= DMS_RSUN_KM) & (R.S.fast_tables != 0);
+	double vesc = fast::sqrt(ok ? solar_vesc2_fast(R.S, r) : 1.0, ok);
+	if(!ok)
+		vesc = solar_vesc_general(R.S, r);
+	const double E = fast::div_const(0.5 * m_dm * fast::div_const(vv - vesc * vesc, DMS_C_KMS * DMS_C_KMS), 1.0e-9);
+	const double drift = fabs(E - L.free_flight_E);
+	if(drift < INFINITY)
+	{
+		if(drift > L.max_drift_eV)
+			L.max_drift_eV = drift;
+		const double ref = fabs(L.free_flight_E);
+		const double scale = ref > DMS_FREE_ENERGY_DRIFT_REL_E_SCALE_EV ? ref : DMS_FREE_ENERGY_DRIFT_REL_E_SCALE_EV;
+		if(drift * (1.0 + 0x1p-50) >= L.max_drift_rel * scale)
+			relative_drift(L, drift, scale);
+	}
 }
 
-__device__ __noinline__ void commit_event(const RunParams& R, double m_dm, StrictLane& L, double2* hist, const Event& local, double r_now, double& E)
+// abort_if_uncaptured_bound on the committed event, src/Simulation_Trajectory.cpp:767-778, 1108: whether
+// its capture energy is not finite and >= 0, whose sign is that of v^2 - v_esc^2.  r and v may be a
+// rounding error off (the propagator's): what is not clearly faster than the escape speed is decided
+// with the event's own radius and speed.
+static __device__ __noinline__ bool not_free_general(const DevSolar& S, double m_dm, const Event& e)
 {
-	commit_event_inline(R, m_dm, L, hist, local, r_now, E);
+	const double E = capture_energy_eV(S, m_dm, ev_radius(e), ev_speed(e));
+	return !(isfinite(E) && E >= 0.0);
+}
+__device__ __forceinline__ bool not_free(const RunParams& R, double m_dm, const Event& e, double r, double v)
+{
+	const bool inside = r <= DMS_RSUN_KM;
+	const double vv = v * v;
+	// outside the Sun v_esc^2 = 2 G M / r, compared without the division
+	const double have = inside ? vv : vv * r;
+	const double need = inside ? solar_vesc2_fast(R.S, r) : 2 * DMS_GMSUN_KM3S2;
+	const bool clear = (have > need * (1.0 + 0x1p-40)) & (vv < 1.0e200) & (r < 0x1p100) & (R.S.fast_tables != 0);
+	return clear ? false : not_free_general(R.S, m_dm, e);
+}
+
+__device__ __noinline__ void commit_event(const RunParams& R, double m_dm, StrictLane& L, double2* hist, const Event& local)
+{
+	commit_event_inline(R, m_dm, L, hist, local.t, ev_radius(local), ev_speed(local));
 }
 
 // Steps of a warp whose depths are formed by the whole warp rather than by each lane: one round of
@@ -512,6 +528,7 @@ __device__ __noinline__ void commit_event(const RunParams& R, double m_dm, Stric
 constexpr int COOP_MAX_STEPS = 15;
 
 // One pass for every lane of the warp (all 32 call it); returns the lane's next phase.
+template <int UNROLL>
 __device__ __forceinline__ int strict_step(const RunParams& R, const DevPoint* __restrict__ P, double m_dm, StrictLane& L, double2* hist, int phase,
                                            double* buffer)
 {
@@ -528,7 +545,7 @@ __device__ __forceinline__ int strict_step(const RunParams& R, const DevPoint* _
 	{
 		q = L.pr;
 		L.rk_inner++;
-		const int rk = rk45_attempt(R.S, q, L.rk_inner);
+		const int rk = rk45_attempt<UNROLL>(R.S, q, L.rk_inner);
 		if(rk == RK_RETRY)
 			L.pr.time_step = q.time_step;
 		else
@@ -589,14 +606,12 @@ __device__ __forceinline__ int strict_step(const RunParams& R, const DevPoint* _
 	if(interior)
 	{
 		const double scale = d.dtau > DMS_OPTICAL_DEPTH_ABS_TOL ? d.dtau : DMS_OPTICAL_DEPTH_ABS_TOL;
-		const double apart = fabs(d.dtau - d.tau2);
-		const bool reject_depth = d.dtau > tau_limit;
-		if(reject_depth || apart > (DMS_OPTICAL_DEPTH_REL_TOL * (1.0 - 0x1p-50)) * scale)
+		const double apart = capture_mode ? 0.0 : fabs(d.dtau - d.tau2);
+		if((d.dtau > tau_limit) | (!capture_mode & (apart > (DMS_OPTICAL_DEPTH_REL_TOL * (1.0 - 0x1p-50)) * scale)))
 		{
-			const double rel = apart / scale;
-			const bool reject_acc = !capture_mode && rel > DMS_OPTICAL_DEPTH_REL_TOL;
-			if(reject_depth || reject_acc)
-				return depth_reject(L, c.before, d.dtau, rel, reject_acc, c.dt, tau_limit);
+			const int rejected = depth_reject(L, c.before, d.dtau, apart, scale, capture_mode != 0, c.dt, tau_limit);
+			if(rejected != PH_CONTINUE)
+				return rejected;
 		}
 		if(d.dtau >= L.tau)
 		{
@@ -618,12 +633,15 @@ __device__ __forceinline__ int strict_step(const RunParams& R, const DevPoint* _
 	L.seg_steps++;
 	L.steps++;
 	L.retries = 0;
-	const double r_now = ev_radius(accepted);
-	double E;
-	commit_event_inline(R, m_dm, L, hist, accepted, r_now, E);
-	// abort_if_uncaptured_bound on the committed event, src/Simulation_Trajectory.cpp:767-778, 1108
-	const bool bound = !L.is_captured && !(isfinite(E) && E >= 0.0);
-	if(bound | scattering | (boundary == BOUNDARY_ESCAPE))
+	const bool plain = !scattering && boundary == BOUNDARY_INSIDE;
+	// the committed event's own radius and speed; in Capture mode a plain step only asks whether the
+	// particle is still free, which the propagator's decide
+	double r_now = c.r_after, v_now = c.v_after;
+	if(!capture_mode | L.is_captured | !plain)
+		sqrt2(dot3(accepted.x, accepted.x), dot3(accepted.v, accepted.v), r_now, v_now);
+	commit_event_inline(R, m_dm, L, hist, accepted.t, r_now, v_now);
+	const bool bound = !L.is_captured && not_free(R, m_dm, accepted, r_now, v_now);
+	if(bound | !plain)
 	{
 		L.cur = accepted;
 		L.cur.t += L.origin;
@@ -681,14 +699,16 @@ __global__ void __launch_bounds__(128) initial_state_kernel(const RunParams R)
 	R.init[w] = st;
 }
 
+template <bool LOCKSTEP>
 struct StrictStep
 {
+	static constexpr bool lockstep = LOCKSTEP;
 	static constexpr bool collective = true;  // the whole warp makes a pass
 	static constexpr int buffer = COOP_BUFFER;
 	__device__ __forceinline__ int operator()(const RunParams& R, const DevPoint* __restrict__ P, double m_dm, StrictLane& L, double2* hist, int phase,
 	                                          double* buffer) const
 	{
-		return strict_step(R, P, m_dm, L, hist, phase, buffer);
+		return strict_step<LOCKSTEP ? 1 : 6>(R, P, m_dm, L, hist, phase, buffer);
 	}
 	__device__ __forceinline__ double channel(const DevSolar& S, const DevPoint* __restrict__ P, int i, double dr, double T, double v, int k) const
 	{
@@ -700,9 +720,16 @@ struct StrictStep
 	}
 };
 
+// The throughput form: up to 16 warps per SM in lockstep, 128 registers each.
 __global__ void __launch_bounds__(MAX_THREADS, 1) trajectory_kernel(const RunParams R)
 {
-	lane_loop<StrictLane>(R, StrictStep());
+	lane_loop<StrictLane>(R, StrictStep<true>());
+}
+
+// The latency form: one warp per scheduler, no spills (176 registers).
+__global__ void __launch_bounds__(LATENCY_THREADS, 1) trajectory_kernel_latency(const RunParams R)
+{
+	lane_loop<StrictLane>(R, StrictStep<false>());
 }
 
 __global__ void rate_grid_kernel(const DevSolar S, const DevPoint* __restrict__ P, double* grid, int n)
@@ -868,7 +895,10 @@ void Launch_Initial_States(const RunParams& p, cudaStream_t stream)
 
 void Launch_Trajectories(const RunParams& p, int blocks, int threads, cudaStream_t stream)
 {
-	trajectory_kernel<<<blocks, threads, 0, stream>>>(p);
+	if(threads <= LATENCY_THREADS)
+		trajectory_kernel_latency<<<blocks, threads, 0, stream>>>(p);
+	else
+		trajectory_kernel<<<blocks, threads, 0, stream>>>(p);
 }
 
 void Launch_Rate_Grid(const DevSolar& S, const DevPoint* point, double* grid, int n, cudaStream_t stream)
@@ -883,22 +913,6 @@ void Launch_Rate_Query(const DevSolar& S, const DevPoint* point, int interpolate
 	const int blocks = static_cast<int>((n + threads - 1) / threads);
 	if(blocks > 0)
 		rate_query_kernel<<<blocks, threads, 0, stream>>>(S, point, interpolated, r, v, out, n);
-}
-
-int Trajectory_Max_Blocks_Per_SM(int threads)
-{
-	int n = 0;
-	if(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, trajectory_kernel, threads, 0) != cudaSuccess)
-		return 0;
-	return n;
-}
-
-int Trajectory_Kernel_Registers()
-{
-	cudaFuncAttributes a;
-	if(cudaFuncGetAttributes(&a, trajectory_kernel) != cudaSuccess)
-		return -1;
-	return a.numRegs;
 }
 
 unsigned int Take_Bounds_Status()

@@ -10,6 +10,9 @@ namespace dms
 
 // The largest block of the trajectory kernels: all 16 warps that their registers allow per SM.
 constexpr int MAX_THREADS = 512;
+// Blocks of at most this many threads run the latency form of the kernels: one warp per scheduler, so
+// the registers are not shared out among 16 warps.
+constexpr int LATENCY_THREADS = 128;
 
 // Status bits written by the kernels (device status word).
 enum : unsigned int
@@ -119,9 +122,6 @@ void Launch_Rate_Query(const DevSolar& S, const DevPoint* point, int interpolate
 // mixed-precision (batched FP32) trajectory kernel and the FP32 image of a rate grid
 void Launch_Trajectories_Mixed(const RunParams& p, int blocks, int threads, cudaStream_t stream);
 void Launch_To_Float(const double* in, float* out, size_t n, cudaStream_t stream);
-int Trajectory_Mixed_Max_Blocks_Per_SM(int threads);
-int Trajectory_Kernel_Registers();
-int Trajectory_Max_Blocks_Per_SM(int threads);
 double Measure_FP64_Peak(int sm_count, cudaStream_t stream);
 // Self-test of the certified division and square root (dms_fastmath.cuh) against IEEE on n
 // random operand pairs; out (4 device counters, zeroed by the caller) as in dms_check_certified_math.

@@ -355,8 +355,10 @@ __device__ __forceinline__ int free_step_mixed(const RunParams& R, const DevPoin
 	return PH_STEP;
 }
 
+template <bool LOCKSTEP>
 struct MixedStep
 {
+	static constexpr bool lockstep = LOCKSTEP;
 	static constexpr bool collective = false;
 	static constexpr int buffer = 0;
 	__device__ __forceinline__ int operator()(const RunParams& R, const DevPoint* __restrict__ P, double m_dm, MixedLane& L, double2* hist) const
@@ -373,9 +375,15 @@ struct MixedStep
 	}
 };
 
+// The throughput and the latency form, as in dms_kernels.cu.
 __global__ void __launch_bounds__(MAX_THREADS, 1) trajectory_kernel_mixed(const RunParams R)
 {
-	lane_loop<MixedLane>(R, MixedStep());
+	lane_loop<MixedLane>(R, MixedStep<true>());
+}
+
+__global__ void __launch_bounds__(LATENCY_THREADS, 1) trajectory_kernel_mixed_latency(const RunParams R)
+{
+	lane_loop<MixedLane>(R, MixedStep<false>());
 }
 
 __global__ void grid_to_float_kernel(const double* __restrict__ in, float* __restrict__ out, size_t n)
@@ -388,20 +396,15 @@ __global__ void grid_to_float_kernel(const double* __restrict__ in, float* __res
 
 void Launch_Trajectories_Mixed(const RunParams& p, int blocks, int threads, cudaStream_t stream)
 {
-	trajectory_kernel_mixed<<<blocks, threads, 0, stream>>>(p);
+	if(threads <= LATENCY_THREADS)
+		trajectory_kernel_mixed_latency<<<blocks, threads, 0, stream>>>(p);
+	else
+		trajectory_kernel_mixed<<<blocks, threads, 0, stream>>>(p);
 }
 
 void Launch_To_Float(const double* in, float* out, size_t n, cudaStream_t stream)
 {
 	grid_to_float_kernel<<<148 * 4, 256, 0, stream>>>(in, out, n);
-}
-
-int Trajectory_Mixed_Max_Blocks_Per_SM(int threads)
-{
-	int n = 0;
-	if(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, trajectory_kernel_mixed, threads, 0) != cudaSuccess)
-		return 0;
-	return n;
 }
 
 unsigned int Take_Bounds_Status_Mixed()

@@ -690,7 +690,7 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 	double2* hist = R.lane_hist + static_cast<size_t>(warp_id * R.lanes_per_warp + (takes_work ? in_warp : 0)) * DMS_NUM_BINS;
 	// per warp: the 64 channel rates of a scattering, or the steps and rates of Step's own lookups
 	constexpr int BUFFER = Step::buffer > DMS_NUM_TARGETS + 1 ? Step::buffer : DMS_NUM_TARGETS + 1;
-	__shared__ double coop_rates[MAX_THREADS / 32][BUFFER];
+	__shared__ double coop_rates[(Step::lockstep ? MAX_THREADS : LATENCY_THREADS) / 32][BUFFER];
 	double* rates = coop_rates[threadIdx.x >> 5];
 	// Lockstep: the warps of a block with more than one warp per scheduler make every pass together,
 	// so that an instruction fetched once serves all of them.  The block votes on its rare phases:
@@ -699,7 +699,7 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 	__shared__ int votes[2][4];
 	if(threadIdx.x < 8)
 		votes[threadIdx.x >> 2][threadIdx.x & 3] = 0;
-	bool lockstep = blockDim.x > 128;
+	bool lockstep = Step::lockstep;
 	int passes_scatter = 0, passes_final = 0;  // passes since the block's last scattering (termination) phase
 	__syncthreads();
 	Lane L;
@@ -721,7 +721,7 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 	for(uint64_t iter = 0;; iter++)
 	{
 		bool go_scatter = false, go_final = false;
-		if(lockstep)
+		if(Step::lockstep && lockstep)
 		{
 			int* v = votes[iter & 1];
 			const unsigned int b_step = __ballot_sync(FULL_WARP, phase == PH_STEP || phase == PH_FETCH || phase == PH_SEGMENT);

@@ -191,9 +191,10 @@ typedef struct
 	uint64_t max_free_steps;           /* maximum_free_time_steps */
 	double boundary_radius_rsun;       /* initial_and_final_radius / R_sun (2.0) */
 	int32_t precision;                 /* DMS_PRECISION_* */
-	uint32_t threads_per_block;        /* 32, 64, 96 or 128; 0 = chosen by the size of the launch (128
-	                                      when blocks_per_sm is given) */
-	uint32_t blocks_per_sm;            /* resident blocks per SM; 0 = as many as fit */
+	uint32_t threads_per_block;        /* 32, 64, 96 or 128: with blocks_per_sm the most lanes per SM
+	                                      (which run as one block of up to 512 threads); 0 = chosen by
+	                                      the size of the launch (128 when blocks_per_sm is given) */
+	uint32_t blocks_per_sm;            /* blocks per SM; 0 = as many as fit */
 	uint32_t queue_chunk;              /* trajectory ids a lane claims from the work queue at a time
 	                                      (1..1024); 0 = 1 */
 	uint64_t iteration_budget;         /* per-lane loop-iteration bound; 0 = default */

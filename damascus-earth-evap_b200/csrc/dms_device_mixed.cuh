@@ -226,7 +226,7 @@ __device__ __forceinline__ double capture_energy_eV_f(const DevSolar& S, const D
 		const int i = knot_index_f(S, F, rr);
 		vesc2 = __ldg(F.vesc2 + i) + (rr - __ldg(F.r + i)) * __ldg(F.vesc2_s + i);
 	}
-	const float scale = static_cast<float>(0.5 * m_dm / (DMS_C_KMS * DMS_C_KMS) / 1.0e-9);
+	const float scale = static_cast<float>(fast::div_const(fast::div_const(0.5 * m_dm, DMS_C_KMS * DMS_C_KMS), 1.0e-9));
 	return static_cast<double>(scale * (v * v - vesc2));
 }
 

@@ -703,7 +703,6 @@ template <bool LOCKSTEP>
 struct StrictStep
 {
 	static constexpr bool lockstep = LOCKSTEP;
-	static constexpr bool collective = true;  // the whole warp makes a pass
 	static constexpr int buffer = COOP_BUFFER;
 	__device__ __forceinline__ int operator()(const RunParams& R, const DevPoint* __restrict__ P, double m_dm, StrictLane& L, double2* hist, int phase,
 	                                          double* buffer) const

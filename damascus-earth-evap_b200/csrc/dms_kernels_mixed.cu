@@ -17,15 +17,309 @@ using namespace lane;
 using namespace mixed;
 using MixedLane = LaneT<PropF, EventF>;
 
-// commit_accepted_event (src/Simulation_Trajectory.cpp:842-874) for an FP32 event: bincount
-// with FP64 times, capture energy in FP64.  Returns the energy when evaluated, NaN otherwise.
-__device__ __forceinline__ double commit_event_mixed(const DevSolar& S, const DevSolarF& F, double m_dm, int capture_mode, MixedLane& L, double2* hist,
-                                                     const EventF& local)
+// The mixed-precision pass (see dms_kernels.cu for the FP64 one, whose structure this follows, and
+// dms_device_mixed.cuh for what stays FP64): the Propagate_Freely loop body,
+// src/Simulation_Trajectory.cpp:876-1116, split at the RK45 retry loop.
+
+__device__ __forceinline__ DevSolarF tables_f(const RunParams& R) { return DevSolarF{R.sf_r, R.sf_gm, R.sf_gm_s, R.sf_vesc2, R.sf_vesc2_s}; }
+
+__device__ __forceinline__ const float* grid_f(const DevPoint* __restrict__ P)
 {
+	return reinterpret_cast<const float*>(__ldg(reinterpret_cast<const unsigned long long*>(&P->grid_f)));
+}
+
+// The event, speed and scattering rate at the propagator's state, at the start of a free segment.
+static __device__ __noinline__ void fresh_state(const DevSolar& S, const DevPoint* __restrict__ P, MixedLane& L)
+{
+	if(!L.before_valid)
+		L.before = prop_event_f(L.pr);
+	L.before_valid = L.before_valid ? L.before_valid : 1;
+	const double r = prop_radius_f(L.pr);
+	L.next_speed = prop_speed_f(L.pr);
+	L.next_rate = r >= DMS_RSUN_KM ? 0.0 : rate_total_f(S, P, grid_f(P), static_cast<float>(r), static_cast<float>(L.next_speed));
+	L.next_valid = 1;
+}
+
+static __device__ __noinline__ int end_at_propagator(MixedLane& L, int reason)
+{
+	set_final(L, to_event64(prop_event_f(L.pr)), true, reason);
+	return PH_FINAL;
+}
+
+static __device__ __noinline__ double outside_step(const MixedLane& L, double r, double step, double boundary)
+{
+	const double cap = step_cap(r, L.next_speed, boundary);
+	step = step < cap ? step : cap;
+	const double vr = (r > 0.0) ? static_cast<double>(dotf(L.before.x, L.before.v)) / r : 0.0;
+	if(r > DMS_RSUN_KM && vr < 0.0)
+	{
+		const double est = (r - DMS_RSUN_KM) / (-vr);
+		if(isfinite(est) && est > 0.0)
+		{
+			const double lim = est > DMS_RK45_ABS_MIN_STEP_S ? est : DMS_RK45_ABS_MIN_STEP_S;
+			step = lim < step ? lim : step;
+		}
+	}
+	return step;
+}
+
+// Pre-step bounds (src/Simulation_Trajectory.cpp:873-927).
+__device__ __forceinline__ int mixed_begin(const RunParams& R, const DevPoint* __restrict__ P, MixedLane& L)
+{
+	if(!(L.seg_steps < R.max_free_steps))
+	{
+		if(L.before_valid == 2)  // otherwise L.cur holds the last committed event
+		{
+			L.cur = to_event64(L.before);
+			L.cur.t += L.origin;
+		}
+		L.reason = DMS_REASON_MAX_FREE_STEPS;
+		return PH_FINAL;
+	}
+	if(wall_time_exceeded(R, L))  // "before_step", src/Simulation_Trajectory.cpp:873-874
+		return end_at_propagator(L, DMS_REASON_WALL_TIME_LIMIT);
+	if(!L.next_valid)
+		fresh_state(R.S, P, L);
+	const double r = prop_radius_f(L.pr);
+	double step = sanitized_step(L.pr.time_step), rate = 0.0;
+	if(r >= DMS_RSUN_KM)
+		step = outside_step(L, r, step, R.boundary);
+	else
+	{
+		rate = L.next_rate;
+		if(!isfinite(rate) || rate < 0.0)
+			return end_at_propagator(L, DMS_REASON_NUMERICAL_FAILURE);
+		if(rate > 0.0)
+		{
+			const double tau_limit = R.capture_mode ? DMS_CAPTURE_MAX_OPTICAL_DEPTH_STEP : DMS_MAX_OPTICAL_DEPTH_STEP;
+			const float lim = static_cast<float>(tau_limit) / static_cast<float>(rate);
+			if(static_cast<double>(lim) < step)
+				step = static_cast<double>(lim);
+		}
+	}
+	L.rate_before = rate;
+	L.pr.time_step = step;
+	L.in_rk = 1;
+	L.rk_inner = 0;
+	return PH_STEP;
+}
+
+// A step as an accepted attempt leaves it.
+struct StepCtxF
+{
+	EventF before, after;
+	double r_before, r_after, v_after, dt;
+	float s0, s1;
+};
+
+static __device__ __noinline__ bool interior_interval_outside(const EventF& a, const EventF& b, double ra, double rb, float& s0, float& s1)
+{
+	return interior_interval_f(a, b, ra, rb, s0, s1);
+}
+
+// One piece-boundary rate of a step or, with `next`, the scattering rate at the state after it.
+__device__ __forceinline__ float piece_rate_f(const DevSolar& S, const DevPoint* __restrict__ P, const float* __restrict__ grid, const EventF& a,
+                                              const EventF& b, float f, bool next, float ra, float va)
+{
+	f = f < 0.0f ? 0.0f : (f > 1.0f ? 1.0f : f);
+	const float x = a.x.x + f * (b.x.x - a.x.x), vx = a.v.x + f * (b.v.x - a.v.x);
+	const float y = a.x.y + f * (b.x.y - a.x.y), vy = a.v.y + f * (b.v.y - a.v.y);
+	const float z = a.x.z + f * (b.x.z - a.x.z), vz = a.v.z + f * (b.v.z - a.v.z);
+	float r = sqrtf(fmaxf(x * x + y * y + z * z, 0.0f));
+	float v = sqrtf(fmaxf(vx * vx + vy * vy + vz * vz, 0.0f));
+	if(!next && r >= static_cast<float>(DMS_RSUN_KM))
+		return 0.0f;
+	r = next ? ra : r;
+	v = next ? va : v;
+	return rate_total_f(S, P, grid, r, v);
+}
+
+// The optical depth of a step in FP32 (at most 0.1), as in dms_kernels.cu.
+struct DepthF
+{
+	float dtau, tau2, next_rate;
+	bool invalid;
+};
+
+struct DepthSumsF
+{
+	float f_prev, r_prev, f_0, r_0;
+	__device__ __forceinline__ void add(DepthF& d, int i, float f, float rate, float dt)
+	{
+		if(!isfinite(rate) || rate < 0.0f)
+			d.invalid = true;
+		if(i == 0)
+		{
+			f_0 = f;
+			r_0 = rate;
+		}
+		else
+		{
+			if(f > f_prev)
+				d.dtau += 0.5f * (r_prev + rate) * (dt * (f - f_prev));
+			if((i & 1) == 0)
+			{
+				d.tau2 += 0.5f * (r_0 + rate) * (dt * (f - f_0));
+				f_0 = f;
+				r_0 = rate;
+			}
+		}
+		f_prev = f;
+		r_prev = rate;
+	}
+};
+
+__device__ __forceinline__ void lane_depth(const RunParams& R, const DevPoint* __restrict__ P, const StepCtxF& c, float rate_before, bool first_known,
+                                           int pieces, DepthF& d)
+{
+	const float* grid = grid_f(P);
+	const float fraction = pieces == 4 ? 0.25f : 0.5f, span = c.s1 - c.s0, dt = static_cast<float>(c.dt);
+	DepthSumsF sums = {};
+#pragma unroll 1
+	for(int i = 0; i <= pieces + 1; i++)
+	{
+		const float f = c.s0 + static_cast<float>(i) * fraction * span;
+		float rate = rate_before;
+		if(i > 0 || !first_known)
+			rate = piece_rate_f(R.S, P, grid, c.before, c.after, f, i > pieces, static_cast<float>(c.r_after), static_cast<float>(c.v_after));
+		if(i <= pieces)
+			sums.add(d, i, f, rate, dt);
+		else
+			d.next_rate = rate;
+	}
+}
+
+constexpr int COOP_SLOT_F = 18;  // floats of a step handed over (the point's address among them)
+constexpr int COOP_SLOTS_F = 8;
+constexpr int COOP_BUFFER_F = (COOP_SLOT_F * COOP_SLOTS_F + 32) / 2;  // in doubles
+__device__ __forceinline__ void warp_depth(const RunParams& R, const DevPoint* __restrict__ P, const StepCtxF& c, float rate_before, bool first_known,
+                                           int pieces, unsigned int dm, bool mine, float* buffer, DepthF& d)
+{
+	const float fraction = pieces == 4 ? 0.25f : 0.5f, dt = static_cast<float>(c.dt);
+	const int rates = pieces + 2, slots = 32 / rates;
+	const int me = threadIdx.x & 31;
+	const int rank = __popc(dm & ((1u << me) - 1u));
+	const int steps = __popc(dm);
+	const int slot_of_job = pieces == 4 ? (me * 43) >> 8 : me >> 2, j = me - slot_of_job * rates;  // me / rates
+	for(int base = 0; base < steps; base += slots)
+	{
+		const int slot = rank - base;
+		const bool owner = mine && slot >= 0 && slot < slots;
+		if(owner)
+		{
+			float* b = buffer + slot * COOP_SLOT_F;
+			b[0] = c.before.x.x; b[1] = c.before.x.y; b[2] = c.before.x.z;
+			b[3] = c.before.v.x; b[4] = c.before.v.y; b[5] = c.before.v.z;
+			b[6] = c.after.x.x; b[7] = c.after.x.y; b[8] = c.after.x.z;
+			b[9] = c.after.v.x; b[10] = c.after.v.y; b[11] = c.after.v.z;
+			b[12] = c.s0; b[13] = c.s1 - c.s0;
+			b[14] = static_cast<float>(c.r_after); b[15] = static_cast<float>(c.v_after);
+			*reinterpret_cast<const DevPoint**>(b + 16) = P;
+		}
+		__syncwarp();
+		float rate = 0.0f;
+		if(slot_of_job < slots && base + slot_of_job < steps)
+		{
+			const float* b = buffer + slot_of_job * COOP_SLOT_F;
+			const DevPoint* Po = *reinterpret_cast<const DevPoint* const*>(b + 16);
+			const EventF before{0.0, f3(b[0], b[1], b[2]), f3(b[3], b[4], b[5])}, after{0.0, f3(b[6], b[7], b[8]), f3(b[9], b[10], b[11])};
+			rate = piece_rate_f(R.S, Po, grid_f(Po), before, after, b[12] + static_cast<float>(j) * fraction * b[13], j > pieces, b[14], b[15]);
+		}
+		buffer[COOP_SLOT_F * COOP_SLOTS_F + me] = rate;
+		__syncwarp();
+		if(owner)
+		{
+			const float* q = buffer + COOP_SLOT_F * COOP_SLOTS_F + slot * rates;
+			const float span = c.s1 - c.s0;
+			DepthSumsF sums = {};
+			sums.add(d, 0, c.s0, first_known ? rate_before : q[0], dt);
+			sums.add(d, 1, c.s0 + fraction * span, q[1], dt);
+			sums.add(d, 2, c.s0 + 2.0f * fraction * span, q[2], dt);
+			if(pieces == 4)
+			{
+				sums.add(d, 3, c.s0 + 3.0f * fraction * span, q[3], dt);
+				sums.add(d, 4, c.s0 + 4.0f * fraction * span, q[4], dt);
+			}
+			d.next_rate = q[rates - 1];
+		}
+		__syncwarp();
+	}
+}
+
+// A step whose optical depth exceeds the limit or whose two estimates differ too much
+// (src/Simulation_Trajectory.cpp:975-1011).
+constexpr int PH_CONTINUE = -1;
+static __device__ __noinline__ int depth_reject(MixedLane& L, const EventF& before, float dtau_f, float tau2, bool capture_mode, double dt, double tau_limit)
+{
+	const double dtau = static_cast<double>(dtau_f);
+	const float scale = dtau_f > static_cast<float>(DMS_OPTICAL_DEPTH_ABS_TOL) ? dtau_f : static_cast<float>(DMS_OPTICAL_DEPTH_ABS_TOL);
+	const double rel = static_cast<double>(fabsf(dtau_f - tau2) / scale);
+	const bool reject_acc = !capture_mode && rel > DMS_OPTICAL_DEPTH_REL_TOL;
+	if(!(dtau > tau_limit) && !reject_acc)
+		return PH_CONTINUE;
+	L.retries++;
+	if(L.retries > DMS_MAX_OPTICAL_DEPTH_RETRIES)
+	{
+		set_final(L, to_event64(before), true, DMS_REASON_NUMERICAL_FAILURE);
+		return PH_FINAL;
+	}
+	double factor = DMS_RK45_MAX_STEP_FACTOR;
+	if(dtau > tau_limit && dtau > 0.0 && 0.8 * tau_limit / dtau < factor)
+		factor = 0.8 * tau_limit / dtau;
+	if(reject_acc && rel > 0.0 && 0.8 * sqrt(DMS_OPTICAL_DEPTH_REL_TOL / rel) < factor)
+		factor = 0.8 * sqrt(DMS_OPTICAL_DEPTH_REL_TOL / rel);
+	if(factor > 1.0) factor = 1.0;
+	if(factor < DMS_RK45_MIN_STEP_FACTOR) factor = DMS_RK45_MIN_STEP_FACTOR;
+	L.pr.time_step = sanitized_step(factor * dt);
+	return PH_STEP;
+}
+
+// The scattering point (src/Simulation_Trajectory.cpp:1013-1044), the boundary rates formed again.
+static __device__ __noinline__ void scatter_point(const DevSolar& S, const DevPoint* __restrict__ P, const StepCtxF& c, float rate_before, bool first_known,
+                                                  bool depth, int pieces, double remaining, EventF& accepted)
+{
+	if(depth)
+	{
+		const float* grid = grid_f(P);
+		const float fraction = pieces == 4 ? 0.25f : 0.5f, span = c.s1 - c.s0;
+		float f_prev = c.s0, r_prev = rate_before;
+		if(!first_known)
+			r_prev = rate_at_fraction_f(S, P, grid, c.before, c.after, f_prev);
+#pragma unroll 1
+		for(int k = 1; k <= pieces; k++)
+		{
+			const float f = c.s0 + static_cast<float>(k) * fraction * span;
+			const float rate = rate_at_fraction_f(S, P, grid, c.before, c.after, f);
+			if(f > f_prev)
+			{
+				const double pdt = c.dt * static_cast<double>(f - f_prev);
+				const double ptau = 0.5 * static_cast<double>(r_prev + rate) * pdt;
+				if(ptau >= remaining)
+				{
+					const double lf = solve_linear_rate(r_prev, rate, pdt, remaining);
+					accepted = interpolate_event_f(c.before, c.after, f_prev + static_cast<float>(lf) * (f - f_prev));
+					return;
+				}
+				remaining -= ptau;
+			}
+			f_prev = f;
+			r_prev = rate;
+		}
+	}
+	accepted = interpolate_event_f(c.before, c.after, c.s1);
+}
+
+// commit_accepted_event (src/Simulation_Trajectory.cpp:842-874) for an FP32 event: bincount
+// with FP64 times, capture energy of the drift statistics and the uncaptured-bound guard in FP32
+// (m_dm / (2 c^2) in FP64 first).  Returns the energy when evaluated, NaN otherwise.
+__device__ __forceinline__ double commit_event_mixed(const RunParams& R, double m_dm, MixedLane& L, double2* hist, const EventF& local)
+{
+	if(R.capture_mode && !L.is_captured)
+		return NAN;
 	const float rf = normf(local.x), vf = normf(local.v);
 	const double r_now = static_cast<double>(rf);
 	const double v_now = static_cast<double>(vf);
-	if(!capture_mode)
+	if(!R.capture_mode)
 	{
 		if(L.prev_time >= 0.0)
 			accumulate_bincount(L, hist, L.prev_r, L.prev_v2, local.t - L.prev_time);
@@ -34,9 +328,8 @@ __device__ __forceinline__ double commit_event_mixed(const DevSolar& S, const De
 		L.prev_v2 = v_now * v_now;
 	}
 	const double t_abs = local.t + L.origin;
-	if(capture_mode && !L.is_captured)
-		return NAN;
-	const double E = capture_energy_eV_f(S, F, m_dm, rf, vf);
+	const DevSolarF F = tables_f(R);
+	const double E = capture_energy_eV_f(R.S, F, m_dm, rf, vf);
 	if(L.is_captured && isfinite(L.free_flight_E))
 	{
 		const double drift = fabs(E - L.free_flight_E);
@@ -44,314 +337,241 @@ __device__ __forceinline__ double commit_event_mixed(const DevSolar& S, const De
 			L.max_drift_eV = drift;
 		const double ref = fabs(L.free_flight_E);
 		const double scale = ref > DMS_FREE_ENERGY_DRIFT_REL_E_SCALE_EV ? ref : DMS_FREE_ENERGY_DRIFT_REL_E_SCALE_EV;
-		const double rel = drift / scale;
-		if(isfinite(rel) && rel > L.max_drift_rel)
-			L.max_drift_rel = rel;
+		// the quotient is formed only where it can be the larger one
+		if(drift * (1.0 + 0x1p-50) >= L.max_drift_rel * scale)
+		{
+			const double rel = drift / scale;
+			if(isfinite(rel) && rel > L.max_drift_rel)
+				L.max_drift_rel = rel;
+		}
 	}
 	if(L.bound_state && L.is_captured)
 		L.t_last_bound = t_abs;
 	return E;
 }
+static __device__ __noinline__ void commit_event_general(const RunParams& R, double m_dm, MixedLane& L, double2* hist, const EventF& local)
+{
+	commit_event_mixed(R, m_dm, L, hist, local);
+}
 
-// Mixed-precision form of the free step (see dms_kernels.cu for the FP64 form and
-// dms_device_mixed.cuh for what stays FP64).  Propagate_Freely loop body,
-// src/Simulation_Trajectory.cpp:876-1116, split at the
-// RK45 retry loop: when no step is in progress the pre-step bounds are applied and a step is
-// opened; every pass makes one RK45 attempt; only a finished step runs the optical-depth,
-// boundary and commit logic.  Returns the next phase of the lane.
-__device__ __forceinline__ int free_step_mixed(const RunParams& R, const DevPoint* __restrict__ P, double m_dm, MixedLane& L, double2* hist)
+// abort_if_uncaptured_bound (src/Simulation_Trajectory.cpp:767-778, 1108) in Capture mode, where the commit
+// forms no energy: the FP64 energy of the event decides unless the FP32 speeds are far apart.
+static __device__ __noinline__ bool not_free_general(const DevSolar& S, double m_dm, const EventF& e)
+{
+	const Event d = to_event64(e);
+	const double E = capture_energy_eV(S, m_dm, ev_radius(d), ev_speed(d));
+	return !(isfinite(E) && E >= 0.0);
+}
+__device__ __forceinline__ bool not_free(const RunParams& R, double m_dm, const EventF& e)
+{
+	const float r2 = dotf(e.x, e.x), v2 = dotf(e.v, e.v);
+	const float r = sqrtf(r2);
+	const bool inside = r < static_cast<float>(DMS_RSUN_KM * (1.0 - 1.0e-6));
+	const DevSolarF F = tables_f(R);
+	float need = static_cast<float>(2.0 * DMS_GMSUN_KM3S2);
+	if(inside)
+	{
+		const int i = knot_index_f(R.S, F, r);
+		need = __ldg(F.vesc2 + i) + (r - __ldg(F.r + i)) * __ldg(F.vesc2_s + i);
+	}
+	const float have = inside ? v2 : v2 * r;
+	const bool clear = (have > need * 1.001f) & (v2 < 1.0e12f) & (r < 1.0e12f);
+	return clear ? false : not_free_general(R.S, m_dm, e);
+}
+
+// A step that ends at or beyond the boundary radius (src/Simulation_Trajectory.cpp:1046-1086).
+enum Boundary : int
+{
+	BOUNDARY_INSIDE = 0,
+	BOUNDARY_ESCAPE = 1,
+	BOUNDARY_RETURN = 2,
+	BOUNDARY_FAILURE = 3,
+};
+static __device__ __noinline__ int boundary_step(const RunParams& R, double m_dm, MixedLane& L, double2* hist, const StepCtxF& c, EventF& accepted)
 {
 	const DevSolar& S = R.S;
-	const DevSolarF F{R.sf_r, R.sf_gm, R.sf_gm_s, R.sf_vesc2, R.sf_vesc2_s};
-	const float* grid = reinterpret_cast<const float*>(__ldg(reinterpret_cast<const unsigned long long*>(&P->grid_f)));
-	const int capture_mode = R.capture_mode;
-	const double tau_limit = capture_mode ? DMS_CAPTURE_MAX_OPTICAL_DEPTH_STEP : DMS_MAX_OPTICAL_DEPTH_STEP;
-	if(!L.in_rk)
+	EventF ev = c.after;
+	double r_b = c.r_after, v_b = c.v_after;
+	if(c.r_before < R.boundary && c.r_after >= R.boundary && c.r_after > c.r_before)
 	{
-		if(!(L.seg_steps < R.max_free_steps))
-		{
-			L.reason = DMS_REASON_MAX_FREE_STEPS;  // L.cur holds the last committed event
-			return PH_FINAL;
-		}
-		if(wall_time_exceeded(R, L))  // "before_step", src/Simulation_Trajectory.cpp:873-874
-		{
-			set_final(L, to_event64(prop_event_f(L.pr)), true, DMS_REASON_WALL_TIME_LIMIT);
-			return PH_FINAL;
-		}
-		if(!L.before_valid)
-		{
-			L.before = prop_event_f(L.pr);
-			L.before_valid = 1;
-		}
-		const double r_before = prop_radius_f(L.pr);
-		const double v_before = prop_speed_f(L.pr);
-		L.rate_before = 0.0;
-		if(r_before >= DMS_RSUN_KM)
-		{
-			const double cap = step_cap(r_before, v_before, R.boundary);
-			const double ts = sanitized_step(L.pr.time_step);
-			L.pr.time_step = ts < cap ? ts : cap;
-			const double vr = (r_before > 0.0) ? static_cast<double>(dotf(L.before.x, L.before.v)) / r_before : 0.0;
-			if(r_before > DMS_RSUN_KM && vr < 0.0)
-			{
-				const double est = (r_before - DMS_RSUN_KM) / (-vr);
-				if(isfinite(est) && est > 0.0)
-				{
-					const double lim = est > DMS_RK45_ABS_MIN_STEP_S ? est : DMS_RK45_ABS_MIN_STEP_S;
-					if(lim < L.pr.time_step) L.pr.time_step = lim;
-				}
-			}
-		}
+		const double f = (R.boundary - c.r_before) / (c.r_after - c.r_before);
+		ev = interpolate_event_f(c.before, c.after, static_cast<float>(f));
+		r_b = normf(ev.x);
+		v_b = normf(ev.v);
+	}
+	if(!(r_b >= R.boundary && r_b >= c.r_before))
+		return BOUNDARY_INSIDE;
+	if(v_b > solar_vesc(S, r_b))
+	{
+		accepted = ev;
+		return BOUNDARY_ESCAPE;
+	}
+	Event abs_b = to_event64(ev);
+	abs_b.t += L.origin;
+	if(uncaptured_bound(S, m_dm, L, abs_b))
+	{
+		set_final(L, abs_b, false, DMS_REASON_NUMERICAL_FAILURE);
+		return BOUNDARY_FAILURE;
+	}
+	Event inbound;
+	if(!bound_kepler_return(to_event64(ev), inbound))
+		return BOUNDARY_INSIDE;
+	L.seg_steps++;
+	L.steps++;
+	L.retries = 0;
+	commit_event_general(R, m_dm, L, hist, ev);
+	// reset_propagator_at_absolute_event, src/Simulation_Trajectory.cpp:814-822
+	L.cur = inbound;
+	L.cur.t += L.origin;
+	L.origin = L.cur.t;
+	Event local = inbound;
+	local.t = 0.0;
+	prop_init_f(L.pr, local);
+	L.before_valid = 0;
+	L.next_valid = 0;
+	if(!R.capture_mode && L.prev_time >= 0.0)
+		L.prev_time = 0.0;
+	return BOUNDARY_RETURN;
+}
+
+// as in dms_kernels.cu
+constexpr int COOP_MAX_STEPS = 15;
+
+// One pass for every lane of the warp (all 32 call it); returns the lane's next phase.
+template <bool UNROLLED>
+__device__ __forceinline__ int mixed_step(const RunParams& R, const DevPoint* __restrict__ P, double m_dm, MixedLane& L, double2* hist, int phase,
+                                          float* buffer)
+{
+	const int capture_mode = R.capture_mode;
+	const int pieces = capture_mode ? DMS_CAPTURE_OPTICAL_DEPTH_PIECES : DMS_MAX_OPTICAL_DEPTH_PIECES;
+	const double tau_limit = capture_mode ? DMS_CAPTURE_MAX_OPTICAL_DEPTH_STEP : DMS_MAX_OPTICAL_DEPTH_STEP;
+	StepCtxF c;
+	PropF q;
+	bool done = false, interior = false, depth = false;
+	int reason = 0;
+	if(phase == PH_STEP && !L.in_rk)
+		phase = mixed_begin(R, P, L);
+	if(phase == PH_STEP)
+	{
+		q = L.pr;
+		L.rk_inner++;
+		const int rk = rk45_attempt_f<UNROLLED>(R.S, tables_f(R), q, L.rk_inner);
+		if(rk == RK_RETRY)
+			L.pr.time_step = q.time_step;
 		else
 		{
-			L.pr.time_step = sanitized_step(L.pr.time_step);
-			L.rate_before = rate_total_f(S, P, grid, static_cast<float>(r_before), static_cast<float>(v_before));
-			if(!isfinite(L.rate_before) || L.rate_before < 0.0)
+			done = true;
+			L.in_rk = 0;
+			L.attempts += static_cast<uint64_t>(L.rk_inner);
+			c.before = L.before;
+			c.before.t = L.pr.time;
+			c.r_before = prop_radius_f(L.pr);
+			c.dt = q.time - L.pr.time;
+			c.r_after = prop_radius_f(q);
+			c.v_after = prop_speed_f(q);
+			c.after = prop_event_f(q);
+			// the checks after an attempt, src/Simulation_Trajectory.cpp:930-960
+			if(rk == RK_FORCED)
+				reason = DMS_REASON_NUMERICAL_FAILURE;
+			else if(!isfinite(c.r_after) || !isfinite(c.v_after) || !isfinite(c.dt) || c.dt <= 0.0)
+				reason = DMS_REASON_NON_FINITE_STATE;
+			else if(c.v_after > DMS_V_MAX_C * DMS_C_KMS)
+				reason = DMS_REASON_SPEED_LIMIT;
+			else if(wall_time_exceeded(R, L))  // "after_rk45_step", src/Simulation_Trajectory.cpp:953-954
+				reason = DMS_REASON_WALL_TIME_LIMIT;
+			else
 			{
-				set_final(L, to_event64(prop_event_f(L.pr)), true, DMS_REASON_NUMERICAL_FAILURE);
-				return PH_FINAL;
-			}
-			if(L.rate_before > 0.0)
-			{
-				const float lim = static_cast<float>(tau_limit) / static_cast<float>(L.rate_before);
-				if(static_cast<double>(lim) < L.pr.time_step)
-					L.pr.time_step = static_cast<double>(lim);
-			}
-		}
-		// the RK step changes only these propagator fields
-		L.b_time = L.pr.time;
-		L.b_radius = L.pr.radius;
-		L.b_phi = L.pr.phi;
-		L.b_vr = L.pr.v_radial;
-		L.b_step = L.pr.time_step;
-		L.pr.time_step = sanitized_step(L.pr.time_step);  // head of Runge_Kutta_45_Step, :1489
-		L.in_rk = 1;
-		L.rk_inner = 0;
-	}
-	L.rk_inner++;
-	const int rk = rk45_attempt_f<true>(S, F, L.pr, L.rk_inner);
-	if(rk == RK_RETRY)
-		return PH_STEP;
-	L.in_rk = 0;
-	L.attempts += static_cast<uint64_t>(L.rk_inner);
-	const EventF before = L.before;
-	const double r_before = L.b_radius < 0.0 ? 0.0 : L.b_radius;
-	const double rate_before = L.rate_before;
-	const double actual_dt = L.pr.time - L.b_time;
-	const double r_after = prop_radius_f(L.pr);
-	const double v_after = prop_speed_f(L.pr);
-	const EventF after = prop_event_f(L.pr);
-	if(rk == RK_FORCED)
-	{
-		set_final(L, to_event64(after), true, DMS_REASON_NUMERICAL_FAILURE);
-		return PH_FINAL;
-	}
-	if(!isfinite(r_after) || !isfinite(v_after) || !isfinite(actual_dt) || actual_dt <= 0.0)
-	{
-		set_final(L, to_event64(after), true, DMS_REASON_NON_FINITE_STATE);
-		return PH_FINAL;
-	}
-	if(v_after > DMS_V_MAX_C * DMS_C_KMS)
-	{
-		set_final(L, to_event64(after), true, DMS_REASON_SPEED_LIMIT);
-		return PH_FINAL;
-	}
-	if(wall_time_exceeded(R, L))  // "after_rk45_step", src/Simulation_Trajectory.cpp:953-954
-	{
-		set_final(L, to_event64(after), true, DMS_REASON_WALL_TIME_LIMIT);
-		return PH_FINAL;
-	}
-	bool scattering = false, reflection = false;
-	EventF accepted = after;
-	float s0 = 0.0f, s1 = 0.0f;
-	if(interior_interval_f(before, after, r_before, r_after, s0, s1))
-	{
-		// Build_Optical_Depth_Pieces, src/Simulation_Trajectory.cpp:347-414
-		const int pieces = capture_mode ? DMS_CAPTURE_OPTICAL_DEPTH_PIECES : DMS_MAX_OPTICAL_DEPTH_PIECES;
-		const bool use_cached = r_before < DMS_RSUN_KM && s0 <= 1.0e-12f;
-		const float span = s1 - s0;
-		const float adt = static_cast<float>(actual_dt);
-		float fr[DMS_MAX_OPTICAL_DEPTH_PIECES + 1];
-		float rt[DMS_MAX_OPTICAL_DEPTH_PIECES + 1];
-		bool invalid = false;
-		float dtau_f = 0.0f, tau2 = 0.0f;  // optical depths of one step (<= 0.1) in FP32
-		if(s1 > s0 && actual_dt > 0.0)
-		{
-			// one loop over the piece boundaries, trapezoids formed as the rates arrive
-			float fr_prev = 0.0f, rt_prev = 0.0f, fr_0 = 0.0f, rt_0 = 0.0f, fr_2 = 0.0f, rt_2 = 0.0f, tau2_a = 0.0f;
-#pragma unroll 1
-			for(int i = 0; i <= pieces; i++)
-			{
-				const float f = s0 + static_cast<float>(i) / static_cast<float>(pieces) * span;
-				const float rate = (i == 0 && use_cached) ? static_cast<float>(rate_before) : rate_at_fraction_f(S, P, grid, before, after, f);
-				fr[i] = f;
-				rt[i] = rate;
-				if(!isfinite(rate) || rate < 0.0f)
-					invalid = true;
-				if(i > 0 && f > fr_prev)
-					dtau_f += 0.5f * (rt_prev + rate) * (adt * (f - fr_prev));
-				if(pieces >= 4)
+				c.s0 = 0.0f;
+				c.s1 = 1.0f;
+				interior = true;
+				if(!(c.r_before < DMS_RSUN_KM && c.r_after < DMS_RSUN_KM))
 				{
-					if(i == 0)
-					{
-						fr_0 = f;
-						rt_0 = rate;
-					}
-					else if(i == 2)
-					{
-						fr_2 = f;
-						rt_2 = rate;
-						tau2_a = 0.5f * (rt_0 + rt_2) * (adt * (fr_2 - fr_0));
-					}
-					else if(i == 4)
-						tau2 = tau2_a + 0.5f * (rt_2 + rate) * (adt * (f - fr_2));
+					c.s1 = 0.0f;
+					interior = interior_interval_outside(c.before, c.after, c.r_before, c.r_after, c.s0, c.s1);
 				}
-				else if(i > 0)
-					tau2 += 0.5f * (rt_prev + rate) * (adt * (f - fr_prev));
-				fr_prev = f;
-				rt_prev = rate;
+				depth = interior && c.s1 > c.s0;
 			}
 		}
-		const double dtau = static_cast<double>(dtau_f);
-		if(invalid || !isfinite(dtau) || dtau < 0.0)
+	}
+	const unsigned int dm = __ballot_sync(0xffffffffu, depth);
+	DepthF d = {0.0f, 0.0f, 0.0f, false};
+	const bool first_known = depth && c.r_before < DMS_RSUN_KM && c.s0 <= 1.0e-12f;
+	const float rate_before = static_cast<float>(L.rate_before);
+	if(dm != 0u)
+	{
+		if(__popc(dm) <= COOP_MAX_STEPS)
+			warp_depth(R, P, c, rate_before, first_known, pieces, dm, depth, buffer, d);
+		else if(depth)
+			lane_depth(R, P, c, rate_before, first_known, pieces, d);
+	}
+	if(!done)
+		return phase;
+	const double dtau = static_cast<double>(d.dtau);
+	if(reason == 0 && (d.invalid || !isfinite(dtau) || dtau < 0.0))
+		reason = DMS_REASON_NUMERICAL_FAILURE;
+	if(reason != 0)
+	{
+		set_final(L, to_event64(c.after), true, reason);
+		return PH_FINAL;
+	}
+	EventF accepted = c.after;
+	bool scattering = false;
+	if(interior)
+	{
+		// the quotient of the two estimates is formed only where the step may be rejected
+		const float scale = d.dtau > static_cast<float>(DMS_OPTICAL_DEPTH_ABS_TOL) ? d.dtau : static_cast<float>(DMS_OPTICAL_DEPTH_ABS_TOL);
+		if((dtau > tau_limit) | (!capture_mode & (fabsf(d.dtau - d.tau2) > static_cast<float>(DMS_OPTICAL_DEPTH_REL_TOL * 0.999) * scale)))
 		{
-			set_final(L, to_event64(after), true, DMS_REASON_NUMERICAL_FAILURE);
-			return PH_FINAL;
-		}
-		const float scale = dtau_f > static_cast<float>(DMS_OPTICAL_DEPTH_ABS_TOL) ? dtau_f : static_cast<float>(DMS_OPTICAL_DEPTH_ABS_TOL);
-		const double rel = static_cast<double>(fabsf(dtau_f - tau2) / scale);
-		const bool reject_depth = dtau > tau_limit;
-		const bool reject_acc = !capture_mode && rel > DMS_OPTICAL_DEPTH_REL_TOL;
-		if(reject_depth || reject_acc)
-		{
-			L.retries++;
-			if(L.retries > DMS_MAX_OPTICAL_DEPTH_RETRIES)
-			{
-				set_final(L, to_event64(before), true, DMS_REASON_NUMERICAL_FAILURE);
-				return PH_FINAL;
-			}
-			L.pr.time = L.b_time;
-			L.pr.radius = L.b_radius;
-			L.pr.phi = L.b_phi;
-			L.pr.v_radial = L.b_vr;
-			L.pr.time_step = L.b_step;
-			double factor = DMS_RK45_MAX_STEP_FACTOR;
-			if(dtau > tau_limit && dtau > 0.0 && 0.8 * tau_limit / dtau < factor)
-				factor = 0.8 * tau_limit / dtau;
-			if(reject_acc && rel > 0.0 && 0.8 * sqrt(DMS_OPTICAL_DEPTH_REL_TOL / rel) < factor)
-				factor = 0.8 * sqrt(DMS_OPTICAL_DEPTH_REL_TOL / rel);
-			if(factor > 1.0) factor = 1.0;
-			if(factor < DMS_RK45_MIN_STEP_FACTOR) factor = DMS_RK45_MIN_STEP_FACTOR;
-			L.pr.time_step = sanitized_step(factor * actual_dt);
-			return PH_STEP;  // L.before still describes the restored propagator
+			const int rejected = depth_reject(L, c.before, d.dtau, d.tau2, capture_mode != 0, c.dt, tau_limit);
+			if(rejected != PH_CONTINUE)
+				return rejected;
 		}
 		if(dtau >= L.tau)
 		{
-			double remaining = L.tau;
-			for(int k = 0; k < pieces; k++)
-			{
-				if(!(fr[k + 1] > fr[k]))
-					continue;
-				const double pdt = actual_dt * static_cast<double>(fr[k + 1] - fr[k]);
-				const double ptau = 0.5 * static_cast<double>(rt[k] + rt[k + 1]) * pdt;
-				if(ptau >= remaining)
-				{
-					const double lf = solve_linear_rate(rt[k], rt[k + 1], pdt, remaining);
-					const float f = fr[k] + static_cast<float>(lf) * (fr[k + 1] - fr[k]);
-					accepted = interpolate_event_f(before, after, f);
-					scattering = true;
-					break;
-				}
-				remaining -= ptau;
-			}
-			if(!scattering)
-			{
-				accepted = interpolate_event_f(before, after, s1);
-				scattering = true;
-			}
+			scatter_point(R.S, P, c, rate_before, first_known, depth, pieces, L.tau, accepted);
+			scattering = true;
 		}
 		else
 			L.tau -= dtau;
 	}
-	if(!scattering)
+	int boundary = BOUNDARY_INSIDE;
+	if(!scattering && c.r_after >= R.boundary)
 	{
-		EventF boundary_ev = after;
-		double r_b = r_after, v_b = v_after;
-		if(r_before < R.boundary && r_after >= R.boundary && r_after > r_before)
-		{
-			const double f = (R.boundary - r_before) / (r_after - r_before);
-			boundary_ev = interpolate_event_f(before, after, static_cast<float>(f));
-			r_b = normf(boundary_ev.x);
-			v_b = normf(boundary_ev.v);
-		}
-		if(r_b >= R.boundary && r_b >= r_before && v_b > solar_vesc(S, r_b))
-		{
-			accepted = boundary_ev;
-			reflection = true;
-		}
-		else if(r_b >= R.boundary && r_b >= r_before)
-		{
-			Event abs_b = to_event64(boundary_ev);
-			abs_b.t += L.origin;
-			if(uncaptured_bound(S, m_dm, L, abs_b))
-			{
-				set_final(L, abs_b, false, DMS_REASON_NUMERICAL_FAILURE);
-				return PH_FINAL;
-			}
-			Event inbound;
-			if(bound_kepler_return(to_event64(boundary_ev), inbound))
-			{
-				L.seg_steps++;
-				L.steps++;
-				L.retries = 0;
-				commit_event_mixed(S, F, m_dm, capture_mode, L, hist, boundary_ev);
-				// reset_propagator_at_absolute_event, src/Simulation_Trajectory.cpp:814-822
-				L.cur = inbound;
-				L.cur.t += L.origin;
-				L.origin = L.cur.t;
-				Event local = inbound;
-				local.t = 0.0;
-				prop_init_f(L.pr, local);
-				L.before_valid = 0;
-				if(!capture_mode && L.prev_time >= 0.0)
-					L.prev_time = 0.0;
-				return PH_STEP;
-			}
-		}
+		boundary = boundary_step(R, m_dm, L, hist, c, accepted);
+		if(boundary == BOUNDARY_RETURN)
+			return PH_STEP;
+		if(boundary == BOUNDARY_FAILURE)
+			return PH_FINAL;
 	}
 	L.seg_steps++;
 	L.steps++;
 	L.retries = 0;
-	double E = commit_event_mixed(S, F, m_dm, capture_mode, L, hist, accepted);
-	L.cur = to_event64(accepted);
-	L.cur.t += L.origin;
-	if(!L.is_captured)
+	const double E = commit_event_mixed(R, m_dm, L, hist, accepted);
+	const bool bound = !L.is_captured && (isnan(E) ? not_free(R, m_dm, accepted) : !(isfinite(E) && E >= 0.0));
+	if(bound | scattering | (boundary == BOUNDARY_ESCAPE))
 	{
-		// abort_if_uncaptured_bound on the committed event, src/Simulation_Trajectory.cpp:767-778, 1108
-		if(isnan(E))
-			E = capture_energy_eV(S, m_dm, ev_radius(L.cur), ev_speed(L.cur));
-		if(!(isfinite(E) && E >= 0.0))
-		{
+		L.cur = to_event64(accepted);
+		L.cur.t += L.origin;
+		if(bound)
 			L.reason = DMS_REASON_NUMERICAL_FAILURE;
-			return PH_FINAL;
-		}
-	}
-	if(reflection)
-	{
-		L.reason = DMS_REASON_OUTWARD_ESCAPE;
+		else if(!scattering)
+			L.reason = DMS_REASON_OUTWARD_ESCAPE;
+		else if(ev_radius(L.cur) < DMS_RSUN_KM)
+			return PH_SCATTER;  // Simulate, src/Simulation_Trajectory.cpp:1313-1346; Sample_Target runs in the lane loop
+		else
+			L.reason = DMS_REASON_SCATTER;
 		return PH_FINAL;
 	}
-	if(scattering)
-	{
-		// Simulate, src/Simulation_Trajectory.cpp:1313-1346
-		if(!(ev_radius(L.cur) < DMS_RSUN_KM))
-		{
-			L.reason = DMS_REASON_SCATTER;
-			return PH_FINAL;
-		}
-		return PH_SCATTER;  // Sample_Target runs warp-cooperatively in the lane loop
-	}
-	L.before = after;
+	L.pr.time = q.time;
+	L.pr.radius = q.radius;
+	L.pr.phi = q.phi;
+	L.pr.v_radial = q.v_radial;
+	L.pr.time_step = q.time_step;
+	L.before = c.after;
+	L.before_valid = 2;
+	L.next_speed = c.v_after;
+	L.next_rate = static_cast<double>(d.next_rate);
+	L.next_valid = depth || c.r_after >= DMS_RSUN_KM;
 	return PH_STEP;
 }
 
@@ -359,11 +579,11 @@ template <bool LOCKSTEP>
 struct MixedStep
 {
 	static constexpr bool lockstep = LOCKSTEP;
-	static constexpr bool collective = false;
-	static constexpr int buffer = 0;
-	__device__ __forceinline__ int operator()(const RunParams& R, const DevPoint* __restrict__ P, double m_dm, MixedLane& L, double2* hist) const
+	static constexpr int buffer = COOP_BUFFER_F;
+	__device__ __forceinline__ int operator()(const RunParams& R, const DevPoint* __restrict__ P, double m_dm, MixedLane& L, double2* hist, int phase,
+	                                          double* buffer) const
 	{
-		return free_step_mixed(R, P, m_dm, L, hist);
+		return mixed_step<!LOCKSTEP>(R, P, m_dm, L, hist, phase, reinterpret_cast<float*>(buffer));
 	}
 	__device__ __forceinline__ double channel(const DevSolar& S, const DevPoint* __restrict__ P, int i, double dr, double T, double v, int k) const
 	{

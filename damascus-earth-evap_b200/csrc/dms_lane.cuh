@@ -50,7 +50,6 @@ struct LaneT
 	double rate_before;  // scattering rate at the start of the step
 	int next_valid;      // next_speed / next_rate hold the propagator's speed and rate (FP64 form, tail)
 	double next_speed, next_rate;
-	double b_time, b_radius, b_phi, b_vr, b_step;  // propagator fields at the start of the step
 	int shift_ok;
 	int reason;
 	// capture / evaporation state
@@ -855,13 +854,8 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 		}
 		if(phase == PH_SEGMENT)
 			phase = segment_start(R, P, m_dm, L);
-		if constexpr(Step::collective)
-		{
-			if(__any_sync(FULL_WARP, phase == PH_STEP))
-				phase = step(R, P, m_dm, L, hist, phase, rates);
-		}
-		else if(phase == PH_STEP)
-			phase = step(R, P, m_dm, L, hist);
+		if(__any_sync(FULL_WARP, phase == PH_STEP))
+			phase = step(R, P, m_dm, L, hist, phase, rates);
 	}
 	const bool in_trajectory = phase != PH_FETCH && phase != PH_DONE;
 	if(in_trajectory && L.bmax >= L.bmin)

@@ -972,6 +972,17 @@ __device__ __forceinline__ double step_cap(double radius, double speed, double m
 	return cap > DMS_RK45_ABS_MIN_STEP_S ? cap : DMS_RK45_ABS_MIN_STEP_S;
 }
 
+// Whether none of the bounds of a step that starts at or outside the surface (step_cap and the time
+// to the surface, src/Simulation_Trajectory.cpp:65-80, 886-899) is below `step`, by a margin far above
+// their rounding.  along = x . v.
+__device__ __forceinline__ bool outside_step_is_free(double r, double speed, double along, double step, double boundary)
+{
+	const double crossing = (0.25 * boundary > 10.0) ? 0.25 * boundary : 10.0;
+	return (step <= DMS_RK45_ABS_MAX_STEP_S) & (step >= DMS_RK45_ABS_MIN_STEP_S) & (step * speed < crossing * (1.0 - 1.0e-9)) &
+	       (speed > 1.0e-12) & (step * step * (100.0 * DMS_GMSUN_KM3S2) < r * r * r * (1.0 - 1.0e-9)) &
+	       ((along >= 0.0) | ((r - DMS_RSUN_KM) * r * (1.0 - 1.0e-9) > -along * step));
+}
+
 __device__ __forceinline__ double ev_radius(const Event& e) { return norm3(e.x); }
 __device__ __forceinline__ double ev_speed(const Event& e) { return norm3(e.v); }
 

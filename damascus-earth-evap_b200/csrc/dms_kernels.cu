@@ -94,7 +94,10 @@ __device__ __forceinline__ int step_begin(const RunParams& R, const DevPoint* __
 	double step = sanitized_step(L.pr.time_step);
 	double rate = 0.0;
 	if(r >= DMS_RSUN_KM)
-		step = outside_step(L, r, step, R.boundary);
+	{
+		if(!outside_step_is_free(r, L.next_speed, dot3(L.before.x, L.before.v), step, R.boundary))
+			step = outside_step(L, r, step, R.boundary);
+	}
 	else
 	{
 		rate = L.next_rate;
@@ -154,6 +157,17 @@ __device__ __forceinline__ void event_and_speed(const Prop& p, Event& e, double&
 	e.t = p.time;
 	e.x = mk(safe * (cp * p.ax.x + sp * p.ay.x), safe * (cp * p.ax.y + sp * p.ay.y), safe * (cp * p.ax.z + sp * p.ay.z));
 	e.v = mk(vx * p.ax.x + vy * p.ay.x, vx * p.ax.y + vy * p.ay.y, vx * p.ax.z + vy * p.ay.z);
+}
+
+// Whether a chord with both ends clearly outside the Sun passes clear of it: it only recedes from or only
+// approaches the Sun between its ends, or its line misses the Sun.  Solar_Interior_Fraction_Interval
+// then finds no crossing in [0, 1]; the margin of 10^-6 is far above its rounding.
+__device__ __forceinline__ bool chord_stays_outside(const Event& a, const Event& b, double ra, double rb)
+{
+	const Vec3 d = sub3(b.x, a.x);
+	const double ad = dot3(a.x, d), bd = dot3(b.x, d), dd = dot3(d, d);
+	const double lim = DMS_RSUN_KM * (1.0 + 1.0e-6);
+	return (ra > lim) & (rb > lim) & ((ad >= 0.0) | (bd <= 0.0) | ((ra * ra - lim * lim) * dd > ad * ad * (1.0 + 1.0e-6)));
 }
 
 // Solar_Interior_Fraction_Interval for a chord with an end outside the Sun.
@@ -480,8 +494,13 @@ __device__ __forceinline__ void commit_event_inline(const RunParams& R, double m
 	if(!isfinite(L.free_flight_E))
 		return;
 	// capture_energy_eV
-	bool ok = (r <= DMS_RSUN_KM) & (R.S.fast_tables != 0);
-	double vesc = fast::sqrt(ok ? solar_vesc2_fast(R.S, r) : 1.0, ok);
+	bool ok = (R.S.fast_tables != 0) & (r < 0x1p100);
+	double w;  // v_esc^2 before its root
+	if(r <= DMS_RSUN_KM)
+		w = solar_vesc2_fast(R.S, r);
+	else
+		w = fast::div(2 * DMS_GMSUN_KM3S2, fast::recip(r, ok));
+	double vesc = fast::sqrt(w, ok);
 	if(!ok)
 		vesc = solar_vesc_general(R.S, r);
 	const double E = fast::div_const(0.5 * m_dm * fast::div_const(vv - vesc * vesc, DMS_C_KMS * DMS_C_KMS), 1.0e-9);
@@ -576,7 +595,9 @@ __device__ __forceinline__ int strict_step(const RunParams& R, const DevPoint* _
 				if(!(c.r_before < DMS_RSUN_KM && c.r_after < DMS_RSUN_KM))
 				{
 					c.s1 = 0.0;
-					interior = interior_interval_outside(c.before, c.after, c.r_before, c.r_after, c.s0, c.s1);
+					interior = false;
+					if(!chord_stays_outside(c.before, c.after, c.r_before, c.r_after))
+						interior = interior_interval_outside(c.before, c.after, c.r_before, c.r_after, c.s0, c.s1);
 				}
 				depth = interior && c.s1 > c.s0;
 			}

@@ -83,7 +83,10 @@ __device__ __forceinline__ int mixed_begin(const RunParams& R, const DevPoint* _
 	const double r = prop_radius_f(L.pr);
 	double step = sanitized_step(L.pr.time_step), rate = 0.0;
 	if(r >= DMS_RSUN_KM)
-		step = outside_step(L, r, step, R.boundary);
+	{
+		if(!outside_step_is_free(r, L.next_speed, static_cast<double>(dotf(L.before.x, L.before.v)), step, R.boundary))
+			step = outside_step(L, r, step, R.boundary);
+	}
 	else
 	{
 		rate = L.next_rate;
@@ -111,6 +114,17 @@ struct StepCtxF
 	double r_before, r_after, v_after, dt;
 	float s0, s1;
 };
+
+// Whether a chord with both ends clearly outside the Sun passes clear of it (as in dms_kernels.cu, with a
+// margin of 10^-4 for the FP32 events).
+__device__ __forceinline__ bool chord_stays_outside(const EventF& a, const EventF& b, double ra, double rb)
+{
+	const F3 d = f3(b.x.x - a.x.x, b.x.y - a.x.y, b.x.z - a.x.z);
+	const float ad = dotf(a.x, d), bd = dotf(b.x, d), dd = dotf(d, d);
+	const float lim = static_cast<float>(DMS_RSUN_KM * (1.0 + 1.0e-4)), r = static_cast<float>(ra);
+	return (ra > static_cast<double>(lim)) & (rb > static_cast<double>(lim)) &
+	       ((ad >= 0.0f) | (bd <= 0.0f) | ((r - lim) * (r + lim) * dd > ad * ad * 1.0001f));
+}
 
 static __device__ __noinline__ bool interior_interval_outside(const EventF& a, const EventF& b, double ra, double rb, float& s0, float& s1)
 {
@@ -487,7 +501,9 @@ __device__ __forceinline__ int mixed_step(const RunParams& R, const DevPoint* __
 				if(!(c.r_before < DMS_RSUN_KM && c.r_after < DMS_RSUN_KM))
 				{
 					c.s1 = 0.0f;
-					interior = interior_interval_outside(c.before, c.after, c.r_before, c.r_after, c.s0, c.s1);
+					interior = false;
+					if(!chord_stays_outside(c.before, c.after, c.r_before, c.r_after))
+						interior = interior_interval_outside(c.before, c.after, c.r_before, c.r_after, c.s0, c.s1);
 				}
 				depth = interior && c.s1 > c.s0;
 			}

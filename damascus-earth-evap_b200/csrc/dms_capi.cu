@@ -248,14 +248,13 @@ int Launch_And_Wait(dms_ctx* ctx, const dms_run_opts* o, RunParams& p)
 	const bool mixed = o->precision == DMS_PRECISION_MIXED;
 	const int threads = Block_Threads(o, p.total, ctx->sm_count);
 	int blocks = ctx->sm_count;
-	// a launch with fewer trajectories than lanes spreads them over all of its warps: fewer lanes per
-	// warp diverge less, and its idle lanes help in the collective steps
-	const uint64_t warps = static_cast<uint64_t>(blocks) * (threads / 32);
-	p.lanes_per_warp = static_cast<int>(std::min<uint64_t>(32, (p.total + warps - 1) / warps));
-	const uint64_t per_block = static_cast<uint64_t>(threads / 32) * p.lanes_per_warp;
-	blocks = static_cast<int>(std::min<uint64_t>(blocks, (p.total + per_block - 1) / per_block));
+	// a launch with fewer trajectories than lanes spreads them over the SMs and then over the warps: fewer
+	// lanes per warp diverge less, its idle lanes help in the collective steps, and the warps of a block
+	// with a lone lane form a team
+	blocks = static_cast<int>(std::min<uint64_t>(blocks, p.total));
+	p.lanes_per_block = static_cast<int>(std::min<uint64_t>(threads, (p.total + blocks - 1) / blocks));
 	p.lockstep_min = threads / 16;
-	const size_t lanes = static_cast<size_t>(blocks) * (threads / 32) * p.lanes_per_warp;
+	const size_t lanes = static_cast<size_t>(blocks) * p.lanes_per_block;
 	int rc = Ensure_Lanes(ctx, lanes);
 	if(rc != DMS_OK)
 		return rc;
@@ -1307,12 +1306,11 @@ int dms_run_records_noalloc(dms_ctx* ctx, const dms_run_opts* opts, int point_id
 	rc = Noalloc_Scratch(ctx, &scratch);
 	if(rc != DMS_OK)
 		return rc;
-	// one trajectory per warp, four warps per block: the lanes that take work number at most
-	// DMS_NOALLOC_MAX_TRAJECTORIES.  (127 histories: 106 ms in blocks of one full warp.)
-	const int threads = 128;
-	const int blocks = static_cast<int>((count + 3) / 4);
-	const uint64_t lanes = static_cast<uint64_t>(blocks) * 4;
-	static_assert(DMS_NOALLOC_MAX_TRAJECTORIES % 4 == 0, "the lanes of whole blocks fit the scratch");
+	// one trajectory per block of four warps, which make its steps together (127 histories: 106 ms in
+	// blocks of one full warp, 25 ms with one trajectory per warp)
+	const int threads = LATENCY_THREADS;
+	const int blocks = static_cast<int>(count);
+	const uint64_t lanes = count;
 
 	RunParams p{};
 	p.S = ctx->dsolar;
@@ -1337,7 +1335,7 @@ int dms_run_records_noalloc(dms_ctx* ctx, const dms_run_opts* opts, int point_id
 	if(opts->max_trajectory_wall_time_s > 0.0 && p.wall_limit_ns == 0)
 		p.wall_limit_ns = 1;
 	p.ic_max_attempts = 1 << 20;
-	p.lanes_per_warp = 1;
+	p.lanes_per_block = 1;
 	Apply_Lane_Options(p, opts);
 	p.counters = ctx->d_counters;
 	p.hists = ctx->d_hists;

@@ -972,15 +972,38 @@ __device__ __forceinline__ double step_cap(double radius, double speed, double m
 	return cap > DMS_RK45_ABS_MIN_STEP_S ? cap : DMS_RK45_ABS_MIN_STEP_S;
 }
 
-// Whether none of the bounds of a step that starts at or outside the surface (step_cap and the time
-// to the surface, src/Simulation_Trajectory.cpp:65-80, 886-899) is below `step`, by a margin far above
-// their rounding.  along = x . v.
-__device__ __forceinline__ bool outside_step_is_free(double r, double speed, double along, double step, double boundary)
+static __device__ __noinline__ double step_cap_general(double r, double speed, double boundary) { return step_cap(r, speed, boundary); }
+
+// step_cap (src/Simulation_Trajectory.cpp:65-80) applied to `step` at a radius r at or outside the surface,
+// straight-line: the quotients and the root are formed with dms_fastmath.cuh, and only where they can bind.
+__device__ __forceinline__ double capped_step(double r, double speed, double step, double boundary)
 {
+	bool ok = (speed > 0x1p-30) & (speed < 0x1p60) & (r < 0x1p100);
 	const double crossing = (0.25 * boundary > 10.0) ? 0.25 * boundary : 10.0;
-	return (step <= DMS_RK45_ABS_MAX_STEP_S) & (step >= DMS_RK45_ABS_MIN_STEP_S) & (step * speed < crossing * (1.0 - 1.0e-9)) &
-	       (speed > 1.0e-12) & (step * step * (100.0 * DMS_GMSUN_KM3S2) < r * r * r * (1.0 - 1.0e-9)) &
-	       ((along >= 0.0) | ((r - DMS_RSUN_KM) * r * (1.0 - 1.0e-9) > -along * step));
+	double cap = DMS_RK45_ABS_MAX_STEP_S;
+	const double r3 = r * r * r;
+	if(!(step * step * (100.0 * DMS_GMSUN_KM3S2) < r3 * (1.0 - 1.0e-9)))
+	{
+		const double dyn = 0.1 * fast::sqrt(fast::div_const(r3, DMS_GMSUN_KM3S2), ok);
+		cap = dyn < cap ? dyn : cap;
+	}
+	if(!((step < cap ? step : cap) * speed < crossing * (1.0 - 1.0e-9)))
+	{
+		ok &= crossing < 0x1p100;
+		const double q = fast::div(crossing, fast::recip(speed, ok));
+		cap = q < cap ? q : cap;
+	}
+	cap = cap > DMS_RK45_ABS_MIN_STEP_S ? cap : DMS_RK45_ABS_MIN_STEP_S;
+	if(!ok)
+		cap = step_cap_general(r, speed, boundary);
+	return step < cap ? step : cap;
+}
+
+// Whether the time to the surface (src/Simulation_Trajectory.cpp:886-899) of a particle outside it cannot be
+// below `step`, by a margin far above its rounding.  along = x . v.
+__device__ __forceinline__ bool surface_is_far(double r, double along, double step)
+{
+	return (along >= 0.0) | ((r - DMS_RSUN_KM) * r * (1.0 - 1.0e-9) > -along * step);
 }
 
 __device__ __forceinline__ double ev_radius(const Event& e) { return norm3(e.x); }

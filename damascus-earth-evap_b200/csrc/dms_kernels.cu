@@ -54,12 +54,10 @@ static __device__ __noinline__ int end_at_propagator(StrictLane& L, int reason)
 
 static __device__ __noinline__ double div_general(double a, double b) { return a / b; }
 
-// The bounds of a step that starts at or outside the surface.
-static __device__ __noinline__ double outside_step(const StrictLane& L, double r, double step, double boundary)
+// The time to the surface as a bound of a step that starts at or outside it.
+static __device__ __noinline__ double surface_step(const Event& before, double r, double step)
 {
-	const double cap = step_cap(r, L.next_speed, boundary);
-	step = step < cap ? step : cap;
-	const double along = dot3(L.before.x, L.before.v);
+	const double along = dot3(before.x, before.v);
 	if(r > DMS_RSUN_KM && along < 0.0)
 	{
 		const double est = (r - DMS_RSUN_KM) / (-(along / r));
@@ -68,6 +66,22 @@ static __device__ __noinline__ double outside_step(const StrictLane& L, double r
 			const double lim = est > DMS_RK45_ABS_MIN_STEP_S ? est : DMS_RK45_ABS_MIN_STEP_S;
 			step = lim < step ? lim : step;
 		}
+	}
+	return step;
+}
+
+// The optical-depth bound of a step that starts inside the Sun at scattering rate `rate`.
+__device__ __forceinline__ double inside_step(const RunParams& R, double rate, double step)
+{
+	const double tau_limit = R.capture_mode ? DMS_CAPTURE_MAX_OPTICAL_DEPTH_STEP : DMS_MAX_OPTICAL_DEPTH_STEP;
+	// the quotient is formed only where it can be the smaller one
+	if(rate * step * (1.0 + 0x1p-50) > tau_limit)
+	{
+		bool ok = (rate > 0x1p-200) & (rate < 0x1p100);
+		double lim = fast::div(tau_limit, fast::recip(rate, ok));
+		if(!ok)
+			lim = div_general(tau_limit, rate);
+		step = lim < step ? lim : step;
 	}
 	return step;
 }
@@ -95,24 +109,16 @@ __device__ __forceinline__ int step_begin(const RunParams& R, const DevPoint* __
 	double rate = 0.0;
 	if(r >= DMS_RSUN_KM)
 	{
-		if(!outside_step_is_free(r, L.next_speed, dot3(L.before.x, L.before.v), step, R.boundary))
-			step = outside_step(L, r, step, R.boundary);
+		step = capped_step(r, L.next_speed, step, R.boundary);
+		if(!surface_is_far(r, dot3(L.before.x, L.before.v), step))
+			step = surface_step(L.before, r, step);
 	}
 	else
 	{
 		rate = L.next_rate;
 		if(!isfinite(rate) || rate < 0.0)
 			return end_at_propagator(L, DMS_REASON_NUMERICAL_FAILURE);
-		const double tau_limit = R.capture_mode ? DMS_CAPTURE_MAX_OPTICAL_DEPTH_STEP : DMS_MAX_OPTICAL_DEPTH_STEP;
-		// the quotient is formed only where it can be the smaller one
-		if(rate * step * (1.0 + 0x1p-50) > tau_limit)
-		{
-			bool ok = (rate > 0x1p-200) & (rate < 0x1p100);
-			double lim = fast::div(tau_limit, fast::recip(rate, ok));
-			if(!ok)
-				lim = div_general(tau_limit, rate);
-			step = lim < step ? lim : step;
-		}
+		step = inside_step(R, rate, step);
 	}
 	L.rate_before = rate;
 	L.pr.time_step = step;
@@ -546,6 +552,52 @@ __device__ __noinline__ void commit_event(const RunParams& R, double m_dm, Stric
 // which makes 5 (3) of them one after another.
 constexpr int COOP_MAX_STEPS = 15;
 
+// Commits a step whose outcome is decided (src/Simulation_Trajectory.cpp:1088-1116): the event `accepted`, and
+// for a plain step the propagator after it with the scattering rate there (next_known when it was formed).
+__device__ __forceinline__ int finish_step(const RunParams& R, double m_dm, StrictLane& L, double2* hist, const StepCtx& c, const Event& accepted,
+                                           bool scattering, int boundary, double time, double radius, double phi, double v_radial, double time_step,
+                                           double next_rate, bool next_known)
+{
+	L.seg_steps++;
+	L.steps++;
+	L.retries = 0;
+	const bool plain = !scattering && boundary == BOUNDARY_INSIDE;
+	// the committed event's own radius and speed; in Capture mode a plain step only asks whether the
+	// particle is still free, which the propagator's decide
+	double r_now = c.r_after, v_now = c.v_after;
+	if(!R.capture_mode | L.is_captured | !plain)
+		sqrt2(dot3(accepted.x, accepted.x), dot3(accepted.v, accepted.v), r_now, v_now);
+	commit_event_inline(R, m_dm, L, hist, accepted.t, r_now, v_now);
+	const bool bound = !L.is_captured && not_free(R, m_dm, accepted, r_now, v_now);
+	if(bound | !plain)
+	{
+		L.cur = accepted;
+		L.cur.t += L.origin;
+		if(bound)
+			L.reason = DMS_REASON_NUMERICAL_FAILURE;
+		else if(!scattering)
+			L.reason = DMS_REASON_OUTWARD_ESCAPE;
+		else if(r_now < DMS_RSUN_KM)
+			return PH_SCATTER;  // Simulate, src/Simulation_Trajectory.cpp:1313-1346; Sample_Target runs in the lane loop
+		else
+			L.reason = DMS_REASON_SCATTER;
+		return PH_FINAL;
+	}
+	L.pr.time = time;
+	L.pr.radius = radius;
+	L.pr.phi = phi;
+	L.pr.v_radial = v_radial;
+	L.pr.time_step = time_step;
+	L.before = c.after;
+	L.before_valid = 2;
+	// the next step starts from this speed and rate; without a depth the rate at a state inside the
+	// Sun is not known yet
+	L.next_speed = c.v_after;
+	L.next_rate = next_rate;
+	L.next_valid = next_known || c.r_after >= DMS_RSUN_KM;
+	return PH_STEP;
+}
+
 // One pass for every lane of the warp (all 32 call it); returns the lane's next phase.
 template <int UNROLL>
 __device__ __forceinline__ int strict_step(const RunParams& R, const DevPoint* __restrict__ P, double m_dm, StrictLane& L, double2* hist, int phase,
@@ -651,44 +703,269 @@ __device__ __forceinline__ int strict_step(const RunParams& R, const DevPoint* _
 		if(boundary == BOUNDARY_FAILURE)
 			return PH_FINAL;
 	}
-	L.seg_steps++;
-	L.steps++;
-	L.retries = 0;
-	const bool plain = !scattering && boundary == BOUNDARY_INSIDE;
-	// the committed event's own radius and speed; in Capture mode a plain step only asks whether the
-	// particle is still free, which the propagator's decide
-	double r_now = c.r_after, v_now = c.v_after;
-	if(!capture_mode | L.is_captured | !plain)
-		sqrt2(dot3(accepted.x, accepted.x), dot3(accepted.v, accepted.v), r_now, v_now);
-	commit_event_inline(R, m_dm, L, hist, accepted.t, r_now, v_now);
-	const bool bound = !L.is_captured && not_free(R, m_dm, accepted, r_now, v_now);
-	if(bound | !plain)
+	return finish_step(R, m_dm, L, hist, c, accepted, scattering, boundary, q.time, q.radius, q.phi, q.v_radial, q.time_step, d.next_rate, depth);
+}
+
+// ---------------------------------------------------------------------------------------------
+// Team: a lane that runs alone in its block spends its step on one dependent chain, and a warp issues one
+// instruction every 4.4 cycles of it.  Once the other warps of a 128-thread block have run out of work,
+// two of them take over parts of the lone lane's steps, one step apart, with a barrier per step:
+//   propagate  the bounds and the RK45 attempts of the next step, from its own last result
+//   judge      (the lane's own warp) event, optical depth and decisions of the step before
+//   commit     bincount and energy drift of the step before that
+// (9 steps per orbit is common for a lone lane: an orbit that leaves the boundary radius comes back by Kepler's
+// equation, which the lane solves with the team's step in hand.)
+// The propagating warp runs ahead as if every step ended plainly.  A step that does not is not committed:
+// a depth rejection restarts the propagation from the step's start with the shorter step; anything
+// else (a scattering, the boundary, a failure) hands the state at the step's start back to the lane, which
+// makes that step by itself.  Every value is formed by the functions of the one-lane pass from the same
+// arguments, so the results are the same bits.  The barriers count whole warps that all run the same loop;
+// the only wait by polling is that of a warp without work for a team to form, and it is bounded.
+struct TeamState  // the propagator at the start of a step
+{
+	double time, radius, phi, v_radial, step, speed, rate;
+	int inner, ok;  // attempts of the step that led here; whether the propagating warp could make it
+};
+struct TeamBox
+{
+	int word;       // warps without work; TEAM_FORMED once a team has formed, negative when none can
+	int command;    // TEAM_RUN, TEAM_EXIT
+	int verdict[2];
+	int captured, bound, bmin, bmax, cbin;
+	const DevPoint* P;
+	double2* hist;
+	double m_dm, J;
+	Vec3 ax, ay;
+	double origin, prev_time, prev_r, prev_v2, t_last_bound, free_flight_E, max_drift_eV, max_drift_rel;
+	double2 cval;
+	TeamState s[4];  // by step number modulo 4
+	Event e[4];      // the events at those states
+};
+constexpr int TEAM_FORMED = 0x100, TEAM_NEVER = -0x10000, TEAM_RUN = 0, TEAM_EXIT = 1;
+enum Verdict : int
+{
+	VERDICT_PLAIN = 0,
+	VERDICT_RESTART = 1,
+	VERDICT_STOP = 2,
+	VERDICT_BOUNDARY = 3,  // the step ends at or beyond the boundary radius
+};
+#ifndef DMS_TU
+#define DMS_TU 6
+#endif
+constexpr int TEAM_UNROLL = DMS_TU;
+constexpr int TEAM_MAX_STEPS = 512;                      // per call: the lane loop looks at the cancel flag between calls
+constexpr long long TEAM_WAIT_CYCLES = 40000000000ll;   // ~20 s: how long a warp without work waits for a team
+
+__device__ __forceinline__ TeamBox& team_box()
+{
+	__shared__ TeamBox box;
+	return box;
+}
+__device__ __forceinline__ void team_barrier() { asm volatile("bar.sync 1, 96;" ::: "memory"); }
+
+// The propagating warp's step: from s to n.  One lane.
+__device__ __forceinline__ void team_propagate(const RunParams& R, const TeamBox& b, const TeamState& s, TeamState& n)
+{
+	Prop q;
+	q.time = s.time;
+	q.radius = s.radius;
+	q.phi = s.phi;
+	q.v_radial = s.v_radial;
+	q.J = b.J;
+	q.ax = b.ax;
+	q.ay = b.ay;
+	q.radial_mode = 0;
+	// step_begin; the event at the state is only needed where the time to the surface may bind
+	const double r = s.radius;
+	double step = sanitized_step(s.step);
+	bool ok = true;
+	if(r >= DMS_RSUN_KM)
 	{
-		L.cur = accepted;
-		L.cur.t += L.origin;
-		if(bound)
-			L.reason = DMS_REASON_NUMERICAL_FAILURE;
-		else if(!scattering)
-			L.reason = DMS_REASON_OUTWARD_ESCAPE;
-		else if(r_now < DMS_RSUN_KM)
-			return PH_SCATTER;  // Simulate, src/Simulation_Trajectory.cpp:1313-1346; Sample_Target runs in the lane loop
-		else
-			L.reason = DMS_REASON_SCATTER;
-		return PH_FINAL;
+		const double along = r * s.v_radial;
+		step = capped_step(r, s.speed, step, R.boundary);
+		if(!(((along > 1.0e-6 * r) | (along < -1.0e-6 * r)) && surface_is_far(r, along, step)))
+		{
+			Event before;
+			double speed;
+			event_and_speed(q, before, speed);
+			step = surface_step(before, r, step);
+		}
 	}
-	L.pr.time = q.time;
-	L.pr.radius = q.radius;
-	L.pr.phi = q.phi;
-	L.pr.v_radial = q.v_radial;
-	L.pr.time_step = q.time_step;
-	L.before = c.after;
-	L.before_valid = 2;
-	// the next step starts from this speed and rate; without a depth the rate at a state inside the
-	// Sun is not known yet
-	L.next_speed = c.v_after;
-	L.next_rate = d.next_rate;
-	L.next_valid = depth || c.r_after >= DMS_RSUN_KM;
-	return PH_STEP;
+	else
+	{
+		ok = (s.rate >= 0.0) & (s.rate < INFINITY);
+		step = inside_step(R, s.rate, step);
+	}
+	q.time_step = step;
+	int inner = 0, rk = RK_RETRY;
+	while(ok && rk == RK_RETRY && inner <= DMS_RK45_MAX_INNER_RETRIES)
+	{
+		inner++;
+		rk = rk45_attempt<TEAM_UNROLL>(R.S, q, inner);
+	}
+	ok &= rk == RK_ACCEPTED;
+	// prop_speed, as in event_and_speed
+	ok &= fast::in_radius_range(q.radius) & (fabs(q.phi) < 0x1p20);
+	const fast::Recip D = fast::recip(q.radius, ok);
+	n.speed = fast::sqrt(q.v_radial * q.v_radial + fast::div(fast::div(b.J * b.J, D), D), ok);
+	n.rate = ok ? rate_inside(R.S, b.P, q.radius, n.speed) : 0.0;
+	n.time = q.time;
+	n.radius = q.radius;
+	n.phi = q.phi;
+	n.v_radial = q.v_radial;
+	n.step = q.time_step;
+	n.inner = inner;
+	n.ok = ok ? 1 : 0;
+}
+
+// The judging warp's step: from state s with event e to state n, whose event goes to en.  All 32 lanes;
+// `mine` marks the lane whose trajectory it is.
+__device__ __forceinline__ int team_judge(const RunParams& R, const TeamBox& b, TeamState& s, const Event& e, const TeamState& n, Event& en, StrictLane& L,
+                                          bool mine, double* buffer, StepCtx& c)
+{
+	const int capture_mode = R.capture_mode;
+	const int pieces = capture_mode ? DMS_CAPTURE_OPTICAL_DEPTH_PIECES : DMS_MAX_OPTICAL_DEPTH_PIECES;
+	const double tau_limit = capture_mode ? DMS_CAPTURE_MAX_OPTICAL_DEPTH_STEP : DMS_MAX_OPTICAL_DEPTH_STEP;
+	bool interior = false, depth = false, stop = true;
+	if(mine && n.ok)
+	{
+		Prop q;
+		q.time = n.time;
+		q.radius = n.radius;
+		q.phi = n.phi;
+		q.v_radial = n.v_radial;
+		q.J = b.J;
+		q.ax = b.ax;
+		q.ay = b.ay;
+		q.radial_mode = 0;
+		c.before = e;
+		c.r_before = s.radius;
+		c.dt = n.time - s.time;
+		c.r_after = n.radius;
+		event_and_speed(q, c.after, c.v_after);
+		stop = !(isfinite(c.v_after) & (c.dt > 0.0) & (c.dt < INFINITY) & (c.v_after <= DMS_V_MAX_C * DMS_C_KMS) &
+		         (L.seg_steps + 4 < R.max_free_steps));
+		if(!stop)
+		{
+			c.s0 = 0.0;
+			c.s1 = 1.0;
+			interior = true;
+			if(!(c.r_before < DMS_RSUN_KM && c.r_after < DMS_RSUN_KM))
+			{
+				c.s1 = 0.0;
+				interior = false;
+				if(!chord_stays_outside(c.before, c.after, c.r_before, c.r_after))
+					interior = interior_interval_outside(c.before, c.after, c.r_before, c.r_after, c.s0, c.s1);
+			}
+			depth = interior && c.s1 > c.s0;
+		}
+	}
+	const unsigned int dm = __ballot_sync(0xffffffffu, depth);
+	Depth d = {0.0, 0.0, 0.0, false};
+	if(dm != 0u)
+		warp_depth(R, b.P, c, s.rate, c.r_before < DMS_RSUN_KM && c.s0 <= 1.0e-12, pieces, dm, depth, buffer, d);
+	int verdict = VERDICT_STOP;
+	if(mine && !stop)
+	{
+		const double scale = d.dtau > DMS_OPTICAL_DEPTH_ABS_TOL ? d.dtau : DMS_OPTICAL_DEPTH_ABS_TOL;
+		const double apart = capture_mode ? 0.0 : fabs(d.dtau - d.tau2);
+		verdict = VERDICT_PLAIN;
+		if(d.invalid | !(d.dtau >= 0.0) | !(d.dtau < INFINITY) | (interior & (d.dtau >= L.tau)))
+			verdict = VERDICT_STOP;
+		if(interior && ((d.dtau > tau_limit) | (!capture_mode & (apart > (DMS_OPTICAL_DEPTH_REL_TOL * (1.0 - 0x1p-50)) * scale))) && !d.invalid &&
+		   d.dtau >= 0.0 && d.dtau < INFINITY)
+		{
+			// (a rejection comes before the scattering test; the last retry ends the trajectory)
+			verdict = VERDICT_STOP;
+			if(L.retries < DMS_MAX_OPTICAL_DEPTH_RETRIES)
+			{
+				const int rejected = depth_reject(L, c.before, d.dtau, apart, scale, capture_mode != 0, c.dt, tau_limit);
+				verdict = rejected == PH_STEP ? VERDICT_RESTART : (d.dtau >= L.tau ? VERDICT_STOP : VERDICT_PLAIN);
+			}
+		}
+		if(verdict == VERDICT_PLAIN && c.r_after >= R.boundary)
+			verdict = VERDICT_BOUNDARY;
+		if(verdict == VERDICT_PLAIN && !L.is_captured && not_free(R, b.m_dm, c.after, c.r_after, c.v_after))
+			verdict = VERDICT_STOP;
+		if(verdict != VERDICT_STOP)
+			L.attempts += static_cast<uint64_t>(n.inner);
+		if(verdict == VERDICT_RESTART)
+			s.step = L.pr.time_step;
+		if(interior && (verdict == VERDICT_PLAIN || verdict == VERDICT_BOUNDARY))
+			L.tau -= d.dtau;
+		if(verdict == VERDICT_PLAIN)
+		{
+			L.seg_steps++;
+			L.steps++;
+			L.retries = 0;
+			en = c.after;
+		}
+	}
+	return verdict;
+}
+
+// The committing warp's step: the bincount and energy drift of the event e.  One lane, whose own lane
+// state serves as scratch.
+__device__ __forceinline__ void team_commit(const RunParams& R, const TeamBox& b, StrictLane& L, const Event& e)
+{
+	double r, v;
+	if(!R.capture_mode | L.is_captured)
+	{
+		sqrt2(dot3(e.x, e.x), dot3(e.v, e.v), r, v);
+		commit_event_inline(R, b.m_dm, L, b.hist, e.t, r, v);
+	}
+}
+
+// The loop of the three warps: role 0 judges, 1 propagates, 2 commits.  Returns the number of the step at
+// whose start the lane goes on by itself (the states and events are in the box).
+__device__ __forceinline__ int team_loop(const RunParams& R, TeamBox& b, StrictLane& L, int role, bool mine, double* buffer, StepCtx& c, int& last)
+{
+	const bool lane0 = (threadIdx.x & 31) == 0;
+	int j = 0;             // the step to judge
+	bool have = false;     // ... whose result is there
+	bool pending = false;  // step j - 1 is to be committed
+	for(int pass = 0;; pass++)
+	{
+		if(role == 1)
+		{
+			const int from = have ? j + 1 : j;
+			if(lane0)
+				team_propagate(R, b, b.s[from & 3], b.s[(from + 1) & 3]);
+		}
+		else if(role == 0)
+		{
+			if(have)
+			{
+				int v = VERDICT_STOP;
+				if(pass < TEAM_MAX_STEPS)
+					v = team_judge(R, b, b.s[j & 3], b.e[j & 3], b.s[(j + 1) & 3], b.e[(j + 1) & 3], L, mine, buffer, c);
+				if(mine)
+					b.verdict[pass & 1] = v;
+			}
+		}
+		else if(pending && lane0)
+			team_commit(R, b, L, b.e[j & 3]);
+		__syncwarp();
+		team_barrier();
+		pending = false;
+		if(!have)
+		{
+			have = true;
+			continue;
+		}
+		const int v = *reinterpret_cast<volatile int*>(&b.verdict[pass & 1]);
+		last = v;
+		if(v >= VERDICT_STOP)
+			break;
+		if(v == VERDICT_PLAIN)
+		{
+			j++;
+			pending = true;
+		}
+		else
+			have = false;
+	}
+	return j;
 }
 
 // Initial_Conditions + Hyperbolic_Kepler_Shift of every work index (src/Data_Generation.cpp:747-761,
@@ -729,6 +1006,218 @@ struct StrictStep
 	                                          double* buffer) const
 	{
 		return strict_step<LOCKSTEP ? 1 : 6>(R, P, m_dm, L, hist, phase, buffer);
+	}
+	// ---- team (the latency form) ----
+	static constexpr bool team = !LOCKSTEP;
+	__device__ __forceinline__ void team_init() const
+	{
+		team_box().word = 0;
+		team_box().command = TEAM_RUN;
+	}
+	// Called by a whole warp without work: it helps a lone lane of its block, if one forms a team, until that
+	// lane's trajectory has ended.
+	__device__ __noinline__ void team_help(const RunParams& R, StrictLane& L, double* buffer) const
+	{
+		TeamBox& b = team_box();
+		const bool lane0 = (threadIdx.x & 31) == 0;
+		int rank = 0;
+		if(lane0)
+			rank = atomicAdd(&b.word, 1);
+		rank = __shfl_sync(0xffffffffu, rank, 0);
+		if(rank == 3)
+		{
+			team_forgo();  // the last warp of the block: nobody is left to help
+			return;
+		}
+		const long long t0 = clock64();
+		for(unsigned int poll = 1;; poll++)
+		{
+			int word = 0;
+			if(lane0)
+			{
+				word = *reinterpret_cast<volatile int*>(&b.word);
+				bool leave = clock64() - t0 > TEAM_WAIT_CYCLES;
+				if((poll & 255u) == 0u)
+					leave |= *R.cancel != 0;
+				// a warp leaves by putting the count out of reach, which no formed team can follow
+				if(leave && word >= 0 && word < TEAM_FORMED)
+				{
+					const int seen = atomicCAS(&b.word, word, TEAM_NEVER);
+					word = seen == word ? TEAM_NEVER : seen;
+				}
+			}
+			word = __shfl_sync(0xffffffffu, word, 0);
+			if(word < 0)
+				return;
+			if(word >= TEAM_FORMED)
+				break;
+			__nanosleep(1000);
+		}
+		if(rank > 1)
+			return;  // two helpers are enough
+		for(;;)
+		{
+			team_barrier();  // the owner has filled the box
+			if(*reinterpret_cast<volatile int*>(&b.command) == TEAM_EXIT)
+				return;
+			if(rank == 1)
+			{
+				L.is_captured = b.captured;
+				L.bound_state = b.bound;
+				L.bmin = b.bmin;
+				L.bmax = b.bmax;
+				L.cbin = b.cbin;
+				L.cval = b.cval;
+				L.origin = b.origin;
+				L.prev_time = b.prev_time;
+				L.prev_r = b.prev_r;
+				L.prev_v2 = b.prev_v2;
+				L.t_last_bound = b.t_last_bound;
+				L.free_flight_E = b.free_flight_E;
+				L.max_drift_eV = b.max_drift_eV;
+				L.max_drift_rel = b.max_drift_rel;
+			}
+			StepCtx c;
+			int last;
+			team_loop(R, b, L, rank == 0 ? 1 : 2, false, buffer, c, last);
+			if(rank == 1 && lane0)
+			{
+				b.bmin = L.bmin;
+				b.bmax = L.bmax;
+				b.cbin = L.cbin;
+				b.cval = L.cval;
+				b.prev_time = L.prev_time;
+				b.prev_r = L.prev_r;
+				b.prev_v2 = L.prev_v2;
+				b.t_last_bound = L.t_last_bound;
+				b.max_drift_eV = L.max_drift_eV;
+				b.max_drift_rel = L.max_drift_rel;
+			}
+			__syncwarp();
+			team_barrier();  // the owner may read the box
+		}
+	}
+	// Called by the whole warp of a lone lane (`mine` on that lane, at the start of a step): forms the team if the
+	// other three warps are without work.
+	__device__ __forceinline__ bool team_form() const
+	{
+		TeamBox& b = team_box();
+		int formed = 0;
+		if((threadIdx.x & 31) == 0)
+			formed = *reinterpret_cast<volatile int*>(&b.word) == 3 && atomicCAS(&b.word, 3, TEAM_FORMED) == 3 ? 1 : 0;
+		return __shfl_sync(0xffffffffu, formed, 0) != 0;
+	}
+	// A warp that stops in mid-trajectory: no team can form any more.
+	__device__ __forceinline__ void team_forgo() const
+	{
+		if((threadIdx.x & 31) == 0)
+			atomicExch(&team_box().word, TEAM_NEVER);
+	}
+	__device__ __forceinline__ void team_dismiss() const
+	{
+		TeamBox& b = team_box();
+		if((threadIdx.x & 31) == 0)
+			*reinterpret_cast<volatile int*>(&b.command) = TEAM_EXIT;
+		__syncwarp();
+		team_barrier();
+	}
+	// Steps of the lone lane made by the team; the lane's state is that at the start of a step before and
+	// after (or `phase`, its phase, says otherwise).  Returns the number of steps made.
+	__device__ __noinline__ int team_run(const RunParams& R, const DevPoint* __restrict__ P, double m_dm, StrictLane& L, double2* hist, bool mine,
+	                                     double* buffer, int& phase) const
+	{
+		TeamBox& b = team_box();
+		if(mine && !L.next_valid)
+			fresh_state(R.S, P, L);
+		// what the fast functions cover; other states go to the one-lane pass
+		const bool fit = mine && (L.pr.radial_mode == 0) & (L.pr.J > 0x1p-200) & (L.pr.J < 0x1p200) &
+		                                          fast::in_radius_range(L.pr.radius) & (fabs(L.pr.phi) < 0x1p20);
+		if(!__any_sync(0xffffffffu, fit))
+			return 0;
+		if(mine)
+		{
+			b.P = P;
+			b.hist = hist;
+			b.m_dm = m_dm;
+			b.J = L.pr.J;
+			b.ax = L.pr.ax;
+			b.ay = L.pr.ay;
+			b.captured = L.is_captured;
+			b.bound = L.bound_state;
+			b.bmin = L.bmin;
+			b.bmax = L.bmax;
+			b.cbin = L.cbin;
+			b.cval = L.cval;
+			b.origin = L.origin;
+			b.prev_time = L.prev_time;
+			b.prev_r = L.prev_r;
+			b.prev_v2 = L.prev_v2;
+			b.t_last_bound = L.t_last_bound;
+			b.free_flight_E = L.free_flight_E;
+			b.max_drift_eV = L.max_drift_eV;
+			b.max_drift_rel = L.max_drift_rel;
+			TeamState& s = b.s[0];
+			s.time = L.pr.time;
+			s.radius = L.pr.radius;
+			s.phi = L.pr.phi;
+			s.v_radial = L.pr.v_radial;
+			s.step = L.pr.time_step;
+			s.speed = L.next_speed;
+			s.rate = L.next_rate;
+			b.e[0] = L.before;
+			b.e[0].t = L.pr.time;
+		}
+		__syncwarp();
+		team_barrier();
+		StepCtx c;
+		int last = VERDICT_PLAIN;
+		int j = team_loop(R, b, L, 0, mine, buffer, c, last);
+		team_barrier();  // the committing warp has written its part back
+		if(mine)
+		{
+			const TeamState& s = b.s[j & 3];
+			L.pr.time = s.time;
+			L.pr.radius = s.radius;
+			L.pr.phi = s.phi;
+			L.pr.v_radial = s.v_radial;
+			L.pr.time_step = s.step;
+			L.next_speed = s.speed;
+			L.next_rate = s.rate;
+			if(j > 0)
+			{
+				L.before = b.e[j & 3];
+				L.before_valid = 2;
+			}
+			L.bmin = b.bmin;
+			L.bmax = b.bmax;
+			L.cbin = b.cbin;
+			L.cval = b.cval;
+			L.prev_time = b.prev_time;
+			L.prev_r = b.prev_r;
+			L.prev_v2 = b.prev_v2;
+			L.t_last_bound = b.t_last_bound;
+			L.max_drift_eV = b.max_drift_eV;
+			L.max_drift_rel = b.max_drift_rel;
+		}
+		// a step that ends at the boundary is finished here with what the team made of it, as in strict_step
+		if(last == VERDICT_BOUNDARY)
+		{
+			if(mine)
+			{
+				Event accepted = c.after;
+				const int boundary = boundary_step(R, m_dm, L, hist, c, accepted);
+				if(boundary == BOUNDARY_FAILURE)
+					phase = PH_FINAL;
+				else if(boundary != BOUNDARY_RETURN)
+				{
+					const TeamState& n = b.s[(j + 1) & 3];
+					phase = finish_step(R, m_dm, L, hist, c, accepted, false, boundary, n.time, n.radius, n.phi, n.v_radial, n.step, n.rate, true);
+				}
+			}
+			j++;
+		}
+		__syncwarp();
+		return j;
 	}
 	__device__ __forceinline__ double channel(const DevSolar& S, const DevPoint* __restrict__ P, int i, double dr, double T, double v, int k) const
 	{

@@ -69,7 +69,7 @@ struct RunParams
 	// the warp batching of scatterings and terminations
 	uint32_t queue_chunk;
 	int scatter_batch, scatter_wait, final_batch, final_wait;
-	int lanes_per_warp;  // lanes of a warp that take trajectories (32, fewer in a spread launch)
+	int lanes_per_block; // lanes of a block that take trajectories (all, fewer in a spread launch)
 	int lockstep_min;    // lanes at work below which a block's warps leave the lockstep once the queue is empty
 	int ic_max_attempts;
 	// accumulators (accumulate mode)

@@ -46,10 +46,8 @@ static __device__ __noinline__ int end_at_propagator(MixedLane& L, int reason)
 	return PH_FINAL;
 }
 
-static __device__ __noinline__ double outside_step(const MixedLane& L, double r, double step, double boundary)
+static __device__ __noinline__ double surface_step(const MixedLane& L, double r, double step)
 {
-	const double cap = step_cap(r, L.next_speed, boundary);
-	step = step < cap ? step : cap;
 	const double vr = (r > 0.0) ? static_cast<double>(dotf(L.before.x, L.before.v)) / r : 0.0;
 	if(r > DMS_RSUN_KM && vr < 0.0)
 	{
@@ -84,8 +82,9 @@ __device__ __forceinline__ int mixed_begin(const RunParams& R, const DevPoint* _
 	double step = sanitized_step(L.pr.time_step), rate = 0.0;
 	if(r >= DMS_RSUN_KM)
 	{
-		if(!outside_step_is_free(r, L.next_speed, static_cast<double>(dotf(L.before.x, L.before.v)), step, R.boundary))
-			step = outside_step(L, r, step, R.boundary);
+		step = capped_step(r, L.next_speed, step, R.boundary);
+		if(!surface_is_far(r, static_cast<double>(dotf(L.before.x, L.before.v)), step))
+			step = surface_step(L, r, step);
 	}
 	else
 	{
@@ -596,6 +595,7 @@ struct MixedStep
 {
 	static constexpr bool lockstep = LOCKSTEP;
 	static constexpr int buffer = COOP_BUFFER_F;
+	static constexpr bool team = false;
 	__device__ __forceinline__ int operator()(const RunParams& R, const DevPoint* __restrict__ P, double m_dm, MixedLane& L, double2* hist, int phase,
 	                                          double* buffer) const
 	{

@@ -681,12 +681,12 @@ __device__ __forceinline__ int finish_scatter(const RunParams& R, const DevPoint
 template <class Lane, class Step>
 __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 {
-	// the first R.lanes_per_warp lanes of every warp take trajectories (and own a histogram row);
-	// the others only help in the warp's collective steps
+	// R.lanes_per_block lanes of the block take trajectories and own a histogram row, dealt out to the warps
+	// one by one; the others only help in the collective steps
 	const int in_warp = threadIdx.x & 31;
-	const bool takes_work = in_warp < R.lanes_per_warp;
-	const int warp_id = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-	double2* hist = R.lane_hist + static_cast<size_t>(warp_id * R.lanes_per_warp + (takes_work ? in_warp : 0)) * DMS_NUM_BINS;
+	const int slot = in_warp * (blockDim.x >> 5) + (threadIdx.x >> 5);
+	const bool takes_work = slot < R.lanes_per_block;
+	double2* hist = R.lane_hist + (static_cast<size_t>(blockIdx.x) * R.lanes_per_block + (takes_work ? slot : 0)) * DMS_NUM_BINS;
 	// per warp: the 64 channel rates of a scattering, or the steps and rates of Step's own lookups
 	constexpr int BUFFER = Step::buffer > DMS_NUM_TARGETS + 1 ? Step::buffer : DMS_NUM_TARGETS + 1;
 	__shared__ double coop_rates[(Step::lockstep ? MAX_THREADS : LATENCY_THREADS) / 32][BUFFER];
@@ -699,6 +699,11 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 	if(threadIdx.x < 8)
 		votes[threadIdx.x >> 2][threadIdx.x & 3] = 0;
 	bool lockstep = Step::lockstep;
+	bool team = false;  // this warp's lone lane has formed a team
+	uint64_t next_check = 1023;
+	if constexpr(Step::team)
+		if(threadIdx.x == 0)
+			step.team_init();
 	int passes_scatter = 0, passes_final = 0;  // passes since the block's last scattering (termination) phase
 	__syncthreads();
 	Lane L;
@@ -771,19 +776,44 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 		}
 		else
 		{
-			if(__all_sync(FULL_WARP, phase == PH_DONE))
-				break;
-			if((iter & 1023) == 1023)
+			const unsigned int live = __ballot_sync(FULL_WARP, phase != PH_DONE);
+			bool leave = live == 0u;
+			if(iter >= next_check)
 			{
+				next_check = iter + 1024;
 				if(__any_sync(FULL_WARP, *R.cancel != 0))
 				{
 					atomicOr(R.status, STATUS_CANCELLED);
-					break;
+					leave = true;
 				}
 				if(iter > R.iteration_budget)
 				{
 					atomicOr(R.status, STATUS_BUDGET);
-					break;
+					leave = true;
+				}
+			}
+			if(leave)
+			{
+				if constexpr(Step::team)
+				{
+					if(team)
+						step.team_dismiss();
+					else if(live != 0u)
+						step.team_forgo();
+					else if(R.wall_limit_ns == 0 && blockDim.x == 128)
+						step.team_help(R, L, rates);
+				}
+				break;
+			}
+			if constexpr(Step::team)
+			{
+				const bool mine = phase == PH_STEP && !L.in_rk;
+				if((live & (live - 1u)) == 0u && __any_sync(FULL_WARP, mine) && R.wall_limit_ns == 0)
+				{
+					if(!team)
+						team = step.team_form();
+					if(team)
+						iter += step.team_run(R, P, m_dm, L, hist, mine, rates, phase);
 				}
 			}
 			const unsigned int stepping = __ballot_sync(FULL_WARP, phase == PH_STEP || phase == PH_FETCH || phase == PH_SEGMENT);

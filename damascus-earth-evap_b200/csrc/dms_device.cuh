@@ -346,6 +346,46 @@ struct Draws
 	}
 };
 
+// The next uniform draw in [0, 1), out of line.  A scattering makes about ten draws and runs once in some 25
+// to 50 steps of a lane: its code is never in the instruction cache, so its size is what it costs.  (The
+// same reason for the other out-of-line forms below: a lone lane spent 60 us on a scattering, 20 steps' time,
+// with everything inline.)
+static __device__ __noinline__ double draw_unit(Draws& D) { return D.uniform(0.0, 1.0); }
+__device__ __forceinline__ double draw_between(Draws& D, double a, double b)
+{
+	const double u = draw_unit(D);
+	return a + u * (b - a);
+}
+__device__ __forceinline__ double draw_positive(Draws& D)
+{
+	const double u = draw_unit(D);
+	return u > 2.2250738585072014e-308 ? u : 2.2250738585072014e-308;
+}
+static __device__ __noinline__ double log_call(double x) { return dms_log(x); }
+static __device__ __noinline__ void sincos_call(double x, double& s, double& c) { dms_sincos(x, &s, &c); }
+
+// a / n by component: the quotients share one reciprocal where their operands are in its range.
+static __device__ __noinline__ void div3_general(Vec3& a, double n) { a = div3(a, n); }
+__device__ __forceinline__ bool in_quotient_range(double x)
+{
+	const unsigned int e = static_cast<unsigned int>(__double2hiint(x)) & 0x7fffffffu;
+	return (e - 0x14300000u < 0x58f00000u - 0x14300000u) | (x == 0.0);  // 0 or 2^-700 <= |x| < 2^400
+}
+__device__ __forceinline__ double signed_quotient(double a, const fast::Recip& d) { return a == 0.0 ? a : fast::div(a, d); }
+__device__ __forceinline__ Vec3 div3_fast(const Vec3& a, double n)
+{
+	bool ok = (n > 0x1p-100) & (n < 0x1p100) & in_quotient_range(a.x) & in_quotient_range(a.y) & in_quotient_range(a.z);
+	const fast::Recip d = fast::recip(n, ok);
+	Vec3 q = mk(signed_quotient(a.x, d), signed_quotient(a.y, d), signed_quotient(a.z, d));
+	if(!ok)
+	{
+		q = a;
+		div3_general(q, n);
+	}
+	return q;
+}
+__device__ __forceinline__ Vec3 normalized3_fast(const Vec3& a) { return div3_fast(a, norm3(a)); }
+
 // ---------------------------------------------------------------------------------------------
 // Standard Halo Model and initial conditions, src/Simulation_Utilities.cpp:123-249
 __device__ __forceinline__ double halo_pdf_speed(const DevPoint* __restrict__ P, double v)
@@ -544,6 +584,15 @@ struct Prop
 	int radial_mode;
 };
 
+// Build_Stable_Orthonormal_Basis, src/Simulation_Trajectory.cpp:130-142
+static __device__ __noinline__ void stable_basis(Vec3& ax, Vec3& ay)
+{
+	const Vec3 e1 = div3(ax, norm3(ax));
+	const Vec3 ref = (fabs(e1.z) < 0.9) ? mk(0.0, 0.0, 1.0) : mk(1.0, 0.0, 0.0);
+	ax = e1;
+	ay = normalized3(cross3(ref, e1));
+}
+
 static __device__ __noinline__ void prop_init(Prop& p, const Event& e)
 {
 	p.time = e.t;
@@ -560,7 +609,7 @@ static __device__ __noinline__ void prop_init(Prop& p, const Event& e)
 	Vec3 ax;
 	if(isfinite(p.radius) && p.radius > 1.0e-12)
 	{
-		ax = div3(e.x, p.radius);
+		ax = div3_fast(e.x, p.radius);
 		p.v_radial = dot3(e.x, e.v) / p.radius;
 	}
 	else if(isfinite(speed) && speed > 0.0)
@@ -580,13 +629,13 @@ static __device__ __noinline__ void prop_init(Prop& p, const Event& e)
 	Vec3 ay = mk(0.0, 0.0, 0.0);
 	if(!p.radial_mode && isfinite(Ln) && Ln > angular_eps)
 	{
-		const Vec3 az = div3(L, Ln);
+		const Vec3 az = div3_fast(L, Ln);
 		ay = cross3(az, ax);
 		const double ny = norm3(ay);
 		if(isfinite(ny) && ny > 0.0)
 		{
-			ay = div3(ay, ny);
-			ax = normalized3(cross3(ay, az));
+			ay = div3_fast(ay, ny);
+			ax = normalized3_fast(cross3(ay, az));
 			p.J = Ln;
 		}
 		else
@@ -596,11 +645,7 @@ static __device__ __noinline__ void prop_init(Prop& p, const Event& e)
 		p.radial_mode = 1;
 	if(p.radial_mode)
 	{
-		// Build_Stable_Orthonormal_Basis, src/Simulation_Trajectory.cpp:130-142
-		const Vec3 e1 = div3(ax, norm3(ax));
-		const Vec3 ref = (fabs(e1.z) < 0.9) ? mk(0.0, 0.0, 1.0) : mk(1.0, 0.0, 0.0);
-		ax = e1;
-		ay = normalized3(cross3(ref, e1));
+		stable_basis(ax, ay);
 		p.J = 0.0;
 	}
 	p.ax = ax;
@@ -1241,22 +1286,24 @@ static __device__ __noinline__ double solve_linear_rate(double r0, double r1, do
 }
 
 // Unit_Vector_At_Angle_From_Axis, src/Simulation_Trajectory.cpp:109-128
-__device__ __forceinline__ bool unit_vector_at_angle(double cos_theta, double phi, const Vec3& axis, Vec3& out)
+static __device__ __noinline__ bool unit_vector_at_angle(double cos_theta, double phi, const Vec3& axis, Vec3& out)
 {
 	if(!isfinite(cos_theta) || cos_theta < -1.0 - 1.0e-12 || cos_theta > 1.0 + 1.0e-12 || !isfinite(phi))
 		return false;
 	const double n = norm3(axis);
 	if(!isfinite(n) || n <= 0.0)
 		return false;
-	const Vec3 e3 = div3(axis, n);
+	const Vec3 e3 = div3_fast(axis, n);
 	const Vec3 ref = (fabs(e3.z) < 0.9) ? mk(0.0, 0.0, 1.0) : mk(1.0, 0.0, 0.0);
-	const Vec3 e1 = normalized3(cross3(ref, e3));
-	const Vec3 e2 = normalized3(cross3(e3, e1));
+	Vec3 e[2];  // one copy of the cross product and its norm
+#pragma unroll 1
+	for(int k = 0; k < 2; k++) e[k] = normalized3_fast(k == 0 ? cross3(ref, e3) : cross3(e3, e[0]));
+	const Vec3 e1 = e[0], e2 = e[1];
 	cos_theta = clamp_cos(cos_theta);
 	const double st2 = 1.0 - cos_theta * cos_theta;
 	const double st = sqrt(st2 > 0.0 ? st2 : 0.0);
 	double sp, cp;
-	dms_sincos(phi, &sp, &cp);
+	sincos_call(phi, sp, cp);
 	out = mk(cos_theta * e3.x + st * cp * e1.x + st * sp * e2.x, cos_theta * e3.y + st * cp * e1.y + st * sp * e2.y,
 	         cos_theta * e3.z + st * cp * e1.z + st * sp * e2.z);
 	return true;
@@ -1270,8 +1317,8 @@ __device__ __forceinline__ bool unit_vector_at_angle(double cos_theta, double ph
 __device__ __forceinline__ double sample_cos_alpha(const DevPoint* __restrict__ P, Draws& D, int k, double v)
 {
 	if(__ldg(&P->interaction) != DMS_INTERACTION_DARK_PHOTON_GENERAL)
-		return D.uniform(-1.0, 1.0);
-	const double xi = D.uniform(0.0, 1.0);
+		return draw_between(D, -1.0, 1.0);
+	const double xi = draw_unit(D);
 	const double m2 = __ldg(&P->ff_m2);
 	const double q2 = __ldg(&P->q2c[k < 0 ? DMS_NUM_TARGETS : k]) * (v * v);
 	return (m2 * (2.0 * xi - 1.0) + q2 * xi) / (m2 + q2 * xi);
@@ -1301,31 +1348,37 @@ constexpr int TARGET_FAILED = -2;
 __device__ __forceinline__ double channel_total(const double* rates)
 {
 	double total = rates[DMS_NUM_TARGETS];
+#pragma unroll 9
 	for(int k = 0; k < DMS_NUM_TARGETS; k++) total += rates[k];
 	return total;
 }
 
-// The cumulative pick from the fractions q[k] = rate_k / total (q[63] the electrons).
+// The cumulative pick from the fractions q[k] = rate_k / total (q[63] the electrons).  Nine sums at a time:
+// they do not decrease, so the channel is the number of sums not above xi.
 __device__ __forceinline__ int pick_from_fractions(Draws& D, const double* q)
 {
-	const double xi = D.uniform(0.0, 1.0);
-	int target = -1;
+	static_assert(DMS_NUM_TARGETS % 9 == 0, "whole groups of sums");
+	const double xi = draw_unit(D);
 	double sum = q[DMS_NUM_TARGETS];
-	if(!(sum > xi))
+	if(sum > xi)
+		return -1;
+	int target = 0;
+#pragma unroll 1
+	for(int k = 0; k < DMS_NUM_TARGETS; k += 9)
 	{
-		for(int k = 0; k < DMS_NUM_TARGETS; k++)
+		int below = 0;
+#pragma unroll
+		for(int i = 0; i < 9; i++)
 		{
-			sum += q[k];
-			if(sum > xi || k == DMS_NUM_TARGETS - 1)
-			{
-				target = k;
-				break;
-			}
+			sum += q[k + i];
+			below += sum > xi ? 0 : 1;
 		}
+		target = k + below;
+		if(below < 9)
+			break;
 	}
-	return target;
+	return target < DMS_NUM_TARGETS ? target : DMS_NUM_TARGETS - 1;
 }
-
 
 // The rest of Scatter once the target is known: Sample_Target_Velocity, the scattering angle
 // and New_DM_Velocity, src/Simulation_Trajectory.cpp:1160-1269.  Returns
@@ -1364,32 +1417,33 @@ static __device__ __noinline__ bool scatter_with_target(const DevSolar& S, const
 		if(!isfinite(ratio) || ratio < 0.0 || ratio > 1.0 + 1.0e-12)
 			return false;
 		const double accept = ratio < 1.0 ? ratio : 1.0;
-		if(!(accept < D.uniform(0.0, 1.0)))
+		if(!(accept < draw_unit(D)))
 			break;
 		attempts++;
 		if(attempts > DMS_TARGET_VELOCITY_MAX_REJECTIONS)
 			return false;
-		mu = D.uniform(-1.0, 1.0);
-		const double xi1 = D.uniform(0.0, 1.0);
+		mu = draw_between(D, -1.0, 1.0);
+		const double xi1 = draw_unit(D);
 		if(xi1 < 2.0 / (sqrt_pi * y + 2.0))
 		{
-			const double xi2 = D.positive_unit();
-			const double xi3 = D.positive_unit();
-			const double z = -dms_log(xi2) - dms_log(xi3);
+			const double xi2 = draw_positive(D);
+			const double xi3 = draw_positive(D);
+			const double z = -log_call(xi2) - log_call(xi3);
 			x = sqrt(z);
 		}
 		else
 		{
-			const double xi2 = D.positive_unit();
-			const double xi3 = D.uniform(0.0, 1.0);
-			const double xi4 = D.positive_unit();
-			const double c = dms_cos(DMS_PI / 2.0 * xi3);
-			const double z = -dms_log(xi2) - (c * c) * dms_log(xi4);
+			const double xi2 = draw_positive(D);
+			const double xi3 = draw_unit(D);
+			const double xi4 = draw_positive(D);
+			double sine, c;
+			sincos_call(DMS_PI / 2.0 * xi3, sine, c);
+			const double z = -log_call(xi2) - (c * c) * log_call(xi4);
 			x = sqrt(z);
 		}
 	}
 	const double vT = x / kappa;
-	const double phi_t = D.uniform(0.0, 2.0 * DMS_PI);
+	const double phi_t = draw_between(D, 0.0, 2.0 * DMS_PI);
 	Vec3 unit_t;
 	if(!unit_vector_at_angle(mu, phi_t, e.v, unit_t))
 		return false;
@@ -1402,15 +1456,15 @@ static __device__ __noinline__ bool scatter_with_target(const DevSolar& S, const
 	   !isfinite(norm3(e.v)) || !isfinite(norm3(vel_t)))
 		return false;
 	const double ca = clamp_cos(cos_alpha);
-	const double phi_n = D.uniform(0.0, 2.0 * DMS_PI);
+	const double phi_n = draw_between(D, 0.0, 2.0 * DMS_PI);
 	Vec3 n;
 	if(!unit_vector_at_angle(ca, phi_n, e.v, n))
 		return false;
 	const double rel_speed = norm3(sub3(vel_t, e.v));
 	const double mt = m_target;
 	const double sc = mt * rel_speed / (mt + md);
-	const Vec3 out = mk(sc * n.x + (md * e.v.x + mt * vel_t.x) / (mt + md), sc * n.y + (md * e.v.y + mt * vel_t.y) / (mt + md),
-	                    sc * n.z + (md * e.v.z + mt * vel_t.z) / (mt + md));
+	const Vec3 com = div3_fast(mk(md * e.v.x + mt * vel_t.x, md * e.v.y + mt * vel_t.y, md * e.v.z + mt * vel_t.z), mt + md);
+	const Vec3 out = mk(sc * n.x + com.x, sc * n.y + com.y, sc * n.z + com.z);
 	if(!isfinite(norm3(out)))
 		return false;
 	e.v = out;

@@ -512,30 +512,30 @@ static __device__ __noinline__ bool scatter_with_target_f(const DevSolar& S, con
 			return false;
 		const float ratio = sqrtf(fmaxf(raw, 0.0f)) / den;
 		const float accept = ratio < 1.0f ? ratio : 1.0f;
-		if(!(static_cast<double>(accept) < D.uniform(0.0, 1.0)))
+		if(!(static_cast<double>(accept) < draw_unit(D)))
 			break;
 		attempts++;
 		if(attempts > DMS_TARGET_VELOCITY_MAX_REJECTIONS)
 			return false;
-		mu = static_cast<float>(D.uniform(-1.0, 1.0));
-		const double xi1 = D.uniform(0.0, 1.0);
+		mu = static_cast<float>(draw_between(D, -1.0, 1.0));
+		const double xi1 = draw_unit(D);
 		if(xi1 < static_cast<double>(2.0f / (sqrt_pi * y + 2.0f)))
 		{
-			const float xi2 = static_cast<float>(D.positive_unit());
-			const float xi3 = static_cast<float>(D.positive_unit());
+			const float xi2 = static_cast<float>(draw_positive(D));
+			const float xi3 = static_cast<float>(draw_positive(D));
 			x = sqrtf(-logf(xi2) - logf(xi3));
 		}
 		else
 		{
-			const float xi2 = static_cast<float>(D.positive_unit());
-			const float xi3 = static_cast<float>(D.uniform(0.0, 1.0));
-			const float xi4 = static_cast<float>(D.positive_unit());
+			const float xi2 = static_cast<float>(draw_positive(D));
+			const float xi3 = static_cast<float>(draw_unit(D));
+			const float xi4 = static_cast<float>(draw_positive(D));
 			const float c = cosf(1.5707963267948966f * xi3);
 			x = sqrtf(-logf(xi2) - (c * c) * logf(xi4));
 		}
 	}
 	const float vT = x / kappa;
-	const float phi_t = static_cast<float>(D.uniform(0.0, 2.0 * DMS_PI));
+	const float phi_t = static_cast<float>(draw_between(D, 0.0, 2.0 * DMS_PI));
 	F3 unit_t;
 	if(!unit_vector_at_angle_f(mu, phi_t, vd, unit_t))
 		return false;
@@ -544,7 +544,7 @@ static __device__ __noinline__ bool scatter_with_target_f(const DevSolar& S, con
 	const float md = static_cast<float>(__ldg(&P->m_dm));
 	if(!isfinite(normf(vel_t)) || !isfinite(md) || md <= 0.0f)
 		return false;
-	const float phi_n = static_cast<float>(D.uniform(0.0, 2.0 * DMS_PI));
+	const float phi_n = static_cast<float>(draw_between(D, 0.0, 2.0 * DMS_PI));
 	F3 n;
 	if(!unit_vector_at_angle_f(fminf(fmaxf(cos_alpha, -1.0f), 1.0f), phi_n, vd, n))
 		return false;

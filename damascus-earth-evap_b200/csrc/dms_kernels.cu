@@ -748,6 +748,8 @@ enum Verdict : int
 	VERDICT_RESTART = 1,
 	VERDICT_STOP = 2,
 	VERDICT_BOUNDARY = 3,  // the step ends at or beyond the boundary radius
+	VERDICT_SCATTER = 4,   // the remaining optical depth lies in the step
+	VERDICT_PAUSE = 5,     // not judged: the lane loop is due
 };
 #ifndef DMS_TU
 #define DMS_TU 6
@@ -870,8 +872,10 @@ __device__ __forceinline__ int team_judge(const RunParams& R, const TeamBox& b, 
 		const double scale = d.dtau > DMS_OPTICAL_DEPTH_ABS_TOL ? d.dtau : DMS_OPTICAL_DEPTH_ABS_TOL;
 		const double apart = capture_mode ? 0.0 : fabs(d.dtau - d.tau2);
 		verdict = VERDICT_PLAIN;
-		if(d.invalid | !(d.dtau >= 0.0) | !(d.dtau < INFINITY) | (interior & (d.dtau >= L.tau)))
+		if(d.invalid | !(d.dtau >= 0.0) | !(d.dtau < INFINITY))
 			verdict = VERDICT_STOP;
+		else if(interior & (d.dtau >= L.tau))
+			verdict = VERDICT_SCATTER;
 		if(interior && ((d.dtau > tau_limit) | (!capture_mode & (apart > (DMS_OPTICAL_DEPTH_REL_TOL * (1.0 - 0x1p-50)) * scale))) && !d.invalid &&
 		   d.dtau >= 0.0 && d.dtau < INFINITY)
 		{
@@ -880,7 +884,7 @@ __device__ __forceinline__ int team_judge(const RunParams& R, const TeamBox& b, 
 			if(L.retries < DMS_MAX_OPTICAL_DEPTH_RETRIES)
 			{
 				const int rejected = depth_reject(L, c.before, d.dtau, apart, scale, capture_mode != 0, c.dt, tau_limit);
-				verdict = rejected == PH_STEP ? VERDICT_RESTART : (d.dtau >= L.tau ? VERDICT_STOP : VERDICT_PLAIN);
+				verdict = rejected == PH_STEP ? VERDICT_RESTART : (d.dtau >= L.tau ? VERDICT_SCATTER : VERDICT_PLAIN);
 			}
 		}
 		if(verdict == VERDICT_PLAIN && c.r_after >= R.boundary)
@@ -936,7 +940,7 @@ __device__ __forceinline__ int team_loop(const RunParams& R, TeamBox& b, StrictL
 		{
 			if(have)
 			{
-				int v = VERDICT_STOP;
+				int v = VERDICT_PAUSE;
 				if(pass < TEAM_MAX_STEPS)
 					v = team_judge(R, b, b.s[j & 3], b.e[j & 3], b.s[(j + 1) & 3], b.e[(j + 1) & 3], L, mine, buffer, c);
 				if(mine)
@@ -1122,9 +1126,10 @@ struct StrictStep
 		team_barrier();
 	}
 	// Steps of the lone lane made by the team; the lane's state is that at the start of a step before and
-	// after (or `phase`, its phase, says otherwise).  Returns the number of steps made.
-	__device__ __noinline__ int team_run(const RunParams& R, const DevPoint* __restrict__ P, double m_dm, StrictLane& L, double2* hist, bool mine,
-	                                     double* buffer, int& phase) const
+	// after (or `phase`, its phase, says otherwise).  Adds the number of steps to `iter`; returns whether
+	// the lane must make its next step alone.
+	__device__ __noinline__ bool team_run(const RunParams& R, const DevPoint* __restrict__ P, double m_dm, StrictLane& L, double2* hist, bool mine,
+	                                     double* buffer, int& phase, uint64_t& iter) const
 	{
 		TeamBox& b = team_box();
 		if(mine && !L.next_valid)
@@ -1133,7 +1138,7 @@ struct StrictStep
 		const bool fit = mine && (L.pr.radial_mode == 0) & (L.pr.J > 0x1p-200) & (L.pr.J < 0x1p200) &
 		                                          fast::in_radius_range(L.pr.radius) & (fabs(L.pr.phi) < 0x1p20);
 		if(!__any_sync(0xffffffffu, fit))
-			return 0;
+			return true;
 		if(mine)
 		{
 			b.P = P;
@@ -1171,7 +1176,7 @@ struct StrictStep
 		team_barrier();
 		StepCtx c;
 		int last = VERDICT_PLAIN;
-		int j = team_loop(R, b, L, 0, mine, buffer, c, last);
+		const int j = team_loop(R, b, L, 0, mine, buffer, c, last);
 		team_barrier();  // the committing warp has written its part back
 		if(mine)
 		{
@@ -1199,25 +1204,32 @@ struct StrictStep
 			L.max_drift_eV = b.max_drift_eV;
 			L.max_drift_rel = b.max_drift_rel;
 		}
-		// a step that ends at the boundary is finished here with what the team made of it, as in strict_step
-		if(last == VERDICT_BOUNDARY)
+		// a step that ends at the boundary or in a scattering is finished here with what the team made of it,
+		// as in strict_step
+		if(mine && (last == VERDICT_BOUNDARY || last == VERDICT_SCATTER))
 		{
-			if(mine)
+			Event accepted = c.after;
+			int boundary = BOUNDARY_INSIDE;
+			if(last == VERDICT_BOUNDARY)
+				boundary = boundary_step(R, m_dm, L, hist, c, accepted);
+			else
 			{
-				Event accepted = c.after;
-				const int boundary = boundary_step(R, m_dm, L, hist, c, accepted);
-				if(boundary == BOUNDARY_FAILURE)
-					phase = PH_FINAL;
-				else if(boundary != BOUNDARY_RETURN)
-				{
-					const TeamState& n = b.s[(j + 1) & 3];
-					phase = finish_step(R, m_dm, L, hist, c, accepted, false, boundary, n.time, n.radius, n.phi, n.v_radial, n.step, n.rate, true);
-				}
+				const bool depth = c.s1 > c.s0;
+				scatter_point(R.S, P, c, L.next_rate, depth && c.r_before < DMS_RSUN_KM && c.s0 <= 1.0e-12, depth,
+				              R.capture_mode ? DMS_CAPTURE_OPTICAL_DEPTH_PIECES : DMS_MAX_OPTICAL_DEPTH_PIECES, L.tau, accepted);
 			}
-			j++;
+			if(boundary == BOUNDARY_FAILURE)
+				phase = PH_FINAL;
+			else if(boundary != BOUNDARY_RETURN)
+			{
+				const TeamState& n = b.s[(j + 1) & 3];
+				phase = finish_step(R, m_dm, L, hist, c, accepted, last == VERDICT_SCATTER, boundary, n.time, n.radius, n.phi, n.v_radial, n.step,
+				                    n.rate, true);
+			}
 		}
 		__syncwarp();
-		return j;
+		iter += j;
+		return last == VERDICT_STOP;
 	}
 	__device__ __forceinline__ double channel(const DevSolar& S, const DevPoint* __restrict__ P, int i, double dr, double T, double v, int k) const
 	{

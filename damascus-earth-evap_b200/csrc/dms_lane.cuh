@@ -228,7 +228,7 @@ __device__ __forceinline__ int segment_start(const RunParams& R, const DevPoint*
 	Event local = L.cur;
 	local.t = 0.0;
 	init_propagator(L.pr, local);
-	L.tau = -dms_log(L.D.positive_unit());
+	L.tau = -log_call(draw_positive(L.D));
 	L.seg_steps = 0;
 	L.retries = 0;
 	L.before_valid = 0;
@@ -660,13 +660,13 @@ __device__ __forceinline__ int finish_scatter(const RunParams& R, const DevPoint
 		return PH_FINAL;
 	}
 	L.nscat++;
-	const bool captured = update_capture_state(R.S, m_dm, R.capture_mode, L, ev_radius(L.cur), ev_speed(L.cur), L.cur.t, true);
+	const double r = ev_radius(L.cur), v = ev_speed(L.cur);
+	const bool captured = update_capture_state(R.S, m_dm, R.capture_mode, L, r, v, L.cur.t, true);
 	if(!R.capture_mode)
 	{
 		// Reset_Bincount_Anchor, src/Simulation_Trajectory.cpp:671-680
 		L.prev_time = L.cur.t;
-		L.prev_r = ev_radius(L.cur);
-		const double v = ev_speed(L.cur);
+		L.prev_r = r;
 		L.prev_v2 = v * v;
 	}
 	if(R.capture_mode && captured)
@@ -725,6 +725,7 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 	for(uint64_t iter = 0;; iter++)
 	{
 		bool go_scatter = false, go_final = false;
+		bool alone = !team;  // the lanes make this pass's steps themselves
 		if(Step::lockstep && lockstep)
 		{
 			int* v = votes[iter & 1];
@@ -808,12 +809,13 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 			if constexpr(Step::team)
 			{
 				const bool mine = phase == PH_STEP && !L.in_rk;
+				alone |= __any_sync(FULL_WARP, phase == PH_STEP && L.in_rk);
 				if((live & (live - 1u)) == 0u && __any_sync(FULL_WARP, mine) && R.wall_limit_ns == 0)
 				{
 					if(!team)
 						team = step.team_form();
 					if(team)
-						iter += step.team_run(R, P, m_dm, L, hist, mine, rates, phase);
+						alone = step.team_run(R, P, m_dm, L, hist, mine, rates, phase, iter);
 				}
 			}
 			const unsigned int stepping = __ballot_sync(FULL_WARP, phase == PH_STEP || phase == PH_FETCH || phase == PH_SEGMENT);
@@ -884,7 +886,7 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 		}
 		if(phase == PH_SEGMENT)
 			phase = segment_start(R, P, m_dm, L);
-		if(__any_sync(FULL_WARP, phase == PH_STEP))
+		if(alone && __any_sync(FULL_WARP, phase == PH_STEP))
 			phase = step(R, P, m_dm, L, hist, phase, rates);
 	}
 	const bool in_trajectory = phase != PH_FETCH && phase != PH_DONE;

@@ -208,13 +208,18 @@ int Check_Run_Opts(dms_ctx* ctx, const dms_run_opts* o)
 	return DMS_OK;
 }
 
-// The lane-scheduling options of a launch (dms_run_opts, 0 = default).
-void Apply_Lane_Options(RunParams& p, const dms_run_opts* o)
+// The lane-scheduling options of a launch (dms_run_opts, 0 = default).  In lockstep the whole block makes a
+// rare phase together, so larger batches pay.  Measured there (FP64; batch / wait of the scatterings, batch of
+// the terminations: 16 / 32, 8 against 24 / 64, 16): Capture mode m = 0.3 GeV, 1e-36 cm^2, 2^20 trajectories
+// 45.1 / 41.0 ms, m = 1 GeV, 1e-35 cm^2 48.5 / 44.4 ms, steady state at m = 0.1 GeV, 1e-33 cm^2 890 / 949
+// million steps/s.  The mixed form's scatterings are cheaper: its steady states lose 2-6 % by longer waits.
+void Apply_Lane_Options(RunParams& p, const dms_run_opts* o, bool lockstep)
 {
+	const bool patient = lockstep && o->precision == DMS_PRECISION_FP64;
 	p.queue_chunk = o->queue_chunk ? o->queue_chunk : 1u;
-	p.scatter_batch = o->scatter_batch ? static_cast<int>(o->scatter_batch) : 16;
-	p.scatter_wait = o->scatter_wait ? static_cast<int>(o->scatter_wait) : 32;
-	p.final_batch = o->final_batch ? static_cast<int>(o->final_batch) : 8;
+	p.scatter_batch = o->scatter_batch ? static_cast<int>(o->scatter_batch) : patient ? 24 : 16;
+	p.scatter_wait = o->scatter_wait ? static_cast<int>(o->scatter_wait) : patient ? 64 : 32;
+	p.final_batch = o->final_batch ? static_cast<int>(o->final_batch) : lockstep ? 16 : 8;
 	p.final_wait = o->final_wait ? static_cast<int>(o->final_wait) : 32;
 }
 
@@ -244,9 +249,9 @@ int Launch_And_Wait(dms_ctx* ctx, const dms_run_opts* o, RunParams& p)
 	p.wall_limit_ns = static_cast<uint64_t>(o->max_trajectory_wall_time_s * 1.0e9);
 	if(o->max_trajectory_wall_time_s > 0.0 && p.wall_limit_ns == 0)
 		p.wall_limit_ns = 1;
-	Apply_Lane_Options(p, o);
 	const bool mixed = o->precision == DMS_PRECISION_MIXED;
 	const int threads = Block_Threads(o, p.total, ctx->sm_count);
+	Apply_Lane_Options(p, o, threads > LATENCY_THREADS);
 	int blocks = ctx->sm_count;
 	// a launch with fewer trajectories than lanes spreads them over the SMs and then over the warps: fewer
 	// lanes per warp diverge less, its idle lanes help in the collective steps, and the warps of a block
@@ -1336,7 +1341,7 @@ int dms_run_records_noalloc(dms_ctx* ctx, const dms_run_opts* opts, int point_id
 		p.wall_limit_ns = 1;
 	p.ic_max_attempts = 1 << 20;
 	p.lanes_per_block = 1;
-	Apply_Lane_Options(p, opts);
+	Apply_Lane_Options(p, opts, false);
 	p.counters = ctx->d_counters;
 	p.hists = ctx->d_hists;
 	p.events = ctx->d_events;

@@ -385,131 +385,153 @@ __device__ __forceinline__ Vec3 div3_fast(const Vec3& a, double n)
 	return q;
 }
 __device__ __forceinline__ Vec3 normalized3_fast(const Vec3& a) { return div3_fast(a, norm3(a)); }
+static __device__ __noinline__ void normalize_call(Vec3& a) { a = normalized3_fast(a); }
+
+// (2n - 1)^2, (2n)(2n + 1) and the latter's correctly rounded reciprocal, n = 1 ... 30: the term ratios of
+// dms_asin_small.
+struct AsinTerm
+{
+	double square, divisor, inverse;
+};
+#define DMS_ASIN_TERM(n) {(2.0 * (n) - 1.0) * (2.0 * (n) - 1.0), (2.0 * (n)) * (2.0 * (n) + 1.0), 1.0 / ((2.0 * (n)) * (2.0 * (n) + 1.0))}
+__constant__ AsinTerm ASIN_TERMS[30] = {
+	DMS_ASIN_TERM(1), DMS_ASIN_TERM(2), DMS_ASIN_TERM(3), DMS_ASIN_TERM(4), DMS_ASIN_TERM(5), DMS_ASIN_TERM(6),
+	DMS_ASIN_TERM(7), DMS_ASIN_TERM(8), DMS_ASIN_TERM(9), DMS_ASIN_TERM(10), DMS_ASIN_TERM(11), DMS_ASIN_TERM(12),
+	DMS_ASIN_TERM(13), DMS_ASIN_TERM(14), DMS_ASIN_TERM(15), DMS_ASIN_TERM(16), DMS_ASIN_TERM(17), DMS_ASIN_TERM(18),
+	DMS_ASIN_TERM(19), DMS_ASIN_TERM(20), DMS_ASIN_TERM(21), DMS_ASIN_TERM(22), DMS_ASIN_TERM(23), DMS_ASIN_TERM(24),
+	DMS_ASIN_TERM(25), DMS_ASIN_TERM(26), DMS_ASIN_TERM(27), DMS_ASIN_TERM(28), DMS_ASIN_TERM(29), DMS_ASIN_TERM(30)};
+
+// dms_acos out of line, its series as a loop whose quotients by the constants of the table need no division
+// (the same bits: a term too small for the straight-line quotient is lost against the argument).
+static __device__ __noinline__ double acos_call(double x)
+{
+	if(!(x >= -1.0 && x <= 1.0))
+		return NAN;
+	const bool middle = x <= 0.5 && x >= -0.5;
+	const double t = middle ? x : sqrt((x > 0.5 ? 1.0 - x : 1.0 + x) * 0.5);
+	const double z = t * t;
+	double term = t, sum = 0.0;
+#pragma unroll 1
+	for(int n = 0; n < 30; n++)
+	{
+		const AsinTerm& c = ASIN_TERMS[n];
+		const double a = term * z * c.square;
+		const double q = __dmul_rn(a, c.inverse);
+		const double q1 = __fma_rn(__fma_rn(-c.divisor, q, a), c.inverse, q);
+		term = __fma_rn(__fma_rn(-c.divisor, q1, a), c.inverse, q1);
+		sum += term;
+	}
+	const double s = t + sum;
+	return middle ? 0.5 * DMS_PI - s : (x > 0.5 ? 2.0 * s : DMS_PI - 2.0 * s);
+}
 
 // ---------------------------------------------------------------------------------------------
 // Standard Halo Model and initial conditions, src/Simulation_Utilities.cpp:123-249
-__device__ __forceinline__ double halo_pdf_speed(const DevPoint* __restrict__ P, double v)
+// The halo sampler of one trajectory (Initial_Conditions, src/Simulation_Utilities.cpp:176-249) as a state
+// machine of single rejection tries, so that the lanes of a warp can make the same kind of try together.
+// What depends on the point alone is formed once per lane (Sampler); every value is formed by the
+// reference's operations in its order.
+struct Sampler
 {
-	const double v0 = __ldg(&P->v0), vesc = __ldg(&P->vesc_halo), vobs = __ldg(&P->vobs);
-	if(v < 0.0 || v > vesc + vobs)
+	double v0, vesc, vobs, n_esc;
+	Vec3 vo;               // the Sun's velocity in the halo frame
+	Vec3 e1, e2, e3;       // the stable frame about it (libphysica::Spherical_Coordinates restated)
+	double v0v0, fall;     // v0^2; exp(-v_esc^2 / v0^2), the pdf's term beyond the escape speed
+	double speed_norm;     // n_esc sqrt(pi) v0 v_obs
+	double vesc_sun;       // the local escape speed at the surface
+	double flux_norm;      // the normalisation of the flux-weighted speed
+	double v_max, v_sun;
+};
+
+static __device__ __noinline__ void sampler_init(const DevSolar& S, const DevPoint* __restrict__ P, Sampler& h)
+{
+	h.v0 = __ldg(&P->v0);
+	h.vesc = __ldg(&P->vesc_halo);
+	h.vobs = __ldg(&P->vobs);
+	h.n_esc = __ldg(&P->n_esc);
+	h.vo = mk(__ldg(&P->vel_obs[0]), __ldg(&P->vel_obs[1]), __ldg(&P->vel_obs[2]));
+	h.v_sun = norm3(h.vo);
+	h.v_max = h.vesc + h.vobs;
+	h.e3 = (h.v_sun > 0.0) ? h.vo : mk(0.0, 0.0, 1.0);
+	normalize_call(h.e3);
+	h.e1 = cross3((fabs(h.e3.z) < 0.9) ? mk(0.0, 0.0, 1.0) : mk(1.0, 0.0, 0.0), h.e3);
+	normalize_call(h.e1);
+	h.e2 = cross3(h.e3, h.e1);
+	normalize_call(h.e2);
+	h.v0v0 = h.v0 * h.v0;
+	h.fall = exp(-h.vesc * h.vesc / h.v0v0);
+	h.speed_norm = h.n_esc * sqrt(DMS_PI) * h.v0 * h.vobs;
+	h.vesc_sun = solar_vesc(S, DMS_RSUN_KM);
+	h.flux_norm = __ldg(&P->avg_speed) + h.vesc_sun * h.vesc_sun * __ldg(&P->eta0);
+}
+
+// Standard Halo Model speed and velocity densities, src/Simulation_Utilities.cpp:123-175
+static __device__ __noinline__ double halo_pdf_speed(const Sampler& h, double v)
+{
+	if(v < 0.0 || v > h.vesc + h.vobs)
 		return 0.0;
-	const double dm = v - vobs;
-	const double dp = v + vobs;
-	const double a = exp(-dm * dm / (v0 * v0));
-	const double b = (dp <= vesc) ? exp(-dp * dp / (v0 * v0)) : exp(-vesc * vesc / (v0 * v0));
-	return v / (__ldg(&P->n_esc) * sqrt(DMS_PI) * v0 * vobs) * (a - b);
+	const double dm = v - h.vobs;
+	const double dp = v + h.vobs;
+	const double a = exp(-dm * dm / h.v0v0);
+	const double b = (dp <= h.vesc) ? exp(-dp * dp / h.v0v0) : h.fall;
+	return v / h.speed_norm * (a - b);
 }
 
-__device__ __forceinline__ double halo_pdf_velocity(const DevPoint* __restrict__ P, const Vec3& vel)
-{
-	const double v0 = __ldg(&P->v0), vesc = __ldg(&P->vesc_halo);
-	const Vec3 w = add3(vel, mk(__ldg(&P->vel_obs[0]), __ldg(&P->vel_obs[1]), __ldg(&P->vel_obs[2])));
-	const double w2 = dot3(w, w);
-	if(w2 > vesc * vesc)
-		return 0.0;
-	return exp(-w2 / (v0 * v0)) / (__ldg(&P->n_esc) * 5.5683279968317078453 * v0 * v0 * v0);
-}
-
-// libphysica::Spherical_Coordinates restated (stable frame about `axis`)
-__device__ __forceinline__ Vec3 spherical_coordinates(double r, double theta, double phi, const Vec3& axis)
-{
-	const Vec3 e3 = div3(axis, norm3(axis));
-	const Vec3 ref = (fabs(e3.z) < 0.9) ? mk(0.0, 0.0, 1.0) : mk(1.0, 0.0, 0.0);
-	const Vec3 e1 = normalized3(cross3(ref, e3));
-	const Vec3 e2 = normalized3(cross3(e3, e1));
-	double st, ct, sp, cp;
-	dms_sincos(theta, &st, &ct);
-	dms_sincos(phi, &sp, &cp);
-	return mk(r * (st * cp * e1.x + st * sp * e2.x + ct * e3.x), r * (st * cp * e1.y + st * sp * e2.y + ct * e3.y),
-	          r * (st * cp * e1.z + st * sp * e2.z + ct * e3.z));
-}
-
-__device__ __forceinline__ double pdf_initial_speed(const DevSolar& S, const DevPoint* __restrict__ P, double v)
+__device__ __forceinline__ double pdf_initial_speed(const Sampler& h, double v)
 {
 	if(v == 0.0)
 		return 0.0;
-	const double v_esc = solar_vesc(S, DMS_RSUN_KM);
-	const double normalization = __ldg(&P->avg_speed) + v_esc * v_esc * __ldg(&P->eta0);
-	const double f = halo_pdf_speed(P, v);
-	return (f * v + (f / v) * v_esc * v_esc) / normalization;
+	const double f = halo_pdf_speed(h, v);
+	return (f * v + (f / v) * h.vesc_sun * h.vesc_sun) / h.flux_norm;
 }
 
-__device__ __forceinline__ double pdf_cos_theta(const DevPoint* __restrict__ P, double cos_theta, double v)
+// r (sin(theta) cos(phi) e1 + sin(theta) sin(phi) e2 + cos(theta) e3)
+__device__ __forceinline__ Vec3 spherical_vector(const Sampler& h, double r, double theta, double sp, double cp)
 {
-	const double f = halo_pdf_speed(P, v);
-	const double normalization = 2.0 * DMS_PI * v * v / f;
-	const Vec3 vo = mk(__ldg(&P->vel_obs[0]), __ldg(&P->vel_obs[1]), __ldg(&P->vel_obs[2]));
-	const Vec3 axis = (norm3(vo) > 0.0) ? vo : mk(0.0, 0.0, 1.0);
-	const Vec3 vel = spherical_coordinates(v, dms_acos(cos_theta), 0.0, axis);
-	return normalization * halo_pdf_velocity(P, vel);
+	double st, ct;
+	sincos_call(theta, st, ct);
+	return mk(r * (st * cp * h.e1.x + st * sp * h.e2.x + ct * h.e3.x), r * (st * cp * h.e1.y + st * sp * h.e2.y + ct * h.e3.y),
+	          r * (st * cp * h.e1.z + st * sp * h.e2.z + ct * h.e3.z));
 }
 
-// Initial_Conditions, src/Simulation_Utilities.cpp:176-249.  Returns false when a rejection
-// loop exceeds `max_attempts` (the reference loops without bound).
-static __device__ __noinline__ bool initial_conditions(const DevSolar& S, const DevPoint* __restrict__ P, Draws& D, Event& e, int max_attempts)
+// The density of cos(theta) at speed v; normalization = 2 pi v^2 / (halo speed density).
+static __device__ __noinline__ double pdf_cos_theta(const Sampler& h, double cos_theta, double v, double normalization)
 {
-	const double y_max_speed = DMS_IC_SPEED_YMAX_NATURAL / DMS_C_KMS;
-	const double v_max = __ldg(&P->vesc_halo) + __ldg(&P->vobs);
-	double u = 0.0;
-	bool ok = false;
-	for(int a = 0; a < max_attempts; a++)
-	{
-		const double x = D.uniform(0.0, v_max);
-		const double y = D.uniform(0.0, y_max_speed);
-		if(y <= pdf_initial_speed(S, P, x))
-		{
-			u = x;
-			ok = true;
-			break;
-		}
-	}
-	if(!ok)
-		return false;
-	const Vec3 vo = mk(__ldg(&P->vel_obs[0]), __ldg(&P->vel_obs[1]), __ldg(&P->vel_obs[2]));
-	const double v_sun = norm3(vo);
-	const double v_gal = v_max - v_sun;
-	double cos_theta_max = (v_sun == 0.0) ? 1.0 : (v_gal * v_gal - v_sun * v_sun - u * u) / (2.0 * u * v_sun);
-	if(cos_theta_max > 1.0)
-		cos_theta_max = 1.0;
-	const double y_max = pdf_cos_theta(P, -1.0, u);
-	double cos_theta = 0.0;
-	ok = false;
-	for(int a = 0; a < max_attempts; a++)
-	{
-		const double x = D.uniform(-1.0, cos_theta_max);
-		const double y = D.uniform(0.0, y_max);
-		if(y <= pdf_cos_theta(P, x, u))
-		{
-			cos_theta = x;
-			ok = true;
-			break;
-		}
-	}
-	if(!ok)
-		return false;
-	const double phi = D.uniform(0.0, 2.0 * DMS_PI);
-	const Vec3 axis = (v_sun > 0.0) ? vo : mk(0.0, 0.0, 1.0);
-	Vec3 velocity = spherical_coordinates(u, dms_acos(clamp_cos(cos_theta)), phi, axis);
+	const Vec3 w = add3(spherical_vector(h, v, acos_call(cos_theta), 0.0, 1.0), h.vo);
+	const double w2 = dot3(w, w);
+	double density = 0.0;
+	if(!(w2 > h.vesc * h.vesc))
+		density = exp(-w2 / h.v0v0) / (h.n_esc * 5.5683279968317078453 * h.v0 * h.v0 * h.v0);
+	return normalization * density;
+}
+
+// The rest of Initial_Conditions from the accepted speed u and cosine.
+static __device__ __noinline__ void initial_event(const DevSolar& S, const Sampler& h, Draws& D, double u, double cos_theta, Event& e)
+{
+	double s, c;
+	sincos_call(draw_between(D, 0.0, 2.0 * DMS_PI), s, c);
+	Vec3 velocity = spherical_vector(h, u, acos_call(clamp_cos(cos_theta)), s, c);
 	const double asymptotic_distance = DMS_IC_ASYMPTOTIC_DISTANCE_AU * DMS_AU_KM;
 	const double vesc_asymptotic = solar_vesc(S, asymptotic_distance);
 	const double v = sqrt(u * u + vesc_asymptotic * vesc_asymptotic);
-	velocity = scale3(v, normalized3(velocity));
-	const double v_esc = solar_vesc(S, DMS_RSUN_KM);
-	const double b_max = sqrt(u * u + v_esc * v_esc) / v * DMS_RSUN_KM;
-	const Vec3 e_z = scale3(-1.0, normalized3(velocity));
-	const Vec3 ref = (fabs(e_z.z) < 0.9) ? mk(0.0, 0.0, 1.0) : mk(1.0, 0.0, 0.0);
-	const Vec3 e_x = normalized3(cross3(ref, e_z));
-	const Vec3 e_y = normalized3(cross3(e_z, e_x));
-	const double phi_disk = D.uniform(0.0, 2.0 * DMS_PI);
-	const double xi = D.uniform(0.0, 1.0);
+	normalize_call(velocity);
+	velocity = scale3(v, velocity);
+	const double b_max = sqrt(u * u + h.vesc_sun * h.vesc_sun) / v * DMS_RSUN_KM;
+	Vec3 e_z = velocity;
+	normalize_call(e_z);
+	e_z = scale3(-1.0, e_z);
+	Vec3 e_x = cross3((fabs(e_z.z) < 0.9) ? mk(0.0, 0.0, 1.0) : mk(1.0, 0.0, 0.0), e_z);
+	normalize_call(e_x);
+	Vec3 e_y = cross3(e_z, e_x);
+	normalize_call(e_y);
+	const double phi_disk = draw_between(D, 0.0, 2.0 * DMS_PI);
+	const double xi = draw_unit(D);
 	const double b = sqrt(xi) * b_max;
-	double s, c;
-	dms_sincos(phi_disk, &s, &c);
+	sincos_call(phi_disk, s, c);
 	e.t = 0.0;
 	e.x = mk(asymptotic_distance * e_z.x + b * (c * e_x.x + s * e_y.x), asymptotic_distance * e_z.y + b * (c * e_x.y + s * e_y.y),
 	         asymptotic_distance * e_z.z + b * (c * e_x.z + s * e_y.z));
 	e.v = velocity;
-	return true;
 }
 
 __device__ __forceinline__ bool finite_positive(double x) { return isfinite(x) && x > 0.0; }
@@ -537,7 +559,7 @@ static __device__ __noinline__ bool hyperbolic_kepler_shift(Event& e, double R_f
 	const double energy = 0.5 * speed * speed - mu / R_initial;
 	if(!finite_positive(energy))
 		return false;
-	const Vec3 r_hat = div3(e.x, R_initial);
+	const Vec3 r_hat = div3_fast(e.x, R_initial);
 	const Vec3 h_vec = cross3(e.x, e.v);
 	const double h = norm3(h_vec);
 	const double h_scale = R_initial * speed;
@@ -551,24 +573,25 @@ static __device__ __noinline__ bool hyperbolic_kepler_shift(Event& e, double R_f
 		return true;
 	}
 	const double p = h * h / mu;
-	const Vec3 ecc_vec = sub3(div3(cross3(e.v, h_vec), mu), r_hat);
+	const Vec3 ecc_vec = sub3(div3_fast(cross3(e.v, h_vec), mu), r_hat);
 	const double ecc = norm3(ecc_vec);
 	if(!finite_positive(p) || !isfinite(ecc) || ecc <= 1.0)
 		return false;
 	const double cos_final = (p / R_final - 1.0) / ecc;
 	if(!isfinite(cos_final) || cos_final > 1.0 + DMS_KEPLER_DOMAIN_TOLERANCE || cos_final < -1.0 - DMS_KEPLER_DOMAIN_TOLERANCE)
 		return false;
-	Vec3 ax = div3(ecc_vec, ecc);
-	const Vec3 az = div3(h_vec, h);
+	Vec3 ax = div3_fast(ecc_vec, ecc);
+	const Vec3 az = div3_fast(h_vec, h);
 	Vec3 ay = cross3(az, ax);
 	const double ny = norm3(ay);
 	if(!finite_positive(ny))
 		return false;
-	ay = div3(ay, ny);
-	ax = normalized3(cross3(ay, az));
-	const double theta = dir * dms_acos(clamp_cos(cos_final));
+	ay = div3_fast(ay, ny);
+	ax = cross3(ay, az);
+	normalize_call(ax);
+	const double theta = dir * acos_call(clamp_cos(cos_final));
 	double st, ct;
-	dms_sincos(theta, &st, &ct);
+	sincos_call(theta, st, ct);
 	const double sq = sqrt(mu / p);
 	e.x = mk(R_final * (ct * ax.x + st * ay.x), R_final * (ct * ax.y + st * ay.y), R_final * (ct * ax.z + st * ay.z));
 	e.v = mk(sq * (-st * ax.x + (ecc + ct) * ay.x), sq * (-st * ax.y + (ecc + ct) * ay.y), sq * (-st * ax.z + (ecc + ct) * ay.z));
@@ -1089,7 +1112,11 @@ static __device__ __noinline__ bool bound_kepler_return(const Event& out, Event&
 	if(ecc <= 1.0e-14 || ecc >= 1.0)
 		return false;
 	const double cosE = clamp_cos((1.0 - radius / a) / ecc);
-	const double Eanom = dms_acos(cosE);
+#ifdef DMS_FMA_CONTRACTION
+	const double Eanom = dms_acos(cosE);  // contracted across the call in the mixed kernels: in place, for the same bits
+#else
+	const double Eanom = acos_call(cosE);
+#endif
 	const double one_minus = 1.0 - cosE * cosE;
 	const double sinE = sqrt(one_minus > 0.0 ? one_minus : 0.0);
 	const double n = sqrt(mu / (a * a * a));
@@ -1098,7 +1125,7 @@ static __device__ __noinline__ bool bound_kepler_return(const Event& out, Event&
 	const double T = (2.0 * DMS_PI - 2.0 * Eanom + 2.0 * ecc * sinE) / n;
 	if(!isfinite(T) || T <= 0.0)
 		return false;
-	const Vec3 rhat = div3(out.x, radius);
+	const Vec3 rhat = div3_fast(out.x, radius);
 	in = out;
 	in.t += T;
 	in.v = sub3(out.v, scale3(2.0 * vr, rhat));

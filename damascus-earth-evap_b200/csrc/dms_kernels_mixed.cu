@@ -1,5 +1,6 @@
 // Mixed-precision trajectory kernel (the batched-FP32 form).  Compiled with FMA contraction;
 // shares the lane state machine (dms_lane.cuh) with the FP64 kernel.
+#define DMS_FMA_CONTRACTION 1
 #include "dms_device_mixed.cuh"
 #include "dms_lane.cuh"
 

@@ -208,7 +208,8 @@ typedef struct
 	 * a lane that reaches a scattering point (a termination) waits until scatter_batch
 	 * (final_batch) lanes of its warp are there, or it has waited scatter_wait (final_wait)
 	 * loop iterations, or no lane of the warp is stepping; then the warp runs the scattering
-	 * (termination) code once for all of them.  0 = defaults 16 / 32 / 8 / 32; batches up to
+	 * (termination) code once for all of them.  0 = defaults (16 / 32 / 8 / 32, longer in launches that
+	 * fill the GPU, where whole blocks of 512 lanes count in their stead); batches up to
 	 * 32, waits up to 1024. */
 	uint32_t scatter_batch;
 	uint32_t scatter_wait;

@@ -258,7 +258,7 @@ int Launch_And_Wait(dms_ctx* ctx, const dms_run_opts* o, RunParams& p)
 	// with a lone lane form a team
 	blocks = static_cast<int>(std::min<uint64_t>(blocks, p.total));
 	p.lanes_per_block = static_cast<int>(std::min<uint64_t>(threads, (p.total + blocks - 1) / blocks));
-	p.lockstep_min = threads / 16;
+	p.lockstep_min = threads > LATENCY_THREADS ? threads / 16 : 8;
 	const size_t lanes = static_cast<size_t>(blocks) * p.lanes_per_block;
 	int rc = Ensure_Lanes(ctx, lanes);
 	if(rc != DMS_OK)
@@ -1341,6 +1341,7 @@ int dms_run_records_noalloc(dms_ctx* ctx, const dms_run_opts* opts, int point_id
 		p.wall_limit_ns = 1;
 	p.ic_max_attempts = 1 << 20;
 	p.lanes_per_block = 1;
+	p.lockstep_min = 8;
 	Apply_Lane_Options(p, opts, false);
 	p.counters = ctx->d_counters;
 	p.hists = ctx->d_hists;

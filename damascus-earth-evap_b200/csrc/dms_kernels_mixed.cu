@@ -591,16 +591,18 @@ __device__ __forceinline__ int mixed_step(const RunParams& R, const DevPoint* __
 	return PH_STEP;
 }
 
-template <bool LOCKSTEP>
+template <bool THROUGHPUT>
 struct MixedStep
 {
-	static constexpr bool lockstep = LOCKSTEP;
+	static constexpr int threads = THROUGHPUT ? MAX_THREADS : LATENCY_THREADS;
+	// (in the latency form the barriers cost more than the fetches: 16 384 Capture-mode trajectories 2.8 / 3.0 ms)
+	static constexpr bool lockstep = THROUGHPUT;
 	static constexpr int buffer = COOP_BUFFER_F;
 	static constexpr bool team = false;
 	__device__ __forceinline__ int operator()(const RunParams& R, const DevPoint* __restrict__ P, double m_dm, MixedLane& L, double2* hist, int phase,
 	                                          double* buffer) const
 	{
-		return mixed_step<!LOCKSTEP>(R, P, m_dm, L, hist, phase, reinterpret_cast<float*>(buffer));
+		return mixed_step<!THROUGHPUT>(R, P, m_dm, L, hist, phase, reinterpret_cast<float*>(buffer));
 	}
 	__device__ __forceinline__ double channel(const DevSolar& S, const DevPoint* __restrict__ P, int i, double dr, double T, double v, int k) const
 	{

@@ -689,10 +689,10 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 	double2* hist = R.lane_hist + (static_cast<size_t>(blockIdx.x) * R.lanes_per_block + (takes_work ? slot : 0)) * DMS_NUM_BINS;
 	// per warp: the 64 channel rates of a scattering, or the steps and rates of Step's own lookups
 	constexpr int BUFFER = Step::buffer > DMS_NUM_TARGETS + 1 ? Step::buffer : DMS_NUM_TARGETS + 1;
-	__shared__ double coop_rates[(Step::lockstep ? MAX_THREADS : LATENCY_THREADS) / 32][BUFFER];
+	__shared__ double coop_rates[Step::threads / 32][BUFFER];
 	double* rates = coop_rates[threadIdx.x >> 5];
-	// Lockstep: the warps of a block with more than one warp per scheduler make every pass together,
-	// so that an instruction fetched once serves all of them.  The block votes on its rare phases:
+	// Lockstep: the warps of a block make every pass together, so that an instruction fetched once serves
+	// all of them (until few lanes are left: R.lockstep_min).  The block votes on its rare phases:
 	// lanes stepping, at a scattering point and at a termination, counted per pass (two sets, one
 	// being cleared while the other is filled).
 	__shared__ int votes[2][4];
@@ -749,11 +749,11 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 			const int n_step = v[0], n_scatter = v[1], n_final = v[2], flags = v[3];
 			if(threadIdx.x < 3)
 				votes[(iter & 1) ^ 1][threadIdx.x] = 0;
-			const int lanes = blockDim.x >> 5;
+			const int at_work = n_step + n_scatter + n_final, warps = blockDim.x >> 5;
 			passes_scatter++;
 			passes_final++;
-			go_scatter = n_scatter != 0 && (n_scatter >= R.scatter_batch * lanes / 2 || n_step == 0 || passes_scatter >= R.scatter_wait);
-			go_final = n_final != 0 && (n_final >= R.final_batch * lanes / 2 || n_step == 0 || passes_final >= R.final_wait);
+			go_scatter = n_scatter != 0 && (n_scatter >= R.scatter_batch * warps / 2 || n_step == 0 || passes_scatter >= R.scatter_wait);
+			go_final = n_final != 0 && (n_final >= R.final_batch * warps / 2 || n_step == 0 || passes_final >= R.final_wait);
 			if(go_scatter)
 				passes_scatter = 0;
 			if(go_final)
@@ -770,9 +770,9 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 				break;
 			}
 			// few lanes left and no more work: the warps go on by themselves
-			if((flags & 1) && n_step + n_scatter + n_final <= R.lockstep_min)
+			if((flags & 1) && at_work <= R.lockstep_min)
 				lockstep = false;
-			if(n_step + n_scatter + n_final == 0)
+			if(at_work == 0)
 				break;
 		}
 		else
@@ -822,18 +822,19 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 			const unsigned int waiting = __ballot_sync(FULL_WARP, phase == PH_SCATTER);
 			const unsigned int ending = __ballot_sync(FULL_WARP, phase == PH_FINAL);
 			// lanes wait until several lanes of the warp are there, or one has waited long enough, or no
-			// lane is stepping
+			// lane is stepping; batches and waits are for a full warp and shrink with the lanes at work
+			const int at_work = __popc(live);
 			if(waiting != 0u)
 			{
 				passes_scatter++;
-				go_scatter = __popc(waiting) >= R.scatter_batch || stepping == 0u || passes_scatter >= R.scatter_wait;
+				go_scatter = 32 * __popc(waiting) >= R.scatter_batch * at_work || stepping == 0u || 32 * passes_scatter >= R.scatter_wait * at_work;
 				if(go_scatter)
 					passes_scatter = 0;
 			}
 			if(ending != 0u)
 			{
 				passes_final++;
-				go_final = __popc(ending) >= R.final_batch || stepping == 0u || passes_final >= R.final_wait;
+				go_final = 32 * __popc(ending) >= R.final_batch * at_work || stepping == 0u || 32 * passes_final >= R.final_wait * at_work;
 				if(go_final)
 					passes_final = 0;
 			}

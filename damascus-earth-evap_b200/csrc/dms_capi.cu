@@ -58,6 +58,8 @@ struct dms_ctx
 	unsigned long long* d_refl_count = nullptr;
 	uint64_t event_capacity = 1ULL << 20;
 	// run scratch
+	char* d_work = nullptr;         // work ranges or records of a run; kept up to WORKSPACE_KEPT bytes
+	size_t work_capacity = 0;
 	double2* d_lane_hist = nullptr;
 	size_t lane_capacity = 0;
 	InitState* d_init = nullptr;    // initial state of every work index of a launch
@@ -165,6 +167,42 @@ int Grow_Points(dms_ctx* ctx, int needed)
 	return DMS_OK;
 }
 
+// Device memory for the work ranges or the records of one call.  Up to WORKSPACE_KEPT bytes the context's own
+// allocation, grown as needed and kept for the next call (one call runs at a time per context); larger ones
+// (records with histograms: 32 KB per trajectory) are the call's.
+constexpr size_t WORKSPACE_KEPT = size_t{16} << 20;
+struct Workspace
+{
+	char* p = nullptr;
+	bool own = false;
+	~Workspace()
+	{
+		if(own)
+			cudaFree(p);
+	}
+};
+
+int Take_Workspace(dms_ctx* ctx, size_t bytes, Workspace& w)
+{
+	if(bytes > WORKSPACE_KEPT)
+	{
+		DMS_CUDA(ctx, cudaMalloc(reinterpret_cast<void**>(&w.p), bytes));
+		w.own = true;
+		return DMS_OK;
+	}
+	if(bytes > ctx->work_capacity)
+	{
+		cudaFree(ctx->d_work);
+		ctx->d_work = nullptr;
+		ctx->work_capacity = 0;
+		const size_t cap = std::max<size_t>(bytes, 1 << 16);
+		DMS_CUDA(ctx, cudaMalloc(reinterpret_cast<void**>(&ctx->d_work), cap));
+		ctx->work_capacity = cap;
+	}
+	w.p = ctx->d_work;
+	return DMS_OK;
+}
+
 int Ensure_Lanes(dms_ctx* ctx, size_t lanes)
 {
 	if(lanes <= ctx->lane_capacity)
@@ -173,7 +211,7 @@ int Ensure_Lanes(dms_ctx* ctx, size_t lanes)
 	ctx->d_lane_hist = nullptr;
 	ctx->lane_capacity = 0;
 	DMS_CUDA(ctx, cudaMalloc(&ctx->d_lane_hist, sizeof(double2) * DMS_NUM_BINS * lanes));
-	DMS_CUDA(ctx, cudaMemset(ctx->d_lane_hist, 0, sizeof(double2) * DMS_NUM_BINS * lanes));
+	DMS_CUDA(ctx, cudaMemsetAsync(ctx->d_lane_hist, 0, sizeof(double2) * DMS_NUM_BINS * lanes, ctx->stream));
 	ctx->lane_capacity = lanes;
 	return DMS_OK;
 }
@@ -221,6 +259,14 @@ void Apply_Lane_Options(RunParams& p, const dms_run_opts* o, bool lockstep)
 	p.scatter_wait = o->scatter_wait ? static_cast<int>(o->scatter_wait) : patient ? 64 : 32;
 	p.final_batch = o->final_batch ? static_cast<int>(o->final_batch) : lockstep ? 16 : 8;
 	p.final_wait = o->final_wait ? static_cast<int>(o->final_wait) : 32;
+}
+
+// The pause between two looks at a launch in flight: none in its first half millisecond, then a fiftieth of
+// the time it has taken, 200 us at most.  (A fixed 200 us was a third of a small launch's time.)
+void Poll_Pause(std::chrono::steady_clock::duration elapsed)
+{
+	if(elapsed > std::chrono::microseconds(500))
+		std::this_thread::sleep_for(std::min<std::chrono::steady_clock::duration>(elapsed / 50, std::chrono::microseconds(200)));
 }
 
 // Threads of the one block per SM.  With a lane per trajectory in 128 threads, every warp has a
@@ -355,7 +401,7 @@ int Launch_And_Wait(dms_ctx* ctx, const dms_run_opts* o, RunParams& p)
 				cancelled_by_hook = true;
 			}
 		}
-		std::this_thread::sleep_for(std::chrono::microseconds(200));
+		Poll_Pause(now - start);
 	}
 	ctx->running = false;
 	float kernel_ms = 0.0f;
@@ -458,6 +504,7 @@ void dms_destroy(dms_ctx* ctx)
 	cudaFree(ctx->d_refl);
 	cudaFree(ctx->d_refl_count);
 	cudaFree(ctx->d_lane_hist);
+	cudaFree(ctx->d_work);
 	cudaFree(ctx->d_queue);
 	cudaFree(ctx->d_status);
 	if(ctx->h_cancel)
@@ -617,6 +664,7 @@ int dms_load_solar_model(dms_ctx* ctx, const char* path)
 	}
 	cudaFree(ctx->d_tables_f);
 	ctx->d_tables_f = df;
+	DMS_CUDA(ctx, cudaStreamSynchronize(cudaStreamLegacy));
 	ctx->tables = std::move(t);
 	ctx->has_solar = true;
 	return DMS_OK;
@@ -693,6 +741,7 @@ int dms_add_point(dms_ctx* ctx, const dms_point_params* params, int* point_id)
 		cudaFree(grid_f);
 		return Fail(ctx, DMS_ERR_CUDA, cudaGetErrorString(e1));
 	}
+	cudaStreamSynchronize(cudaStreamLegacy);  // the copies above, ahead of what runs on the context's stream
 	if(c.grid_n > 0)
 		Launch_Rate_Grid(ctx->dsolar, ctx->d_points + id, grid, c.grid_n, ctx->stream);
 	const cudaError_t e2 = cudaStreamSynchronize(ctx->stream);
@@ -729,6 +778,7 @@ int dms_set_rate_grid(dms_ctx* ctx, int point_id, const double* grid, uint32_t n
 	if(static_cast<int>(n) != ctx->points[point_id].grid_n)
 		return Fail(ctx, DMS_ERR_INVALID_ARGUMENT, "grid size does not match the point's interpolation_points");
 	DMS_CUDA(ctx, cudaMemcpy(ctx->d_grids[point_id], grid, sizeof(double) * n * n, cudaMemcpyHostToDevice));
+	DMS_CUDA(ctx, cudaStreamSynchronize(cudaStreamLegacy));  // the copy's last part may still be on its way
 	ctx->grid_f_valid[point_id] = 0;
 	return DMS_OK;
 }
@@ -814,19 +864,16 @@ int dms_run(dms_ctx* ctx, const dms_run_opts* opts, const dms_work_range* ranges
 	if(total == 0)
 		return DMS_OK;
 	std::vector<char> buf(sizeof(int32_t) * n_ranges + sizeof(uint64_t) * (2 * n_ranges + 1) + 16);
-	void* d = nullptr;
-	DMS_CUDA(ctx, cudaMalloc(&d, buf.size()));
-	char* dc = static_cast<char*>(d);
+	Workspace work;
+	rc = Take_Workspace(ctx, buf.size(), work);
+	if(rc != DMS_OK)
+		return rc;
+	char* dc = work.p;
 	const size_t off_first = 0, off_offset = sizeof(uint64_t) * n_ranges, off_point = sizeof(uint64_t) * (2 * n_ranges + 1);
 	std::memcpy(buf.data() + off_first, firsts.data(), sizeof(uint64_t) * n_ranges);
 	std::memcpy(buf.data() + off_offset, offsets.data(), sizeof(uint64_t) * (n_ranges + 1));
 	std::memcpy(buf.data() + off_point, pts.data(), sizeof(int32_t) * n_ranges);
-	cudaError_t e = cudaMemcpy(d, buf.data(), buf.size(), cudaMemcpyHostToDevice);
-	if(e != cudaSuccess)
-	{
-		cudaFree(d);
-		return Fail(ctx, DMS_ERR_CUDA, cudaGetErrorString(e));
-	}
+	DMS_CUDA(ctx, cudaMemcpyAsync(dc, buf.data(), buf.size(), cudaMemcpyHostToDevice, ctx->stream));
 	RunParams p{};
 	p.range_first = reinterpret_cast<const uint64_t*>(dc + off_first);
 	p.range_offset = reinterpret_cast<const uint64_t*>(dc + off_offset);
@@ -840,9 +887,7 @@ int dms_run(dms_ctx* ctx, const dms_run_opts* opts, const dms_work_range* ranges
 	p.event_capacity = ctx->event_capacity;
 	p.reflections = ctx->d_refl;
 	p.reflection_count = ctx->d_refl_count;
-	rc = Launch_And_Wait(ctx, opts, p);
-	cudaFree(d);
-	return rc;
+	return Launch_And_Wait(ctx, opts, p);
 }
 
 // ---- autotuner ------------------------------------------------------------------------------
@@ -1044,21 +1089,18 @@ int dms_run_records(dms_ctx* ctx, const dms_run_opts* opts, int point_id, uint64
 	const size_t hist_bytes = want_hist ? sizeof(double) * DMS_NUM_BINS * count : 0;
 	const size_t rec_bytes = sizeof(dms_traj_record) * count;
 	const size_t meta = 64;
-	char* d = nullptr;
-	DMS_CUDA(ctx, cudaMalloc(reinterpret_cast<void**>(&d), meta + rec_bytes + 2 * hist_bytes));
+	Workspace work;
+	rc = Take_Workspace(ctx, meta + rec_bytes + 2 * hist_bytes, work);
+	if(rc != DMS_OK)
+		return rc;
+	char* d = work.p;
 	struct Meta
 	{
 		uint64_t first, off0, off1;
 		int32_t point;
 	} m{first, 0, count, point_id};
-	cudaError_t e = cudaMemcpy(d, &m, sizeof m, cudaMemcpyHostToDevice);
-	if(e == cudaSuccess)
-		e = cudaMemset(d + meta, 0, rec_bytes + 2 * hist_bytes);
-	if(e != cudaSuccess)
-	{
-		cudaFree(d);
-		return Fail(ctx, DMS_ERR_CUDA, cudaGetErrorString(e));
-	}
+	DMS_CUDA(ctx, cudaMemcpyAsync(d, &m, sizeof m, cudaMemcpyHostToDevice, ctx->stream));
+	DMS_CUDA(ctx, cudaMemsetAsync(d + meta, 0, rec_bytes + 2 * hist_bytes, ctx->stream));
 	RunParams p{};
 	p.range_first = reinterpret_cast<const uint64_t*>(d);
 	p.range_offset = reinterpret_cast<const uint64_t*>(d + 8);
@@ -1078,7 +1120,7 @@ int dms_run_records(dms_ctx* ctx, const dms_run_opts* opts, int point_id, uint64
 	rc = Launch_And_Wait(ctx, opts, p);
 	if(rc == DMS_OK || rc == DMS_ERR_CANCELLED || rc == DMS_ERR_BUDGET)
 	{
-		e = cudaMemcpy(records, d + meta, rec_bytes, cudaMemcpyDeviceToHost);
+		cudaError_t e = cudaMemcpy(records, d + meta, rec_bytes, cudaMemcpyDeviceToHost);
 		if(e == cudaSuccess && want_hist)
 			e = cudaMemcpy(hist_dt, d + meta + rec_bytes, hist_bytes, cudaMemcpyDeviceToHost);
 		if(e == cudaSuccess && want_hist)
@@ -1086,7 +1128,6 @@ int dms_run_records(dms_ctx* ctx, const dms_run_opts* opts, int point_id, uint64
 		if(e != cudaSuccess)
 			rc = Fail(ctx, DMS_ERR_CUDA, cudaGetErrorString(e));
 	}
-	cudaFree(d);
 	return rc;
 }
 
@@ -1133,12 +1174,16 @@ int dms_reset_results(dms_ctx* ctx, int point_id)
 	if(point_id < 0 || point_id >= static_cast<int>(ctx->points.size()))
 		return Fail(ctx, DMS_ERR_NO_POINT, "no such point");
 	DMS_CUDA(ctx, cudaSetDevice(ctx->device));
-	DMS_CUDA(ctx, cudaMemset(ctx->d_counters + static_cast<size_t>(point_id) * DMS_NUM_COUNTERS, 0, sizeof(unsigned long long) * DMS_NUM_COUNTERS));
-	DMS_CUDA(ctx, cudaMemset(ctx->d_hists + static_cast<size_t>(point_id) * DMS_NUM_HISTS * DMS_NUM_BINS, 0, sizeof(double) * DMS_NUM_HISTS * DMS_NUM_BINS));
-	DMS_CUDA(ctx, cudaMemset(ctx->d_event_count + point_id, 0, sizeof(unsigned long long)));
-	DMS_CUDA(ctx, cudaMemset(ctx->d_refl_count + point_id, 0, sizeof(unsigned long long)));
-	DMS_CUDA(ctx, cudaMemset(ctx->d_events + static_cast<size_t>(point_id) * ctx->event_capacity, 0,
-	                         sizeof(dms_evaporation_event) * ctx->event_capacity));
+	// on the context's stream, ahead of the next launch; done before a reader looks
+	DMS_CUDA(ctx, cudaMemsetAsync(ctx->d_counters + static_cast<size_t>(point_id) * DMS_NUM_COUNTERS, 0, sizeof(unsigned long long) * DMS_NUM_COUNTERS,
+	                              ctx->stream));
+	DMS_CUDA(ctx, cudaMemsetAsync(ctx->d_hists + static_cast<size_t>(point_id) * DMS_NUM_HISTS * DMS_NUM_BINS, 0,
+	                              sizeof(double) * DMS_NUM_HISTS * DMS_NUM_BINS, ctx->stream));
+	DMS_CUDA(ctx, cudaMemsetAsync(ctx->d_event_count + point_id, 0, sizeof(unsigned long long), ctx->stream));
+	DMS_CUDA(ctx, cudaMemsetAsync(ctx->d_refl_count + point_id, 0, sizeof(unsigned long long), ctx->stream));
+	DMS_CUDA(ctx, cudaMemsetAsync(ctx->d_events + static_cast<size_t>(point_id) * ctx->event_capacity, 0,
+	                              sizeof(dms_evaporation_event) * ctx->event_capacity, ctx->stream));
+	DMS_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
 	return DMS_OK;
 }
 
@@ -1377,13 +1422,13 @@ int dms_run_records_noalloc(dms_ctx* ctx, const dms_run_opts* opts, int point_id
 			break;
 		if(q != cudaErrorNotReady)
 			return Fail(ctx, DMS_ERR_CUDA, std::string("trajectory kernel: ") + cudaGetErrorString(q));
-		if(opts->time_limit_s > 0.0 && !cancelled_by_limit &&
-		   std::chrono::duration<double>(std::chrono::steady_clock::now() - start).count() > opts->time_limit_s)
+		const auto elapsed = std::chrono::steady_clock::now() - start;
+		if(opts->time_limit_s > 0.0 && !cancelled_by_limit && std::chrono::duration<double>(elapsed).count() > opts->time_limit_s)
 		{
 			*reinterpret_cast<volatile int*>(ctx->h_cancel) = 1;
 			cancelled_by_limit = true;
 		}
-		std::this_thread::sleep_for(std::chrono::microseconds(200));
+		Poll_Pause(elapsed);
 	}
 	float kernel_ms = 0.0f;
 	DMS_CUDA(ctx, cudaEventElapsedTime(&kernel_ms, ctx->ev_start, ctx->ev_stop));

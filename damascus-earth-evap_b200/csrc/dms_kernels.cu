@@ -1108,6 +1108,7 @@ __global__ void __launch_bounds__(128) initial_state_kernel(const RunParams R, i
 template <bool THROUGHPUT>
 struct StrictStep
 {
+	static constexpr bool throughput = THROUGHPUT;
 	static constexpr int threads = THROUGHPUT ? MAX_THREADS : LATENCY_THREADS;
 	// in both forms: four warps with a scheduler each share the instruction cache too (4 096 histories of
 	// m = 1 GeV, 1e-35 cm^2 cut at 300 scatterings 196 -> 173 ms, 8 192 273 -> 208 ms)

@@ -13,6 +13,8 @@ constexpr int MAX_THREADS = 512;
 // Blocks of at most this many threads run the latency form of the kernels: one warp per scheduler, so
 // the registers are not shared out among 16 warps.
 constexpr int LATENCY_THREADS = 128;
+// Room for one parked lane state.
+constexpr size_t PARKED_BYTES = 1024;
 
 // Status bits written by the kernels (device status word).
 enum : unsigned int
@@ -70,7 +72,12 @@ struct RunParams
 	uint32_t queue_chunk;
 	int scatter_batch, scatter_wait, final_batch, final_wait;
 	int lanes_per_block; // lanes of a block that take trajectories (all, fewer in a spread launch)
-	int lockstep_min;    // lanes at work below which a block's warps leave the lockstep once the queue is empty
+	int lockstep_min;    // lanes at work at which a block's warps leave the lockstep once the queue is empty
+	// The tail of a throughput launch: a block with at most lockstep_min lanes at work and no more work parks
+	// their states (PARKED_BYTES each) and ends; a latency launch behind it resumes them.
+	unsigned char* parked;
+	unsigned int* parked_count;
+	int resume;          // 1: the lanes take the parked states instead of work indices
 	int ic_max_attempts;
 	// accumulators (accumulate mode)
 	unsigned long long* counters;   // n_points x DMS_NUM_COUNTERS

@@ -594,6 +594,7 @@ __device__ __forceinline__ int mixed_step(const RunParams& R, const DevPoint* __
 template <bool THROUGHPUT>
 struct MixedStep
 {
+	static constexpr bool throughput = THROUGHPUT;
 	static constexpr int threads = THROUGHPUT ? MAX_THREADS : LATENCY_THREADS;
 	// (in the latency form the barriers cost more than the fetches: 16 384 Capture-mode trajectories 2.8 / 3.0 ms)
 	static constexpr bool lockstep = THROUGHPUT;

@@ -678,6 +678,17 @@ __device__ __forceinline__ int finish_scatter(const RunParams& R, const DevPoint
 }
 
 
+// A trajectory in flight, handed from a throughput launch to the latency launch behind it.
+template <class Lane>
+struct Parked
+{
+	Lane L;
+	double2* hist;          // its histogram row
+	uint64_t q_next, q_end; // its lane's claimed ids
+	uint64_t iter;
+	int phase;
+};
+
 template <class Lane, class Step>
 __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 {
@@ -713,16 +724,47 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 	const DevPoint* P = R.points;
 	double m_dm = 0.0;
 	int phase = takes_work ? PH_FETCH : PH_DONE;
+	uint64_t iter = 0;
 	// the lane's claimed ids [q_next, q_end): R.queue_chunk ids per claim
 	uint64_t q_next = 0, q_end = 0;
 	const unsigned int lane_bit = 1u << (threadIdx.x & 31);
+	static_assert(sizeof(Parked<Lane>) <= PARKED_BYTES, "a parked state fits its slot");
+	if constexpr(!Step::throughput)
+		if(R.resume)
+		{
+			// the parked trajectories dealt out to the blocks one by one, and to the warps within
+			const unsigned int item = static_cast<unsigned int>(slot) * gridDim.x + blockIdx.x;
+			phase = PH_DONE;
+			if(item < *R.parked_count)
+			{
+				const Parked<Lane>& s = *reinterpret_cast<const Parked<Lane>*>(R.parked + item * PARKED_BYTES);
+				L = s.L;
+				hist = s.hist;
+				q_next = s.q_next;
+				q_end = s.q_end;
+				phase = s.phase;
+				iter = s.iter;
+				P = R.points + L.point;
+				m_dm = __ldg(&P->m_dm);
+			}
+			// one count per block: the warps in lockstep agree on it
+			__shared__ unsigned long long first_iter;
+			if(threadIdx.x == 0)
+				first_iter = 0;
+			__syncthreads();
+			atomicMax(&first_iter, static_cast<unsigned long long>(iter));
+			__syncthreads();
+			iter = first_iter;
+			next_check = iter + 1023;
+		}
 	// Every lane stays in the loop until its whole warp is done (a lane without work waits in
 	// PH_DONE), and leaves only together with the others.  So the warp's collective steps
 	// below (batching votes, cooperative target sampling into the warp's shared rates, the
 	// histogram flush) always run with all 32 lanes, a fixed mask, instead of whichever lanes
 	// happen to be converged at that point.
 	constexpr unsigned int FULL_WARP = 0xffffffffu;
-	for(uint64_t iter = 0;; iter++)
+	bool drained = false;
+	for(;; iter++)
 	{
 		bool go_scatter = false, go_final = false;
 		bool alone = !team;  // the lanes make this pass's steps themselves
@@ -749,11 +791,15 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 			const int n_step = v[0], n_scatter = v[1], n_final = v[2], flags = v[3];
 			if(threadIdx.x < 3)
 				votes[(iter & 1) ^ 1][threadIdx.x] = 0;
-			const int at_work = n_step + n_scatter + n_final, warps = blockDim.x >> 5;
+			drained |= (flags & 1) != 0;
+			// batches and waits are for a full block; in the tail of a throughput launch they shrink with the
+			// lanes at work
+			const int at_work = n_step + n_scatter + n_final, lanes = blockDim.x;
+			const int full = Step::throughput && drained ? at_work : lanes;
 			passes_scatter++;
 			passes_final++;
-			go_scatter = n_scatter != 0 && (n_scatter >= R.scatter_batch * warps / 2 || n_step == 0 || passes_scatter >= R.scatter_wait);
-			go_final = n_final != 0 && (n_final >= R.final_batch * warps / 2 || n_step == 0 || passes_final >= R.final_wait);
+			go_scatter = n_scatter != 0 && (64 * n_scatter >= R.scatter_batch * full || n_step == 0 || passes_scatter * lanes >= R.scatter_wait * full);
+			go_final = n_final != 0 && (64 * n_final >= R.final_batch * full || n_step == 0 || passes_final * lanes >= R.final_wait * full);
 			if(go_scatter)
 				passes_scatter = 0;
 			if(go_final)
@@ -769,11 +815,29 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 				atomicOr(R.status, STATUS_BUDGET);
 				break;
 			}
-			// few lanes left and no more work: the warps go on by themselves
-			if((flags & 1) && at_work <= R.lockstep_min)
-				lockstep = false;
 			if(at_work == 0)
 				break;
+			// few lanes left and no more work: their trajectories go on in the latency launch, or the warps by
+			// themselves
+			if(drained && at_work <= R.lockstep_min)
+			{
+				if constexpr(Step::throughput)
+				{
+					if(phase != PH_DONE && !(phase == PH_FETCH && q_next >= q_end))
+					{
+						Parked<Lane>& s = *reinterpret_cast<Parked<Lane>*>(R.parked + atomicAdd(R.parked_count, 1u) * PARKED_BYTES);
+						s.L = L;
+						s.hist = hist;
+						s.q_next = q_next;
+						s.q_end = q_end;
+						s.phase = phase;
+						s.iter = iter;
+					}
+					phase = PH_DONE;
+					break;
+				}
+				lockstep = false;
+			}
 		}
 		else
 		{

@@ -41,7 +41,7 @@ struct dms_ctx
 	SolarTables tables;
 	void* d_tables = nullptr;
 	DevSolar dsolar{};
-	float* d_tables_f = nullptr;    // FP32 r, G*M, G*M slope for the mixed-precision kernel
+	float* d_tables_f = nullptr;    // FP32 knots, v_esc^2 slopes and buckets for the mixed-precision kernel
 	// points
 	std::vector<PointConstants> points;
 	std::vector<double*> d_grids;
@@ -354,11 +354,11 @@ int Launch_And_Wait(dms_ctx* ctx, const dms_run_opts* o, RunParams& p)
 				DMS_CUDA(ctx, cudaGetLastError());
 				ctx->grid_f_valid[i] = 1;
 			}
-		p.sf_r = ctx->d_tables_f;
-		p.sf_gm = ctx->d_tables_f + ctx->dsolar.n;
-		p.sf_gm_s = ctx->d_tables_f + 2 * static_cast<size_t>(ctx->dsolar.n);
-		p.sf_vesc2 = ctx->d_tables_f + 3 * static_cast<size_t>(ctx->dsolar.n);
+		p.sf_knots = reinterpret_cast<const float4*>(ctx->d_tables_f);
 		p.sf_vesc2_s = ctx->d_tables_f + 4 * static_cast<size_t>(ctx->dsolar.n);
+		p.sf_bucket = reinterpret_cast<const uint16_t*>(ctx->d_tables_f + 5 * static_cast<size_t>(ctx->dsolar.n));
+		p.sf_scale = ctx->tables.bucket_scale_f;
+		p.sf_single_step = ctx->tables.bucket_single_step_f;
 	}
 #ifdef DMS_CHECKED
 	// bits left by a launch that does not report them (dms_run_records_noalloc) are dropped
@@ -667,17 +667,18 @@ int dms_load_solar_model(dms_ctx* ctx, const char* path)
 	S.nt_s = dd + offsets[10];
 	S.target_mass = dd + off_mass;
 	S.bucket = reinterpret_cast<const uint16_t*>(dd + off);
-	// FP32 images of the tables the mixed-precision kernel reads every step: knots, G*M and
-	// v_esc^2 with their slopes
-	std::vector<float> hf(5 * n);
+	// FP32 images of the tables the mixed-precision kernel reads every step: {r, G*M, its slope, v_esc^2} per
+	// knot, the slopes of v_esc^2, and the bucket table
+	std::vector<float> hf(5 * n + (t.bucket_index_f.size() + 1) / 2);
 	for(size_t i = 0; i < n; i++)
 	{
-		hf[i] = static_cast<float>(t.r[i]);
-		hf[n + i] = static_cast<float>(t.gm[i]);
-		hf[2 * n + i] = static_cast<float>(t.gm_s[i]);
-		hf[3 * n + i] = static_cast<float>(t.vesc2[i]);
-		hf[4 * n + i] = static_cast<float>(t.vesc2_s[i]);
+		hf[4 * i + 0] = i + 1 < n ? static_cast<float>(t.r[i]) : INFINITY;
+		hf[4 * i + 1] = static_cast<float>(t.gm[i]);
+		hf[4 * i + 2] = i + 1 < n ? static_cast<float>(t.gm_s[i]) : 0.0f;
+		hf[4 * i + 3] = static_cast<float>(t.vesc2[i]);
+		hf[4 * n + i] = i + 1 < n ? static_cast<float>(t.vesc2_s[i]) : 0.0f;
 	}
+	std::memcpy(hf.data() + 5 * n, t.bucket_index_f.data(), sizeof(uint16_t) * t.bucket_index_f.size());
 	float* df = nullptr;
 	DMS_CUDA(ctx, cudaMalloc(&df, sizeof(float) * hf.size()));
 	const cudaError_t cf = cudaMemcpy(df, hf.data(), sizeof(float) * hf.size(), cudaMemcpyHostToDevice);

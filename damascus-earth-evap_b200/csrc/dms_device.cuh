@@ -338,12 +338,6 @@ struct Draws
 		const double u = dms_draw_uniform(seed, point, traj, index++);
 		return a + u * (b - a);
 	}
-	// Positive_Unit_Uniform, src/Simulation_Trajectory.cpp:103-107
-	__device__ __forceinline__ double positive_unit()
-	{
-		const double u = uniform(0.0, 1.0);
-		return u > 2.2250738585072014e-308 ? u : 2.2250738585072014e-308;
-	}
 };
 
 // The next uniform draw in [0, 1), out of line.  A scattering makes about ten draws and runs once in some 25

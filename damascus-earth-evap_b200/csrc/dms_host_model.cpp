@@ -268,6 +268,28 @@ std::string Load_Solar_Tables(const std::string& path, SolarTables& t)
 	for(int i = 0; i < n; i++)
 		if(!in_range(t.gm[i]) || (i < n - 1 && !in_range(t.gm_s[i])))
 			t.fast_tables = 0;
+
+	// The FP32 form: the base of bucket b is the last knot of an earlier bucket (x -> bucket never falls, so
+	// that knot lies at or below every x of the bucket).  The product is the device's one
+	// rounded multiply.
+	t.bucket_scale_f = static_cast<float>(scale);
+	t.bucket_index_f.assign(t.nbuckets + 1, 0);
+	t.bucket_single_step_f = 1;
+	for(int b = 0, i = 0; b <= t.nbuckets + 1; b++)
+	{
+		const int base = i;
+		for(; i + 1 < n - 1; i++)
+		{
+			const float x = static_cast<float>(t.r[i + 1]) * t.bucket_scale_f;
+			if(static_cast<int>(std::floor(std::min<float>(x, static_cast<float>(t.nbuckets)))) >= b)
+				break;
+		}
+		// i: the last interval that begins in a bucket before b
+		if(b > 0 && i > base + 1)
+			t.bucket_single_step_f = 0;
+		if(b <= t.nbuckets)
+			t.bucket_index_f[b] = static_cast<uint16_t>(i);
+	}
 	return "";
 }
 

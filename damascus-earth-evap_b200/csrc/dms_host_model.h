@@ -37,6 +37,10 @@ struct SolarTables
 	// device's straight-line division (dms_fastmath.cuh)
 	int fast_tables = 0;
 	std::vector<uint16_t> bucket_index;
+	// the same for the knots rounded to float and the device's FP32 bucket floor(x * bucket_scale_f)
+	float bucket_scale_f = 0.0f;
+	int bucket_single_step_f = 0;
+	std::vector<uint16_t> bucket_index_f;
 };
 
 // Loads the solar model file; returns an empty string on success, else the error.

@@ -751,10 +751,7 @@ enum Verdict : int
 	VERDICT_SCATTER = 4,   // the remaining optical depth lies in the step
 	VERDICT_PAUSE = 5,     // not judged: the lane loop is due
 };
-#ifndef DMS_TU
-#define DMS_TU 6
-#endif
-constexpr int TEAM_UNROLL = DMS_TU;
+constexpr int TEAM_UNROLL = 6;
 constexpr int TEAM_MAX_STEPS = 512;                      // per call: the lane loop looks at the cancel flag between calls
 constexpr long long TEAM_WAIT_CYCLES = 40000000000ll;   // ~20 s: how long a warp without work waits for a team
 

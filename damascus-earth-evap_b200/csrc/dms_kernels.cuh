@@ -45,11 +45,11 @@ struct RunParams
 {
 	DevSolar S;
 	// FP32 images of the knot, G*M and G*M-slope tables (mixed-precision kernel only)
-	const float* sf_r;
-	const float* sf_gm;
-	const float* sf_gm_s;
-	const float* sf_vesc2;
+	const float4* sf_knots;
 	const float* sf_vesc2_s;
+	const uint16_t* sf_bucket;
+	float sf_scale;
+	int sf_single_step;
 	const DevPoint* points;
 	int n_points;
 	// work: ranges and their prefix offsets (n_ranges + 1)

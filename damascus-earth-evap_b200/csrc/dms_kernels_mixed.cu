@@ -22,7 +22,7 @@ using MixedLane = LaneT<PropF, EventF>;
 // dms_device_mixed.cuh for what stays FP64): the Propagate_Freely loop body,
 // src/Simulation_Trajectory.cpp:876-1116, split at the RK45 retry loop.
 
-__device__ __forceinline__ DevSolarF tables_f(const RunParams& R) { return DevSolarF{R.sf_r, R.sf_gm, R.sf_gm_s, R.sf_vesc2, R.sf_vesc2_s}; }
+__device__ __forceinline__ DevSolarF tables_f(const RunParams& R) { return DevSolarF{R.sf_knots, R.sf_vesc2_s, R.sf_bucket, R.sf_scale, R.S.nbuckets, R.sf_single_step, R.S.n}; }
 
 __device__ __forceinline__ const float* grid_f(const DevPoint* __restrict__ P)
 {
@@ -343,7 +343,7 @@ __device__ __forceinline__ double commit_event_mixed(const RunParams& R, double 
 	}
 	const double t_abs = local.t + L.origin;
 	const DevSolarF F = tables_f(R);
-	const double E = capture_energy_eV_f(R.S, F, m_dm, rf, vf);
+	const double E = capture_energy_eV_f(F, m_dm, rf, vf);
 	if(L.is_captured && isfinite(L.free_flight_E))
 	{
 		const double drift = fabs(E - L.free_flight_E);
@@ -384,10 +384,7 @@ __device__ __forceinline__ bool not_free(const RunParams& R, double m_dm, const 
 	const DevSolarF F = tables_f(R);
 	float need = static_cast<float>(2.0 * DMS_GMSUN_KM3S2);
 	if(inside)
-	{
-		const int i = knot_index_f(R.S, F, r);
-		need = __ldg(F.vesc2 + i) + (r - __ldg(F.r + i)) * __ldg(F.vesc2_s + i);
-	}
+		need = vesc2_f(F, r);
 	const float have = inside ? v2 : v2 * r;
 	const bool clear = (have > need * 1.001f) & (v2 < 1.0e12f) & (r < 1.0e12f);
 	return clear ? false : not_free_general(R.S, m_dm, e);
@@ -469,7 +466,7 @@ __device__ __forceinline__ int mixed_step(const RunParams& R, const DevPoint* __
 	{
 		q = L.pr;
 		L.rk_inner++;
-		const int rk = rk45_attempt_f<UNROLLED>(R.S, tables_f(R), q, L.rk_inner);
+		const int rk = rk45_attempt_f<UNROLLED>(tables_f(R), q, L.rk_inner);
 		if(rk == RK_RETRY)
 			L.pr.time_step = q.time_step;
 		else

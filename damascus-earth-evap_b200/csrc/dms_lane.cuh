@@ -48,7 +48,7 @@ struct LaneT
 	int in_rk;           // an RK45 step is in progress (retry pending)
 	int rk_inner;        // passes of the current RK45 step
 	double rate_before;  // scattering rate at the start of the step
-	int next_valid;      // next_speed / next_rate hold the propagator's speed and rate (FP64 form, tail)
+	int next_valid;      // next_speed / next_rate hold the propagator's speed and rate
 	double next_speed, next_rate;
 	int shift_ok;
 	int reason;

@@ -278,17 +278,19 @@ void Poll_Pause(std::chrono::steady_clock::duration elapsed)
 
 // Threads of the one block per SM.  With a lane per trajectory in 128 threads, every warp has a
 // scheduler of its own and a pass is bound by its dependent chain (the latency form of the kernel);
-// beyond that, 512 threads run their 16 warps in lockstep (the throughput form, dms_lane.cuh).
+// beyond that, 512 (640 in a large mixed launch) run their warps in lockstep (the throughput form, dms_lane.cuh).
 // Measured, Capture mode m = 1 GeV, sigma = 1e-35 cm^2, FP64, 128 against 512 threads: 1 024 trajectories
 // 2.1 / 2.3 ms, 4 096 2.9 / 3.2 ms, 16 384 4.2 / 4.1 ms, 65 536 10.6 / 6.3 ms.  threads_per_block and
 // blocks_per_sm ask for the lanes per SM: blocks of one SM run as one block.
 int Block_Threads(const dms_run_opts* o, uint64_t total, int sm_count)
 {
-	const int fitting = total <= LATENCY_THREADS * static_cast<uint64_t>(sm_count) ? LATENCY_THREADS : MAX_THREADS;
+	const bool more = o->precision == DMS_PRECISION_MIXED && total >= 2 * MAX_THREADS_MIXED * static_cast<uint64_t>(sm_count);
+	const int max_threads = more ? MAX_THREADS_MIXED : MAX_THREADS;
+	const int fitting = total <= LATENCY_THREADS * static_cast<uint64_t>(sm_count) ? LATENCY_THREADS : max_threads;
 	if(o->threads_per_block == 0 && o->blocks_per_sm == 0)
 		return fitting;
 	const int threads = o->threads_per_block ? static_cast<int>(o->threads_per_block) : LATENCY_THREADS;
-	const int most = MAX_THREADS / threads;
+	const int most = max_threads / threads;
 	const int per_sm = o->blocks_per_sm ? static_cast<int>(std::min<uint32_t>(o->blocks_per_sm, most)) : most;
 	return std::min(threads * per_sm, fitting);
 }

@@ -10,6 +10,7 @@
 // per-lane scratch row (touched bin range tracked) and is flushed once, at termination, into
 // the per-point sums and sums of squares (src/Data_Generation.cpp:787-822).
 #include "dms_lane.cuh"
+#include "dms_team.cuh"
 
 namespace dms
 {
@@ -707,73 +708,13 @@ __device__ __forceinline__ int strict_step(const RunParams& R, const DevPoint* _
 }
 
 // ---------------------------------------------------------------------------------------------
-// Team: a lane that runs alone in its block spends its step on one dependent chain, and a warp issues one
-// instruction every 4.4 cycles of it.  Once the other warps of a 128-thread block have run out of work,
-// two of them take over parts of the lone lane's steps, one step apart, with a barrier per step:
-//   propagate  the bounds and the RK45 attempts of the next step, from its own last result
-//   judge      (the lane's own warp) event, optical depth and decisions of the step before
-//   commit     bincount and energy drift of the step before that
-// (9 steps per orbit is common for a lone lane: an orbit that leaves the boundary radius comes back by Kepler's
-// equation, which the lane solves with the team's step in hand.)
-// The propagating warp runs ahead as if every step ended plainly.  A step that does not is not committed:
-// a depth rejection restarts the propagation from the step's start with the shorter step; anything
-// else (a scattering, the boundary, a failure) hands the state at the step's start back to the lane, which
-// makes that step by itself.  Every value is formed by the functions of the one-lane pass from the same
-// arguments, so the results are the same bits.  The barriers count whole warps that all run the same loop;
-// the only wait by polling is that of a warp without work for a team to form, and it is bounded.
-struct TeamState  // the propagator at the start of a step
-{
-	double time, radius, phi, v_radial, step, speed, rate;
-	int inner, ok;  // attempts of the step that led here; whether the propagating warp could make it
-};
-struct TeamBox
-{
-	int word;       // warps without work; TEAM_FORMED once a team has formed, negative when none can
-	int command;    // TEAM_RUN, TEAM_EXIT
-	int verdict[2];
-	int captured, bound, bmin, bmax, cbin;
-	const DevPoint* P;
-	double2* hist;
-	double m_dm, J;
-	Vec3 ax, ay;
-	double origin, prev_time, prev_r, prev_v2, t_last_bound, free_flight_E, max_drift_eV, max_drift_rel;
-	double2 cval;
-	TeamState s[4];  // by step number modulo 4
-	Event e[4];      // the events at those states
-};
-constexpr int TEAM_FORMED = 0x100, TEAM_NEVER = -0x10000, TEAM_RUN = 0, TEAM_EXIT = 1;
-enum Verdict : int
-{
-	VERDICT_PLAIN = 0,
-	VERDICT_RESTART = 1,
-	VERDICT_STOP = 2,
-	VERDICT_BOUNDARY = 3,  // the step ends at or beyond the boundary radius
-	VERDICT_SCATTER = 4,   // the remaining optical depth lies in the step
-	VERDICT_PAUSE = 5,     // not judged: the lane loop is due
-};
-constexpr int TEAM_UNROLL = 6;
-constexpr int TEAM_MAX_STEPS = 512;                      // per call: the lane loop looks at the cancel flag between calls
-constexpr long long TEAM_WAIT_CYCLES = 40000000000ll;   // ~20 s: how long a warp without work waits for a team
-
-__device__ __forceinline__ TeamBox& team_box()
-{
-	__shared__ TeamBox box;
-	return box;
-}
-__device__ __forceinline__ void team_barrier() { asm volatile("bar.sync 1, 96;" ::: "memory"); }
+// The three parts of a step made by a team (dms_team.cuh).
+using StrictBox = TeamBox<Prop, Event>;
 
 // The propagating warp's step: from s to n.  One lane.
-__device__ __forceinline__ void team_propagate(const RunParams& R, const TeamBox& b, const TeamState& s, TeamState& n)
+__device__ __forceinline__ void strict_propagate(const RunParams& R, const StrictBox& b, const TeamState& s, TeamState& n)
 {
-	Prop q;
-	q.time = s.time;
-	q.radius = s.radius;
-	q.phi = s.phi;
-	q.v_radial = s.v_radial;
-	q.J = b.J;
-	q.ax = b.ax;
-	q.ay = b.ay;
-	q.radial_mode = 0;
+	Prop q = team_prop(b, s);
 	// step_begin; the event at the state is only needed where the time to the surface may bind
 	const double r = s.radius;
 	double step = sanitized_step(s.step);
@@ -800,13 +741,13 @@ __device__ __forceinline__ void team_propagate(const RunParams& R, const TeamBox
 	while(ok && rk == RK_RETRY && inner <= DMS_RK45_MAX_INNER_RETRIES)
 	{
 		inner++;
-		rk = rk45_attempt<TEAM_UNROLL>(R.S, q, inner);
+		rk = rk45_attempt<6>(R.S, q, inner);
 	}
 	ok &= rk == RK_ACCEPTED;
 	// prop_speed, as in event_and_speed
 	ok &= fast::in_radius_range(q.radius) & (fabs(q.phi) < 0x1p20);
 	const fast::Recip D = fast::recip(q.radius, ok);
-	n.speed = fast::sqrt(q.v_radial * q.v_radial + fast::div(fast::div(b.J * b.J, D), D), ok);
+	n.speed = fast::sqrt(q.v_radial * q.v_radial + fast::div(fast::div(b.pr.J * b.pr.J, D), D), ok);
 	n.rate = ok ? rate_inside(R.S, b.P, q.radius, n.speed) : 0.0;
 	n.time = q.time;
 	n.radius = q.radius;
@@ -819,7 +760,7 @@ __device__ __forceinline__ void team_propagate(const RunParams& R, const TeamBox
 
 // The judging warp's step: from state s with event e to state n, whose event goes to en.  All 32 lanes;
 // `mine` marks the lane whose trajectory it is.
-__device__ __forceinline__ int team_judge(const RunParams& R, const TeamBox& b, TeamState& s, const Event& e, const TeamState& n, Event& en, StrictLane& L,
+__device__ __forceinline__ int strict_judge(const RunParams& R, const StrictBox& b, TeamState& s, const Event& e, const TeamState& n, Event& en, StrictLane& L,
                                           bool mine, double* buffer, StepCtx& c)
 {
 	const int capture_mode = R.capture_mode;
@@ -828,15 +769,7 @@ __device__ __forceinline__ int team_judge(const RunParams& R, const TeamBox& b, 
 	bool interior = false, depth = false, stop = true;
 	if(mine && n.ok)
 	{
-		Prop q;
-		q.time = n.time;
-		q.radius = n.radius;
-		q.phi = n.phi;
-		q.v_radial = n.v_radial;
-		q.J = b.J;
-		q.ax = b.ax;
-		q.ay = b.ay;
-		q.radial_mode = 0;
+		const Prop q = team_prop(b, n);
 		c.before = e;
 		c.r_before = s.radius;
 		c.dt = n.time - s.time;
@@ -907,7 +840,7 @@ __device__ __forceinline__ int team_judge(const RunParams& R, const TeamBox& b, 
 
 // The committing warp's step: the bincount and energy drift of the event e.  One lane, whose own lane
 // state serves as scratch.
-__device__ __forceinline__ void team_commit(const RunParams& R, const TeamBox& b, StrictLane& L, const Event& e)
+__device__ __forceinline__ void strict_commit(const RunParams& R, const StrictBox& b, StrictLane& L, const Event& e)
 {
 	double r, v;
 	if(!R.capture_mode | L.is_captured)
@@ -917,57 +850,44 @@ __device__ __forceinline__ void team_commit(const RunParams& R, const TeamBox& b
 	}
 }
 
-// The loop of the three warps: role 0 judges, 1 propagates, 2 commits.  Returns the number of the step at
-// whose start the lane goes on by itself (the states and events are in the box).
-__device__ __forceinline__ int team_loop(const RunParams& R, TeamBox& b, StrictLane& L, int role, bool mine, double* buffer, StepCtx& c, int& last)
+struct StrictTeam
 {
-	const bool lane0 = (threadIdx.x & 31) == 0;
-	int j = 0;             // the step to judge
-	bool have = false;     // ... whose result is there
-	bool pending = false;  // step j - 1 is to be committed
-	for(int pass = 0;; pass++)
+	using Lane = StrictLane;
+	using Box = StrictBox;
+	using Ctx = StepCtx;
+	static __device__ __forceinline__ void fresh(const RunParams& R, const DevPoint* __restrict__ P, StrictLane& L) { fresh_state(R.S, P, L); }
+	// what the fast functions cover; other states go to the one-lane pass
+	static __device__ __forceinline__ bool fits(const StrictLane& L)
 	{
-		if(role == 1)
-		{
-			const int from = have ? j + 1 : j;
-			if(lane0)
-				team_propagate(R, b, b.s[from & 3], b.s[(from + 1) & 3]);
-		}
-		else if(role == 0)
-		{
-			if(have)
-			{
-				int v = VERDICT_PAUSE;
-				if(pass < TEAM_MAX_STEPS)
-					v = team_judge(R, b, b.s[j & 3], b.e[j & 3], b.s[(j + 1) & 3], b.e[(j + 1) & 3], L, mine, buffer, c);
-				if(mine)
-					b.verdict[pass & 1] = v;
-			}
-		}
-		else if(pending && lane0)
-			team_commit(R, b, L, b.e[j & 3]);
-		__syncwarp();
-		team_barrier();
-		pending = false;
-		if(!have)
-		{
-			have = true;
-			continue;
-		}
-		const int v = *reinterpret_cast<volatile int*>(&b.verdict[pass & 1]);
-		last = v;
-		if(v >= VERDICT_STOP)
-			break;
-		if(v == VERDICT_PLAIN)
-		{
-			j++;
-			pending = true;
-		}
-		else
-			have = false;
+		return (L.pr.radial_mode == 0) & (L.pr.J > 0x1p-200) & (L.pr.J < 0x1p200) & fast::in_radius_range(L.pr.radius) & (fabs(L.pr.phi) < 0x1p20);
 	}
-	return j;
-}
+	static __device__ __forceinline__ void propagate(const RunParams& R, const Box& b, const TeamState& s, TeamState& n) { strict_propagate(R, b, s, n); }
+	static __device__ __forceinline__ int judge(const RunParams& R, const Box& b, TeamState& s, const Event& e, const TeamState& n, Event& en, StrictLane& L,
+	                                            bool mine, double* buffer, StepCtx& c)
+	{
+		return strict_judge(R, b, s, e, n, en, L, mine, buffer, c);
+	}
+	static __device__ __forceinline__ void commit(const RunParams& R, const Box& b, StrictLane& L, const Event& e) { strict_commit(R, b, L, e); }
+	// The end of a step that reaches the boundary or a scattering, as in strict_step: `phase` is the lane's next.
+	static __device__ __forceinline__ void finish(const RunParams& R, const DevPoint* __restrict__ P, double m_dm, StrictLane& L, double2* hist, StepCtx& c,
+	                                              const TeamState& n, bool scattering, int& phase)
+	{
+		Event accepted = c.after;
+		int boundary = BOUNDARY_INSIDE;
+		if(!scattering)
+			boundary = boundary_step(R, m_dm, L, hist, c, accepted);
+		else
+		{
+			const bool depth = c.s1 > c.s0;
+			scatter_point(R.S, P, c, L.next_rate, depth && c.r_before < DMS_RSUN_KM && c.s0 <= 1.0e-12, depth,
+			              R.capture_mode ? DMS_CAPTURE_OPTICAL_DEPTH_PIECES : DMS_MAX_OPTICAL_DEPTH_PIECES, L.tau, accepted);
+		}
+		if(boundary == BOUNDARY_FAILURE)
+			phase = PH_FINAL;
+		else if(boundary != BOUNDARY_RETURN)
+			phase = finish_step(R, m_dm, L, hist, c, accepted, scattering, boundary, n.time, n.radius, n.phi, n.v_radial, n.step, n.rate, true);
+	}
+};
 
 // Initial_Conditions + Hyperbolic_Kepler_Shift of every work index (src/Data_Generation.cpp:747-761,
 // src/Simulation_Utilities.cpp:123-321), ahead of the trajectory launch.  A lane takes every n-th work index
@@ -1103,7 +1023,7 @@ __global__ void __launch_bounds__(128) initial_state_kernel(const RunParams R, i
 }
 
 template <bool THROUGHPUT>
-struct StrictStep
+struct StrictStep : Team<StrictTeam>
 {
 	static constexpr bool throughput = THROUGHPUT;
 	static constexpr int threads = THROUGHPUT ? MAX_THREADS : LATENCY_THREADS;
@@ -1116,226 +1036,7 @@ struct StrictStep
 	{
 		return strict_step<THROUGHPUT ? 1 : 6>(R, P, m_dm, L, hist, phase, buffer);
 	}
-	// ---- team (the latency form) ----
 	static constexpr bool team = !THROUGHPUT;
-	__device__ __forceinline__ void team_init() const
-	{
-		team_box().word = 0;
-		team_box().command = TEAM_RUN;
-	}
-	// Called by a whole warp without work: it helps a lone lane of its block, if one forms a team, until that
-	// lane's trajectory has ended.
-	__device__ __noinline__ void team_help(const RunParams& R, StrictLane& L, double* buffer) const
-	{
-		TeamBox& b = team_box();
-		const bool lane0 = (threadIdx.x & 31) == 0;
-		int rank = 0;
-		if(lane0)
-			rank = atomicAdd(&b.word, 1);
-		rank = __shfl_sync(0xffffffffu, rank, 0);
-		if(rank == 3)
-		{
-			team_forgo();  // the last warp of the block: nobody is left to help
-			return;
-		}
-		const long long t0 = clock64();
-		for(unsigned int poll = 1;; poll++)
-		{
-			int word = 0;
-			if(lane0)
-			{
-				word = *reinterpret_cast<volatile int*>(&b.word);
-				bool leave = clock64() - t0 > TEAM_WAIT_CYCLES;
-				if((poll & 255u) == 0u)
-					leave |= *R.cancel != 0;
-				// a warp leaves by putting the count out of reach, which no formed team can follow
-				if(leave && word >= 0 && word < TEAM_FORMED)
-				{
-					const int seen = atomicCAS(&b.word, word, TEAM_NEVER);
-					word = seen == word ? TEAM_NEVER : seen;
-				}
-			}
-			word = __shfl_sync(0xffffffffu, word, 0);
-			if(word < 0)
-				return;
-			if(word >= TEAM_FORMED)
-				break;
-			__nanosleep(1000);
-		}
-		if(rank > 1)
-			return;  // two helpers are enough
-		for(;;)
-		{
-			team_barrier();  // the owner has filled the box
-			if(*reinterpret_cast<volatile int*>(&b.command) == TEAM_EXIT)
-				return;
-			if(rank == 1)
-			{
-				L.is_captured = b.captured;
-				L.bound_state = b.bound;
-				L.bmin = b.bmin;
-				L.bmax = b.bmax;
-				L.cbin = b.cbin;
-				L.cval = b.cval;
-				L.origin = b.origin;
-				L.prev_time = b.prev_time;
-				L.prev_r = b.prev_r;
-				L.prev_v2 = b.prev_v2;
-				L.t_last_bound = b.t_last_bound;
-				L.free_flight_E = b.free_flight_E;
-				L.max_drift_eV = b.max_drift_eV;
-				L.max_drift_rel = b.max_drift_rel;
-			}
-			StepCtx c;
-			int last;
-			team_loop(R, b, L, rank == 0 ? 1 : 2, false, buffer, c, last);
-			if(rank == 1 && lane0)
-			{
-				b.bmin = L.bmin;
-				b.bmax = L.bmax;
-				b.cbin = L.cbin;
-				b.cval = L.cval;
-				b.prev_time = L.prev_time;
-				b.prev_r = L.prev_r;
-				b.prev_v2 = L.prev_v2;
-				b.t_last_bound = L.t_last_bound;
-				b.max_drift_eV = L.max_drift_eV;
-				b.max_drift_rel = L.max_drift_rel;
-			}
-			__syncwarp();
-			team_barrier();  // the owner may read the box
-		}
-	}
-	// Called by the whole warp of a lone lane (`mine` on that lane, at the start of a step): forms the team if the
-	// other three warps are without work.
-	__device__ __forceinline__ bool team_form() const
-	{
-		TeamBox& b = team_box();
-		int formed = 0;
-		if((threadIdx.x & 31) == 0)
-			formed = *reinterpret_cast<volatile int*>(&b.word) == 3 && atomicCAS(&b.word, 3, TEAM_FORMED) == 3 ? 1 : 0;
-		return __shfl_sync(0xffffffffu, formed, 0) != 0;
-	}
-	// A warp that stops in mid-trajectory: no team can form any more.
-	__device__ __forceinline__ void team_forgo() const
-	{
-		if((threadIdx.x & 31) == 0)
-			atomicExch(&team_box().word, TEAM_NEVER);
-	}
-	__device__ __forceinline__ void team_dismiss() const
-	{
-		TeamBox& b = team_box();
-		if((threadIdx.x & 31) == 0)
-			*reinterpret_cast<volatile int*>(&b.command) = TEAM_EXIT;
-		__syncwarp();
-		team_barrier();
-	}
-	// Steps of the lone lane made by the team; the lane's state is that at the start of a step before and
-	// after (or `phase`, its phase, says otherwise).  Adds the number of steps to `iter`; returns whether
-	// the lane must make its next step alone.
-	__device__ __noinline__ bool team_run(const RunParams& R, const DevPoint* __restrict__ P, double m_dm, StrictLane& L, double2* hist, bool mine,
-	                                     double* buffer, int& phase, uint64_t& iter) const
-	{
-		TeamBox& b = team_box();
-		if(mine && !L.next_valid)
-			fresh_state(R.S, P, L);
-		// what the fast functions cover; other states go to the one-lane pass
-		const bool fit = mine && (L.pr.radial_mode == 0) & (L.pr.J > 0x1p-200) & (L.pr.J < 0x1p200) &
-		                                          fast::in_radius_range(L.pr.radius) & (fabs(L.pr.phi) < 0x1p20);
-		if(!__any_sync(0xffffffffu, fit))
-			return true;
-		if(mine)
-		{
-			b.P = P;
-			b.hist = hist;
-			b.m_dm = m_dm;
-			b.J = L.pr.J;
-			b.ax = L.pr.ax;
-			b.ay = L.pr.ay;
-			b.captured = L.is_captured;
-			b.bound = L.bound_state;
-			b.bmin = L.bmin;
-			b.bmax = L.bmax;
-			b.cbin = L.cbin;
-			b.cval = L.cval;
-			b.origin = L.origin;
-			b.prev_time = L.prev_time;
-			b.prev_r = L.prev_r;
-			b.prev_v2 = L.prev_v2;
-			b.t_last_bound = L.t_last_bound;
-			b.free_flight_E = L.free_flight_E;
-			b.max_drift_eV = L.max_drift_eV;
-			b.max_drift_rel = L.max_drift_rel;
-			TeamState& s = b.s[0];
-			s.time = L.pr.time;
-			s.radius = L.pr.radius;
-			s.phi = L.pr.phi;
-			s.v_radial = L.pr.v_radial;
-			s.step = L.pr.time_step;
-			s.speed = L.next_speed;
-			s.rate = L.next_rate;
-			b.e[0] = L.before;
-			b.e[0].t = L.pr.time;
-		}
-		__syncwarp();
-		team_barrier();
-		StepCtx c;
-		int last = VERDICT_PLAIN;
-		const int j = team_loop(R, b, L, 0, mine, buffer, c, last);
-		team_barrier();  // the committing warp has written its part back
-		if(mine)
-		{
-			const TeamState& s = b.s[j & 3];
-			L.pr.time = s.time;
-			L.pr.radius = s.radius;
-			L.pr.phi = s.phi;
-			L.pr.v_radial = s.v_radial;
-			L.pr.time_step = s.step;
-			L.next_speed = s.speed;
-			L.next_rate = s.rate;
-			if(j > 0)
-			{
-				L.before = b.e[j & 3];
-				L.before_valid = 2;
-			}
-			L.bmin = b.bmin;
-			L.bmax = b.bmax;
-			L.cbin = b.cbin;
-			L.cval = b.cval;
-			L.prev_time = b.prev_time;
-			L.prev_r = b.prev_r;
-			L.prev_v2 = b.prev_v2;
-			L.t_last_bound = b.t_last_bound;
-			L.max_drift_eV = b.max_drift_eV;
-			L.max_drift_rel = b.max_drift_rel;
-		}
-		// a step that ends at the boundary or in a scattering is finished here with what the team made of it,
-		// as in strict_step
-		if(mine && (last == VERDICT_BOUNDARY || last == VERDICT_SCATTER))
-		{
-			Event accepted = c.after;
-			int boundary = BOUNDARY_INSIDE;
-			if(last == VERDICT_BOUNDARY)
-				boundary = boundary_step(R, m_dm, L, hist, c, accepted);
-			else
-			{
-				const bool depth = c.s1 > c.s0;
-				scatter_point(R.S, P, c, L.next_rate, depth && c.r_before < DMS_RSUN_KM && c.s0 <= 1.0e-12, depth,
-				              R.capture_mode ? DMS_CAPTURE_OPTICAL_DEPTH_PIECES : DMS_MAX_OPTICAL_DEPTH_PIECES, L.tau, accepted);
-			}
-			if(boundary == BOUNDARY_FAILURE)
-				phase = PH_FINAL;
-			else if(boundary != BOUNDARY_RETURN)
-			{
-				const TeamState& n = b.s[(j + 1) & 3];
-				phase = finish_step(R, m_dm, L, hist, c, accepted, last == VERDICT_SCATTER, boundary, n.time, n.radius, n.phi, n.v_radial, n.step,
-				                    n.rate, true);
-			}
-		}
-		__syncwarp();
-		iter += j;
-		return last == VERDICT_STOP;
-	}
 	__device__ __forceinline__ double channel(const DevSolar& S, const DevPoint* __restrict__ P, int i, double dr, double T, double v, int k) const
 	{
 		return channel_rate(S, P, i, dr, T, v, k);

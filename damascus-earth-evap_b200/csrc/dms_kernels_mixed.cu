@@ -588,19 +588,19 @@ __device__ __forceinline__ int mixed_step(const RunParams& R, const DevPoint* __
 	return PH_STEP;
 }
 
-template <bool THROUGHPUT>
+template <int THREADS>
 struct MixedStep
 {
-	static constexpr bool throughput = THROUGHPUT;
-	static constexpr int threads = THROUGHPUT ? MAX_THREADS : LATENCY_THREADS;
+	static constexpr int threads = THREADS;
+	static constexpr bool throughput = THREADS > LATENCY_THREADS;
 	// (in the latency form the barriers cost more than the fetches: 16 384 Capture-mode trajectories 2.8 / 3.0 ms)
-	static constexpr bool lockstep = THROUGHPUT;
+	static constexpr bool lockstep = throughput;
 	static constexpr int buffer = COOP_BUFFER_F;
 	static constexpr bool team = false;
 	__device__ __forceinline__ int operator()(const RunParams& R, const DevPoint* __restrict__ P, double m_dm, MixedLane& L, double2* hist, int phase,
 	                                          double* buffer) const
 	{
-		return mixed_step<!THROUGHPUT>(R, P, m_dm, L, hist, phase, reinterpret_cast<float*>(buffer));
+		return mixed_step<!throughput>(R, P, m_dm, L, hist, phase, reinterpret_cast<float*>(buffer));
 	}
 	__device__ __forceinline__ double channel(const DevSolar& S, const DevPoint* __restrict__ P, int i, double dr, double T, double v, int k) const
 	{
@@ -613,14 +613,15 @@ struct MixedStep
 };
 
 // The throughput and the latency form, as in dms_kernels.cu.
-__global__ void __launch_bounds__(MAX_THREADS, 1) trajectory_kernel_mixed(const RunParams R)
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, 1) trajectory_kernel_mixed(const RunParams R)
 {
-	lane_loop<MixedLane>(R, MixedStep<true>());
+	lane_loop<MixedLane>(R, MixedStep<THREADS>());
 }
 
 __global__ void __launch_bounds__(LATENCY_THREADS, 1) trajectory_kernel_mixed_latency(const RunParams R)
 {
-	lane_loop<MixedLane>(R, MixedStep<false>());
+	lane_loop<MixedLane>(R, MixedStep<LATENCY_THREADS>());
 }
 
 __global__ void grid_to_float_kernel(const double* __restrict__ in, float* __restrict__ out, size_t n)
@@ -635,8 +636,10 @@ void Launch_Trajectories_Mixed(const RunParams& p, int blocks, int threads, cuda
 {
 	if(threads <= LATENCY_THREADS)
 		trajectory_kernel_mixed_latency<<<blocks, threads, 0, stream>>>(p);
+	else if(threads <= MAX_THREADS)
+		trajectory_kernel_mixed<MAX_THREADS><<<blocks, threads, 0, stream>>>(p);
 	else
-		trajectory_kernel_mixed<<<blocks, threads, 0, stream>>>(p);
+		trajectory_kernel_mixed<MAX_THREADS_MIXED><<<blocks, threads, 0, stream>>>(p);
 }
 
 void Launch_To_Float(const double* in, float* out, size_t n, cudaStream_t stream)

@@ -192,7 +192,8 @@ typedef struct
 	double boundary_radius_rsun;       /* initial_and_final_radius / R_sun (2.0) */
 	int32_t precision;                 /* DMS_PRECISION_* */
 	uint32_t threads_per_block;        /* 32, 64, 96 or 128: with blocks_per_sm the most lanes per SM
-	                                      (which run as one block of up to 512 threads); 0 = chosen by
+	                                      (which run as one block, of up to 512 threads,
+	                                      or 640 in a large mixed launch); 0 = chosen by
 	                                      the size of the launch (128 when blocks_per_sm is given) */
 	uint32_t blocks_per_sm;            /* blocks per SM; 0 = as many as fit */
 	uint32_t queue_chunk;              /* trajectory ids a lane claims from the work queue at a time
@@ -209,7 +210,7 @@ typedef struct
 	 * (final_batch) lanes of its warp are there, or it has waited scatter_wait (final_wait)
 	 * loop iterations, or no lane of the warp is stepping; then the warp runs the scattering
 	 * (termination) code once for all of them.  0 = defaults (16 / 32 / 8 / 32, longer in launches that
-	 * fill the GPU, where whole blocks of 512 lanes count in their stead); batches up to
+	 * fill the GPU, where the lanes of whole blocks count in their stead); batches up to
 	 * 32, waits up to 1024. */
 	uint32_t scatter_batch;
 	uint32_t scatter_wait;

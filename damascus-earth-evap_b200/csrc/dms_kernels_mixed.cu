@@ -3,6 +3,7 @@
 #define DMS_FMA_CONTRACTION 1
 #include "dms_device_mixed.cuh"
 #include "dms_lane.cuh"
+#include "dms_team.cuh"
 
 namespace dms
 {
@@ -47,9 +48,9 @@ static __device__ __noinline__ int end_at_propagator(MixedLane& L, int reason)
 	return PH_FINAL;
 }
 
-static __device__ __noinline__ double surface_step(const MixedLane& L, double r, double step)
+static __device__ __noinline__ double surface_step(const EventF& before, double r, double step)
 {
-	const double vr = (r > 0.0) ? static_cast<double>(dotf(L.before.x, L.before.v)) / r : 0.0;
+	const double vr = (r > 0.0) ? static_cast<double>(dotf(before.x, before.v)) / r : 0.0;
 	if(r > DMS_RSUN_KM && vr < 0.0)
 	{
 		const double est = (r - DMS_RSUN_KM) / (-vr);
@@ -58,6 +59,19 @@ static __device__ __noinline__ double surface_step(const MixedLane& L, double r,
 			const double lim = est > DMS_RK45_ABS_MIN_STEP_S ? est : DMS_RK45_ABS_MIN_STEP_S;
 			step = lim < step ? lim : step;
 		}
+	}
+	return step;
+}
+
+// The bound of a step inside the Sun by its optical depth.
+__device__ __forceinline__ double inside_step(const RunParams& R, double rate, double step)
+{
+	if(rate > 0.0)
+	{
+		const double tau_limit = R.capture_mode ? DMS_CAPTURE_MAX_OPTICAL_DEPTH_STEP : DMS_MAX_OPTICAL_DEPTH_STEP;
+		const float lim = static_cast<float>(tau_limit) / static_cast<float>(rate);
+		if(static_cast<double>(lim) < step)
+			step = static_cast<double>(lim);
 	}
 	return step;
 }
@@ -85,20 +99,14 @@ __device__ __forceinline__ int mixed_begin(const RunParams& R, const DevPoint* _
 	{
 		step = capped_step(r, L.next_speed, step, R.boundary);
 		if(!surface_is_far(r, static_cast<double>(dotf(L.before.x, L.before.v)), step))
-			step = surface_step(L, r, step);
+			step = surface_step(L.before, r, step);
 	}
 	else
 	{
 		rate = L.next_rate;
 		if(!isfinite(rate) || rate < 0.0)
 			return end_at_propagator(L, DMS_REASON_NUMERICAL_FAILURE);
-		if(rate > 0.0)
-		{
-			const double tau_limit = R.capture_mode ? DMS_CAPTURE_MAX_OPTICAL_DEPTH_STEP : DMS_MAX_OPTICAL_DEPTH_STEP;
-			const float lim = static_cast<float>(tau_limit) / static_cast<float>(rate);
-			if(static_cast<double>(lim) < step)
-				step = static_cast<double>(lim);
-		}
+		step = inside_step(R, rate, step);
 	}
 	L.rate_before = rate;
 	L.pr.time_step = step;
@@ -448,6 +456,43 @@ static __device__ __noinline__ int boundary_step(const RunParams& R, double m_dm
 // as in dms_kernels.cu
 constexpr int COOP_MAX_STEPS = 15;
 
+// The end of a step that has not been rejected, for the committed event `accepted` and the propagator after it.
+__device__ __forceinline__ int finish_step(const RunParams& R, double m_dm, MixedLane& L, double2* hist, const StepCtxF& c, const EventF& accepted,
+                                           bool scattering, int boundary, double time, double radius, double phi, double v_radial, double time_step,
+                                           double next_rate, bool next_known)
+{
+	L.seg_steps++;
+	L.steps++;
+	L.retries = 0;
+	const double E = commit_event_mixed(R, m_dm, L, hist, accepted);
+	const bool bound = !L.is_captured && (isnan(E) ? not_free(R, m_dm, accepted) : !(isfinite(E) && E >= 0.0));
+	if(bound | scattering | (boundary == BOUNDARY_ESCAPE))
+	{
+		L.cur = to_event64(accepted);
+		L.cur.t += L.origin;
+		if(bound)
+			L.reason = DMS_REASON_NUMERICAL_FAILURE;
+		else if(!scattering)
+			L.reason = DMS_REASON_OUTWARD_ESCAPE;
+		else if(ev_radius(L.cur) < DMS_RSUN_KM)
+			return PH_SCATTER;  // Simulate, src/Simulation_Trajectory.cpp:1313-1346; Sample_Target runs in the lane loop
+		else
+			L.reason = DMS_REASON_SCATTER;
+		return PH_FINAL;
+	}
+	L.pr.time = time;
+	L.pr.radius = radius;
+	L.pr.phi = phi;
+	L.pr.v_radial = v_radial;
+	L.pr.time_step = time_step;
+	L.before = c.after;
+	L.before_valid = 2;
+	L.next_speed = c.v_after;
+	L.next_rate = next_rate;
+	L.next_valid = next_known || c.r_after >= DMS_RSUN_KM;
+	return PH_STEP;
+}
+
 // One pass for every lane of the warp (all 32 call it); returns the lane's next phase.
 template <bool UNROLLED>
 __device__ __forceinline__ int mixed_step(const RunParams& R, const DevPoint* __restrict__ P, double m_dm, MixedLane& L, double2* hist, int phase,
@@ -556,47 +601,166 @@ __device__ __forceinline__ int mixed_step(const RunParams& R, const DevPoint* __
 		if(boundary == BOUNDARY_FAILURE)
 			return PH_FINAL;
 	}
-	L.seg_steps++;
-	L.steps++;
-	L.retries = 0;
-	const double E = commit_event_mixed(R, m_dm, L, hist, accepted);
-	const bool bound = !L.is_captured && (isnan(E) ? not_free(R, m_dm, accepted) : !(isfinite(E) && E >= 0.0));
-	if(bound | scattering | (boundary == BOUNDARY_ESCAPE))
-	{
-		L.cur = to_event64(accepted);
-		L.cur.t += L.origin;
-		if(bound)
-			L.reason = DMS_REASON_NUMERICAL_FAILURE;
-		else if(!scattering)
-			L.reason = DMS_REASON_OUTWARD_ESCAPE;
-		else if(ev_radius(L.cur) < DMS_RSUN_KM)
-			return PH_SCATTER;  // Simulate, src/Simulation_Trajectory.cpp:1313-1346; Sample_Target runs in the lane loop
-		else
-			L.reason = DMS_REASON_SCATTER;
-		return PH_FINAL;
-	}
-	L.pr.time = q.time;
-	L.pr.radius = q.radius;
-	L.pr.phi = q.phi;
-	L.pr.v_radial = q.v_radial;
-	L.pr.time_step = q.time_step;
-	L.before = c.after;
-	L.before_valid = 2;
-	L.next_speed = c.v_after;
-	L.next_rate = static_cast<double>(d.next_rate);
-	L.next_valid = depth || c.r_after >= DMS_RSUN_KM;
-	return PH_STEP;
+	return finish_step(R, m_dm, L, hist, c, accepted, scattering, boundary, q.time, q.radius, q.phi, q.v_radial, q.time_step,
+	                   static_cast<double>(d.next_rate), depth);
 }
 
+// The three parts of a step made by a team (dms_team.cuh), as in dms_kernels.cu.
+struct MixedTeam
+{
+	using Lane = MixedLane;
+	using Box = TeamBox<PropF, EventF>;
+	using Ctx = StepCtxF;
+	static __device__ __forceinline__ void fresh(const RunParams& R, const DevPoint* __restrict__ P, MixedLane& L) { fresh_state(R.S, P, L); }
+	static __device__ __forceinline__ bool fits(const MixedLane& L) { return L.pr.radial_mode == 0; }
+
+	static __device__ __forceinline__ void propagate(const RunParams& R, const Box& b, const TeamState& s, TeamState& n)
+	{
+		PropF q = team_prop(b, s);
+		const double r = prop_radius_f(q);
+		double step = sanitized_step(s.step);
+		bool ok = true;
+		if(r >= DMS_RSUN_KM)
+		{
+			const EventF before = prop_event_f(q);
+			step = capped_step(r, s.speed, step, R.boundary);
+			if(!surface_is_far(r, static_cast<double>(dotf(before.x, before.v)), step))
+				step = surface_step(before, r, step);
+		}
+		else
+		{
+			ok = (s.rate >= 0.0) & (s.rate < INFINITY);
+			step = inside_step(R, s.rate, step);
+		}
+		q.time_step = step;
+		int inner = 0, rk = RK_RETRY;
+		while(ok && rk == RK_RETRY && inner <= DMS_RK45_MAX_INNER_RETRIES)
+		{
+			inner++;
+			rk = rk45_attempt_f<true>(tables_f(R), q, inner);
+		}
+		const double r_after = prop_radius_f(q);
+		n.speed = prop_speed_f(q);
+		ok &= (rk == RK_ACCEPTED) & (r_after < INFINITY) & (n.speed < INFINITY);
+		n.rate = ok && r_after < DMS_RSUN_KM ? static_cast<double>(rate_total_f(R.S, b.P, grid_f(b.P), static_cast<float>(r_after), static_cast<float>(n.speed))) : 0.0;
+		n.time = q.time;
+		n.radius = q.radius;
+		n.phi = q.phi;
+		n.v_radial = q.v_radial;
+		n.step = q.time_step;
+		n.inner = inner;
+		n.ok = ok ? 1 : 0;
+	}
+
+	static __device__ __forceinline__ int judge(const RunParams& R, const Box& b, TeamState& s, const EventF& e, const TeamState& n, EventF& en, MixedLane& L,
+	                                            bool mine, double* buffer, StepCtxF& c)
+	{
+		const int capture_mode = R.capture_mode;
+		const int pieces = capture_mode ? DMS_CAPTURE_OPTICAL_DEPTH_PIECES : DMS_MAX_OPTICAL_DEPTH_PIECES;
+		const double tau_limit = capture_mode ? DMS_CAPTURE_MAX_OPTICAL_DEPTH_STEP : DMS_MAX_OPTICAL_DEPTH_STEP;
+		bool interior = false, depth = false, stop = true;
+		if(mine && n.ok)
+		{
+			const PropF q = team_prop(b, n);
+			c.before = e;
+			c.r_before = s.radius < 0.0 ? 0.0 : s.radius;
+			c.dt = n.time - s.time;
+			c.r_after = prop_radius_f(q);
+			c.v_after = n.speed;
+			c.after = prop_event_f(q);
+			stop = !((c.dt > 0.0) & (c.dt < INFINITY) & (c.v_after <= DMS_V_MAX_C * DMS_C_KMS) & (L.seg_steps + 4 < R.max_free_steps));
+			if(!stop)
+			{
+				c.s0 = 0.0f;
+				c.s1 = 1.0f;
+				interior = true;
+				if(!(c.r_before < DMS_RSUN_KM && c.r_after < DMS_RSUN_KM))
+				{
+					c.s1 = 0.0f;
+					interior = false;
+					if(!chord_stays_outside(c.before, c.after, c.r_before, c.r_after))
+						interior = interior_interval_outside(c.before, c.after, c.r_before, c.r_after, c.s0, c.s1);
+				}
+				depth = interior && c.s1 > c.s0;
+			}
+		}
+		const unsigned int dm = __ballot_sync(0xffffffffu, depth);
+		DepthF d = {0.0f, 0.0f, 0.0f, false};
+		if(dm != 0u)
+			warp_depth(R, b.P, c, static_cast<float>(s.rate), c.r_before < DMS_RSUN_KM && c.s0 <= 1.0e-12f, pieces, dm, depth,
+			           reinterpret_cast<float*>(buffer), d);
+		int verdict = VERDICT_STOP;
+		const double dtau = static_cast<double>(d.dtau);
+		if(mine && !stop && !d.invalid && (dtau >= 0.0) & (dtau < INFINITY))
+		{
+			verdict = interior & (dtau >= L.tau) ? VERDICT_SCATTER : VERDICT_PLAIN;
+			const float scale = d.dtau > static_cast<float>(DMS_OPTICAL_DEPTH_ABS_TOL) ? d.dtau : static_cast<float>(DMS_OPTICAL_DEPTH_ABS_TOL);
+			if(interior && ((dtau > tau_limit) | (!capture_mode & (fabsf(d.dtau - d.tau2) > static_cast<float>(DMS_OPTICAL_DEPTH_REL_TOL * 0.999) * scale))))
+			{
+				// (a rejection comes before the scattering test; the last retry ends the trajectory)
+				if(L.retries >= DMS_MAX_OPTICAL_DEPTH_RETRIES)
+					verdict = VERDICT_STOP;
+				else if(depth_reject(L, c.before, d.dtau, d.tau2, capture_mode != 0, c.dt, tau_limit) == PH_STEP)
+					verdict = VERDICT_RESTART;
+			}
+			if(verdict == VERDICT_PLAIN && c.r_after >= R.boundary)
+				verdict = VERDICT_BOUNDARY;
+			if(verdict == VERDICT_PLAIN && !L.is_captured)
+			{
+				// the energy that commit_event_mixed forms, or that of not_free
+				const double E = capture_mode ? NAN : capture_energy_eV_f(tables_f(R), b.m_dm, normf(c.after.x), normf(c.after.v));
+				if(isnan(E) ? not_free(R, b.m_dm, c.after) : !(isfinite(E) && E >= 0.0))
+					verdict = VERDICT_STOP;
+			}
+			if(verdict != VERDICT_STOP)
+				L.attempts += static_cast<uint64_t>(n.inner);
+			if(verdict == VERDICT_RESTART)
+				s.step = L.pr.time_step;
+			if(interior && (verdict == VERDICT_PLAIN || verdict == VERDICT_BOUNDARY))
+				L.tau -= dtau;
+			if(verdict == VERDICT_PLAIN)
+			{
+				L.seg_steps++;
+				L.steps++;
+				L.retries = 0;
+				en = c.after;
+			}
+		}
+		return verdict;
+	}
+
+	static __device__ __forceinline__ void commit(const RunParams& R, const Box& b, MixedLane& L, const EventF& e) { commit_event_mixed(R, b.m_dm, L, b.hist, e); }
+
+	// The end of a step that reaches the boundary or a scattering, as in mixed_step: `phase` is the lane's next.
+	static __device__ __forceinline__ void finish(const RunParams& R, const DevPoint* __restrict__ P, double m_dm, MixedLane& L, double2* hist, StepCtxF& c,
+	                                              const TeamState& n, bool scattering, int& phase)
+	{
+		EventF accepted = c.after;
+		int boundary = BOUNDARY_INSIDE;
+		if(!scattering)
+			boundary = boundary_step(R, m_dm, L, hist, c, accepted);
+		else
+		{
+			const bool depth = c.s1 > c.s0;
+			scatter_point(R.S, P, c, static_cast<float>(L.next_rate), depth && c.r_before < DMS_RSUN_KM && c.s0 <= 1.0e-12f, depth,
+			              R.capture_mode ? DMS_CAPTURE_OPTICAL_DEPTH_PIECES : DMS_MAX_OPTICAL_DEPTH_PIECES, L.tau, accepted);
+		}
+		if(boundary == BOUNDARY_FAILURE)
+			phase = PH_FINAL;
+		else if(boundary != BOUNDARY_RETURN)
+			phase = finish_step(R, m_dm, L, hist, c, accepted, scattering, boundary, n.time, n.radius, n.phi, n.v_radial, n.step, n.rate, true);
+	}
+};
+
 template <int THREADS>
-struct MixedStep
+struct MixedStep : Team<MixedTeam>
 {
 	static constexpr int threads = THREADS;
 	static constexpr bool throughput = THREADS > LATENCY_THREADS;
 	// (in the latency form the barriers cost more than the fetches: 16 384 Capture-mode trajectories 2.8 / 3.0 ms)
 	static constexpr bool lockstep = throughput;
 	static constexpr int buffer = COOP_BUFFER_F;
-	static constexpr bool team = false;
+	static constexpr bool team = !throughput;
 	__device__ __forceinline__ int operator()(const RunParams& R, const DevPoint* __restrict__ P, double m_dm, MixedLane& L, double2* hist, int phase,
 	                                          double* buffer) const
 	{

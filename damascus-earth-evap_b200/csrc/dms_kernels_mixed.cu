@@ -31,24 +31,24 @@ __device__ __forceinline__ const float* grid_f(const DevPoint* __restrict__ P)
 }
 
 // The event, speed and scattering rate at the propagator's state, at the start of a free segment.
-static __device__ __noinline__ void fresh_state(const DevSolar& S, const DevPoint* __restrict__ P, MixedLane& L)
+__device__ __forceinline__ void fresh_state(const DevSolar& S, const DevPoint* __restrict__ P, MixedLane& L)
 {
-	if(!L.before_valid)
-		L.before = prop_event_f(L.pr);
-	L.before_valid = L.before_valid ? L.before_valid : 1;
-	const double r = prop_radius_f(L.pr);
-	L.next_speed = prop_speed_f(L.pr);
-	L.next_rate = r >= DMS_RSUN_KM ? 0.0 : rate_total_f(S, P, grid_f(P), static_cast<float>(r), static_cast<float>(L.next_speed));
-	L.next_valid = 1;
+	if(!L.hot().before_valid)
+		L.hot().before = prop_event_f(L.hot().pr);
+	L.hot().before_valid = L.hot().before_valid ? L.hot().before_valid : 1;
+	const double r = prop_radius_f(L.hot().pr);
+	L.hot().next_speed = prop_speed_f(L.hot().pr);
+	L.hot().next_rate = r >= DMS_RSUN_KM ? 0.0 : rate_total_f(S, P, grid_f(P), static_cast<float>(r), static_cast<float>(L.hot().next_speed));
+	L.hot().next_valid = 1;
 }
 
 static __device__ __noinline__ int end_at_propagator(MixedLane& L, int reason)
 {
-	set_final(L, to_event64(prop_event_f(L.pr)), true, reason);
+	set_final(L, to_event64(prop_event_f(L.hot().pr)), true, reason);
 	return PH_FINAL;
 }
 
-static __device__ __noinline__ double surface_step(const EventF& before, double r, double step)
+__device__ __forceinline__ double surface_step(const EventF& before, double r, double step)
 {
 	const double vr = (r > 0.0) ? static_cast<double>(dotf(before.x, before.v)) / r : 0.0;
 	if(r > DMS_RSUN_KM && vr < 0.0)
@@ -79,46 +79,47 @@ __device__ __forceinline__ double inside_step(const RunParams& R, double rate, d
 // Pre-step bounds (src/Simulation_Trajectory.cpp:873-927).
 __device__ __forceinline__ int mixed_begin(const RunParams& R, const DevPoint* __restrict__ P, MixedLane& L)
 {
-	if(!(L.seg_steps < R.max_free_steps))
+	if(!(L.hot().seg_steps < R.max_free_steps))
 	{
-		if(L.before_valid == 2)  // otherwise L.cur holds the last committed event
+		if(L.hot().before_valid == 2)  // otherwise L.cur holds the last committed event
 		{
-			L.cur = to_event64(L.before);
-			L.cur.t += L.origin;
+			L.cur = to_event64(L.hot().before);
+			L.cur.t += L.hot().origin;
 		}
 		L.reason = DMS_REASON_MAX_FREE_STEPS;
 		return PH_FINAL;
 	}
 	if(wall_time_exceeded(R, L))  // "before_step", src/Simulation_Trajectory.cpp:873-874
 		return end_at_propagator(L, DMS_REASON_WALL_TIME_LIMIT);
-	if(!L.next_valid)
+	if(!L.hot().next_valid)
 		fresh_state(R.S, P, L);
-	const double r = prop_radius_f(L.pr);
-	double step = sanitized_step(L.pr.time_step), rate = 0.0;
+	const double r = prop_radius_f(L.hot().pr);
+	double step = sanitized_step(L.hot().pr.time_step), rate = 0.0;
 	if(r >= DMS_RSUN_KM)
 	{
-		step = capped_step(r, L.next_speed, step, R.boundary);
-		if(!surface_is_far(r, static_cast<double>(dotf(L.before.x, L.before.v)), step))
-			step = surface_step(L.before, r, step);
+		step = capped_step(r, L.hot().next_speed, step, R.boundary);
+		if(!surface_is_far(r, static_cast<double>(dotf(L.hot().before.x, L.hot().before.v)), step))
+			step = surface_step(L.hot().before, r, step);
 	}
 	else
 	{
-		rate = L.next_rate;
+		rate = L.hot().next_rate;
 		if(!isfinite(rate) || rate < 0.0)
 			return end_at_propagator(L, DMS_REASON_NUMERICAL_FAILURE);
 		step = inside_step(R, rate, step);
 	}
-	L.rate_before = rate;
-	L.pr.time_step = step;
-	L.in_rk = 1;
-	L.rk_inner = 0;
+	L.hot().rate_before = rate;
+	L.hot().pr.time_step = step;
+	L.hot().in_rk = 1;
+	L.hot().rk_inner = 0;
 	return PH_STEP;
 }
 
 // A step as an accepted attempt leaves it.
 struct StepCtxF
 {
-	EventF before, after;
+	const EventF* before;  // the lane's own, not a copy
+	EventF after;
 	double r_before, r_after, v_after, dt;
 	float s0, s1;
 };
@@ -134,7 +135,7 @@ __device__ __forceinline__ bool chord_stays_outside(const EventF& a, const Event
 	       ((ad >= 0.0f) | (bd <= 0.0f) | ((r - lim) * (r + lim) * dd > ad * ad * 1.0001f));
 }
 
-static __device__ __noinline__ bool interior_interval_outside(const EventF& a, const EventF& b, double ra, double rb, float& s0, float& s1)
+__device__ __forceinline__ bool interior_interval_outside(const EventF& a, const EventF& b, double ra, double rb, float& s0, float& s1)
 {
 	return interior_interval_f(a, b, ra, rb, s0, s1);
 }
@@ -203,7 +204,7 @@ __device__ __forceinline__ void lane_depth(const RunParams& R, const DevPoint* _
 		const float f = c.s0 + static_cast<float>(i) * fraction * span;
 		float rate = rate_before;
 		if(i > 0 || !first_known)
-			rate = piece_rate_f(R.S, P, grid, c.before, c.after, f, i > pieces, static_cast<float>(c.r_after), static_cast<float>(c.v_after));
+			rate = piece_rate_f(R.S, P, grid, *c.before, c.after, f, i > pieces, static_cast<float>(c.r_after), static_cast<float>(c.v_after));
 		if(i <= pieces)
 			sums.add(d, i, f, rate, dt);
 		else
@@ -230,8 +231,8 @@ __device__ __forceinline__ void warp_depth(const RunParams& R, const DevPoint* _
 		if(owner)
 		{
 			float* b = buffer + slot * COOP_SLOT_F;
-			b[0] = c.before.x.x; b[1] = c.before.x.y; b[2] = c.before.x.z;
-			b[3] = c.before.v.x; b[4] = c.before.v.y; b[5] = c.before.v.z;
+			b[0] = c.before->x.x; b[1] = c.before->x.y; b[2] = c.before->x.z;
+			b[3] = c.before->v.x; b[4] = c.before->v.y; b[5] = c.before->v.z;
 			b[6] = c.after.x.x; b[7] = c.after.x.y; b[8] = c.after.x.z;
 			b[9] = c.after.v.x; b[10] = c.after.v.y; b[11] = c.after.v.z;
 			b[12] = c.s0; b[13] = c.s1 - c.s0;
@@ -271,7 +272,7 @@ __device__ __forceinline__ void warp_depth(const RunParams& R, const DevPoint* _
 // A step whose optical depth exceeds the limit or whose two estimates differ too much
 // (src/Simulation_Trajectory.cpp:975-1011).
 constexpr int PH_CONTINUE = -1;
-static __device__ __noinline__ int depth_reject(MixedLane& L, const EventF& before, float dtau_f, float tau2, bool capture_mode, double dt, double tau_limit)
+__device__ __forceinline__ int depth_reject(MixedLane& L, const EventF& before, float dtau_f, float tau2, bool capture_mode, double dt, double tau_limit)
 {
 	const double dtau = static_cast<double>(dtau_f);
 	const float scale = dtau_f > static_cast<float>(DMS_OPTICAL_DEPTH_ABS_TOL) ? dtau_f : static_cast<float>(DMS_OPTICAL_DEPTH_ABS_TOL);
@@ -279,8 +280,8 @@ static __device__ __noinline__ int depth_reject(MixedLane& L, const EventF& befo
 	const bool reject_acc = !capture_mode && rel > DMS_OPTICAL_DEPTH_REL_TOL;
 	if(!(dtau > tau_limit) && !reject_acc)
 		return PH_CONTINUE;
-	L.retries++;
-	if(L.retries > DMS_MAX_OPTICAL_DEPTH_RETRIES)
+	L.hot().retries++;
+	if(L.hot().retries > DMS_MAX_OPTICAL_DEPTH_RETRIES)
 	{
 		set_final(L, to_event64(before), true, DMS_REASON_NUMERICAL_FAILURE);
 		return PH_FINAL;
@@ -292,12 +293,12 @@ static __device__ __noinline__ int depth_reject(MixedLane& L, const EventF& befo
 		factor = 0.8 * sqrt(DMS_OPTICAL_DEPTH_REL_TOL / rel);
 	if(factor > 1.0) factor = 1.0;
 	if(factor < DMS_RK45_MIN_STEP_FACTOR) factor = DMS_RK45_MIN_STEP_FACTOR;
-	L.pr.time_step = sanitized_step(factor * dt);
+	L.hot().pr.time_step = sanitized_step(factor * dt);
 	return PH_STEP;
 }
 
 // The scattering point (src/Simulation_Trajectory.cpp:1013-1044), the boundary rates formed again.
-static __device__ __noinline__ void scatter_point(const DevSolar& S, const DevPoint* __restrict__ P, const StepCtxF& c, float rate_before, bool first_known,
+__device__ __forceinline__ void scatter_point(const DevSolar& S, const DevPoint* __restrict__ P, const StepCtxF& c, float rate_before, bool first_known,
                                                   bool depth, int pieces, double remaining, EventF& accepted)
 {
 	if(depth)
@@ -306,12 +307,12 @@ static __device__ __noinline__ void scatter_point(const DevSolar& S, const DevPo
 		const float fraction = pieces == 4 ? 0.25f : 0.5f, span = c.s1 - c.s0;
 		float f_prev = c.s0, r_prev = rate_before;
 		if(!first_known)
-			r_prev = rate_at_fraction_f(S, P, grid, c.before, c.after, f_prev);
+			r_prev = rate_at_fraction_f(S, P, grid, *c.before, c.after, f_prev);
 #pragma unroll 1
 		for(int k = 1; k <= pieces; k++)
 		{
 			const float f = c.s0 + static_cast<float>(k) * fraction * span;
-			const float rate = rate_at_fraction_f(S, P, grid, c.before, c.after, f);
+			const float rate = rate_at_fraction_f(S, P, grid, *c.before, c.after, f);
 			if(f > f_prev)
 			{
 				const double pdt = c.dt * static_cast<double>(f - f_prev);
@@ -319,7 +320,7 @@ static __device__ __noinline__ void scatter_point(const DevSolar& S, const DevPo
 				if(ptau >= remaining)
 				{
 					const double lf = solve_linear_rate(r_prev, rate, pdt, remaining);
-					accepted = interpolate_event_f(c.before, c.after, f_prev + static_cast<float>(lf) * (f - f_prev));
+					accepted = interpolate_event_f(*c.before, c.after, f_prev + static_cast<float>(lf) * (f - f_prev));
 					return;
 				}
 				remaining -= ptau;
@@ -328,7 +329,7 @@ static __device__ __noinline__ void scatter_point(const DevSolar& S, const DevPo
 			r_prev = rate;
 		}
 	}
-	accepted = interpolate_event_f(c.before, c.after, c.s1);
+	accepted = interpolate_event_f(*c.before, c.after, c.s1);
 }
 
 // commit_accepted_event (src/Simulation_Trajectory.cpp:842-874) for an FP32 event: bincount
@@ -336,7 +337,7 @@ static __device__ __noinline__ void scatter_point(const DevSolar& S, const DevPo
 // (m_dm / (2 c^2) in FP64 first).  Returns the energy when evaluated, NaN otherwise.
 __device__ __forceinline__ double commit_event_mixed(const RunParams& R, double m_dm, MixedLane& L, double2* hist, const EventF& local)
 {
-	if(R.capture_mode && !L.is_captured)
+	if(R.capture_mode && !L.hot().is_captured)
 		return NAN;
 	const float rf = normf(local.x), vf = normf(local.v);
 	const double r_now = static_cast<double>(rf);
@@ -349,10 +350,10 @@ __device__ __forceinline__ double commit_event_mixed(const RunParams& R, double 
 		L.prev_r = r_now;
 		L.prev_v2 = v_now * v_now;
 	}
-	const double t_abs = local.t + L.origin;
+	const double t_abs = local.t + L.hot().origin;
 	const DevSolarF F = tables_f(R);
 	const double E = capture_energy_eV_f(F, m_dm, rf, vf);
-	if(L.is_captured && isfinite(L.free_flight_E))
+	if(L.hot().is_captured && isfinite(L.free_flight_E))
 	{
 		const double drift = fabs(E - L.free_flight_E);
 		if(isfinite(drift) && drift > L.max_drift_eV)
@@ -367,7 +368,7 @@ __device__ __forceinline__ double commit_event_mixed(const RunParams& R, double 
 				L.max_drift_rel = rel;
 		}
 	}
-	if(L.bound_state && L.is_captured)
+	if(L.bound_state && L.hot().is_captured)
 		L.t_last_bound = t_abs;
 	return E;
 }
@@ -378,7 +379,7 @@ static __device__ __noinline__ void commit_event_general(const RunParams& R, dou
 
 // abort_if_uncaptured_bound (src/Simulation_Trajectory.cpp:767-778, 1108) in Capture mode, where the commit
 // forms no energy: the FP64 energy of the event decides unless the FP32 speeds are far apart.
-static __device__ __noinline__ bool not_free_general(const DevSolar& S, double m_dm, const EventF& e)
+__device__ __forceinline__ bool not_free_general(const DevSolar& S, double m_dm, const EventF& e)
 {
 	const Event d = to_event64(e);
 	const double E = capture_energy_eV(S, m_dm, ev_radius(d), ev_speed(d));
@@ -406,7 +407,7 @@ enum Boundary : int
 	BOUNDARY_RETURN = 2,
 	BOUNDARY_FAILURE = 3,
 };
-static __device__ __noinline__ int boundary_step(const RunParams& R, double m_dm, MixedLane& L, double2* hist, const StepCtxF& c, EventF& accepted)
+static __device__ __noinline__ int boundary_step(const RunParams& R, double m_dm, MixedLane& L, double2* hist, StepCtxF& c)
 {
 	const DevSolar& S = R.S;
 	EventF ev = c.after;
@@ -414,7 +415,7 @@ static __device__ __noinline__ int boundary_step(const RunParams& R, double m_dm
 	if(c.r_before < R.boundary && c.r_after >= R.boundary && c.r_after > c.r_before)
 	{
 		const double f = (R.boundary - c.r_before) / (c.r_after - c.r_before);
-		ev = interpolate_event_f(c.before, c.after, static_cast<float>(f));
+		ev = interpolate_event_f(*c.before, c.after, static_cast<float>(f));
 		r_b = normf(ev.x);
 		v_b = normf(ev.v);
 	}
@@ -422,11 +423,11 @@ static __device__ __noinline__ int boundary_step(const RunParams& R, double m_dm
 		return BOUNDARY_INSIDE;
 	if(v_b > solar_vesc(S, r_b))
 	{
-		accepted = ev;
+		c.after = ev;
 		return BOUNDARY_ESCAPE;
 	}
 	Event abs_b = to_event64(ev);
-	abs_b.t += L.origin;
+	abs_b.t += L.hot().origin;
 	if(uncaptured_bound(S, m_dm, L, abs_b))
 	{
 		set_final(L, abs_b, false, DMS_REASON_NUMERICAL_FAILURE);
@@ -435,19 +436,19 @@ static __device__ __noinline__ int boundary_step(const RunParams& R, double m_dm
 	Event inbound;
 	if(!bound_kepler_return(to_event64(ev), inbound))
 		return BOUNDARY_INSIDE;
-	L.seg_steps++;
-	L.steps++;
-	L.retries = 0;
+	L.hot().seg_steps++;
+	L.hot().steps++;
+	L.hot().retries = 0;
 	commit_event_general(R, m_dm, L, hist, ev);
 	// reset_propagator_at_absolute_event, src/Simulation_Trajectory.cpp:814-822
 	L.cur = inbound;
-	L.cur.t += L.origin;
-	L.origin = L.cur.t;
+	L.cur.t += L.hot().origin;
+	L.hot().origin = L.cur.t;
 	Event local = inbound;
 	local.t = 0.0;
-	prop_init_f(L.pr, local);
-	L.before_valid = 0;
-	L.next_valid = 0;
+	prop_init_f(L.hot().pr, local);
+	L.hot().before_valid = 0;
+	L.hot().next_valid = 0;
 	if(!R.capture_mode && L.prev_time >= 0.0)
 		L.prev_time = 0.0;
 	return BOUNDARY_RETURN;
@@ -456,20 +457,20 @@ static __device__ __noinline__ int boundary_step(const RunParams& R, double m_dm
 // as in dms_kernels.cu
 constexpr int COOP_MAX_STEPS = 15;
 
-// The end of a step that has not been rejected, for the committed event `accepted` and the propagator after it.
-__device__ __forceinline__ int finish_step(const RunParams& R, double m_dm, MixedLane& L, double2* hist, const StepCtxF& c, const EventF& accepted,
+// The end of a step that has not been rejected, for the committed event c.after and the propagator after it.
+__device__ __forceinline__ int finish_step(const RunParams& R, double m_dm, MixedLane& L, double2* hist, const StepCtxF& c,
                                            bool scattering, int boundary, double time, double radius, double phi, double v_radial, double time_step,
                                            double next_rate, bool next_known)
 {
-	L.seg_steps++;
-	L.steps++;
-	L.retries = 0;
-	const double E = commit_event_mixed(R, m_dm, L, hist, accepted);
-	const bool bound = !L.is_captured && (isnan(E) ? not_free(R, m_dm, accepted) : !(isfinite(E) && E >= 0.0));
+	L.hot().seg_steps++;
+	L.hot().steps++;
+	L.hot().retries = 0;
+	const double E = commit_event_mixed(R, m_dm, L, hist, c.after);
+	const bool bound = !L.hot().is_captured && (isnan(E) ? not_free(R, m_dm, c.after) : !(isfinite(E) && E >= 0.0));
 	if(bound | scattering | (boundary == BOUNDARY_ESCAPE))
 	{
-		L.cur = to_event64(accepted);
-		L.cur.t += L.origin;
+		L.cur = to_event64(c.after);
+		L.cur.t += L.hot().origin;
 		if(bound)
 			L.reason = DMS_REASON_NUMERICAL_FAILURE;
 		else if(!scattering)
@@ -480,16 +481,16 @@ __device__ __forceinline__ int finish_step(const RunParams& R, double m_dm, Mixe
 			L.reason = DMS_REASON_SCATTER;
 		return PH_FINAL;
 	}
-	L.pr.time = time;
-	L.pr.radius = radius;
-	L.pr.phi = phi;
-	L.pr.v_radial = v_radial;
-	L.pr.time_step = time_step;
-	L.before = c.after;
-	L.before_valid = 2;
-	L.next_speed = c.v_after;
-	L.next_rate = next_rate;
-	L.next_valid = next_known || c.r_after >= DMS_RSUN_KM;
+	L.hot().pr.time = time;
+	L.hot().pr.radius = radius;
+	L.hot().pr.phi = phi;
+	L.hot().pr.v_radial = v_radial;
+	L.hot().pr.time_step = time_step;
+	L.hot().before = c.after;
+	L.hot().before_valid = 2;
+	L.hot().next_speed = c.v_after;
+	L.hot().next_rate = next_rate;
+	L.hot().next_valid = next_known || c.r_after >= DMS_RSUN_KM;
 	return PH_STEP;
 }
 
@@ -505,24 +506,23 @@ __device__ __forceinline__ int mixed_step(const RunParams& R, const DevPoint* __
 	PropF q;
 	bool done = false, interior = false, depth = false;
 	int reason = 0;
-	if(phase == PH_STEP && !L.in_rk)
+	if(phase == PH_STEP && !L.hot().in_rk)
 		phase = mixed_begin(R, P, L);
 	if(phase == PH_STEP)
 	{
-		q = L.pr;
-		L.rk_inner++;
-		const int rk = rk45_attempt_f<UNROLLED>(tables_f(R), q, L.rk_inner);
+		q = L.hot().pr;
+		L.hot().rk_inner++;
+		const int rk = rk45_attempt_f<UNROLLED>(tables_f(R), q, L.hot().rk_inner);
 		if(rk == RK_RETRY)
-			L.pr.time_step = q.time_step;
+			L.hot().pr.time_step = q.time_step;
 		else
 		{
 			done = true;
-			L.in_rk = 0;
-			L.attempts += static_cast<uint64_t>(L.rk_inner);
-			c.before = L.before;
-			c.before.t = L.pr.time;
-			c.r_before = prop_radius_f(L.pr);
-			c.dt = q.time - L.pr.time;
+			L.hot().in_rk = 0;
+			L.hot().attempts += static_cast<uint64_t>(L.hot().rk_inner);
+			c.before = &L.hot().before;
+			c.r_before = prop_radius_f(L.hot().pr);
+			c.dt = q.time - L.hot().pr.time;
 			c.r_after = prop_radius_f(q);
 			c.v_after = prop_speed_f(q);
 			c.after = prop_event_f(q);
@@ -544,8 +544,8 @@ __device__ __forceinline__ int mixed_step(const RunParams& R, const DevPoint* __
 				{
 					c.s1 = 0.0f;
 					interior = false;
-					if(!chord_stays_outside(c.before, c.after, c.r_before, c.r_after))
-						interior = interior_interval_outside(c.before, c.after, c.r_before, c.r_after, c.s0, c.s1);
+					if(!chord_stays_outside(*c.before, c.after, c.r_before, c.r_after))
+						interior = interior_interval_outside(*c.before, c.after, c.r_before, c.r_after, c.s0, c.s1);
 				}
 				depth = interior && c.s1 > c.s0;
 			}
@@ -554,7 +554,7 @@ __device__ __forceinline__ int mixed_step(const RunParams& R, const DevPoint* __
 	const unsigned int dm = __ballot_sync(0xffffffffu, depth);
 	DepthF d = {0.0f, 0.0f, 0.0f, false};
 	const bool first_known = depth && c.r_before < DMS_RSUN_KM && c.s0 <= 1.0e-12f;
-	const float rate_before = static_cast<float>(L.rate_before);
+	const float rate_before = static_cast<float>(L.hot().rate_before);
 	if(dm != 0u)
 	{
 		if(__popc(dm) <= COOP_MAX_STEPS)
@@ -572,7 +572,6 @@ __device__ __forceinline__ int mixed_step(const RunParams& R, const DevPoint* __
 		set_final(L, to_event64(c.after), true, reason);
 		return PH_FINAL;
 	}
-	EventF accepted = c.after;
 	bool scattering = false;
 	if(interior)
 	{
@@ -580,28 +579,28 @@ __device__ __forceinline__ int mixed_step(const RunParams& R, const DevPoint* __
 		const float scale = d.dtau > static_cast<float>(DMS_OPTICAL_DEPTH_ABS_TOL) ? d.dtau : static_cast<float>(DMS_OPTICAL_DEPTH_ABS_TOL);
 		if((dtau > tau_limit) | (!capture_mode & (fabsf(d.dtau - d.tau2) > static_cast<float>(DMS_OPTICAL_DEPTH_REL_TOL * 0.999) * scale)))
 		{
-			const int rejected = depth_reject(L, c.before, d.dtau, d.tau2, capture_mode != 0, c.dt, tau_limit);
+			const int rejected = depth_reject(L, *c.before, d.dtau, d.tau2, capture_mode != 0, c.dt, tau_limit);
 			if(rejected != PH_CONTINUE)
 				return rejected;
 		}
-		if(dtau >= L.tau)
+		if(dtau >= L.hot().tau)
 		{
-			scatter_point(R.S, P, c, rate_before, first_known, depth, pieces, L.tau, accepted);
+			scatter_point(R.S, P, c, rate_before, first_known, depth, pieces, L.hot().tau, c.after);
 			scattering = true;
 		}
 		else
-			L.tau -= dtau;
+			L.hot().tau -= dtau;
 	}
 	int boundary = BOUNDARY_INSIDE;
 	if(!scattering && c.r_after >= R.boundary)
 	{
-		boundary = boundary_step(R, m_dm, L, hist, c, accepted);
+		boundary = boundary_step(R, m_dm, L, hist, c);
 		if(boundary == BOUNDARY_RETURN)
 			return PH_STEP;
 		if(boundary == BOUNDARY_FAILURE)
 			return PH_FINAL;
 	}
-	return finish_step(R, m_dm, L, hist, c, accepted, scattering, boundary, q.time, q.radius, q.phi, q.v_radial, q.time_step,
+	return finish_step(R, m_dm, L, hist, c, scattering, boundary, q.time, q.radius, q.phi, q.v_radial, q.time_step,
 	                   static_cast<double>(d.next_rate), depth);
 }
 
@@ -612,7 +611,7 @@ struct MixedTeam
 	using Box = TeamBox<PropF, EventF>;
 	using Ctx = StepCtxF;
 	static __device__ __forceinline__ void fresh(const RunParams& R, const DevPoint* __restrict__ P, MixedLane& L) { fresh_state(R.S, P, L); }
-	static __device__ __forceinline__ bool fits(const MixedLane& L) { return L.pr.radial_mode == 0; }
+	static __device__ __forceinline__ bool fits(const MixedLane& L) { return L.hot().pr.radial_mode == 0; }
 
 	static __device__ __forceinline__ void propagate(const RunParams& R, const Box& b, const TeamState& s, TeamState& n)
 	{
@@ -662,13 +661,13 @@ struct MixedTeam
 		if(mine && n.ok)
 		{
 			const PropF q = team_prop(b, n);
-			c.before = e;
+			c.before = &e;
 			c.r_before = s.radius < 0.0 ? 0.0 : s.radius;
 			c.dt = n.time - s.time;
 			c.r_after = prop_radius_f(q);
 			c.v_after = n.speed;
 			c.after = prop_event_f(q);
-			stop = !((c.dt > 0.0) & (c.dt < INFINITY) & (c.v_after <= DMS_V_MAX_C * DMS_C_KMS) & (L.seg_steps + 4 < R.max_free_steps));
+			stop = !((c.dt > 0.0) & (c.dt < INFINITY) & (c.v_after <= DMS_V_MAX_C * DMS_C_KMS) & (L.hot().seg_steps + 4 < R.max_free_steps));
 			if(!stop)
 			{
 				c.s0 = 0.0f;
@@ -678,8 +677,8 @@ struct MixedTeam
 				{
 					c.s1 = 0.0f;
 					interior = false;
-					if(!chord_stays_outside(c.before, c.after, c.r_before, c.r_after))
-						interior = interior_interval_outside(c.before, c.after, c.r_before, c.r_after, c.s0, c.s1);
+					if(!chord_stays_outside(*c.before, c.after, c.r_before, c.r_after))
+						interior = interior_interval_outside(*c.before, c.after, c.r_before, c.r_after, c.s0, c.s1);
 				}
 				depth = interior && c.s1 > c.s0;
 			}
@@ -693,19 +692,19 @@ struct MixedTeam
 		const double dtau = static_cast<double>(d.dtau);
 		if(mine && !stop && !d.invalid && (dtau >= 0.0) & (dtau < INFINITY))
 		{
-			verdict = interior & (dtau >= L.tau) ? VERDICT_SCATTER : VERDICT_PLAIN;
+			verdict = interior & (dtau >= L.hot().tau) ? VERDICT_SCATTER : VERDICT_PLAIN;
 			const float scale = d.dtau > static_cast<float>(DMS_OPTICAL_DEPTH_ABS_TOL) ? d.dtau : static_cast<float>(DMS_OPTICAL_DEPTH_ABS_TOL);
 			if(interior && ((dtau > tau_limit) | (!capture_mode & (fabsf(d.dtau - d.tau2) > static_cast<float>(DMS_OPTICAL_DEPTH_REL_TOL * 0.999) * scale))))
 			{
 				// (a rejection comes before the scattering test; the last retry ends the trajectory)
-				if(L.retries >= DMS_MAX_OPTICAL_DEPTH_RETRIES)
+				if(L.hot().retries >= DMS_MAX_OPTICAL_DEPTH_RETRIES)
 					verdict = VERDICT_STOP;
-				else if(depth_reject(L, c.before, d.dtau, d.tau2, capture_mode != 0, c.dt, tau_limit) == PH_STEP)
+				else if(depth_reject(L, *c.before, d.dtau, d.tau2, capture_mode != 0, c.dt, tau_limit) == PH_STEP)
 					verdict = VERDICT_RESTART;
 			}
 			if(verdict == VERDICT_PLAIN && c.r_after >= R.boundary)
 				verdict = VERDICT_BOUNDARY;
-			if(verdict == VERDICT_PLAIN && !L.is_captured)
+			if(verdict == VERDICT_PLAIN && !L.hot().is_captured)
 			{
 				// the energy that commit_event_mixed forms, or that of not_free
 				const double E = capture_mode ? NAN : capture_energy_eV_f(tables_f(R), b.m_dm, normf(c.after.x), normf(c.after.v));
@@ -713,16 +712,16 @@ struct MixedTeam
 					verdict = VERDICT_STOP;
 			}
 			if(verdict != VERDICT_STOP)
-				L.attempts += static_cast<uint64_t>(n.inner);
+				L.hot().attempts += static_cast<uint64_t>(n.inner);
 			if(verdict == VERDICT_RESTART)
-				s.step = L.pr.time_step;
+				s.step = L.hot().pr.time_step;
 			if(interior && (verdict == VERDICT_PLAIN || verdict == VERDICT_BOUNDARY))
-				L.tau -= dtau;
+				L.hot().tau -= dtau;
 			if(verdict == VERDICT_PLAIN)
 			{
-				L.seg_steps++;
-				L.steps++;
-				L.retries = 0;
+				L.hot().seg_steps++;
+				L.hot().steps++;
+				L.hot().retries = 0;
 				en = c.after;
 			}
 		}
@@ -735,20 +734,19 @@ struct MixedTeam
 	static __device__ __forceinline__ void finish(const RunParams& R, const DevPoint* __restrict__ P, double m_dm, MixedLane& L, double2* hist, StepCtxF& c,
 	                                              const TeamState& n, bool scattering, int& phase)
 	{
-		EventF accepted = c.after;
 		int boundary = BOUNDARY_INSIDE;
 		if(!scattering)
-			boundary = boundary_step(R, m_dm, L, hist, c, accepted);
+			boundary = boundary_step(R, m_dm, L, hist, c);
 		else
 		{
 			const bool depth = c.s1 > c.s0;
-			scatter_point(R.S, P, c, static_cast<float>(L.next_rate), depth && c.r_before < DMS_RSUN_KM && c.s0 <= 1.0e-12f, depth,
-			              R.capture_mode ? DMS_CAPTURE_OPTICAL_DEPTH_PIECES : DMS_MAX_OPTICAL_DEPTH_PIECES, L.tau, accepted);
+			scatter_point(R.S, P, c, static_cast<float>(L.hot().next_rate), depth && c.r_before < DMS_RSUN_KM && c.s0 <= 1.0e-12f, depth,
+			              R.capture_mode ? DMS_CAPTURE_OPTICAL_DEPTH_PIECES : DMS_MAX_OPTICAL_DEPTH_PIECES, L.hot().tau, c.after);
 		}
 		if(boundary == BOUNDARY_FAILURE)
 			phase = PH_FINAL;
 		else if(boundary != BOUNDARY_RETURN)
-			phase = finish_step(R, m_dm, L, hist, c, accepted, scattering, boundary, n.time, n.radius, n.phi, n.v_radial, n.step, n.rate, true);
+			phase = finish_step(R, m_dm, L, hist, c, scattering, boundary, n.time, n.radius, n.phi, n.v_radial, n.step, n.rate, true);
 	}
 };
 
@@ -798,12 +796,10 @@ __global__ void grid_to_float_kernel(const double* __restrict__ in, float* __res
 
 void Launch_Trajectories_Mixed(const RunParams& p, int blocks, int threads, cudaStream_t stream)
 {
-	if(threads <= LATENCY_THREADS)
-		trajectory_kernel_mixed_latency<<<blocks, threads, 0, stream>>>(p);
-	else if(threads <= MAX_THREADS)
-		trajectory_kernel_mixed<MAX_THREADS><<<blocks, threads, 0, stream>>>(p);
-	else
-		trajectory_kernel_mixed<MAX_THREADS_MIXED><<<blocks, threads, 0, stream>>>(p);
+	const auto kernel = threads <= LATENCY_THREADS ? trajectory_kernel_mixed_latency
+	                    : threads <= MAX_THREADS   ? trajectory_kernel_mixed<MAX_THREADS>
+	                                               : trajectory_kernel_mixed<MAX_THREADS_MIXED>;
+	Launch_With_Hot_States<MixedLane>(kernel, p, blocks, threads, stream);
 }
 
 void Launch_To_Float(const double* in, float* out, size_t n, cudaStream_t stream)

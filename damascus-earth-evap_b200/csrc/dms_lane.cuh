@@ -23,6 +23,43 @@ enum Phase : int
 };
 
 
+// The part of a lane's state that every pass reads and writes.  It lies in shared memory (127 KB of a full FP64
+// block): the states of a block's lanes are larger than its L1 cache, and in local memory more than half of
+// their reads went to L2, the longest of the kernel's waits.  An odd number of 8-byte words keeps the lanes
+// of a warp on different banks.  Together with the calls written out in the pass (dms_kernels.cu), 2^20
+// Capture-mode trajectories take 40.9 -> 36.5 ms in FP64 and 25.3 -> 23.5 ms in the mixed form, the steady state
+// of Parameter-point mode 855 -> 932 and 1 305 -> 1 407 Msteps/s; with the bincount and drift fields here too
+// (160 KB) the tables lose their place in L1: 39.1 against 38.5 ms.
+template <class PropT, class EvT>
+struct HotFields
+{
+	PropT pr;            // propagator of the current free segment (local time)
+	EvT before;          // Event_In_3D of the propagator at the start of the step (cached)
+	double origin;       // absolute time of the segment's local t = 0
+	double tau;          // remaining optical depth to the next scattering (minus_log_xi)
+	double rate_before;  // scattering rate at the start of the step
+	double next_speed, next_rate;
+	uint64_t seg_steps;
+	uint64_t steps;      // accepted free steps of the whole trajectory (work counter)
+	uint64_t attempts;   // RK45 attempts of the whole trajectory (work counter)
+	unsigned int retries;
+	int before_valid;
+	int in_rk;           // an RK45 step is in progress (retry pending)
+	int rk_inner;        // passes of the current RK45 step
+	int next_valid;      // next_speed / next_rate hold the propagator's speed and rate
+	int is_captured;
+};
+template <class PropT, class EvT, bool EVEN = sizeof(HotFields<PropT, EvT>) / 8 % 2 == 0>
+struct HotState : HotFields<PropT, EvT>
+{
+};
+template <class PropT, class EvT>
+struct HotState<PropT, EvT, true> : HotFields<PropT, EvT>
+{
+	double unused;
+};
+extern __shared__ double lane_hot_states[];
+
 // Trajectory state of a lane (TrajectoryBincount + Trajectory_Simulator members,
 // include/Simulation_Trajectory.hpp:53-154).
 template <class PropT, class EvT>
@@ -31,29 +68,17 @@ struct LaneT
 	// the FP64 form bins by the reference's division; the mixed form multiplies by the
 	// reciprocal bin width (a bin edge can then move by one ulp)
 	static constexpr bool exact_bins = std::is_same<PropT, Prop>::value;
+	using Hot = HotState<PropT, EvT>;
+	static_assert(sizeof(Hot) / 8 % 2 == 1, "lanes on different banks");
+	static __device__ __forceinline__ Hot& hot() { return reinterpret_cast<Hot*>(lane_hot_states)[threadIdx.x]; }
 	uint64_t work;
 	int point;
 	Draws D;
 	Event cur;           // absolute event at segment boundaries and at termination
-	PropT pr;            // propagator of the current free segment (local time)
-	EvT before;          // Event_In_3D of the propagator at the start of the step (cached)
-	double origin;       // absolute time of the segment's local t = 0
-	double tau;          // remaining optical depth to the next scattering (minus_log_xi)
-	uint64_t seg_steps;
 	uint64_t nscat;
-	uint64_t steps;      // accepted free steps of the whole trajectory (work counter)
-	uint64_t attempts;   // RK45 attempts of the whole trajectory (work counter)
-	unsigned int retries;
-	int before_valid;
-	int in_rk;           // an RK45 step is in progress (retry pending)
-	int rk_inner;        // passes of the current RK45 step
-	double rate_before;  // scattering rate at the start of the step
-	int next_valid;      // next_speed / next_rate hold the propagator's speed and rate
-	double next_speed, next_rate;
 	int shift_ok;
 	int reason;
 	// capture / evaporation state
-	int is_captured;
 	int bound_state;
 	double t_capture, t_last_bound, t_final_unbinding;
 	double free_flight_E;
@@ -140,13 +165,13 @@ __device__ __forceinline__ void write_back_bin(Lane& L, double2* hist)
 template <class Lane>
 __device__ __forceinline__ bool update_capture_state(const DevSolar& S, double m_dm, int capture_mode, Lane& L, double r, double v, double t, bool allow_new)
 {
-	if(capture_mode && !allow_new && !L.is_captured)
+	if(capture_mode && !allow_new && !L.hot().is_captured)
 		return false;
 	const double E = capture_energy_eV(S, m_dm, r, v);
 	const bool negative = E < 0.0;
 	if(!allow_new)
 	{
-		if(L.is_captured && isfinite(L.free_flight_E))
+		if(L.hot().is_captured && isfinite(L.free_flight_E))
 		{
 			const double drift = fabs(E - L.free_flight_E);
 			if(isfinite(drift) && drift > L.max_drift_eV)
@@ -157,7 +182,7 @@ __device__ __forceinline__ bool update_capture_state(const DevSolar& S, double m
 			if(isfinite(rel) && rel > L.max_drift_rel)
 				L.max_drift_rel = rel;
 		}
-		if(L.bound_state && L.is_captured)
+		if(L.bound_state && L.hot().is_captured)
 			L.t_last_bound = t;
 		return false;
 	}
@@ -166,9 +191,9 @@ __device__ __forceinline__ bool update_capture_state(const DevSolar& S, double m
 	L.free_flight_E = E;
 	if(negative)
 	{
-		if(!L.is_captured)
+		if(!L.hot().is_captured)
 		{
-			L.is_captured = 1;
+			L.hot().is_captured = 1;
 			L.t_capture = t;
 			L.t_last_bound = t;
 		}
@@ -177,7 +202,7 @@ __device__ __forceinline__ bool update_capture_state(const DevSolar& S, double m
 		L.t_last_bound = t;
 		return true;
 	}
-	if(was_bound && L.is_captured)
+	if(was_bound && L.hot().is_captured)
 		L.t_final_unbinding = t;
 	return false;
 }
@@ -185,7 +210,7 @@ __device__ __forceinline__ bool update_capture_state(const DevSolar& S, double m
 template <class Lane>
 __device__ __forceinline__ bool uncaptured_bound(const DevSolar& S, double m_dm, const Lane& L, const Event& e)
 {
-	if(L.is_captured)
+	if(L.hot().is_captured)
 		return false;
 	const double E = capture_energy_eV(S, m_dm, ev_radius(e), ev_speed(e));
 	if(isfinite(E) && E >= 0.0)
@@ -198,7 +223,7 @@ __device__ __forceinline__ void set_final(Lane& L, const Event& local_or_abs, bo
 {
 	L.cur = local_or_abs;
 	if(is_local)
-		L.cur.t += L.origin;
+		L.cur.t += L.hot().origin;
 	L.reason = reason;
 }
 
@@ -224,16 +249,16 @@ __device__ __forceinline__ int segment_start(const RunParams& R, const DevPoint*
 		L.reason = DMS_REASON_NUMERICAL_FAILURE;
 		return PH_FINAL;
 	}
-	L.origin = L.cur.t;
+	L.hot().origin = L.cur.t;
 	Event local = L.cur;
 	local.t = 0.0;
-	init_propagator(L.pr, local);
-	L.tau = -log_call(draw_positive(L.D));
-	L.seg_steps = 0;
-	L.retries = 0;
-	L.before_valid = 0;
-	L.next_valid = 0;
-	L.in_rk = 0;
+	init_propagator(L.hot().pr, local);
+	L.hot().tau = -log_call(draw_positive(L.D));
+	L.hot().seg_steps = 0;
+	L.hot().retries = 0;
+	L.hot().before_valid = 0;
+	L.hot().next_valid = 0;
+	L.hot().in_rk = 0;
 	if(!R.capture_mode && L.prev_time >= 0.0)
 		L.prev_time = 0.0;
 	return PH_STEP;
@@ -278,7 +303,7 @@ __device__ __noinline__ void finalize(const RunParams& R, const DevPoint* __rest
 	if(L.shift_ok)
 	{
 		flags |= DMS_REC_SHIFT_OK;
-		if(L.is_captured)
+		if(L.hot().is_captured)
 		{
 			const double r_f = ev_radius(L.cur), v_f = ev_speed(L.cur);
 			const double vesc_f = solar_vesc(S, r_f);
@@ -311,18 +336,18 @@ __device__ __noinline__ void finalize(const RunParams& R, const DevPoint* __rest
 			case DMS_REASON_UNKNOWN: survival_valid = 0; break;
 			default: break;
 		}
-		if(L.is_captured && !event_observed)
+		if(L.hot().is_captured && !event_observed)
 		{
 			L.t_final_unbinding = NAN;
 			if(reason != DMS_REASON_CAPTURE_MODE)
 				survival_valid = 0;
 		}
-		if(L.is_captured) flags |= DMS_REC_CAPTURED;
+		if(L.hot().is_captured) flags |= DMS_REC_CAPTURED;
 		if(event_observed) flags |= DMS_REC_EVENT_OBSERVED;
 		if(survival_valid) flags |= DMS_REC_SURVIVAL_VALID;
 		if(boundary_escape) flags |= DMS_REC_BOUNDARY_ESCAPE;
 		if(invalid_escape) flags |= DMS_REC_INVALID_ESCAPE;
-		if(!L.is_captured && reason == DMS_REASON_OUTWARD_ESCAPE)
+		if(!L.hot().is_captured && reason == DMS_REASON_OUTWARD_ESCAPE)
 		{
 			if(L.nscat == 0)
 				flags |= DMS_REC_FREE;
@@ -370,7 +395,7 @@ __device__ __noinline__ void finalize(const RunParams& R, const DevPoint* __rest
 	const bool valid = survival_valid && !invalid;
 	const bool observed = valid && event_observed;
 	const double life = observed ? L.t_final_unbinding - L.t_capture : -1.0;
-	const double lifetime = (L.is_captured && isfinite(life) && life >= 0.0) ? life : -1.0;
+	const double lifetime = (L.hot().is_captured && isfinite(life) && life >= 0.0) ? life : -1.0;
 
 	job.b0 = L.bmin;
 	job.b1 = L.bmax;
@@ -409,8 +434,8 @@ __device__ __noinline__ void finalize(const RunParams& R, const DevPoint* __rest
 		unsigned long long* c = R.counters + static_cast<size_t>(L.point) * DMS_NUM_COUNTERS;
 		atomicAdd(c + DMS_CNT_TRAJECTORIES, 1ULL);
 		atomicAdd(c + DMS_CNT_TOTAL_SCATTERINGS, static_cast<unsigned long long>(L.nscat));
-		atomicAdd(c + DMS_CNT_RK_STEPS, static_cast<unsigned long long>(L.steps));
-		atomicAdd(c + DMS_CNT_RK_ATTEMPTS, static_cast<unsigned long long>(L.attempts));
+		atomicAdd(c + DMS_CNT_RK_STEPS, static_cast<unsigned long long>(L.hot().steps));
+		atomicAdd(c + DMS_CNT_RK_ATTEMPTS, static_cast<unsigned long long>(L.hot().attempts));
 		atomicAdd(c + DMS_CNT_REASON_BASE + reason, 1ULL);
 		if(!L.shift_ok)
 		{
@@ -422,7 +447,7 @@ __device__ __noinline__ void finalize(const RunParams& R, const DevPoint* __rest
 		if(is_computational_truncation(reason))
 			atomicAdd(c + DMS_CNT_COMPUTATIONAL_TRUNCATIONS, 1ULL);
 		int hist_slot = -1;
-		if(L.is_captured)
+		if(L.hot().is_captured)
 		{
 			atomicAdd(c + DMS_CNT_CAPTURED, 1ULL);
 			if(!R.capture_mode)
@@ -543,10 +568,10 @@ __device__ __forceinline__ int start_trajectory(const RunParams& R, Lane& L, uin
 	L.D.traj = R.range_first[k] + (w - R.range_offset[k]);
 	L.D.index = 0;
 	L.nscat = 0;
-	L.steps = 0;
-	L.attempts = 0;
+	L.hot().steps = 0;
+	L.hot().attempts = 0;
 	L.wall_start = R.wall_limit_ns != 0 ? global_timer_ns() : 0;
-	L.is_captured = 0;
+	L.hot().is_captured = 0;
 	L.bound_state = 0;
 	L.t_capture = -1.0;
 	L.t_last_bound = -1.0;
@@ -683,6 +708,7 @@ template <class Lane>
 struct Parked
 {
 	Lane L;
+	typename Lane::Hot hot;
 	double2* hist;          // its histogram row
 	uint64_t q_next, q_end; // its lane's claimed ids
 	uint64_t iter;
@@ -739,6 +765,7 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 			{
 				const Parked<Lane>& s = *reinterpret_cast<const Parked<Lane>*>(R.parked + item * PARKED_BYTES);
 				L = s.L;
+				L.hot() = s.hot;
 				hist = s.hist;
 				q_next = s.q_next;
 				q_end = s.q_end;
@@ -827,6 +854,7 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 					{
 						Parked<Lane>& s = *reinterpret_cast<Parked<Lane>*>(R.parked + atomicAdd(R.parked_count, 1u) * PARKED_BYTES);
 						s.L = L;
+						s.hot = L.hot();
 						s.hist = hist;
 						s.q_next = q_next;
 						s.q_end = q_end;
@@ -872,8 +900,8 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 			}
 			if constexpr(Step::team)
 			{
-				const bool mine = phase == PH_STEP && !L.in_rk;
-				alone |= __any_sync(FULL_WARP, phase == PH_STEP && L.in_rk);
+				const bool mine = phase == PH_STEP && !L.hot().in_rk;
+				alone |= __any_sync(FULL_WARP, phase == PH_STEP && L.hot().in_rk);
 				if((live & (live - 1u)) == 0u && __any_sync(FULL_WARP, mine) && R.wall_limit_ns == 0)
 				{
 					if(!team)
@@ -963,9 +991,19 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 		unsigned long long* c = R.counters + static_cast<size_t>(L.point) * DMS_NUM_COUNTERS;
 		atomicAdd(c + DMS_CNT_UNFINISHED_TRAJECTORIES, 1ULL);
 		atomicAdd(c + DMS_CNT_UNFINISHED_SCATTERINGS, static_cast<unsigned long long>(L.nscat));
-		atomicAdd(c + DMS_CNT_UNFINISHED_RK_STEPS, static_cast<unsigned long long>(L.steps));
-		atomicAdd(c + DMS_CNT_UNFINISHED_RK_ATTEMPTS, static_cast<unsigned long long>(L.attempts));
+		atomicAdd(c + DMS_CNT_UNFINISHED_RK_STEPS, static_cast<unsigned long long>(L.hot().steps));
+		atomicAdd(c + DMS_CNT_UNFINISHED_RK_ATTEMPTS, static_cast<unsigned long long>(L.hot().attempts));
 	}
+}
+
+// The launch of a kernel that runs lane_loop, with the shared memory of its lanes.
+template <class Lane>
+void Launch_With_Hot_States(void (*kernel)(const RunParams), const RunParams& p, int blocks, int threads, cudaStream_t stream)
+{
+	const size_t bytes = sizeof(typename Lane::Hot) * threads;
+	// (a refusal shows as the launch's error)
+	cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+	kernel<<<blocks, threads, bytes, stream>>>(p);
 }
 
 }	// namespace lane

@@ -191,13 +191,13 @@ struct Team
 				return;
 			if(rank == 1)
 			{
-				L.is_captured = b.captured;
+				L.hot().is_captured = b.captured;
 				L.bound_state = b.bound;
 				L.bmin = b.bmin;
 				L.bmax = b.bmax;
 				L.cbin = b.cbin;
 				L.cval = b.cval;
-				L.origin = b.origin;
+				L.hot().origin = b.origin;
 				L.prev_time = b.prev_time;
 				L.prev_r = b.prev_r;
 				L.prev_v2 = b.prev_v2;
@@ -257,7 +257,7 @@ struct Team
 	                                     double* buffer, int& phase, uint64_t& iter) const
 	{
 		Box& b = box();
-		if(mine && !L.next_valid)
+		if(mine && !L.hot().next_valid)
 			T::fresh(R, P, L);
 		const bool fit = mine && T::fits(L);
 		if(!__any_sync(0xffffffffu, fit))
@@ -267,14 +267,14 @@ struct Team
 			b.P = P;
 			b.hist = hist;
 			b.m_dm = m_dm;
-			b.pr = L.pr;
-			b.captured = L.is_captured;
+			b.pr = L.hot().pr;
+			b.captured = L.hot().is_captured;
 			b.bound = L.bound_state;
 			b.bmin = L.bmin;
 			b.bmax = L.bmax;
 			b.cbin = L.cbin;
 			b.cval = L.cval;
-			b.origin = L.origin;
+			b.origin = L.hot().origin;
 			b.prev_time = L.prev_time;
 			b.prev_r = L.prev_r;
 			b.prev_v2 = L.prev_v2;
@@ -283,15 +283,15 @@ struct Team
 			b.max_drift_eV = L.max_drift_eV;
 			b.max_drift_rel = L.max_drift_rel;
 			TeamState& s = b.s[0];
-			s.time = L.pr.time;
-			s.radius = L.pr.radius;
-			s.phi = L.pr.phi;
-			s.v_radial = L.pr.v_radial;
-			s.step = L.pr.time_step;
-			s.speed = L.next_speed;
-			s.rate = L.next_rate;
-			b.e[0] = L.before;
-			b.e[0].t = L.pr.time;
+			s.time = L.hot().pr.time;
+			s.radius = L.hot().pr.radius;
+			s.phi = L.hot().pr.phi;
+			s.v_radial = L.hot().pr.v_radial;
+			s.step = L.hot().pr.time_step;
+			s.speed = L.hot().next_speed;
+			s.rate = L.hot().next_rate;
+			b.e[0] = L.hot().before;
+			b.e[0].t = L.hot().pr.time;
 		}
 		__syncwarp();
 		team_barrier();
@@ -302,17 +302,17 @@ struct Team
 		if(mine)
 		{
 			const TeamState& s = b.s[j & 3];
-			L.pr.time = s.time;
-			L.pr.radius = s.radius;
-			L.pr.phi = s.phi;
-			L.pr.v_radial = s.v_radial;
-			L.pr.time_step = s.step;
-			L.next_speed = s.speed;
-			L.next_rate = s.rate;
+			L.hot().pr.time = s.time;
+			L.hot().pr.radius = s.radius;
+			L.hot().pr.phi = s.phi;
+			L.hot().pr.v_radial = s.v_radial;
+			L.hot().pr.time_step = s.step;
+			L.hot().next_speed = s.speed;
+			L.hot().next_rate = s.rate;
 			if(j > 0)
 			{
-				L.before = b.e[j & 3];
-				L.before_valid = 2;
+				L.hot().before = b.e[j & 3];
+				L.hot().before_valid = 2;
 			}
 			L.bmin = b.bmin;
 			L.bmax = b.bmax;

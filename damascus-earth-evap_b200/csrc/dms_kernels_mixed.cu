@@ -372,10 +372,6 @@ __device__ __forceinline__ double commit_event_mixed(const RunParams& R, double 
 		L.t_last_bound = t_abs;
 	return E;
 }
-static __device__ __noinline__ void commit_event_general(const RunParams& R, double m_dm, MixedLane& L, double2* hist, const EventF& local)
-{
-	commit_event_mixed(R, m_dm, L, hist, local);
-}
 
 // abort_if_uncaptured_bound (src/Simulation_Trajectory.cpp:767-778, 1108) in Capture mode, where the commit
 // forms no energy: the FP64 energy of the event decides unless the FP32 speeds are far apart.
@@ -439,7 +435,8 @@ static __device__ __noinline__ int boundary_step(const RunParams& R, double m_dm
 	L.hot().seg_steps++;
 	L.hot().steps++;
 	L.hot().retries = 0;
-	commit_event_general(R, m_dm, L, hist, ev);
+	// (in place: its radius is contracted as r_b is, so that both lie on the same side of the outermost bin's edge)
+	commit_event_mixed(R, m_dm, L, hist, ev);
 	// reset_propagator_at_absolute_event, src/Simulation_Trajectory.cpp:814-822
 	L.cur = inbound;
 	L.cur.t += L.hot().origin;

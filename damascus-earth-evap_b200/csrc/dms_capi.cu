@@ -280,7 +280,8 @@ void Poll_Pause(std::chrono::steady_clock::duration elapsed)
 // scheduler of its own and a pass is bound by its dependent chain (the latency form of the kernel);
 // beyond that, 512 (640 in a large mixed launch) run their warps in lockstep (the throughput form, dms_lane.cuh).
 // Measured, Capture mode m = 1 GeV, sigma = 1e-35 cm^2, FP64, 128 against 512 threads: 1 024 trajectories
-// 2.1 / 2.3 ms, 4 096 2.9 / 3.2 ms, 16 384 4.2 / 4.1 ms, 65 536 10.6 / 6.3 ms.  threads_per_block and
+// 2.1 / 2.3 ms, 4 096 2.9 / 3.2 ms, 16 384 4.2 / 4.1 ms, 65 536 10.6 / 6.3 ms (when the line was drawn; 16 384 and
+// 65 536 now take 2.9 and 5.0 ms).  threads_per_block and
 // blocks_per_sm ask for the lanes per SM: blocks of one SM run as one block.
 int Block_Threads(const dms_run_opts* o, uint64_t total, int sm_count)
 {

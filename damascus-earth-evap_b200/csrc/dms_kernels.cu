@@ -1,6 +1,7 @@
 // Kernels of the trajectory engine.
 //
-// trajectory_kernel: one persistent launch per dms_run.  Every thread is a lane that owns one
+// trajectory_kernel, trajectory_kernel_latency: a persistent launch per dms_run, and for a large one a second
+// that finishes its last trajectories.  Every thread is a lane that owns one
 // trajectory at a time; lanes claim work indices from a global queue (one warp-aggregated
 // atomic per claim), and refill as soon as their trajectory terminates, so trajectories of
 // wildly different length (0 to 10^6 scatterings) never hold a whole batch back.  A lane's
@@ -218,7 +219,10 @@ __device__ __forceinline__ bool interior_interval_outside_here(const Event& a, c
 {
 	return interior_interval(a, b, ra, rb, s0, s1);
 }
-static __device__ __noinline__ bool interior_interval_outside_called(const Event& a, const Event& b, double ra, double rb, double& s0, double& s1) { return interior_interval_outside_here(a, b, ra, rb, s0, s1); }
+static __device__ __noinline__ bool interior_interval_outside_called(const Event& a, const Event& b, double ra, double rb, double& s0, double& s1)
+{
+	return interior_interval_outside_here(a, b, ra, rb, s0, s1);
+}
 template <bool CALL>
 __device__ __forceinline__ bool interior_interval_outside(const Event& a, const Event& b, double ra, double rb, double& s0, double& s1)
 {
@@ -423,9 +427,14 @@ __device__ __forceinline__ int depth_reject_here(StrictLane& L, const Event& bef
 	L.hot().pr.time_step = sanitized_step(factor * dt);
 	return PH_STEP;  // L.hot().before and the speed and rate at it still describe the propagator
 }
-static __device__ __noinline__ int depth_reject_called(StrictLane& L, const Event& before, double dtau, double apart, double scale, bool capture_mode, double dt, double tau_limit) { return depth_reject_here(L, before, dtau, apart, scale, capture_mode, dt, tau_limit); }
+static __device__ __noinline__ int depth_reject_called(StrictLane& L, const Event& before, double dtau, double apart, double scale,
+                                                       bool capture_mode, double dt, double tau_limit)
+{
+	return depth_reject_here(L, before, dtau, apart, scale, capture_mode, dt, tau_limit);
+}
 template <bool CALL>
-__device__ __forceinline__ int depth_reject(StrictLane& L, const Event& before, double dtau, double apart, double scale, bool capture_mode, double dt, double tau_limit)
+__device__ __forceinline__ int depth_reject(StrictLane& L, const Event& before, double dtau, double apart, double scale, bool capture_mode,
+                                            double dt, double tau_limit)
 {
 	if constexpr(CALL)
 		return depth_reject_called(L, before, dtau, apart, scale, capture_mode, dt, tau_limit);
@@ -467,9 +476,14 @@ __device__ __forceinline__ void scatter_point_here(const DevSolar& S, const DevP
 	}
 	accepted = interpolate_event(*c.before, c.after, c.s1);
 }
-static __device__ __noinline__ void scatter_point_called(const DevSolar& S, const DevPoint* __restrict__ P, const StepCtx& c, double rate_before, bool first_known, bool depth, int pieces, double remaining, Event& accepted) { scatter_point_here(S, P, c, rate_before, first_known, depth, pieces, remaining, accepted); }
+static __device__ __noinline__ void scatter_point_called(const DevSolar& S, const DevPoint* __restrict__ P, const StepCtx& c, double rate_before,
+                                                         bool first_known, bool depth, int pieces, double remaining, Event& accepted)
+{
+	scatter_point_here(S, P, c, rate_before, first_known, depth, pieces, remaining, accepted);
+}
 template <bool CALL>
-__device__ __forceinline__ void scatter_point(const DevSolar& S, const DevPoint* __restrict__ P, const StepCtx& c, double rate_before, bool first_known, bool depth, int pieces, double remaining, Event& accepted)
+__device__ __forceinline__ void scatter_point(const DevSolar& S, const DevPoint* __restrict__ P, const StepCtx& c, double rate_before,
+                                              bool first_known, bool depth, int pieces, double remaining, Event& accepted)
 {
 	if constexpr(CALL)
 		scatter_point_called(S, P, c, rate_before, first_known, depth, pieces, remaining, accepted);
@@ -1190,8 +1204,8 @@ __device__ __forceinline__ double random_double(uint64_t bits, int lo, int hi)
 }
 
 // Self-test of the certified division and square root against IEEE `/` and sqrt on n random
-// operand pairs: out[0] quotients whose certificate held but whose bits differ from IEEE (must
-// be 0), out[1] quotients whose certificate failed, out[2] and out[3] the same for the root.
+// operand pairs: out[0] quotients inside the straight-line range whose bits differ from IEEE (must
+// be 0), out[1] pairs outside that range, out[2] and out[3] the same for the root.
 // Operands: random exponents in the ranges of the trajectory arithmetic, arbitrary bit patterns
 // (NaN, infinities, subnormals, zeros), quotients within a few ulp of representable values,
 // and exact quotients (a power-of-two divisor).  Division and square root never land exactly

@@ -11,10 +11,9 @@ namespace dms
 // The largest block of the trajectory kernels: all 16 warps that their registers allow per SM.
 constexpr int MAX_THREADS = 512;
 // The mixed form keeps less per lane: a launch with at least two trajectories for each lane of 20 warps runs
-// that many, with 96 registers each.  2^20 Capture-mode trajectories with 512 / 640 / 768 / 1 024 threads take 27.0 /
-// 25.3 / 25.9 / 27.3 ms; with 512 / 640
-// 2^19 14.6 / 14.2, 2^18 8.5 / 8.3, 200 000 6.9 / 7.0, 2^17 5.3 / 5.5, 2^16 3.7 / 4.0; the FP64 form takes 40.9 / 41.4 / 44.6 / 48.6 ms
-// for the first (448 / 384: 42.7 / 44.3).
+// that many, with 96 registers each.  2^20 Capture-mode trajectories with 512 / 640 / 768 / 1 024 threads took
+// 27.0 / 25.3 / 25.9 / 27.3 ms; with 512 / 640 2^19 took 14.6 / 14.2, 2^18 8.5 / 8.3, 200 000 6.9 / 7.0, 2^17
+// 5.3 / 5.5, 2^16 3.7 / 4.0.  The FP64 form took 40.9 / 41.4 / 44.6 / 48.6 ms for the first (448 / 384: 42.7 / 44.3).
 constexpr int MAX_THREADS_MIXED = 640;
 // Blocks of at most this many threads run the latency form of the kernels: one warp per scheduler, so
 // the registers are not shared out among 16 warps.

@@ -22,7 +22,7 @@ namespace lane
 // makes that step by itself.  Every value is formed by the functions of the one-lane pass from the same
 // arguments, so the results are the same bits.  The barriers count whole warps that all run the same loop;
 // the only wait by polling is that of a warp without work for a team to form, and it is bounded.
-// A lone lane's step takes 5.7 -> 3.3 us in FP64 and 4.4 -> 3.1 us in the mixed form; 16 384 Parameter-point
+// A lone lane's step takes 5.7 -> 3.3 us in FP64 and 4.4 -> 3.0 us in the mixed form; 16 384 Parameter-point
 // trajectories of m = 0.3 GeV, 1e-36 cm^2 426 -> 259 ms in the mixed form, 128 25 -> 18 ms.
 struct TeamState  // the propagator at the start of a step
 {

@@ -45,11 +45,11 @@ WORKLOAD = ("Parameter-point evaporation (config 1): SI contact m=0.3 GeV sigma_
 # (64-channel rate sum, free-gas target velocity, kinematics) and per trajectory (initial
 # conditions, Kepler shift, classification).
 FLOP_PER_ATTEMPT, FLOP_PER_STEP, FLOP_PER_SCATTER, FLOP_PER_TRAJ = 214.8, 622.3, 2455.0, 3374.0
-# DRAM bytes (read + write) of the FP64 trajectory kernel per trajectory of this point, from one
-# ncu capture of one 65 536-trajectory batch (ids 0-65 535: 2.671 GB read + 6.777 GB written, 635
-# bytes per accepted step): the lane state's local-memory traffic and the termination flush of
-# the per-lane histogram rows.
-TRAFFIC_PER_TRAJECTORY = (2.671374e9 + 6.777167e9) / 65536
+# DRAM bytes (read + write) of the FP64 trajectory kernels per trajectory of this point, from one
+# ncu capture of one 65 536-trajectory batch (ids 0-65 535: 2.399 GB read + 2.180 GB written by its
+# two launches, 308 bytes per accepted step): local memory, and the reads, writes and termination
+# flush of the per-lane histogram rows.
+TRAFFIC_PER_TRAJECTORY = (2.399485e9 + 2.179577e9) / 65536
 
 
 def hbm_peak_gbs():
@@ -348,7 +348,7 @@ def run_engine_arm(args):
             o = dms_b200.run_opts(seed=SEED, capture_mode=False, max_scatterings=MAX_SCAT, time_limit_s=seconds,
                                   precision=prec)
             try:
-                engine.run([(solo, 1 << 40, 1 << 23)], o)
+                engine.run([(solo, 1 << 40, 1 << 25)], o)
             except dms_b200.EngineError as e:
                 if "cancelled" not in str(e):
                     raise
@@ -413,7 +413,7 @@ def run_engine_arm(args):
                     "d2h_bytes_per_step": int(d2h_bytes / max(K, 1)),
                     "seconds": spread([r[0] for r in e2e_runs]),
                     "work": "the timed launch's trajectory ids, recomputed, host wall clock"},
-            "gpu_launches": 2,
+            "gpu_launches": 3,
             "roofline": {"bound": "fp64", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                          "frac": achieved / peak if peak > 0 else None,
                          "frac_of": "measured DFMA peak of this run (MEASURED_PEAKS.json holds no FP64 figure)",
@@ -450,7 +450,7 @@ def run_engine_arm(args):
                                                       "mean_scatterings_rel_error")},
                 "reference_gates": {k: {"pass": bool(ok), "value": v} for k, (ok, v) in gates.items()},
                 "clocks": mix_clocks,
-                "gpu_launches": 2,
+                "gpu_launches": 3,
             }
         if tuning:
             line["autotune"] = dict(tuning, note="0 = the library default; trials of %.2f s over fresh ids, scored by "

@@ -6,6 +6,7 @@
 #include <type_traits>
 
 #include "dms_kernels.cuh"
+#include "dms_lane_rules.h"
 
 namespace dms
 {
@@ -729,12 +730,13 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 	__shared__ double coop_rates[Step::threads / 32][BUFFER];
 	double* rates = coop_rates[threadIdx.x >> 5];
 	// Lockstep: the warps of a block make every pass together, so that an instruction fetched once serves
-	// all of them (until few lanes are left: R.lockstep_min).  The block votes on its rare phases:
-	// lanes stepping, at a scattering point and at a termination, counted per pass (two sets, one
-	// being cleared while the other is filled).
-	__shared__ int votes[2][4];
-	if(threadIdx.x < 8)
+	// all of them (until few lanes are left: R.lockstep_min).  The block votes on its rare phases: lanes
+	// stepping, at a scattering point and at a termination, counted per pass in the sets of
+	// dms_lane_rules.h in turn.
+	__shared__ int votes[VOTE_SETS][4];
+	if(threadIdx.x < VOTE_SETS * 4)
 		votes[threadIdx.x >> 2][threadIdx.x & 3] = 0;
+	int vote_set = 0;
 	bool lockstep = Step::lockstep;
 	bool team = false;  // this warp's lone lane has formed a team
 	uint64_t next_check = 1023;
@@ -797,7 +799,10 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 		bool alone = !team;  // the lanes make this pass's steps themselves
 		if(Step::lockstep && lockstep)
 		{
-			int* v = votes[iter & 1];
+			int* v = votes[vote_set];
+			vote_set = next_vote_set(vote_set);
+			if(threadIdx.x < 3)
+				votes[vote_set][threadIdx.x] = 0;
 			const unsigned int b_step = __ballot_sync(FULL_WARP, phase == PH_STEP || phase == PH_FETCH || phase == PH_SEGMENT);
 			const unsigned int b_scatter = __ballot_sync(FULL_WARP, phase == PH_SCATTER);
 			const unsigned int b_final = __ballot_sync(FULL_WARP, phase == PH_FINAL);
@@ -816,8 +821,6 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 			}
 			__syncthreads();
 			const int n_step = v[0], n_scatter = v[1], n_final = v[2], flags = v[3];
-			if(threadIdx.x < 3)
-				votes[(iter & 1) ^ 1][threadIdx.x] = 0;
 			drained |= (flags & 1) != 0;
 			// batches and waits are for a full block; in the tail of a throughput launch they shrink with the
 			// lanes at work

@@ -1061,13 +1061,6 @@ __device__ __forceinline__ double capped_step(double r, double speed, double ste
 	return step < cap ? step : cap;
 }
 
-// Whether the time to the surface (src/Simulation_Trajectory.cpp:886-899) of a particle outside it cannot be
-// below `step`, by a margin far above its rounding.  along = x . v.
-__device__ __forceinline__ bool surface_is_far(double r, double along, double step)
-{
-	return (along >= 0.0) | ((r - DMS_RSUN_KM) * r * (1.0 - 1.0e-9) > -along * step);
-}
-
 __device__ __forceinline__ double ev_radius(const Event& e) { return norm3(e.x); }
 __device__ __forceinline__ double ev_speed(const Event& e) { return norm3(e.v); }
 

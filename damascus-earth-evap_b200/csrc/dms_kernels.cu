@@ -808,9 +808,8 @@ __device__ __forceinline__ void strict_propagate(const RunParams& R, const Stric
 	bool ok = true;
 	if(r >= DMS_RSUN_KM)
 	{
-		const double along = r * s.v_radial;
 		step = capped_step(r, s.speed, step, R.boundary);
-		if(!(((along > 1.0e-6 * r) | (along < -1.0e-6 * r)) && surface_is_far(r, along, step)))
+		if(!surface_is_far_by_speed(r, s.v_radial, s.speed, step))
 		{
 			Event before;
 			double speed;

@@ -1,6 +1,9 @@
 // Rules of the lane loop that need nothing of the device, so that they can be tested on the CPU.
 #pragma once
 
+#include <cmath>
+
+#include "dms_constants.h"
 #include "dms_philox.h"
 
 namespace dms
@@ -15,6 +18,21 @@ namespace lane
 // warp with an almost empty pass may already be adding.
 constexpr int VOTE_SETS = 3;
 DMS_HD int next_vote_set(int set) { return set + 1 == VOTE_SETS ? 0 : set + 1; }
+
+// Whether the time to the surface (src/Simulation_Trajectory.cpp:886-899) of a particle outside it cannot be
+// below `step`, by a margin far above its rounding.  along = x . v.
+DMS_HD bool surface_is_far(double r, double along, double step)
+{
+	return (along >= 0.0) | ((r - DMS_RSUN_KM) * r * (1.0 - 1.0e-9) > -along * step);
+}
+
+// The same from the propagator's radial speed, for a state whose event has not been formed.  The event's
+// x . v is off r v_radial by some 1e-15 r speed, since its components and axes are rounded: far below
+// the margin only above 1e-4 of the speed.  False below that, where the event decides.
+DMS_HD bool surface_is_far_by_speed(double r, double v_radial, double speed, double step)
+{
+	return (fabs(v_radial) > 1.0e-4 * speed) & surface_is_far(r, r * v_radial, step);
+}
 
 }	// namespace lane
 }	// namespace dms

@@ -8,10 +8,59 @@ import pytest
 from dms_ctypes import PACKAGE_DIR, REPO
 
 SHIM = r"""
+#include <cstdint>
 #include "dms_lane_rules.h"
+#include "dms_math.h"
 extern "C" {
 int vote_sets() { return dms::lane::VOTE_SETS; }
 int next_vote_set(int set) { return dms::lane::next_vote_set(set); }
+}
+
+struct V { double x, y, z; };
+static double dot(const V& a, const V& b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+static V cross(const V& a, const V& b) { return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x}; }
+static V unit(const V& a) { const double n = sqrt(dot(a, a)); return {a.x / n, a.y / n, a.z / n}; }
+static uint64_t seed_;
+static double uniform(double a, double b)
+{
+	uint64_t x = seed_ += 0x9e3779b97f4a7c15ULL;
+	x = (x ^ (x >> 30)) * 0xbf58476d1ce4e5b9ULL;
+	x = (x ^ (x >> 27)) * 0x94d049bb133111ebULL;
+	return a + (b - a) * (static_cast<double>((x ^ (x >> 31)) >> 11) * 0x1p-53);
+}
+
+// States outside the surface, down to grazing ones, with steps about the time to the surface: how many of those that
+// the radial speed calls far does the event's time to the surface bind all the same (*wrong)?  Returns how many it calls far.
+extern "C" int far_from_surface(int n, uint64_t seed, int* wrong)
+{
+	seed_ = seed;
+	int far = 0;
+	*wrong = 0;
+	for(int i = 0; i < n; i++)
+	{
+		// axes as prop_init makes them
+		V ax = unit({uniform(-1, 1), uniform(-1, 1), uniform(-1, 1)});
+		const V az = unit(cross(ax, {uniform(-1, 1), uniform(-1, 1), uniform(-1, 1)}));
+		const V ay = unit(cross(az, ax));
+		ax = unit(cross(ay, az));
+		const double r = DMS_RSUN_KM * (1.0 + pow(10.0, uniform(-9, 0))), J = r * uniform(10.0, 2000.0), v_radial = -pow(10.0, uniform(-8, 3));
+		double sp, cp;
+		dms_sincos(uniform(0.0, 100.0), &sp, &cp);
+		const double vt = J / r, vx = v_radial * cp - vt * sp, vy = v_radial * sp + vt * cp;
+		const V x = {r * (cp * ax.x + sp * ay.x), r * (cp * ax.y + sp * ay.y), r * (cp * ax.z + sp * ay.z)};
+		const V v = {vx * ax.x + vy * ay.x, vx * ax.y + vy * ay.y, vx * ax.z + vy * ay.z};
+		const double speed = sqrt(v_radial * v_radial + J * J / r / r), along = dot(x, v);
+		if(!(along < 0.0))
+			continue;
+		const double time = (r - DMS_RSUN_KM) / (-(along / r)), by_speed = (r - DMS_RSUN_KM) / -v_radial;
+		const double step = i & 1 ? time + uniform(0.0, 1.0) * (by_speed - time) : time * (1.0 + pow(10.0, uniform(-16, -6)) * uniform(-1, 1));
+		if(dms::lane::surface_is_far_by_speed(r, v_radial, speed, step))
+		{
+			far++;
+			*wrong += time < step;
+		}
+	}
+	return far;
 }
 """
 
@@ -77,3 +126,12 @@ def test_two_vote_sets_are_too_few():
         return 1 - s
     assert wrong_count_possible(2, 3, 2, other, clear_after_barrier=True)
     assert wrong_count_possible(2, 3, 2, other, clear_after_barrier=False)
+
+
+def test_radial_speed_calls_no_step_far_that_the_surface_binds(rules):
+    """A team bounds a step outside the Sun without the event where it may; the step has to be that of a lone lane."""
+    wrong = ctypes.c_int()
+    rules.far_from_surface.argtypes = [ctypes.c_int, ctypes.c_uint64, ctypes.POINTER(ctypes.c_int)]
+    far = rules.far_from_surface(2_000_000, 1, ctypes.byref(wrong))
+    assert far > 10_000  # the states reach the rule
+    assert wrong.value == 0

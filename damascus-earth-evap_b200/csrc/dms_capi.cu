@@ -150,6 +150,7 @@ int Grow_Points(dms_ctx* ctx, int needed)
 			                         sizeof(dms_reflection) * ctx->event_capacity, cudaMemcpyDeviceToDevice));
 		DMS_CUDA(ctx, cudaMemcpy(nrc, ctx->d_refl_count, sizeof(unsigned long long) * old, cudaMemcpyDeviceToDevice));
 	}
+	DMS_CUDA(ctx, cudaStreamSynchronize(cudaStreamLegacy));  // ahead of what runs on the context's stream
 	cudaFree(ctx->d_points);
 	cudaFree(ctx->d_counters);
 	cudaFree(ctx->d_hists);
@@ -762,14 +763,23 @@ int dms_add_point(dms_ctx* ctx, const dms_point_params* params, int* point_id)
 	DevPoint d;
 	Fill_Dev_Point(c, grid, d);
 	d.grid_f = grid_f;
-	const cudaError_t e1 = cudaMemcpy(ctx->d_points + id, &d, sizeof d, cudaMemcpyHostToDevice);
+	// on the context's stream, ahead of the launches that read and add to them
+	cudaError_t e1 = cudaMemcpyAsync(ctx->d_points + id, &d, sizeof d, cudaMemcpyHostToDevice, ctx->stream);
+	const auto clear = [&](void* p, size_t bytes) {
+		if(e1 == cudaSuccess)
+			e1 = cudaMemsetAsync(p, 0, bytes, ctx->stream);
+	};
+	clear(ctx->d_counters + static_cast<size_t>(id) * DMS_NUM_COUNTERS, sizeof(unsigned long long) * DMS_NUM_COUNTERS);
+	clear(ctx->d_hists + static_cast<size_t>(id) * DMS_NUM_HISTS * DMS_NUM_BINS, sizeof(double) * DMS_NUM_HISTS * DMS_NUM_BINS);
+	clear(ctx->d_event_count + id, sizeof(unsigned long long));
+	clear(ctx->d_refl_count + id, sizeof(unsigned long long));
 	if(e1 != cudaSuccess)
 	{
+		cudaStreamSynchronize(ctx->stream);
 		cudaFree(grid);
 		cudaFree(grid_f);
 		return Fail(ctx, DMS_ERR_CUDA, cudaGetErrorString(e1));
 	}
-	cudaStreamSynchronize(cudaStreamLegacy);  // the copies above, ahead of what runs on the context's stream
 	if(c.grid_n > 0)
 		Launch_Rate_Grid(ctx->dsolar, ctx->d_points + id, grid, c.grid_n, ctx->stream);
 	const cudaError_t e2 = cudaStreamSynchronize(ctx->stream);
@@ -783,10 +793,6 @@ int dms_add_point(dms_ctx* ctx, const dms_point_params* params, int* point_id)
 	ctx->d_grids.push_back(grid);
 	ctx->d_grids_f.push_back(grid_f);
 	ctx->grid_f_valid.push_back(c.grid_n > 0 ? 0 : 1);
-	DMS_CUDA(ctx, cudaMemset(ctx->d_counters + static_cast<size_t>(id) * DMS_NUM_COUNTERS, 0, sizeof(unsigned long long) * DMS_NUM_COUNTERS));
-	DMS_CUDA(ctx, cudaMemset(ctx->d_hists + static_cast<size_t>(id) * DMS_NUM_HISTS * DMS_NUM_BINS, 0, sizeof(double) * DMS_NUM_HISTS * DMS_NUM_BINS));
-	DMS_CUDA(ctx, cudaMemset(ctx->d_event_count + id, 0, sizeof(unsigned long long)));
-	DMS_CUDA(ctx, cudaMemset(ctx->d_refl_count + id, 0, sizeof(unsigned long long)));
 	if(point_id)
 		*point_id = id;
 	return DMS_OK;
@@ -836,9 +842,9 @@ int dms_rate(dms_ctx* ctx, int point_id, int interpolated, const double* r_km, c
 		return DMS_OK;
 	double* d = nullptr;
 	DMS_CUDA(ctx, cudaMalloc(&d, sizeof(double) * 3 * n));
-	cudaError_t e = cudaMemcpy(d, r_km, sizeof(double) * n, cudaMemcpyHostToDevice);
+	cudaError_t e = cudaMemcpyAsync(d, r_km, sizeof(double) * n, cudaMemcpyHostToDevice, ctx->stream);
 	if(e == cudaSuccess)
-		e = cudaMemcpy(d + n, v_kms, sizeof(double) * n, cudaMemcpyHostToDevice);
+		e = cudaMemcpyAsync(d + n, v_kms, sizeof(double) * n, cudaMemcpyHostToDevice, ctx->stream);
 	if(e == cudaSuccess)
 	{
 		Launch_Rate_Query(ctx->dsolar, ctx->d_points + point_id, interpolated, d, d + n, d + 2 * n, n, ctx->stream);
@@ -961,7 +967,7 @@ double Tune_Trial(dms_ctx* ctx, const dms_run_opts& o, const std::vector<int32_t
 	std::memcpy(buf.data(), firsts.data(), sizeof(uint64_t) * n);
 	std::memcpy(buf.data() + off_offset, offsets.data(), sizeof(uint64_t) * (n + 1));
 	std::memcpy(buf.data() + off_point, pts.data(), sizeof(int32_t) * n);
-	if(cudaMemcpy(d_ranges, buf.data(), buf.size(), cudaMemcpyHostToDevice) != cudaSuccess)
+	if(cudaMemcpyAsync(d_ranges, buf.data(), buf.size(), cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess)
 		return -1.0;
 	RunParams p{};
 	p.range_first = reinterpret_cast<const uint64_t*>(dc);

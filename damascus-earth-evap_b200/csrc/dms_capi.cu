@@ -322,6 +322,7 @@ int Launch_And_Wait(dms_ctx* ctx, const dms_run_opts* o, RunParams& p)
 	{
 		if(ctx->d_parked == nullptr)
 			DMS_CUDA(ctx, cudaMalloc(reinterpret_cast<void**>(&ctx->d_parked), 256 + PARKED_BYTES * PARKED_PER_BLOCK * ctx->sm_count));
+		p.parked_capacity = static_cast<unsigned int>(PARKED_PER_BLOCK * ctx->sm_count);
 		p.parked_count = reinterpret_cast<unsigned int*>(ctx->d_parked);
 		p.parked = ctx->d_parked + 256;
 		DMS_CUDA(ctx, cudaMemsetAsync(p.parked_count, 0, sizeof(unsigned int), ctx->stream));
@@ -436,6 +437,8 @@ int Launch_And_Wait(dms_ctx* ctx, const dms_run_opts* o, RunParams& p)
 	ctx->last_kernel_ms = kernel_ms;
 	unsigned int status = 0;
 	DMS_CUDA(ctx, cudaMemcpy(&status, ctx->d_status, sizeof status, cudaMemcpyDeviceToHost));
+	if(status & STATUS_PARKED_FULL)
+		return Fail(ctx, DMS_ERR_STATE, "trajectories between the two launches of the run exceeded their buffer");
 	if(status & STATUS_CANCELLED)
 		return Fail(ctx, DMS_ERR_CANCELLED, cancelled_by_limit ? "run cancelled: wall-clock limit reached"
 		                                    : cancelled_by_hook ? "run cancelled by the progress callback" : "run cancelled");

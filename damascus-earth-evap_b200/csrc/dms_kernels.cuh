@@ -28,6 +28,7 @@ enum : unsigned int
 	STATUS_BUDGET = 2u,
 	STATUS_IC_REJECTION = 4u,
 	STATUS_BAD_RANGE = 8u,
+	STATUS_PARKED_FULL = 16u,  // more parked states than RunParams::parked_capacity
 };
 
 // Initial state of one work item, computed for the whole launch before the persistent kernel
@@ -81,6 +82,7 @@ struct RunParams
 	// The tail of a throughput launch: a block with at most lockstep_min lanes at work and no more work parks
 	// their states (PARKED_BYTES each) and ends; a latency launch behind it resumes them.
 	unsigned char* parked;
+	unsigned int parked_capacity;
 	unsigned int* parked_count;
 	int resume;          // 1: the lanes take the parked states instead of work indices
 	int ic_max_attempts;

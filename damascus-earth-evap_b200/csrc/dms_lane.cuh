@@ -763,7 +763,7 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 			// the parked trajectories dealt out to the blocks one by one, and to the warps within
 			const unsigned int item = static_cast<unsigned int>(slot) * gridDim.x + blockIdx.x;
 			phase = PH_DONE;
-			if(item < *R.parked_count)
+			if(item < *R.parked_count && item < R.parked_capacity)
 			{
 				const Parked<Lane>& s = *reinterpret_cast<const Parked<Lane>*>(R.parked + item * PARKED_BYTES);
 				L = s.L;
@@ -853,18 +853,28 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 			{
 				if constexpr(Step::throughput)
 				{
+					// (at most lockstep_min lanes of a block come here, and the slots are for as many of every
+					// block; a lane without one would end the run with an error)
+					bool room = true;
 					if(phase != PH_DONE && !(phase == PH_FETCH && q_next >= q_end))
 					{
-						Parked<Lane>& s = *reinterpret_cast<Parked<Lane>*>(R.parked + atomicAdd(R.parked_count, 1u) * PARKED_BYTES);
-						s.L = L;
-						s.hot = L.hot();
-						s.hist = hist;
-						s.q_next = q_next;
-						s.q_end = q_end;
-						s.phase = phase;
-						s.iter = iter;
+						const unsigned int at = atomicAdd(R.parked_count, 1u);
+						room = at < R.parked_capacity;
+						if(room)
+						{
+							Parked<Lane>& s = *reinterpret_cast<Parked<Lane>*>(R.parked + at * PARKED_BYTES);
+							s.L = L;
+							s.hot = L.hot();
+							s.hist = hist;
+							s.q_next = q_next;
+							s.q_end = q_end;
+							s.phase = phase;
+							s.iter = iter;
+						}
+						else
+							atomicOr(R.status, STATUS_PARKED_FULL);
 					}
-					phase = PH_DONE;
+					phase = room ? PH_DONE : phase;
 					break;
 				}
 				lockstep = false;

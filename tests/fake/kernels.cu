@@ -20,6 +20,7 @@ struct FakeLaunch
 	uint64_t total, done, parked_room;
 	int32_t blocks, threads, mixed, resume, lanes_per_block, lockstep_min;
 	uint32_t queue_chunk;
+	uint32_t parked_capacity;
 	int32_t options[4];  // scatter_batch, scatter_wait, final_batch, final_wait
 };
 double fake_rate = 1e9;
@@ -65,6 +66,7 @@ void launch(const RunParams& p, int blocks, int threads, cudaStream_t s, int mix
 	l.total = p.total;
 	l.done = ~0ULL;
 	l.parked_room = p.parked ? fake_room(p.parked) : 0;
+	l.parked_capacity = p.parked_capacity;
 	l.blocks = blocks;
 	l.threads = threads;
 	l.mixed = mixed;

@@ -20,7 +20,7 @@ import dms_b200
 class Launch(ctypes.Structure):
     _fields_ = [("total", ctypes.c_uint64), ("done", ctypes.c_uint64), ("parked_room", ctypes.c_uint64)] + [
         (n, ctypes.c_int32) for n in ("blocks", "threads", "mixed", "resume", "lanes_per_block", "lockstep_min")] + [
-        ("queue_chunk", ctypes.c_uint32), ("options", ctypes.c_int32 * 4)]
+        ("queue_chunk", ctypes.c_uint32), ("parked_capacity", ctypes.c_uint32), ("options", ctypes.c_int32 * 4)]
 lib = dms_b200.library()
 def launches():
     a = (Launch * 4096)()
@@ -88,5 +88,26 @@ buffer = (ctypes.c_char * (ctypes.sizeof(dms_b200.TrajRecord) * 4))()
 pid = point(e)
 e.run_records_noalloc(pid, 0, 4, small, ctypes.addressof(buffer))
 ordered("no-alloc records after add_point")
+e.close()
+""")
+
+
+def test_parked_states_have_room(host):
+    """A large launch hands at most lockstep_min lanes of each block to the launch behind it."""
+    host(r"""
+e = dms_b200.Engine(0)
+pid = point(e)
+for precision in (dms_b200.PRECISION_FP64, dms_b200.PRECISION_MIXED):
+    for count in (128 * 148 + 1, 512 * 148, 2 * 640 * 148):
+        e.run([(pid, 0, count)], dms_b200.run_opts(seed=1, precision=precision))
+        first, second = launches()
+        assert (first.resume, second.resume) == (0, 1) and second.threads == 128
+        for l in (first, second):
+            assert l.parked_capacity * 1024 <= l.parked_room
+            assert l.parked_capacity >= first.blocks * first.lockstep_min
+        assert second.blocks * second.threads >= second.parked_capacity
+e.run([(pid, 0, 128 * 148)], dms_b200.run_opts(seed=1))
+only, = launches()
+assert only.threads == 128 and not only.resume
 e.close()
 """)

@@ -1,16 +1,16 @@
 // FP64 division and square root as straight-line code, equal to IEEE `/` and sqrt() bit for bit.
 //
-// Why: an IEEE double division or square root compiles to a sequence with a slow-path branch, about
-// 24 (32) instructions at every place it is used.  An RK45 attempt holds forty-odd of them, and the
-// trajectory kernel is bound by instruction supply: its step has to fit the SM's 32 KB instruction
-// cache.  The quotients of one stage share a divisor, so one correctly rounded reciprocal (6
-// instructions) serves all of them at 5 instructions each, without a branch, and the compiler can
-// interleave independent stages.
+// Why: an RK45 attempt holds forty-odd divisions, and the trajectory kernel is bound by instruction
+// supply: its step has to fit the SM's 32 KB instruction cache.  `/` has to allow for every operand at every
+// place it is used.  Here the quotients of one stage share a divisor, so one correctly rounded reciprocal (10
+// operations) serves all of them at 4 operations each, without a branch, and the compiler can interleave
+// independent stages.
 //
 // Method (published, restated here from the mathematics):
-//  * reciprocal: the hardware approximation (PTX rcp.approx.ftz.f64) refined by a third-order and a
-//    second-order Newton-Raphson step written with fused multiply-add.  After the first the value
-//    is within one ulp of 1/b; the second then returns RN(1/b) unless the significand of b is all
+//  * reciprocal: Newton's iteration for 1/y - b = 0, y <- y + y (1 - b y), which squares the relative error,
+//    written with fused multiply-add and started from the hardware approximation (PTX
+//    rcp.approx.ftz.f64, error at most 2^-23 by its documentation): 2^-46 after one step, and after two within
+//    one ulp of 1/b.  The third step then returns RN(1/b) unless the significand of b is all
 //    ones (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000
 //    processor", IBM J. Res. Dev. 34, 1990; J.-M. Muller et al., "Handbook of Floating-Point
 //    Arithmetic", 2010, sec. 4.7).
@@ -59,11 +59,9 @@ __device__ __forceinline__ Recip recip(double b, bool& ok)
 	Recip r;
 	r.b = b;
 	double y = rcp_approx(b);
-	double e = __fma_rn(-b, y, 1.0);
-	e = __fma_rn(e, e, e);
-	y = __fma_rn(y, e, y);
-	e = __fma_rn(-b, y, 1.0);
-	r.y = __fma_rn(y, e, y);
+	y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);
+	y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);
+	r.y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);
 	r.l = __dmul_rn(__fma_rn(-b, r.y, 1.0), r.y);
 	ok &= __double2loint(b) != -1;
 	return r;

@@ -15,9 +15,8 @@
 //    processor", IBM J. Res. Dev. 34, 1990; J.-M. Muller et al., "Handbook of Floating-Point
 //    Arithmetic", 2010, sec. 4.7).
 //  * quotient: with y = RN(1/b) and its residual l = (1 - b y) y, q0 = RN(a y + RN(a l)) is within one ulp of
-//    a / b, and Markstein's theorem then gives q = RN(q0 + (a - b q0) y) = RN(a / b).  Neither operand,
-//    quotient nor remainder may leave the normal range; the callers keep 1 <= b < 2^100 and a = 0 or
-//    2^-700 <= |a| <= 2^400.  A zero dividend gives +0.
+//    a / b, and Markstein's theorem then gives q = RN(q0 + (a - b q0) y) = RN(a / b).  No operand,
+//    quotient or remainder may leave the normal range: see in_division_range.  A zero dividend gives +0.
 //  * square root: Goldschmidt iterations from rsqrt.approx.ftz.f64 and Markstein's correction step
 //    s = RN(g + (x - g^2) h), with a certificate instead of a theorem: the rounding error of that
 //    last sum, which is exactly representable, must stay below half the spacing of the doubles
@@ -67,7 +66,17 @@ __device__ __forceinline__ Recip recip(double b, bool& ok)
 	return r;
 }
 
-// RN(a / b) for operands in the range above.
+// Whether (a, b) lie in the range of div: 2^-200 < |b| < 2^400, a = 0 or 2^-700 <= |a| <= 2^400, and a quotient of at
+// least 2^-900, so that the remainder a - b q and its products stay normal.  The callers divide by radii and
+// speeds in [1, 2^100), by norms in (2^-100, 2^100), by rates in (2^-200, 2^100) and by errors of an RK45
+// attempt in [1e-14, 2^400).
+__device__ __forceinline__ bool in_division_range(double a, double b)
+{
+	const double aa = fabs(a), ab = fabs(b);
+	return (ab > 0x1p-200) & (ab < 0x1p400) & ((a == 0.0) | ((aa >= 0x1p-700) & (aa <= 0x1p400) & (aa >= 0x1p-900 * ab)));
+}
+
+// RN(a / b) for operands in that range.
 __device__ __forceinline__ double div(double a, const Recip& d)
 {
 	const double q = __fma_rn(a, d.y, __dmul_rn(a, d.l));

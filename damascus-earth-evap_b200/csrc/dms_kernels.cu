@@ -1206,8 +1206,8 @@ __device__ __forceinline__ double random_double(uint64_t bits, int lo, int hi)
 // operand pairs: out[0] quotients inside the straight-line range whose bits differ from IEEE (must
 // be 0), out[1] pairs outside that range, out[2] and out[3] the same for the root.
 // Operands: random exponents in the ranges of the trajectory arithmetic, arbitrary bit patterns
-// (NaN, infinities, subnormals, zeros), quotients within a few ulp of representable values,
-// and exact quotients (a power-of-two divisor).  Division and square root never land exactly
+// (NaN, infinities, subnormals, zeros), quotients within a few ulp of representable values, exact
+// quotients (a power-of-two divisor), and the whole range of fast::div.  Division and square root never land exactly
 // halfway between two doubles, so round-to-nearest has no ties to test.
 __global__ void certified_math_check_kernel(uint64_t n, uint64_t seed, unsigned long long* out)
 {
@@ -1216,7 +1216,7 @@ __global__ void certified_math_check_kernel(uint64_t n, uint64_t seed, unsigned 
 	{
 		const uint64_t h1 = splitmix64(seed ^ (k * 0x2545f4914f6cdd1dULL)), h2 = splitmix64(h1), h3 = splitmix64(h2);
 		double a, b;
-		switch(k & 3)
+		switch((k & 7) == 7 ? 4 : static_cast<int>(k & 3))
 		{
 			case 0:  // the trajectory ranges: km, km/s, s, km^3/s^2
 				a = random_double(h1, -40, 70);
@@ -1234,19 +1234,22 @@ __global__ void certified_math_check_kernel(uint64_t n, uint64_t seed, unsigned 
 				a = __longlong_as_double(__double_as_longlong(__dmul_rn(b, q)) + d);
 				break;
 			}
-			default:
+			case 3:
 			{  // exact quotients: a power-of-two divisor
 				const double m = random_double(h1, -10, 10);
 				b = ldexp(1.0, static_cast<int>(h2 % 41) - 20);
 				a = __dmul_rn(b, m);
 				break;
 			}
+			default:  // the ends of the range
+				a = random_double(h1, -700, 400);
+				b = random_double(h2, -200, 399);
+				break;
 		}
 		if(h3 & 1)
 			a = -a;
-		// the operand range of fast::div: other pairs count as fallbacks
-		const double aa = fabs(a), ab = fabs(b);
-		bool ok = (ab >= 0x1p-100) & (ab < 0x1p100) & (((aa >= 0x1p-700) & (aa <= 0x1p400)) | (__double_as_longlong(a) == 0));
+		// pairs outside the range of fast::div count as fallbacks (a zero dividend's quotient has no sign there)
+		bool ok = fast::in_division_range(a, b) & ((a != 0.0) | (__double_as_longlong(a) == 0 && b > 0.0));
 		const double q = fast::div(a, fast::recip(b, ok));
 		const double ref = a / b;
 		if(!ok)

@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -930,9 +931,22 @@ int dms_run(dms_ctx* ctx, const dms_run_opts* opts, const dms_work_range* ranges
 // ---- autotuner ------------------------------------------------------------------------------
 namespace
 {
-// One trial of the autotuner: a launch stopped after `seconds` over fresh ids (from 2^40) of the
-// given points, its results in the scratch accumulators `scratch`; returns accepted free steps
-// per second (finished and unfinished trajectories), or a negative value on failure.
+// Most ids of a trial when its points are few: their initial states take 2.1 GB.
+constexpr uint64_t TRIAL_IDS = 1ULL << 25;
+
+// What the options make of a launch of `total` trajectories: two settings of the same form are the same launch.
+std::array<int64_t, 6> Launch_Form(const dms_run_opts* o, uint64_t total, int sm_count)
+{
+	const int threads = Block_Threads(o, total, sm_count);
+	RunParams p{};
+	Apply_Lane_Options(p, o, threads > LATENCY_THREADS);
+	return {threads, p.queue_chunk, p.scatter_batch, p.scatter_wait, p.final_batch, p.final_wait};
+}
+
+// One trial of the autotuner: a launch stopped after the time limit of `o` over fresh ids (from 2^40) of the
+// given points, its results in the scratch accumulators `t`; returns accepted free steps
+// per second (finished and unfinished trajectories), or a negative value on failure.  `taken` receives the
+// number of ids that the lanes have claimed.
 struct TuneScratch
 {
 	unsigned long long* counters = nullptr;
@@ -954,7 +968,7 @@ struct TuneScratch
 };
 
 double Tune_Trial(dms_ctx* ctx, const dms_run_opts& o, const std::vector<int32_t>& pts, uint64_t per_point, uint64_t first,
-                  const TuneScratch& t, void* d_ranges)
+                  const TuneScratch& t, void* d_ranges, uint64_t& taken)
 {
 	const int n = static_cast<int>(pts.size());
 	const size_t np = ctx->points.size();
@@ -989,8 +1003,11 @@ double Tune_Trial(dms_ctx* ctx, const dms_run_opts& o, const std::vector<int32_t
 	if(rc != DMS_OK && rc != DMS_ERR_CANCELLED)
 		return -1.0;
 	std::vector<unsigned long long> c(DMS_NUM_COUNTERS * np);
-	if(cudaMemcpy(c.data(), t.counters, sizeof(unsigned long long) * c.size(), cudaMemcpyDeviceToHost) != cudaSuccess)
+	unsigned long long head = 0;
+	if(cudaMemcpy(c.data(), t.counters, sizeof(unsigned long long) * c.size(), cudaMemcpyDeviceToHost) != cudaSuccess ||
+	   cudaMemcpy(&head, ctx->d_queue, sizeof head, cudaMemcpyDeviceToHost) != cudaSuccess)
 		return -1.0;
+	taken = head;
 	double steps = 0.0;
 	for(int32_t pt : pts)
 	{
@@ -1026,13 +1043,21 @@ int dms_autotune(dms_ctx* ctx, const dms_run_opts* base, const dms_work_range* r
 	struct Guard
 	{
 		TuneScratch& t;
+		dms_ctx* ctx;
+		uint64_t init_capacity;
 		void* ranges = nullptr;
 		~Guard()
 		{
 			t.Free();
 			cudaFree(ranges);
+			if(ctx->init_capacity > init_capacity)  // the trials' initial states are not kept
+			{
+				cudaFree(ctx->d_init);
+				ctx->d_init = nullptr;
+				ctx->init_capacity = 0;
+			}
 		}
-	} guard{t};
+	} guard{t, ctx, ctx->init_capacity};
 	DMS_CUDA(ctx, cudaMalloc(&t.counters, sizeof(unsigned long long) * DMS_NUM_COUNTERS * np));
 	DMS_CUDA(ctx, cudaMalloc(&t.hists, sizeof(double) * DMS_NUM_HISTS * DMS_NUM_BINS * np));
 	DMS_CUDA(ctx, cudaMalloc(&t.events, sizeof(dms_evaporation_event) * t.capacity * np));
@@ -1040,8 +1065,7 @@ int dms_autotune(dms_ctx* ctx, const dms_run_opts* base, const dms_work_range* r
 	DMS_CUDA(ctx, cudaMalloc(&t.refl, sizeof(dms_reflection) * t.capacity * np));
 	DMS_CUDA(ctx, cudaMalloc(&t.refl_count, sizeof(unsigned long long) * np));
 	DMS_CUDA(ctx, cudaMalloc(&guard.ranges, (sizeof(uint64_t) * 2 + sizeof(int32_t)) * (pts.size() + 1)));
-	// enough ids that no trial drains its queue: a million per point, fresh for every trial
-	const uint64_t per_point = 1ULL << 20;
+	uint64_t per_point = 1ULL << 20, taken = 0;
 	dms_run_opts best = *base;
 	best.time_limit_s = trial_seconds;
 	best.iteration_budget = 0;
@@ -1049,13 +1073,28 @@ int dms_autotune(dms_ctx* ctx, const dms_run_opts* base, const dms_work_range* r
 	uint64_t next_first = 1ULL << 40;
 	auto score = [&](const dms_run_opts& o) {
 		n_trials++;
-		const double v = Tune_Trial(ctx, o, pts, per_point, next_first, t, guard.ranges);
+		const double v = Tune_Trial(ctx, o, pts, per_point, next_first, t, guard.ranges, taken);
 		next_first += per_point;
 		return v;
 	};
-	double best_score = score(best);
-	if(!(best_score > 0.0))
-		return Fail(ctx, DMS_ERR_CUDA, "autotune: the first trial launch failed");
+	// A trial whose queue runs dry times the last trajectories instead of the steady state.  So the base setting has
+	// to leave half of the ids of a trial: more ids, and from TRIAL_IDS on a shorter trial, until it does.  (The
+	// bench's point takes 2^20 ids in 0.25 s in FP64 and 0.16 s in the mixed form.)
+	double best_score = -1.0;
+	for(;;)
+	{
+		best_score = score(best);
+		if(!(best_score > 0.0))
+			return Fail(ctx, DMS_ERR_CUDA, "autotune: the first trial launch failed");
+		const uint64_t total = per_point * pts.size();
+		if(2 * taken <= total || best.time_limit_s < 1.0e-3)
+			break;
+		if(2 * total <= TRIAL_IDS)
+			per_point *= 2;
+		else
+			best.time_limit_s *= 0.5;
+	}
+	const uint64_t total = per_point * pts.size();
 	struct Knob
 	{
 		uint32_t dms_run_opts::*field;
@@ -1078,10 +1117,10 @@ int dms_autotune(dms_ctx* ctx, const dms_run_opts* base, const dms_work_range* r
 		for(const Knob& k : knobs)
 			for(uint32_t v : k.values)
 			{
-				if(best.*(k.field) == v)
-					continue;
 				dms_run_opts trial = best;
 				trial.*(k.field) = v;
+				if(Launch_Form(&trial, total, ctx->sm_count) == Launch_Form(&best, total, ctx->sm_count))
+					continue;
 				const double sc = score(trial);
 				if(sc > 1.02 * best_score)
 				{

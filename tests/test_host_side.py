@@ -111,3 +111,28 @@ only, = launches()
 assert only.threads == 128 and not only.resume
 e.close()
 """)
+
+
+@pytest.mark.parametrize("per_second, seconds", [(2 ** 17 / 0.02, 0.02), (2 ** 21 / 0.02, 0.02), (2 ** 22 / 0.02, 0.08), (2 ** 26 / 0.04, 0.08)])
+def test_autotuner_times_the_steady_state_of_different_launches(host, per_second, seconds):
+    """No setting is timed on a launch whose queue has run dry, and none that is the launch of the best one so far."""
+    host("per_second, seconds = %r, %r" % (per_second, seconds) + r"""
+rate.value = per_second
+e = dms_b200.Engine(0)
+pid = point(e)
+tuned, trials = e.autotune([(pid, 0, 100)], dms_b200.run_opts(seed=1), trial_seconds=seconds)
+trial = [l for l in launches() if not l.resume]
+assert len(trial) == trials
+form = lambda l: (l.threads, l.queue_chunk) + tuple(l.options)
+base = form(trial[0])
+sized = [l for l in trial if form(l) == base]
+others = trial[len(sized):]
+# every setting runs at the same speed here: the base stays the best, and nothing but it is launched twice in a pass
+assert all(form(l) != base for l in others)
+assert len(others) >= 8 and len(set(map(form, others))) == len(others)
+assert dms_b200.lane_options(tuned) == dms_b200.lane_options(dms_b200.run_opts(seed=1))
+assert len(set(l.total for l in others)) == 1 and others[0].total <= 2 ** 25
+assert sized[-1].done <= others[0].total // 2
+assert all(l.done < l.total for l in others)
+e.close()
+""")

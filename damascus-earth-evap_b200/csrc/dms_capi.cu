@@ -250,8 +250,8 @@ int Check_Run_Opts(dms_ctx* ctx, const dms_run_opts* o)
 }
 
 // The lane-scheduling options of a launch (dms_run_opts, 0 = default).  In lockstep the whole block makes a
-// rare phase together, so larger batches pay.  Measured there (FP64; batch / wait of the scatterings, batch of
-// the terminations: 16 / 32, 8 against 24 / 64, 16): Capture mode m = 0.3 GeV, 1e-36 cm^2, 2^20 trajectories
+// rare phase together, so larger batches pay.  Measured there (FP64; batch in lanes of 64 / wait of the scatterings,
+// batch of the terminations: 16 / 32, 8 against 24 / 64, 16): Capture mode m = 0.3 GeV, 1e-36 cm^2, 2^20 trajectories
 // 45.1 / 41.0 ms, m = 1 GeV, 1e-35 cm^2 48.5 / 44.4 ms, steady state at m = 0.1 GeV, 1e-33 cm^2 890 / 949
 // million steps/s.  The mixed form's scatterings are cheaper: its steady states lose 2-6 % by longer waits.
 void Apply_Lane_Options(RunParams& p, const dms_run_opts* o, bool lockstep)
@@ -262,6 +262,9 @@ void Apply_Lane_Options(RunParams& p, const dms_run_opts* o, bool lockstep)
 	p.scatter_wait = o->scatter_wait ? static_cast<int>(o->scatter_wait) : patient ? 64 : 32;
 	p.final_batch = o->final_batch ? static_cast<int>(o->final_batch) : lockstep ? 16 : 8;
 	p.final_wait = o->final_wait ? static_cast<int>(o->final_wait) : 32;
+	// in a block, half of the default batches per warp; a batch that the caller sets is the same share of the block
+	p.block_scatter_batch = o->scatter_batch ? 2 * p.scatter_batch : p.scatter_batch;
+	p.block_final_batch = o->final_batch ? 2 * p.final_batch : p.final_batch;
 }
 
 // Lanes at work at which a block of a throughput launch with no more work parks them for the latency launch.
@@ -935,12 +938,12 @@ namespace
 constexpr uint64_t TRIAL_IDS = 1ULL << 25;
 
 // What the options make of a launch of `total` trajectories: two settings of the same form are the same launch.
-std::array<int64_t, 6> Launch_Form(const dms_run_opts* o, uint64_t total, int sm_count)
+std::array<int64_t, 8> Launch_Form(const dms_run_opts* o, uint64_t total, int sm_count)
 {
 	const int threads = Block_Threads(o, total, sm_count);
 	RunParams p{};
 	Apply_Lane_Options(p, o, threads > LATENCY_THREADS);
-	return {threads, p.queue_chunk, p.scatter_batch, p.scatter_wait, p.final_batch, p.final_wait};
+	return {threads, p.queue_chunk, p.scatter_batch, p.scatter_wait, p.final_batch, p.final_wait, p.block_scatter_batch, p.block_final_batch};
 }
 
 // One trial of the autotuner: a launch stopped after the time limit of `o` over fresh ids (from 2^40) of the
@@ -1104,9 +1107,9 @@ int dms_autotune(dms_ctx* ctx, const dms_run_opts* base, const dms_work_range* r
 		{&dms_run_opts::threads_per_block, {64, 96, 128}},
 		{&dms_run_opts::blocks_per_sm, {2, 3, 4}},
 		{&dms_run_opts::queue_chunk, {1, 2, 4}},
-		{&dms_run_opts::scatter_batch, {8, 16, 24, 32}},
+		{&dms_run_opts::scatter_batch, {4, 8, 12, 16, 24, 32}},
 		{&dms_run_opts::scatter_wait, {16, 32, 64, 128}},
-		{&dms_run_opts::final_batch, {4, 8, 16}},
+		{&dms_run_opts::final_batch, {2, 4, 8, 16}},
 		{&dms_run_opts::final_wait, {16, 32, 64}},
 	};
 	// coordinate descent: a value replaces the current one only when it is at least 2 % faster

@@ -77,6 +77,7 @@ struct RunParams
 	// the warp batching of scatterings and terminations
 	uint32_t queue_chunk;
 	int scatter_batch, scatter_wait, final_batch, final_wait;
+	int block_scatter_batch, block_final_batch;  // the batches of a block in lockstep, in lanes of 64
 	int lanes_per_block; // lanes of a block that take trajectories (all, fewer in a spread launch)
 	int lockstep_min;    // lanes at work at which a block's warps leave the lockstep once the queue is empty
 	// The tail of a throughput launch: a block with at most lockstep_min lanes at work and no more work parks

@@ -743,7 +743,7 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 	if constexpr(Step::team)
 		if(threadIdx.x == 0)
 			step.team_init();
-	int passes_scatter = 0, passes_final = 0;  // passes since the block's last scattering (termination) phase
+	int scatter_passes = 0, final_passes = 0;  // as rare_phase_due counts them
 	__syncthreads();
 	Lane L;
 	FlushJob job;
@@ -826,14 +826,8 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 			// lanes at work
 			const int at_work = n_step + n_scatter + n_final, lanes = blockDim.x;
 			const int full = Step::throughput && drained ? at_work : lanes;
-			passes_scatter++;
-			passes_final++;
-			go_scatter = n_scatter != 0 && (64 * n_scatter >= R.scatter_batch * full || n_step == 0 || passes_scatter * lanes >= R.scatter_wait * full);
-			go_final = n_final != 0 && (64 * n_final >= R.final_batch * full || n_step == 0 || passes_final * lanes >= R.final_wait * full);
-			if(go_scatter)
-				passes_scatter = 0;
-			if(go_final)
-				passes_final = 0;
+			go_scatter = rare_phase_due(scatter_passes, n_scatter, n_step, R.block_scatter_batch, 64, R.scatter_wait, lanes, full);
+			go_final = rare_phase_due(final_passes, n_final, n_step, R.block_final_batch, 64, R.final_wait, lanes, full);
 			if(flags & 2)
 			{
 				if(in_warp == 0)
@@ -926,23 +920,10 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 			const unsigned int stepping = __ballot_sync(FULL_WARP, phase == PH_STEP || phase == PH_FETCH || phase == PH_SEGMENT);
 			const unsigned int waiting = __ballot_sync(FULL_WARP, phase == PH_SCATTER);
 			const unsigned int ending = __ballot_sync(FULL_WARP, phase == PH_FINAL);
-			// lanes wait until several lanes of the warp are there, or one has waited long enough, or no
-			// lane is stepping; batches and waits are for a full warp and shrink with the lanes at work
+			// batches and waits are for a full warp and shrink with the lanes at work
 			const int at_work = __popc(live);
-			if(waiting != 0u)
-			{
-				passes_scatter++;
-				go_scatter = 32 * __popc(waiting) >= R.scatter_batch * at_work || stepping == 0u || 32 * passes_scatter >= R.scatter_wait * at_work;
-				if(go_scatter)
-					passes_scatter = 0;
-			}
-			if(ending != 0u)
-			{
-				passes_final++;
-				go_final = 32 * __popc(ending) >= R.final_batch * at_work || stepping == 0u || 32 * passes_final >= R.final_wait * at_work;
-				if(go_final)
-					passes_final = 0;
-			}
+			go_scatter = rare_phase_due(scatter_passes, __popc(waiting), static_cast<int>(stepping), R.scatter_batch, 32, R.scatter_wait, 32, at_work);
+			go_final = rare_phase_due(final_passes, __popc(ending), static_cast<int>(stepping), R.final_batch, 32, R.final_wait, 32, at_work);
 		}
 		// Scatterings and terminations run for many lanes at once.  A lane's draws do not depend on
 		// when it scatters.

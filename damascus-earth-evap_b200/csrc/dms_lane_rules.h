@@ -19,6 +19,21 @@ namespace lane
 constexpr int VOTE_SETS = 3;
 DMS_HD int next_vote_set(int set) { return set + 1 == VOTE_SETS ? 0 : set + 1; }
 
+// When lanes that wait for a rare phase (scatterings, terminations) get it, asked once per pass: when `waiting` of them
+// reach `batch` in `per` lanes of a full group, when the first of them has waited `wait` passes, or when no lane is
+// stepping.  `passes` counts since the first of them arrived (0 before it).  `lanes` is the size of the group;
+// with fewer lanes at work, `full`, batch and wait shrink.
+DMS_HD bool rare_phase_due(int& passes, int waiting, int stepping, int batch, int per, int wait, int lanes, int full)
+{
+	if(waiting == 0)
+		return false;
+	passes++;
+	const bool go = per * waiting >= batch * full || stepping == 0 || passes * lanes >= wait * full;
+	if(go)
+		passes = 0;
+	return go;
+}
+
 // Whether the time to the surface (src/Simulation_Trajectory.cpp:886-899) of a particle outside it cannot be
 // below `step`, by a margin far above its rounding.  along = x . v.
 DMS_HD bool surface_is_far(double r, double along, double step)

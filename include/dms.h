@@ -209,9 +209,10 @@ typedef struct
 	 * a lane that reaches a scattering point (a termination) waits until scatter_batch
 	 * (final_batch) lanes of its warp are there, or it has waited scatter_wait (final_wait)
 	 * loop iterations, or no lane of the warp is stepping; then the warp runs the scattering
-	 * (termination) code once for all of them.  0 = defaults (16 / 32 / 8 / 32, longer in launches that
-	 * fill the GPU, where the lanes of whole blocks count in their stead); batches up to
-	 * 32, waits up to 1024. */
+	 * (termination) code once for all of them.  Where the warps of a block run in step, its lanes
+	 * count in their stead: scatter_batch of every 32 lanes of the block.  0 = defaults (of a warp 16 / 32 /
+	 * 8 / 32, of a block half of the batches; batches and waits longer in launches that fill the GPU);
+	 * batches up to 32, waits up to 1024. */
 	uint32_t scatter_batch;
 	uint32_t scatter_wait;
 	uint32_t final_batch;

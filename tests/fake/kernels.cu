@@ -21,7 +21,7 @@ struct FakeLaunch
 	int32_t blocks, threads, mixed, resume, lanes_per_block, lockstep_min;
 	uint32_t queue_chunk;
 	uint32_t parked_capacity;
-	int32_t options[4];  // scatter_batch, scatter_wait, final_batch, final_wait
+	int32_t options[6];  // scatter_batch, scatter_wait, final_batch, final_wait; the batches of a block
 };
 double fake_rate = 1e9;
 }
@@ -78,6 +78,8 @@ void launch(const RunParams& p, int blocks, int threads, cudaStream_t s, int mix
 	l.options[1] = p.scatter_wait;
 	l.options[2] = p.final_batch;
 	l.options[3] = p.final_wait;
+	l.options[4] = p.block_scatter_batch;
+	l.options[5] = p.block_final_batch;
 	launches.push_back(l);
 	if(!p.resume)
 	{

@@ -20,7 +20,7 @@ import dms_b200
 class Launch(ctypes.Structure):
     _fields_ = [("total", ctypes.c_uint64), ("done", ctypes.c_uint64), ("parked_room", ctypes.c_uint64)] + [
         (n, ctypes.c_int32) for n in ("blocks", "threads", "mixed", "resume", "lanes_per_block", "lockstep_min")] + [
-        ("queue_chunk", ctypes.c_uint32), ("parked_capacity", ctypes.c_uint32), ("options", ctypes.c_int32 * 4)]
+        ("queue_chunk", ctypes.c_uint32), ("parked_capacity", ctypes.c_uint32), ("options", ctypes.c_int32 * 6)]
 lib = dms_b200.library()
 def launches():
     a = (Launch * 4096)()
@@ -134,5 +134,20 @@ assert dms_b200.lane_options(tuned) == dms_b200.lane_options(dms_b200.run_opts(s
 assert len(set(l.total for l in others)) == 1 and others[0].total <= 2 ** 25
 assert sized[-1].done <= others[0].total // 2
 assert all(l.done < l.total for l in others)
+e.close()
+""")
+
+
+@pytest.mark.parametrize("precision", ["FP64", "MIXED"])
+def test_a_batch_that_is_set_is_the_same_share_of_a_warp_and_of_a_block(host, precision):
+    host("precision = dms_b200.PRECISION_%s" % precision + r"""
+e = dms_b200.Engine(0)
+pid = point(e)
+for count in (100, 100000):
+    for scatter, final in ((1, 1), (32, 32), (8, 3)):
+        e.run([(pid, 0, count)], dms_b200.run_opts(seed=1, precision=precision, scatter_batch=scatter, final_batch=final,
+                                                   scatter_wait=5, final_wait=1024))
+        for l in launches():
+            assert tuple(l.options) == (scatter, 5, final, 1024, 2 * scatter, 2 * final)  # of 32 lanes, of 64
 e.close()
 """)

@@ -14,6 +14,10 @@ SHIM = r"""
 extern "C" {
 int vote_sets() { return dms::lane::VOTE_SETS; }
 int next_vote_set(int set) { return dms::lane::next_vote_set(set); }
+int rare_phase_due(int* passes, int waiting, int stepping, int batch, int per, int wait, int lanes, int full)
+{
+	return dms::lane::rare_phase_due(*passes, waiting, stepping, batch, per, wait, lanes, full);
+}
 }
 
 struct V { double x, y, z; };
@@ -135,3 +139,24 @@ def test_radial_speed_calls_no_step_far_that_the_surface_binds(rules):
     far = rules.far_from_surface(2_000_000, 1, ctypes.byref(wrong))
     assert far > 10_000  # the states reach the rule
     assert wrong.value == 0
+
+
+@pytest.mark.parametrize("lanes, per, unit", [(32, 32, 1), (128, 64, 2), (512, 64, 2), (640, 64, 2)])
+@pytest.mark.parametrize("batch", [1, 8, 32])
+@pytest.mark.parametrize("wait", [1, 5, 32])
+def test_lanes_wait_for_their_batch_or_their_passes(rules, lanes, per, unit, batch, wait):
+    """A batch of b lanes of 32 starts a phase, or the first lane's passes since it arrived; quiet passes before do not count."""
+    def passes_until(waiting, quiet, stepping=1):
+        state, n = ctypes.c_int(0), 0
+        for _ in range(quiet):
+            assert not rules.rare_phase_due(ctypes.byref(state), 0, stepping, unit * batch, per, wait, lanes, lanes)
+        while True:
+            n += 1
+            if rules.rare_phase_due(ctypes.byref(state), waiting, stepping, unit * batch, per, wait, lanes, lanes):
+                assert state.value == 0
+                return n
+    enough = batch * lanes // 32
+    for quiet in (0, 1, 1000):
+        assert passes_until(enough, quiet) == 1
+        assert passes_until(enough - 1, quiet) == wait if enough > 1 else True
+        assert passes_until(1, quiet, stepping=0) == 1

@@ -603,6 +603,19 @@ int dms_check_certified_math(dms_ctx* ctx, uint64_t n, uint64_t seed, uint64_t* 
 	return DMS_OK;
 }
 
+#ifdef DMS_CHECKED
+// Checked build: the counts of forms (FORM_*) since the last call, for the kernels of one precision.
+int dms_checked_form_counts(dms_ctx* ctx, int precision, unsigned long long* counts)
+{
+	if(!ctx || !counts)
+		return DMS_ERR_INVALID_ARGUMENT;
+	DMS_NOT_IN_FLIGHT(ctx);
+	DMS_CUDA(ctx, cudaSetDevice(ctx->device));
+	const bool ok = precision == DMS_PRECISION_MIXED ? Take_Form_Counts_Mixed(counts) : Take_Form_Counts(counts);
+	return ok ? DMS_OK : Fail(ctx, DMS_ERR_CUDA, "form counts");
+}
+#endif
+
 int dms_last_kernel_ms(const dms_ctx* ctx, double* ms)
 {
 	if(!ctx || !ms)

@@ -33,8 +33,20 @@ enum : unsigned int
 	BOUNDS_RANGE = 16u,
 	BOUNDS_TARGET = 32u,
 };
+// The checked build also counts the forms that trajectories went through, for its tests.
+enum : int
+{
+	FORM_TEAMS = 0,
+	FORM_TEAM_STEPS = 1,
+	FORM_HELPERS_GAVE_UP = 2,  // warps that stopped waiting for a team to form
+	FORM_PARKED = 3,
+	FORM_RESUMED = 4,
+	FORM_COUNTS = 5,
+};
 #ifdef DMS_CHECKED
 static __device__ unsigned int dms_bounds_status;
+static __device__ unsigned long long dms_form_counts[FORM_COUNTS];
+#define DMS_COUNT_FORM(which, n) atomicAdd(&dms_form_counts[which], static_cast<unsigned long long>(n))
 #define DMS_CHECK_INDEX(i, lo, hi, bit)                                  \
 	do                                                                   \
 	{                                                                    \
@@ -45,6 +57,7 @@ static __device__ unsigned int dms_bounds_status;
 		}                                                                \
 	} while(0)
 #else
+#define DMS_COUNT_FORM(which, n) static_cast<void>(n)
 #define DMS_CHECK_INDEX(i, lo, hi, bit) \
 	do                                  \
 	{                                   \

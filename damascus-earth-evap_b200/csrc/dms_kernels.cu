@@ -1334,6 +1334,15 @@ void Launch_Rate_Query(const DevSolar& S, const DevPoint* point, int interpolate
 		rate_query_kernel<<<blocks, threads, 0, stream>>>(S, point, interpolated, r, v, out, n);
 }
 
+#ifdef DMS_CHECKED
+bool Take_Form_Counts(unsigned long long* counts)
+{
+	const unsigned long long zero[FORM_COUNTS] = {};
+	return cudaMemcpyFromSymbol(counts, dms_form_counts, sizeof zero) == cudaSuccess &&
+	       cudaMemcpyToSymbol(dms_form_counts, zero, sizeof zero) == cudaSuccess && cudaStreamSynchronize(cudaStreamLegacy) == cudaSuccess;
+}
+#endif
+
 unsigned int Take_Bounds_Status()
 {
 #ifdef DMS_CHECKED

@@ -127,6 +127,12 @@ __device__ __forceinline__ int find_range(const RunParams& R, uint64_t w)
 unsigned int Take_Bounds_Status();
 unsigned int Take_Bounds_Status_Mixed();
 
+#ifdef DMS_CHECKED
+// The same for the counts of forms.
+bool Take_Form_Counts(unsigned long long* counts);
+bool Take_Form_Counts_Mixed(unsigned long long* counts);
+#endif
+
 // Initial states of all p.total work indices into p.init (one thread per work index); the
 // trajectory kernels read them.  Launched on the same stream before every trajectory launch.
 void Launch_Initial_States(const RunParams& p, cudaStream_t stream);

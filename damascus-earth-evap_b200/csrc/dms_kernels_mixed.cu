@@ -804,6 +804,15 @@ void Launch_To_Float(const double* in, float* out, size_t n, cudaStream_t stream
 	grid_to_float_kernel<<<148 * 4, 256, 0, stream>>>(in, out, n);
 }
 
+#ifdef DMS_CHECKED
+bool Take_Form_Counts_Mixed(unsigned long long* counts)
+{
+	const unsigned long long zero[FORM_COUNTS] = {};
+	return cudaMemcpyFromSymbol(counts, dms_form_counts, sizeof zero) == cudaSuccess &&
+	       cudaMemcpyToSymbol(dms_form_counts, zero, sizeof zero) == cudaSuccess && cudaStreamSynchronize(cudaStreamLegacy) == cudaSuccess;
+}
+#endif
+
 unsigned int Take_Bounds_Status_Mixed()
 {
 #ifdef DMS_CHECKED

@@ -775,6 +775,7 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 				iter = s.iter;
 				P = R.points + L.point;
 				m_dm = __ldg(&P->m_dm);
+				DMS_COUNT_FORM(FORM_RESUMED, 1);
 			}
 			// one count per block: the warps in lockstep agree on it
 			__shared__ unsigned long long first_iter;
@@ -864,6 +865,7 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 							s.q_end = q_end;
 							s.phase = phase;
 							s.iter = iter;
+							DMS_COUNT_FORM(FORM_PARKED, 1);
 						}
 						else
 							atomicOr(R.status, STATUS_PARKED_FULL);

@@ -56,7 +56,12 @@ enum Verdict : int
 	VERDICT_PAUSE = 5,     // not judged: the lane loop is due
 };
 constexpr int TEAM_MAX_STEPS = 512;                      // per call: the lane loop looks at the cancel flag between calls
-constexpr long long TEAM_WAIT_CYCLES = 40000000000ll;   // ~20 s: how long a warp without work waits for a team
+// How long a warp without work waits for a team (~20 s; the checked build's tests see it run out in ~50 ms).
+#ifdef DMS_CHECKED
+constexpr long long TEAM_WAIT_CYCLES = 100000000ll;
+#else
+constexpr long long TEAM_WAIT_CYCLES = 40000000000ll;
+#endif
 
 __device__ __forceinline__ void team_barrier() { asm volatile("bar.sync 1, 96;" ::: "memory"); }
 
@@ -166,12 +171,15 @@ struct Team
 			{
 				word = *reinterpret_cast<volatile int*>(&b.word);
 				bool leave = clock64() - t0 > TEAM_WAIT_CYCLES;
+				const bool gave_up = leave;
 				if((poll & 255u) == 0u)
 					leave |= *R.cancel != 0;
 				// a warp leaves by putting the count out of reach, which no formed team can follow
 				if(leave && word >= 0 && word < TEAM_FORMED)
 				{
 					const int seen = atomicCAS(&b.word, word, TEAM_NEVER);
+					if(gave_up && seen == word)
+						DMS_COUNT_FORM(FORM_HELPERS_GAVE_UP, 1);
 					word = seen == word ? TEAM_NEVER : seen;
 				}
 			}
@@ -234,6 +242,8 @@ struct Team
 		int formed = 0;
 		if((threadIdx.x & 31) == 0)
 			formed = *reinterpret_cast<volatile int*>(&b.word) == 3 && atomicCAS(&b.word, 3, TEAM_FORMED) == 3 ? 1 : 0;
+		if(formed)
+			DMS_COUNT_FORM(FORM_TEAMS, 1);
 		return __shfl_sync(0xffffffffu, formed, 0) != 0;
 	}
 	// A warp that stops in mid-trajectory: no team can form any more.
@@ -301,6 +311,7 @@ struct Team
 		team_barrier();  // the committing warp has written its part back
 		if(mine)
 		{
+			DMS_COUNT_FORM(FORM_TEAM_STEPS, j);
 			const TeamState& s = b.s[j & 3];
 			L.hot().pr.time = s.time;
 			L.hot().pr.radius = s.radius;

@@ -883,6 +883,8 @@ __device__ __forceinline__ void lane_loop(const RunParams& R, Step step)
 			if(iter >= next_check)
 			{
 				next_check = iter + 1024;
+				if constexpr(Step::team)
+					step.team_alive();
 				if(__any_sync(FULL_WARP, *R.cancel != 0))
 				{
 					atomicOr(R.status, STATUS_CANCELLED);

@@ -21,7 +21,8 @@ namespace lane
 // else (a scattering, the boundary, a failure) hands the state at the step's start back to the lane, which
 // makes that step by itself.  Every value is formed by the functions of the one-lane pass from the same
 // arguments, so the results are the same bits.  The barriers count whole warps that all run the same loop;
-// the only wait by polling is that of a warp without work for a team to form, and it is bounded.
+// the only wait by polling is that of a warp without work for a team to form, and it ends some time after the
+// block's last sign of life.
 // A lone lane's step takes 5.7 -> 3.3 us in FP64 and 4.4 -> 3.0 us in the mixed form; 16 384 Parameter-point
 // trajectories of m = 0.3 GeV, 1e-36 cm^2 426 -> 259 ms in the mixed form, 128 25 -> 18 ms.
 struct TeamState  // the propagator at the start of a step
@@ -33,6 +34,7 @@ template <class PropT, class EvT>
 struct TeamBox
 {
 	int word;       // warps without work; TEAM_FORMED once a team has formed, negative when none can
+	int alive;      // raised now and then by the warps that make steps
 	int command;    // TEAM_RUN, TEAM_EXIT
 	int verdict[2];
 	int captured, bound, bmin, bmax, cbin;
@@ -56,7 +58,8 @@ enum Verdict : int
 	VERDICT_PAUSE = 5,     // not judged: the lane loop is due
 };
 constexpr int TEAM_MAX_STEPS = 512;                      // per call: the lane loop looks at the cancel flag between calls
-// How long a warp without work waits for a team (~20 s; the checked build's tests see it run out in ~50 ms).
+// How long a warp without work waits for a team after the last sign of life of its block, which the warps at
+// work give every 1 024 passes, some 10 ms (~20 s; in the checked build ~50 ms, for its tests).
 #ifdef DMS_CHECKED
 constexpr long long TEAM_WAIT_CYCLES = 100000000ll;
 #else
@@ -146,7 +149,14 @@ struct Team
 	__device__ __forceinline__ void team_init() const
 	{
 		box().word = 0;
+		box().alive = 0;
 		box().command = TEAM_RUN;
+	}
+	// Called now and then by a whole warp at work, for those that wait.
+	__device__ __forceinline__ void team_alive() const
+	{
+		if((threadIdx.x & 31) == 0)
+			atomicAdd(&box().alive, 1);
 	}
 	// Called by a whole warp without work: it helps a lone lane of its block, if one forms a team, until that
 	// lane's trajectory has ended.
@@ -163,13 +173,20 @@ struct Team
 			team_forgo();  // the last warp of the block: nobody is left to help
 			return;
 		}
-		const long long t0 = clock64();
+		long long t0 = clock64();
+		int seen_alive = 0;
 		for(unsigned int poll = 1;; poll++)
 		{
 			int word = 0;
 			if(lane0)
 			{
 				word = *reinterpret_cast<volatile int*>(&b.word);
+				const int alive = *reinterpret_cast<volatile int*>(&b.alive);
+				if(alive != seen_alive)
+				{
+					seen_alive = alive;
+					t0 = clock64();
+				}
 				bool leave = clock64() - t0 > TEAM_WAIT_CYCLES;
 				const bool gave_up = leave;
 				if((poll & 255u) == 0u)

@@ -75,3 +75,16 @@ for capture in (True, False):
 e.run([(pid, 10 ** 6, 128 * SMS)], opts(capture_mode=True, max_scatterings=20))
 assert forms()["parked"] == 0
 """)
+
+
+@pytest.mark.parametrize("precision", ["FP64", "MIXED"])
+def test_helpers_wait_while_their_block_makes_steps(precision):
+    """Two lanes in each block, for longer than a warp without work waits for a block that shows no life."""
+    run(precision, r"""
+heavy = e.add_point(dms_b200.point_params(1.0, 1e-35, interpolation_points=200))
+e.run([(heavy, 0, 2 * SMS)], opts(max_scatterings=2000))
+f = forms()
+print(f, e.last_kernel_ms())
+assert e.last_kernel_ms() > 200.0  # four times as long as the wait
+assert f["teams"] > 0 and f["gave_up"] == 0
+""")

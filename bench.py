@@ -15,7 +15,7 @@ Arms:
   default            the CUDA engine through its C ABI (libdms_cuda.so)
   --impl reference   the reference's own CPU implementation of the path (oracle/_ref: the
                      reference sources compiled against restated third-party shims), all host
-                     cores, bounded per-step samples of the same workload
+                     cores, the same trajectories; without that build one line that says so
 """
 import argparse
 import json
@@ -170,6 +170,11 @@ def cpu_step(pool, point, first, count=TRAJECTORIES, chunk=64):
 def run_reference_arm(args):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
+        return
+    if cpu_kind() != "reference":
+        # the C oracle is this repository's own code: its time is not the reference's
+        print(json.dumps({"impl": "reference", "unavailable": "the reference build oracle/_ref/libdms_ref.so is not there: it is "
+                          "compiled from the reference sources, which this machine does not have"}), flush=True)
         return
     cores = os.cpu_count() or 1
     t_setup = time.perf_counter()

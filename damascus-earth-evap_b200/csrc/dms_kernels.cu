@@ -1138,7 +1138,7 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) trajectory_kernel(const RunPar
 	lane_loop<StrictLane>(R, StrictStep<true>());
 }
 
-// The latency form: one warp per scheduler, no spills (176 registers).
+// The latency form: one warp per scheduler, no spills (196 registers).
 __global__ void __launch_bounds__(LATENCY_THREADS, 1) trajectory_kernel_latency(const RunParams R)
 {
 	lane_loop<StrictLane>(R, StrictStep<false>());

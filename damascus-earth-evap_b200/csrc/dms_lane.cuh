@@ -108,13 +108,6 @@ __device__ __forceinline__ bool wall_time_exceeded(const RunParams& R, const Lan
 	return R.wall_limit_ns != 0 && global_timer_ns() - L.wall_start > R.wall_limit_ns;
 }
 
-// Position of the (n+1)-th set bit of m (n from 0); m must have more than n set bits.
-__device__ __forceinline__ int nth_set_bit(unsigned int m, int n)
-{
-	for(int t = 0; t < n; t++) m &= m - 1u;
-	return __ffs(m) - 1;
-}
-
 template <class Lane>
 __device__ __forceinline__ void accumulate_bincount(Lane& L, double2* hist, double r, double v2, double dt)
 {

@@ -311,7 +311,13 @@ int Launch_And_Wait(dms_ctx* ctx, const dms_run_opts* o, RunParams& p)
 	if(o->max_trajectory_wall_time_s > 0.0 && p.wall_limit_ns == 0)
 		p.wall_limit_ns = 1;
 	const bool mixed = o->precision == DMS_PRECISION_MIXED;
-	const int threads = Block_Threads(o, p.total, ctx->sm_count);
+	int threads = Block_Threads(o, p.total, ctx->sm_count);
+	// where the rows of the wide mixed form (3.0 GB) do not fit, those of the other may
+	if(threads > MAX_THREADS && Ensure_Lanes(ctx, static_cast<size_t>(threads) * ctx->sm_count) != DMS_OK)
+	{
+		(void)cudaGetLastError();
+		threads = MAX_THREADS;
+	}
 	Apply_Lane_Options(p, o, threads > LATENCY_THREADS);
 	int blocks = ctx->sm_count;
 	// a launch with fewer trajectories than lanes spreads them over the SMs and then over the warps: fewer

@@ -87,8 +87,11 @@ cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) { *v = 148; retu
 cudaError_t cudaGetLastError(void) { return cudaSuccess; }
 const char* cudaGetErrorString(cudaError_t) { return "fake error"; }
 
+size_t fake_malloc_limit = ~size_t{0};  // a larger allocation fails
 cudaError_t cudaMalloc(void** p, size_t n)
 {
+	if(n > fake_malloc_limit)
+		return cudaErrorMemoryAllocation;
 	*p = calloc(n ? n : 1, 1);
 	allocations[static_cast<char*>(*p)] = n;
 	return *p ? cudaSuccess : cudaErrorMemoryAllocation;

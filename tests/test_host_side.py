@@ -151,3 +151,29 @@ for count in (100, 100000):
             assert tuple(l.options) == (scatter, 5, final, 1024, 2 * scatter, 2 * final)  # of 32 lanes, of 64
 e.close()
 """)
+
+
+def test_a_large_mixed_launch_takes_the_rows_that_there_is_memory_for(host):
+    """640 lanes per SM need 3.0 GB of histogram rows; where only the 2.4 GB of 512 are there, 512 run."""
+    host(r"""
+limit = ctypes.c_size_t.in_dll(lib, "fake_malloc_limit")
+row, wide = 2000 * 16, [(0, 0, 2 * 640 * 148)]
+mixed = dms_b200.run_opts(seed=1, precision=dms_b200.PRECISION_MIXED)
+e = dms_b200.Engine(0)
+point(e)
+for lanes in (512, 640):
+    limit.value = lanes * 148 * row
+    e.run(wide, mixed)
+    first, second = launches()
+    assert (first.threads, first.lanes_per_block) == (lanes, lanes)
+limit.value = 128 * 148 * row
+e = dms_b200.Engine(0)
+point(e)
+try:
+    e.run(wide, mixed)
+except dms_b200.EngineError as error:
+    assert "CUDA error" in str(error)
+else:
+    raise AssertionError("ran without rows")
+assert not launches()
+""")

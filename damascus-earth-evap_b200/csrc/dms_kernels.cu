@@ -1349,7 +1349,8 @@ unsigned int Take_Bounds_Status()
 	unsigned int bits = 0;
 	const unsigned int zero = 0;
 	if(cudaMemcpyFromSymbol(&bits, dms_bounds_status, sizeof bits) != cudaSuccess ||
-	   cudaMemcpyToSymbol(dms_bounds_status, &zero, sizeof zero) != cudaSuccess)
+	   cudaMemcpyToSymbol(dms_bounds_status, &zero, sizeof zero) != cudaSuccess ||
+	   cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess)  // ahead of what runs on the context's stream
 		return ~0u;
 	return bits;
 #else

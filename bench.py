@@ -46,10 +46,10 @@ WORKLOAD = ("Parameter-point evaporation (config 1): SI contact m=0.3 GeV sigma_
 # conditions, Kepler shift, classification).
 FLOP_PER_ATTEMPT, FLOP_PER_STEP, FLOP_PER_SCATTER, FLOP_PER_TRAJ = 214.8, 622.3, 2455.0, 3374.0
 # DRAM bytes (read + write) of the FP64 trajectory kernels per trajectory of this point, from one
-# ncu capture of one 65 536-trajectory batch (ids 0-65 535: 2.399 GB read + 2.180 GB written by its
-# two launches, 308 bytes per accepted step): local memory, and the reads, writes and termination
+# ncu capture of one 65 536-trajectory batch (ids 0-65 535: 2.398 GB read + 2.210 GB written by its
+# two launches, 310 bytes per accepted step): local memory, and the reads, writes and termination
 # flush of the per-lane histogram rows.
-TRAFFIC_PER_TRAJECTORY = (2.399485e9 + 2.179577e9) / 65536
+TRAFFIC_PER_TRAJECTORY = (2.397908e9 + 2.209972e9) / 65536
 
 
 def hbm_peak_gbs():

@@ -233,8 +233,9 @@ void dms_default_run_opts(dms_run_opts* opts);
  * queue_chunk and the warp-batching thresholds (the lane-compaction interval of the persistent
  * kernel) for the points of `ranges` and the precision of `base`.  Each trial is a launch of
  * trial_seconds wall time over fresh trajectory ids of those points (ids from 2^40 on, results
- * kept in a scratch accumulator, so the points' own results are untouched), scored by accepted
- * free steps per second; the parameters are searched one at a time from the defaults
+ * kept in a scratch accumulator, so the points' own results are untouched), or of less where the
+ * base setting would take more than half of 2^25 ids in that time; it is scored by accepted
+ * free steps per second, and settings that make the same launch are tried once; the parameters are searched one at a time from the defaults
  * (coordinate descent, two passes).  *tuned receives `base` with the best setting; the chosen
  * setting changes throughput only, never results (every draw is keyed by trajectory id).
  * trials (may be NULL) receives the number of trial launches. */

@@ -113,7 +113,7 @@ e.close()
 """)
 
 
-@pytest.mark.parametrize("per_second, seconds", [(2 ** 17 / 0.02, 0.02), (2 ** 21 / 0.02, 0.02), (2 ** 22 / 0.02, 0.08), (2 ** 26 / 0.04, 0.08)])
+@pytest.mark.parametrize("per_second, seconds", [(2 ** 17 / 0.1, 0.1), (2 ** 21 / 0.1, 0.1), (2 ** 24 / 0.1, 0.1), (2 ** 26 / 0.4, 0.8)])
 def test_autotuner_times_the_steady_state_of_different_launches(host, per_second, seconds):
     """No setting is timed on a launch whose queue has run dry, and none that is the launch of the best one so far."""
     host("per_second, seconds = %r, %r" % (per_second, seconds) + r"""
